@@ -61,42 +61,50 @@ __device__ __forceinline__ void store_halfs(const LaunchArgs& p, __half* dst, co
     }
 }
 
-// features of group `g` (relative to all groups) for one point -> its plane
+// Features of group `g` (relative to all groups) for the points `i` of a warp -> their planes. Lanes work in pairs (see
+// grid.cuh): both lanes gather half of the corners of the even lane's point, then of the odd lane's, and each ends up
+// with the sum for its own point. `in0` / `in1`: input rows of the pair's two points; all lanes of the warp take part.
 template <class Spec, int E>
-__device__ __forceinline__ void encode_group(const LaunchArgs& p, int g, const RowReader& in, long long local)
+__device__ __forceinline__ void encode_group(const LaunchArgs& p, int g, const RowReader& in0, const RowReader& in1, long long local, bool valid)
 {
     if constexpr (E < Spec::NUM_ENCODINGS) {
         using Enc = typename Spec::template Enc<E>;
         using PG = PlaneGroups<Spec, E>;
         if (g >= PG::before() + PG::own()) {
-            encode_group<Spec, E + 1>(p, g, in, local);
+            encode_group<Spec, E + 1>(p, g, in0, in1, local, valid);
             return;
         }
+        const int side = threadIdx.x & 1;
         if constexpr (!Enc::IS_GRID) {
+            const RowReader& in = side ? in1 : in0;
             float v[Enc::N];
 #pragma unroll
             for (int i = 0; i < Enc::N; ++i) v[i] = in(i + Enc::START);
-            store_halfs<Enc::N>(p, p.planes + p.planeStride * Enc::OUT_OFF + local * Enc::N, v);
+            if (valid) store_halfs<Enc::N>(p, p.planes + p.planeStride * Enc::OUT_OFF + local * Enc::N, v);
         } else {
+            constexpr int D = Enc::D, F = Enc::F;
             const GridP& grid = p.grids[Enc::SLOT];
-            float pos[Enc::D];
-            grid_position<Enc::D, Enc::START>(grid, in, pos);
-            float feat[Enc::F];
-            if constexpr (Enc::CONCAT) {
-                const int l = g - PG::before();
-                grid_level_forward<Enc::D, Enc::F, Enc::HALF_TABLE>(grid, grid.levels[l], pos, feat);
-                store_halfs<Enc::F>(p, p.planes + p.planeStride * (Enc::OUT_OFF + l * Enc::F) + local * Enc::F, feat);
-            } else {
+            float pos0[D], pos1[D];
+            grid_position<D, Enc::START>(grid, in0, pos0);
+            grid_position<D, Enc::START>(grid, in1, pos1);
+            float feat[F];
 #pragma unroll
-                for (int i = 0; i < Enc::F; ++i) feat[i] = 0.f;
-                for (int l = 0; l < Enc::L; ++l) {
-                    float f[Enc::F];
-                    grid_level_forward<Enc::D, Enc::F, Enc::HALF_TABLE>(grid, grid.levels[l], pos, f);
-#pragma unroll
-                    for (int i = 0; i < Enc::F; ++i) feat[i] += f[i];
+            for (int i = 0; i < F; ++i) feat[i] = 0.f;
+            const int first = Enc::CONCAT ? g - PG::before() : 0, end = Enc::CONCAT ? first + 1 : Enc::L;
+            for (int l = first; l < end; ++l) {
+                const GridLevelP& lv = grid.levels[l];
+                float f0[F], f1[F];
+                if (lv.hashed) {
+                    grid_half_forward<D, F, Enc::HALF_TABLE, 0>(grid, lv, pos0, side, f0);
+                    grid_half_forward<D, F, Enc::HALF_TABLE, 0>(grid, lv, pos1, side, f1);
+                } else {
+                    grid_half_forward<D, F, Enc::HALF_TABLE, D - 1>(grid, lv, pos0, side, f0);
+                    grid_half_forward<D, F, Enc::HALF_TABLE, D - 1>(grid, lv, pos1, side, f1);
                 }
-                store_halfs<Enc::F>(p, p.planes + p.planeStride * Enc::OUT_OFF + local * Enc::F, feat);
+#pragma unroll
+                for (int i = 0; i < F; ++i) feat[i] += (side ? f1[i] : f0[i]) + __shfl_xor_sync(0xffffffffu, side ? f0[i] : f1[i], 1);
             }
+            if (valid) store_halfs<F>(p, p.planes + p.planeStride * (Enc::OUT_OFF + (Enc::CONCAT ? first * F : 0)) + local * F, feat);
         }
     }
 }
@@ -129,10 +137,13 @@ template <class Spec>
 __global__ void __launch_bounds__(256, plane_min_blocks<Spec>()) encode_planes_kernel(const __grid_constant__ LaunchArgs p)
 {
     const int g = blockIdx.y;
-    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < p.numel;
-         i += static_cast<long long>(gridDim.x) * blockDim.x) {
-        RowReader in{p.input + i * p.inS0, p.inS1};
-        encode_group<Spec, 0>(p, g, in, i);
+    // whole warps stay together (the lanes of a pair exchange sums): lanes past the end repeat the last point
+    for (long long base = blockIdx.x * static_cast<long long>(blockDim.x) + (threadIdx.x & ~31); base < p.numel;
+         base += static_cast<long long>(gridDim.x) * blockDim.x) {
+        const long long i = base + (threadIdx.x & 31), last = p.numel - 1;
+        const long long i0 = i & ~1ll;
+        const RowReader in0{p.input + (i0 < last ? i0 : last) * p.inS0, p.inS1}, in1{p.input + (i0 + 1 < last ? i0 + 1 : last) * p.inS0, p.inS1};
+        encode_group<Spec, 0>(p, g, in0, in1, i, i < p.numel);
     }
 }
 
@@ -161,38 +172,56 @@ __host__ __device__ constexpr int scatter_group_count()
     return ScatterGroups<Spec, Spec::NUM_ENCODINGS - 1>::before() + ScatterGroups<Spec, Spec::NUM_ENCODINGS - 1>::own();
 }
 
+// lanes in pairs: both lanes of a pair scatter half of the corners of the even lane's point, then of the odd lane's
 template <class Spec, int E>
-__device__ __forceinline__ void scatter_group(const LaunchArgs& p, int g, const RowReader& in, long long point)
+__device__ __forceinline__ void scatter_group(const LaunchArgs& p, int g, const RowReader& in0, const RowReader& in1, long long point, bool valid)
 {
     if constexpr (E < Spec::NUM_ENCODINGS) {
         using Enc = typename Spec::template Enc<E>;
         using SG = ScatterGroups<Spec, E>;
         if (g >= SG::before() + SG::own()) {
-            scatter_group<Spec, E + 1>(p, g, in, point);
+            scatter_group<Spec, E + 1>(p, g, in0, in1, point, valid);
             return;
         }
         if constexpr (Enc::IS_GRID) {
             const GridP& grid = p.grids[Enc::SLOT];
             if (grid.grad == nullptr) return;
+            constexpr int D = Enc::D, F = Enc::F;
+            const int side = threadIdx.x & 1;
             const int l = g - SG::before();
-            const int c0 = Enc::OUT_OFF + (Enc::CONCAT ? l * Enc::F : 0);
-            const __half* src = p.planes + p.planeStride * c0 + point * Enc::F;
-            if (!scratch_ok(p, src - p.planes, Enc::F, p.planeHalfs, STATUS_PLANES)) return;
-            float adjF[Enc::F];
-            if constexpr (Enc::F == 2) {
-                const float2 x = __half22float2(u32_as_h2(*reinterpret_cast<const uint32_t*>(src)));
-                adjF[0] = x.x; adjF[1] = x.y;
-            } else if constexpr (Enc::F == 4) {
-                const uint2 u = *reinterpret_cast<const uint2*>(src);
-                const float2 x = __half22float2(u32_as_h2(u.x)), y = __half22float2(u32_as_h2(u.y));
-                adjF[0] = x.x; adjF[1] = x.y; adjF[2] = y.x; adjF[3] = y.y;
-            } else {
+            const int c0 = Enc::OUT_OFF + (Enc::CONCAT ? l * F : 0);
+            const __half* src = p.planes + p.planeStride * c0 + point * F;
+            if (!scratch_ok(p, src - p.planes, F, p.planeHalfs, STATUS_PLANES)) valid = false;
+            uint32_t own[(F + 1) / 2];
 #pragma unroll
-                for (int i = 0; i < Enc::F; ++i) adjF[i] = __half2float(src[i]);
+            for (int i = 0; i < (F + 1) / 2; ++i) own[i] = 0u;
+            if (valid) {
+                if constexpr (F == 2) {
+                    own[0] = *reinterpret_cast<const uint32_t*>(src);
+                } else if constexpr (F == 4) {
+                    const uint2 u = *reinterpret_cast<const uint2*>(src);
+                    own[0] = u.x; own[1] = u.y;
+                } else {
+#pragma unroll
+                    for (int i = 0; i < F; ++i) own[i / 2] |= static_cast<uint32_t>(__half_as_ushort(src[i])) << (16 * (i & 1));
+                }
             }
-            float pos[Enc::D];
-            grid_position<Enc::D, Enc::START>(grid, in, pos);
-            grid_level_scatter_paired<Enc::D, Enc::F>(grid, grid.levels[l], pos, adjF);
+            const GridLevelP& lv = grid.levels[l];
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+                float pos[D], adjF[F];
+                grid_position<D, Enc::START>(grid, s == 0 ? in0 : in1, pos);
+                const bool ok = __shfl_sync(0xffffffffu, valid ? 1 : 0, (threadIdx.x & 30) + s) != 0;
+#pragma unroll
+                for (int i = 0; i < (F + 1) / 2; ++i) {
+                    const float2 x = __half22float2(u32_as_h2(__shfl_sync(0xffffffffu, own[i], (threadIdx.x & 30) + s)));
+                    adjF[2 * i] = x.x;
+                    if (2 * i + 1 < F) adjF[2 * i + 1] = x.y;
+                }
+                if (!ok) continue;
+                if (lv.hashed) grid_half_scatter<D, F, 0>(grid, lv, pos, side, adjF);
+                else grid_half_scatter<D, F, D - 1>(grid, lv, pos, side, adjF);
+            }
         }
     }
 }
@@ -214,13 +243,13 @@ __global__ void __launch_bounds__(SCATTER_THREADS, 1024 / SCATTER_THREADS) scatt
     // CTAs on one small level, reductions to the same row queue up behind each other).
     const int first = static_cast<int>(blockIdx.x % count);
     for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {
-        const long long i = t * SCATTER_THREADS + threadIdx.x;
-        if (i >= p.numel) continue;
-        RowReader in{p.input + i * p.inS0, p.inS1};
+        const long long i = t * SCATTER_THREADS + threadIdx.x, i0 = i & ~1ll, last = p.numel - 1;
+        if ((i & ~31ll) >= p.numel) continue;   // whole warps stay together
+        const RowReader in0{p.input + (i0 < last ? i0 : last) * p.inS0, p.inS1}, in1{p.input + (i0 + 1 < last ? i0 + 1 : last) * p.inS0, p.inS1};
         for (int gi = 0; gi < count; ++gi) {
             int g = first + gi;
             if (g >= count) g -= count;
-            scatter_group<Spec, 0>(p, begin + g, in, i);
+            scatter_group<Spec, 0>(p, begin + g, in0, in1, i, i < p.numel);
         }
     }
 }

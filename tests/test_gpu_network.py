@@ -163,6 +163,49 @@ def test_level_major_encoding_pass(name, half_tables):
     helpers.assert_close(out_planes[-m:].cpu().numpy(), emu, f"{name} planes vs oracle", max_violations=0.01)
 
 
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 255, 257])
+@pytest.mark.parametrize("name", ["config3_small", "config4_small", "config5_small", "grid2d_add_plus_identity"])
+def test_lane_pairs_of_the_plane_kernels(name, n):
+    """The plane kernels give a point to two neighbouring lanes: batches that end inside a pair, a warp or a CTA, for both
+    pairing dimensions (hashed and dense levels), concatenating and adding grids. Features through the inference output,
+    table gradients against the scatter inside the backward kernel."""
+    import torch
+    from qmlp import _capi, bindings
+    from qmlp._capi import check, lib, wrap
+    cfg, rng, spec, net, params, tables, acts, t_params, t_tables = _setup(name)
+    x = helpers.uniform(43, 1, (n, spec.num_inputs), *rng)
+    tx = torch.from_numpy(x).cuda()
+    tadj = torch.from_numpy(helpers.uniform(43, 2, (n, spec.num_outputs), -1.0, 1.0)).cuda()
+    out = torch.empty((n, spec.num_outputs), device="cuda")
+    fwd = torch.empty((net.forward_memory(n),), dtype=torch.uint8, device="cuda")
+    bwd = torch.empty((net.adjoint_memory(n, 6),), dtype=torch.uint8, device="cuda")
+    expected = oracle.network_forward(spec, params, x, tables, half=True, activations=acts)
+    results = []
+    try:
+        bindings.QuickMLP.set_kernel_path(2)
+        helpers.assert_close(net.inference(tx, t_params, t_tables).cpu().numpy(), expected, f"{name} n={n}", max_violations=0.01)
+        bindings.QuickMLP.set_tuning("split_scatter", 1)
+        for path in (2, 1):
+            bindings.QuickMLP.set_kernel_path(path)
+            grads = [torch.zeros_like(t) if t is not None else None for t in t_tables]
+            net._bind(t_params, t_tables)
+            for i, g in enumerate(grads):
+                if g is not None:
+                    net.encoding(i).set_parameter(g, _capi.QMLP_GRADIENTS)
+            check(lib().qmlp_network_forward(net._h, wrap(tx), wrap(out), fwd.data_ptr(), None))
+            check(lib().qmlp_network_adjoint(net._h, wrap(tx), wrap(tadj), 4, None, fwd.data_ptr(), bwd.data_ptr(), None))
+            torch.cuda.synchronize()
+            results.append(grads)
+    finally:
+        bindings.QuickMLP.set_kernel_path(0)
+        bindings.QuickMLP.set_tuning("split_scatter", -1)
+    for a, b in zip(*results):
+        if a is not None:
+            # the same fp32 terms in another order: at most a few dozen per row
+            helpers.assert_close(a.cpu().numpy(), b.cpu().numpy(), f"{name} n={n} table gradient", rtol=1e-4,
+                                 atol=1e-5 * float(b.abs().max()))
+
+
 @pytest.mark.parametrize("name,n,chunk", [("config2", 100_003, 0), ("config2", 5000, 1024), ("config3_small", 70_001, 4096),
                                           ("config1", 17, 0), ("config1", 0, 0)])
 def test_inference_from_host_memory(name, n, chunk):
