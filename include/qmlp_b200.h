@@ -242,6 +242,9 @@ QMLP_API int qmlp_activation_adjoint(qmlp_activation_t* act, const qmlp_tensor_t
  * src_cpp/src/activation.cpp:76-92). Needs the compiler, not a GPU. */
 QMLP_API int qmlp_activation_compile(qmlp_activation_t* act);
 
+/* fp32 vector -> fp16 copy (a caller that keeps fp32 master weights binds such a copy for a call). */
+QMLP_API int qmlp_convert_half(const float* src, uint16_t* dst, int64_t count, qmlp_stream_t stream);
+
 /* ---- fused training step ---------------------------------------------------------------------
  * Not a single function in the reference: there the loss and optimiser are user PyTorch code
  * (tests_py/qmlp_tests/test_network_image.py:41-55: mse_loss + torch.optim.Adam around FusedNetwork.forward). These

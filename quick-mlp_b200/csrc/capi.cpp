@@ -890,6 +890,15 @@ int qmlp_activation_adjoint(qmlp_activation_t* act, const qmlp_tensor_t* input, 
     QMLP_CATCH
 }
 
+int qmlp_convert_half(const float* src, uint16_t* dst, int64_t count, qmlp_stream_t stream)
+{
+    QMLP_TRY
+    if (count < 0 || (count > 0 && (!src || !dst))) throw std::runtime_error("null buffer");
+    if (count > 0)
+        checkCuda(kernel::launchRefreshHalf(src, dst, count, Library::instance().smCount(), static_cast<cudaStream_t>(stream)), "convert_half");
+    QMLP_CATCH
+}
+
 } // extern "C"
 
 // ---- fused training step -------------------------------------------------------------------------------------------

@@ -84,9 +84,20 @@ cudaError_t launchAdam(float* master, float* grad, float* m, float* v, uint16_t*
     return cudaGetLastError();
 }
 
+__global__ void __launch_bounds__(256) convert_half_kernel(const float* __restrict__ src, __half* __restrict__ dst, long long count)
+{
+    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < count;
+         i += static_cast<long long>(gridDim.x) * blockDim.x)
+        dst[i] = __float2half(src[i]);
+}
+
 cudaError_t launchRefreshHalf(const float* master, uint16_t* halfCopy, long long count, int numSMs, cudaStream_t stream)
 {
     const long long count4 = count / 4;
+    if (count % 4 != 0 || (reinterpret_cast<uintptr_t>(master) & 15) != 0 || (reinterpret_cast<uintptr_t>(halfCopy) & 7) != 0) {
+        convert_half_kernel<<<gridFor(count, numSMs), 256, 0, stream>>>(master, reinterpret_cast<__half*>(halfCopy), count);
+        return cudaGetLastError();
+    }
     refresh_half_kernel<<<gridFor(count4, numSMs), 256, 0, stream>>>(reinterpret_cast<const float4*>(master),
                                                                      reinterpret_cast<uint2*>(halfCopy), count4);
     return cudaGetLastError();

@@ -541,10 +541,14 @@ struct TcLaunchers {
         constexpr int threads = TL::warpgroups() * 128;
         static DeviceOnce once;   // function attributes are per device
         auto k = fused_forward_tc_kernel<Spec, PLANES>;
-        TcWeightMaps<Spec> maps;
-        {
+        // the maps depend on the address of the parameter vector alone: the ones of this thread's last call usually serve
+        static thread_local TcWeightMaps<Spec> maps;
+        static thread_local const __half* mapsOf = nullptr;
+        if (mapsOf != a.weights) {
+            mapsOf = nullptr;
             const cudaError_t e = encodeWeightMaps(a.weights, maps);
             if (e != cudaSuccess) return e;
+            mapsOf = a.weights;
         }
         {
             const cudaError_t e = once.run([&] { return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); });

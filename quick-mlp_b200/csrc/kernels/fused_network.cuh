@@ -1062,6 +1062,23 @@ struct DeviceOnce {
     }
 };
 
+// A per-device value that costs driver calls to find out (resident CTAs of a kernel), kept after the first launch.
+struct PerDevice {
+    std::atomic<int> value[64] = {};   // 0: not known yet
+    template <class F>
+    cudaError_t get(int& out, F find)
+    {
+        int d = 0;
+        cudaError_t e = cudaGetDevice(&d);
+        if (e != cudaSuccess) return e;
+        out = value[d & 63].load(std::memory_order_acquire);
+        if (out != 0) return cudaSuccess;
+        e = find(out);
+        if (e == cudaSuccess) value[d & 63].store(out, std::memory_order_release);
+        return e;
+    }
+};
+
 template <class Spec> struct TcLaunchers;
 template <class Spec> struct PlaneLaunchers;
 template <class Spec> struct SortLaunchers;
@@ -1074,20 +1091,27 @@ struct NetworkLaunchers {
         return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     }
 
+    template <class K>
+    static cudaError_t residentCtas(K kernel, int threads, int smem, int& perSM)
+    {
+        const cudaError_t e = setSmem(kernel, smem);
+        if (e != cudaSuccess) return e;
+        const cudaError_t o = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, kernel, threads, smem);
+        if (perSM < 1) perSM = 1;
+        return o;
+    }
+
     template <int MODE>
     static cudaError_t forward(const LaunchArgs& a, cudaStream_t s)
     {
         constexpr int smem = SmemLayout<Spec>::totalBytes();
-        static DeviceOnce once;   // function attributes are per device
+        static PerDevice resident;
         auto k = fused_forward_kernel<Spec, MODE>;
+        int perSM = 1;
         {
-            const cudaError_t e = once.run([&] { return setSmem(k, smem); });
+            const cudaError_t e = resident.get(perSM, [&](int& n) { return residentCtas(k, Spec::WARPS * 32, smem, n); });
             if (e != cudaSuccess) return e;
         }
-        int perSM = 0;
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k, Spec::WARPS * 32, smem);
-        if (e != cudaSuccess) return e;
-        if (perSM < 1) perSM = 1;
         const long long tiles = (a.numel + TILE_POINTS - 1) / TILE_POINTS;
         long long blocks = (tiles + Spec::WARPS - 1) / Spec::WARPS;
         const long long cap = static_cast<long long>(a.numSMs) * perSM;
@@ -1101,16 +1125,13 @@ struct NetworkLaunchers {
     static cudaError_t backwardT(const LaunchArgs& a, cudaStream_t s)
     {
         constexpr int smem = SmemLayout<Spec>::totalBytes();
-        static DeviceOnce once;   // function attributes are per device
+        static PerDevice resident;
         auto k = fused_backward_kernel<Spec, FLAGS>;
+        int perSM = 1;
         {
-            const cudaError_t e = once.run([&] { return setSmem(k, smem); });
+            const cudaError_t e = resident.get(perSM, [&](int& n) { return residentCtas(k, Spec::WARPS * 32, smem, n); });
             if (e != cudaSuccess) return e;
         }
-        int perSM = 0;
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k, Spec::WARPS * 32, smem);
-        if (e != cudaSuccess) return e;
-        if (perSM < 1) perSM = 1;
         const long long tiles = (a.numel + TILE_POINTS - 1) / TILE_POINTS;
         long long blocks = (tiles + Spec::WARPS - 1) / Spec::WARPS;
         const long long cap = static_cast<long long>(a.numSMs) * perSM;

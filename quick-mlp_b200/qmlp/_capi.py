@@ -5,6 +5,7 @@ This is the layer the reference fills with its TorchScript custom classes
 The library must be present: there is no fallback path.
 """
 import ctypes as C
+import importlib.util
 import os
 
 import torch
@@ -106,6 +107,7 @@ SIGNATURES = {
     "qmlp_activation_to_json": (C.c_char_p, [_P]),
     "qmlp_activation_forward": (C.c_int, [_P, _TP, _TP, _P]),
     "qmlp_activation_adjoint": (C.c_int, [_P, _TP, _TP, _TP, _P]),
+    "qmlp_convert_half": (C.c_int, [_P, _P, C.c_int64, _P]),
     "qmlp_trainer_create": (C.c_int, [_P, C.POINTER(TrainerConfig), C.POINTER(_P)]),
     "qmlp_trainer_destroy": (None, [_P]),
     "qmlp_trainer_fused_count": (C.c_int64, [_P]),
@@ -135,6 +137,26 @@ def lib():
             fn.argtypes = args
         _lib = handle
     return _lib
+
+
+_calls = None
+
+
+def calls():
+    """The native call path (csrc/torch/calls.cpp) over the loaded library; raises if it has not been built
+    (python quick-mlp_b200/build_torch_ext.py)."""
+    global _calls
+    if _calls is None:
+        path = os.path.abspath(os.path.join(_HERE, "..", "lib", "torch_ext", "qmlp_calls.so"))
+        if not os.path.exists(path):
+            raise ImportError(f"{path} not found: build it with `python quick-mlp_b200/build_torch_ext.py`")
+        lib()
+        spec = importlib.util.spec_from_file_location("qmlp_calls", path)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        module.load(os.path.abspath(os.environ.get("QMLP_B200_LIBRARY", LIB_PATH)), QmlpError, ConfigurationError)
+        _calls = module
+    return _calls
 
 
 def check(status: int):

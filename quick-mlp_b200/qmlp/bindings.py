@@ -5,9 +5,7 @@ Autograd support mirrors NetworkBindings::forward (bind_network.cpp:120-321),
 EncodingBindings (bind_encoding.cpp:134-163) and ActivationBindings (bind_activation.cpp:52-79).
 """
 import ctypes as C
-import json
-import threading
-from typing import List, Optional, Sequence
+from typing import Optional, Sequence
 
 import torch
 
@@ -259,15 +257,9 @@ class Network:
         h = C.c_void_p()
         check(lib().qmlp_network_create(cfg.encode(), parent.encode(), C.byref(h)))
         self._h = h
-        self._mutex = threading.Lock()   # parameter pointers are instance state, bind_network.h:20
-
-    def __del__(self):
-        try:
-            if getattr(self, "_h", None) and _capi._lib is not None:
-                _capi._lib.qmlp_network_destroy(self._h)
-                self._h = None
-        except Exception:   # interpreter shutdown: module globals may already be gone
-            pass
+        # owns the handle and serialises the calls (the bound parameter pointers are state of the network, bind_network.h:20)
+        self._calls = _capi.calls().NetworkCalls(h.value)
+        self._channels = (lib().qmlp_network_channels_in(h), lib().qmlp_network_channels_out(h))
 
     def cfg(self) -> str:
         return self._cfg
@@ -302,10 +294,10 @@ class Network:
         return Encoding(_handle=h, _owner=self)
 
     def channels_in(self) -> int:
-        return lib().qmlp_network_channels_in(self._h)
+        return self._channels[0]
 
     def channels_out(self) -> int:
-        return lib().qmlp_network_channels_out(self._h)
+        return self._channels[1]
 
     def num_layers(self) -> int:
         return lib().qmlp_network_num_layers(self._h)
@@ -344,25 +336,11 @@ class Network:
 
     # -- launches ----------------------------------------------------------------------------------------------------
     def _bind(self, network_parameters, encoding_parameters: Sequence[Optional[torch.Tensor]]):
-        if network_parameters is not None:
-            check(lib().qmlp_network_set_parameter(self._h, wrap(network_parameters), _capi.QMLP_INFERENCE))
-        for i in range(min(len(encoding_parameters), self.num_encodings())):
-            p = encoding_parameters[i]
-            if p is not None:
-                self.encoding(i).set_parameter(p, _capi.QMLP_INFERENCE)
-
-    @staticmethod
-    def _half(p: torch.Tensor) -> torch.Tensor:
-        return p if p.dtype == torch.float16 else p.to(torch.float16)
+        _capi.calls().network_bind(self._calls, network_parameters, list(encoding_parameters))
 
     def inference(self, input: torch.Tensor, network_parameters: torch.Tensor,
                   encoding_parameters: Sequence[Optional[torch.Tensor]] = ()) -> torch.Tensor:
-        with self._mutex:
-            output = torch.empty((input.shape[0], self.channels_out()), dtype=torch.float32, device=input.device)
-            np_half = self._half(network_parameters)
-            self._bind(np_half, encoding_parameters)
-            check(lib().qmlp_network_inference(self._h, wrap(input), wrap(output), current_stream()))
-            return output
+        return _capi.calls().network_inference(self._calls, input, network_parameters, encoding_parameters)
 
     def inference_host(self, input: torch.Tensor, network_parameters: torch.Tensor,
                        encoding_parameters: Sequence[Optional[torch.Tensor]] = (),
@@ -372,29 +350,19 @@ class Network:
         device tensors as in `inference`. Uploads, kernels and downloads of successive chunks overlap
         (qmlp_network_inference_host); the result is complete once the current CUDA stream is."""
         assert input.device.type == "cpu" and input.dtype == torch.float32 and input.is_contiguous()
-        with self._mutex:
-            n = input.shape[0]
-            if output is None:
-                output = torch.empty((n, self.channels_out()), dtype=torch.float32, pin_memory=True)
-            assert output.device.type == "cpu" and output.dtype == torch.float32 and output.is_contiguous()
-            assert tuple(output.shape) == (n, self.channels_out()) and input.shape[1] == self.channels_in()
-            self._bind(self._half(network_parameters), encoding_parameters)
-            check(lib().qmlp_network_inference_host(self._h, input.data_ptr(), output.data_ptr(), n, int(chunk_points),
-                                                    current_stream()))
-            return output
+        n = input.shape[0]
+        if output is None:
+            output = torch.empty((n, self.channels_out()), dtype=torch.float32, pin_memory=True)
+        assert output.device.type == "cpu" and output.dtype == torch.float32 and output.is_contiguous()
+        assert tuple(output.shape) == (n, self.channels_out()) and input.shape[1] == self.channels_in()
+        _capi.calls().network_inference_host(self._calls, input, network_parameters, encoding_parameters, output, int(chunk_points))
+        return output
 
     def forward(self, input: torch.Tensor, network_parameters: torch.Tensor,
                 encoding_parameters: Sequence[Optional[torch.Tensor]] = ()) -> torch.Tensor:
-        flags = 0
-        if input.requires_grad:
-            flags |= _capi.GRADIENTS_INPUT
-        if network_parameters is not None and network_parameters.requires_grad:
-            flags |= _capi.GRADIENTS_NETWORK_WEIGHTS
-        if any(p is not None and p.requires_grad for p in encoding_parameters):
-            flags |= _capi.GRADIENTS_INPUT_ENCODINGS
-        if flags == 0 or not torch.is_grad_enabled():
-            return self.inference(input, network_parameters, encoding_parameters)
-        return _NetworkFunction.apply(self, flags, input, network_parameters, *encoding_parameters)
+        """Inference, or - when gradients are enabled and one of the tensors requires them - an autograd node
+        (csrc/torch/calls.cpp)."""
+        return _capi.calls().network_forward(self._calls, input, network_parameters, encoding_parameters)
 
     def forward_memory(self, n: int, flags: int = 7) -> int:
         b = C.c_size_t()
@@ -417,51 +385,3 @@ class Network:
 
     def __setstate__(self, state):
         self.__init__(*state)
-
-
-class _NetworkFunction(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, net: Network, flags: int, input, network_parameters, *encoding_parameters):
-        np_half = Network._half(network_parameters.detach())
-        tmp = torch.empty((max(net.forward_memory(input.shape[0], flags), 16),), dtype=torch.uint8, device=input.device)
-        output = torch.empty((input.shape[0], net.channels_out()), dtype=torch.float32, device=input.device)
-        with net._mutex:
-            net._bind(np_half, [p.detach() if p is not None else None for p in encoding_parameters])
-            check(lib().qmlp_network_forward(net._h, wrap(input.detach()), wrap(output), tmp.data_ptr(), current_stream()))
-        ctx.net, ctx.flags = net, flags
-        ctx.param_dtype = network_parameters.dtype
-        ctx.num_enc = len(encoding_parameters)
-        ctx.enc_defined = [p is not None for p in encoding_parameters]
-        ctx.save_for_backward(input, np_half, tmp, *[p for p in encoding_parameters if p is not None])
-        return output
-
-    @staticmethod
-    def backward(ctx, grad_output):
-        net, flags = ctx.net, ctx.flags
-        saved = ctx.saved_tensors
-        input, np_half, tmp = saved[0], saved[1], saved[2]
-        enc_saved = list(saved[3:])
-        enc_params: List[Optional[torch.Tensor]] = [enc_saved.pop(0) if d else None for d in ctx.enc_defined]
-        grad_output = grad_output.contiguous()
-        adj_input = torch.zeros_like(input) if flags & _capi.GRADIENTS_INPUT else None
-        adj_params = None
-        adj_enc: List[Optional[torch.Tensor]] = [None] * ctx.num_enc
-        with net._mutex:
-            net._bind(np_half, enc_params)
-            if flags & _capi.GRADIENTS_NETWORK_WEIGHTS:
-                adj_params = torch.zeros(np_half.shape, dtype=torch.float32, device=np_half.device)
-                check(lib().qmlp_network_set_parameter(net._h, wrap(adj_params), _capi.QMLP_GRADIENTS))
-            if flags & _capi.GRADIENTS_INPUT_ENCODINGS:
-                for i, p in enumerate(enc_params):
-                    if p is not None and p.requires_grad:
-                        adj_enc[i] = torch.zeros(p.shape, dtype=torch.float32, device=p.device)
-                        net.encoding(i).set_parameter(adj_enc[i], _capi.QMLP_GRADIENTS)
-                    elif i < net.num_encodings():
-                        net.encoding(i).set_parameter(None, _capi.QMLP_GRADIENTS)
-            adj_tmp = torch.empty((max(net.adjoint_memory(input.shape[0], flags), 16),), dtype=torch.uint8, device=input.device)
-            ai = wrap(adj_input)
-            check(lib().qmlp_network_adjoint(net._h, wrap(input), wrap(grad_output), flags, C.byref(ai), tmp.data_ptr(),
-                                             adj_tmp.data_ptr(), current_stream()))
-        if adj_params is not None:
-            adj_params = adj_params.to(ctx.param_dtype)
-        return (None, None, adj_input, adj_params, *adj_enc)

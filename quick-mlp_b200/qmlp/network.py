@@ -29,6 +29,7 @@ class FusedNetwork(torch.nn.Module):
         self._num_encodings = self._network.num_encodings()
         assert self._num_encodings > 0
         self._encodings = [self._network.encoding(i) for i in range(self._num_encodings)]
+        self._encoding_has_parameters = [e.has_parameters() for e in self._encodings]
         params = []
         for e in self._encodings:
             if e.has_parameters():
@@ -92,7 +93,7 @@ class FusedNetwork(torch.nn.Module):
         if self.weights.requires_grad and self.weights.dtype == torch.float16 and torch.is_grad_enabled():
             warnings.warn("Attempt to train network with 16-bit weights: the gradient tensor will also have 16-bit "
                           "precision. Consider weight_dtype=torch.float32.")
-        enc = [p if e.has_parameters() else None for p, e in zip(self.encoding_parameters, self._encodings)]
+        enc = [self.encoding_parameters[i] if has else None for i, has in enumerate(self._encoding_has_parameters)]
         return self._network.forward(x, self.weights, enc)
 
     def __repr__(self):

@@ -39,6 +39,7 @@ class _CudaStep:
         self.segments = [lib().qmlp_trainer_segment_start(h, i) for i in range(1 + network.num_encodings())]
         self.device = device
         self._workspace = None
+        self._workspace_points = -1
 
     def __del__(self):
         try:
@@ -70,16 +71,17 @@ class _CudaStep:
         """parts: 1 = forward, backward, table gradients; 2 = weight/bias gradients of the layers; 3 = both;
         4 = forward and backward with the scatter deferred; 8 | first << 8 | end << 16 = scatter of grid levels
         [first, end)."""
-        b = C.c_size_t()
-        check(lib().qmlp_trainer_workspace_bytes(self._h, x.shape[0], C.byref(b)))
-        if self._workspace is None or self._workspace.numel() < b.value:
-            self._workspace = torch.empty((b.value,), dtype=torch.uint8, device=x.device)
-        check(lib().qmlp_trainer_gradients_part(self._h, wrap(x), wrap(target), global_points, self._workspace.data_ptr(),
-                                                self._workspace.numel(), loss_sum.data_ptr() if loss_sum is not None else None,
-                                                parts, current_stream()))
+        calls = _capi.calls()
+        n = x.shape[0]
+        if n != self._workspace_points:
+            need = calls.trainer_workspace_bytes(self._h.value, n)
+            if self._workspace is None or self._workspace.numel() < need:
+                self._workspace = torch.empty((need,), dtype=torch.uint8, device=x.device)
+            self._workspace_points = n
+        calls.trainer_gradients(self._h.value, x, target, global_points, self._workspace, loss_sum, parts)
 
     def update(self, step, grad_scale):
-        check(lib().qmlp_trainer_update(self._h, step, grad_scale, current_stream()))
+        _capi.calls().trainer_update(self._h.value, step, grad_scale)
 
 
 class FusedTrainer:

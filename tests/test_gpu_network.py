@@ -463,3 +463,15 @@ def test_argument_errors():
         bindings.Network(json.dumps(bad))
     out = net.inference(torch.zeros((0, 3), device="cuda"), t_params)             # empty batch is a no-op
     assert out.shape == (0, 1)
+
+
+@pytest.mark.parametrize("n,offset", [(1, 0), (3, 0), (4, 0), (1024, 0), (1023, 0), (1024, 1), (4097, 2)])
+def test_convert_half(n, offset):
+    """fp32 -> fp16 copy of a parameter vector: vector and scalar kernels, lengths and alignments either side of the rule."""
+    import torch
+    from qmlp._capi import check, lib
+    src = torch.from_numpy(helpers.uniform(44, 1, (n + offset,), -3.0, 3.0)).cuda()[offset:]
+    dst = torch.zeros((n + offset + 1,), dtype=torch.float16, device="cuda")
+    check(lib().qmlp_convert_half(src.data_ptr(), dst[offset:].data_ptr(), n, None))
+    torch.cuda.synchronize()
+    assert torch.equal(dst[offset:offset + n], src.half()) and float(dst[offset + n]) == 0.0
