@@ -220,6 +220,14 @@ QMLP_API int qmlp_encoding_forward(qmlp_encoding_t* enc, const qmlp_tensor_t* in
 QMLP_API int qmlp_encoding_adjoint(qmlp_encoding_t* enc, const qmlp_tensor_t* input, const qmlp_tensor_t* adj_output,
                                    qmlp_tensor_t* adj_input, qmlp_stream_t stream, const qmlp_tensor_t* parameters,
                                    qmlp_tensor_t* parameter_gradients, int adjoint_mode);
+/* The same with optional scratch memory (qmlp_encoding_adjoint_memory() bytes, 16-byte aligned, contents irrelevant): large
+ * batches on small grid levels then scatter into copies of the gradient that are summed afterwards, instead of queueing up
+ * on a few cache lines. Results are the same up to the order of the fp32 sums. */
+QMLP_API int qmlp_encoding_adjoint_memory(qmlp_encoding_t* enc, int64_t num_elements, int adjoint_mode, size_t* bytes);
+QMLP_API int qmlp_encoding_adjoint_with_memory(qmlp_encoding_t* enc, const qmlp_tensor_t* input, const qmlp_tensor_t* adj_output,
+                                               qmlp_tensor_t* adj_input, qmlp_stream_t stream, const qmlp_tensor_t* parameters,
+                                               qmlp_tensor_t* parameter_gradients, int adjoint_mode, void* tmp_memory,
+                                               size_t tmp_bytes);
 
 /* Instantiate the stand-alone kernels of this encoding now (replaces the lazy NVRTC compile inside IEncoding::forward,
  * src_cpp/src/iencoding.cpp:26-63). half_table selects the fp16-table variant. Needs the compiler, not a GPU. */

@@ -767,9 +767,30 @@ int qmlp_encoding_forward(qmlp_encoding_t* enc, const qmlp_tensor_t* input, qmlp
     QMLP_CATCH
 }
 
+int qmlp_encoding_adjoint_memory(qmlp_encoding_t* enc, int64_t num_elements, int adjoint_mode, size_t* bytes)
+{
+    QMLP_TRY
+    if (!bytes) throw std::runtime_error("null argument");
+    *bytes = 0;
+    auto* g = dynamic_cast<EncodingHashGrid*>(enc->impl.get());
+    if (g && (adjoint_mode & QMLP_ENCODING_PARAM_GRADIENTS)) {
+        kernel::GradReplicas r;
+        g->planReplicas(num_elements, r);
+        *bytes = static_cast<size_t>(r.total) * sizeof(float);
+    }
+    QMLP_CATCH
+}
+
 int qmlp_encoding_adjoint(qmlp_encoding_t* enc, const qmlp_tensor_t* input, const qmlp_tensor_t* adj_output,
                           qmlp_tensor_t* adj_input, qmlp_stream_t stream, const qmlp_tensor_t* parameters,
                           qmlp_tensor_t* parameter_gradients, int adjoint_mode)
+{
+    return qmlp_encoding_adjoint_with_memory(enc, input, adj_output, adj_input, stream, parameters, parameter_gradients, adjoint_mode, nullptr, 0);
+}
+
+int qmlp_encoding_adjoint_with_memory(qmlp_encoding_t* enc, const qmlp_tensor_t* input, const qmlp_tensor_t* adj_output,
+                                      qmlp_tensor_t* adj_input, qmlp_stream_t stream, const qmlp_tensor_t* parameters,
+                                      qmlp_tensor_t* parameter_gradients, int adjoint_mode, void* tmp_memory, size_t tmp_bytes)
 {
     QMLP_TRY
     Encoding& e = *enc->impl;
@@ -807,6 +828,12 @@ int qmlp_encoding_adjoint(qmlp_encoding_t* enc, const qmlp_tensor_t* input, cons
             a.aiS1 = adj_input->strides[1];
         }
         a.flags = (gIn ? 1 : 0) | (gP ? 2 : 0);
+        if (auto* g = dynamic_cast<EncodingHashGrid*>(&e); g && gP && tmp_memory) {
+            if ((reinterpret_cast<uintptr_t>(tmp_memory) & 15) != 0) throw std::runtime_error("scratch memory must be 16-byte aligned");
+            g->planReplicas(a.numel, a.replicas);
+            if (a.replicas.total > 0 && static_cast<size_t>(a.replicas.total) * sizeof(float) <= tmp_bytes) a.replicas.base = static_cast<float*>(tmp_memory);
+            else std::memset(&a.replicas, 0, sizeof a.replicas);
+        }
         if (a.numel > 0 && a.flags != 0) {
             auto m = e.standaloneModule(e.paramInference.precision == QMLP_HALF && e.isGrid());
             checkLaunch(m->launch(kernel::KERNEL_ENCODING_ADJOINT, &a, static_cast<cudaStream_t>(stream), nullptr), "kernel launch failed");

@@ -168,6 +168,8 @@ public:
     void setParameter(const qmlp_tensor_t* t, int usage) override;
     void fillGrid(kernel::GridP& g) const override;
     const std::vector<GridLevel>& levelTable() const { return table_; }
+    // copies of the gradients of small levels for a batch of `points` (kernel::GradReplicas; base is left null)
+    void planReplicas(int64_t points, kernel::GradReplicas& r) const;
     int features() const { return features_; }
     int dimension() const { return dim_; }
     Json gridJson() const;   // the hash grid's own configuration (id "HashGrid")

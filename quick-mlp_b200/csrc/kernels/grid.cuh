@@ -413,14 +413,53 @@ __device__ __forceinline__ void grid_half_forward(const GridP& g, const GridLeve
     }
 }
 
-template <int D, int F, int PD>
-__device__ __forceinline__ void grid_half_scatter(const GridP& g, const GridLevelP& lv, const float (&pos)[D], int side, const float (&adjF)[F])
+// table gradient (into `grad`) and, when requested, the gradient with respect to the unit-cube position (see
+// grid_level_adjoint) from this lane's half of the corners; adjPos receives this lane's share of the sum
+template <int D, int F, bool HALF, bool PARAM_GRAD, bool INPUT_GRAD, int PD>
+__device__ __forceinline__ void grid_half_adjoint(const GridP& g, float* grad, const GridLevelP& lv, const float (&pos)[D], int side,
+                                                  const float (&adjF)[F], float (&adjPos)[D])
 {
     const GridHalfCell<D, PD> c(pos, lv.resolution, side);
     const bool vec = g.vecOk != 0;
+    float lvl[D];
 #pragma unroll
-    for (int h = 0; h < (1 << (D - 1)); ++h)
-        grid_scatter_row<F>(g.grad, c.template index<F>(g, lv, h), vec, c.weight(h), adjF);
+    for (int k = 0; k < D; ++k) lvl[k] = 0.f;
+#pragma unroll
+    for (int h = 0; h < (1 << (D - 1)); ++h) {
+        const unsigned int e = c.template index<F>(g, lv, h);
+        if constexpr (PARAM_GRAD) grid_scatter_row<F>(grad, e, vec, c.weight(h), adjF);
+        if constexpr (INPUT_GRAD) {
+            float row[F];
+            grid_load_row<F, HALF>(g.table, e, vec, row);
+            float dot = 0.f;
+#pragma unroll
+            for (int i = 0; i < F; ++i) dot += adjF[i] * row[i];
+#pragma unroll
+            for (int k = 0; k < D; ++k) {
+                float wk = 1.f;   // weight without dimension k
+#pragma unroll
+                for (int j = D - 1, b = D - 2; j >= 0; --j) {
+                    const int bit = j == PD ? 0 : b--;
+                    if (j == k) continue;
+                    wk *= j == PD ? c.wp : ((h >> bit) & 1) ? c.c.f[j] : (1.f - c.c.f[j]);
+                }
+                // bit of dimension k: its position among the dimensions other than PD
+                const bool high = k == PD ? side != 0 : ((h >> (k > PD ? k - 1 : k)) & 1) != 0;
+                lvl[k] += (high ? wk : -wk) * dot;
+            }
+        }
+    }
+    if constexpr (INPUT_GRAD) {
+#pragma unroll
+        for (int k = 0; k < D; ++k) adjPos[k] += lvl[k] * static_cast<float>(lv.resolution - 1);
+    }
+}
+
+template <int D, int F, int PD>
+__device__ __forceinline__ void grid_half_scatter(const GridP& g, const GridLevelP& lv, const float (&pos)[D], int side, const float (&adjF)[F])
+{
+    float none[D];
+    grid_half_adjoint<D, F, false, true, false, PD>(g, g.grad, lv, pos, side, adjF, none);
 }
 
 } // namespace kernel

@@ -55,6 +55,15 @@ constexpr int FLAG_GRAD_ENCODINGS = 4;
 // FLAG_GRAD_INPUT.
 constexpr int FLAG_SPLIT_SCATTER = 8;
 
+// Copies of the gradients of small grid levels. Reductions to one 128-byte line execute one after the other in its L2 slice
+// (about nine clocks each): a level of a few lines that a large batch keeps hitting holds the whole kernel up. Such
+// levels are scattered into several copies, picked by the CTA, which are added up afterwards.
+struct GradReplicas {
+    float* base;                            // copies of all such levels, level by level (null: none)
+    long long total;                        // elements
+    unsigned char log2Copies[MAX_GRID_LEVELS];   // 0: the level has no copies
+};
+
 struct LaunchArgs {
     long long numel;
     const float* input;     long long inS0, inS1;
@@ -85,6 +94,7 @@ struct LaunchArgs {
     float* sortedTarget;                           // (numel, NUM_OUTPUTS) row-major, may be null
     int scatterLevelBegin, scatterLevelEnd;        // KERNEL_SCATTER_PLANES: grid levels (counted over all grids) to scatter; 0, 0 = all
     int runAggregation;                            // 0: every point of every level scatters straight to the gradient table
+    GradReplicas replicas;                         // KERNEL_ENCODING_ADJOINT
     GridP grids[MAX_GRIDS];
 };
 
@@ -131,4 +141,4 @@ extern "C" {
 typedef int (*qmlp_spec_launch_fn)(int kernel, const void* args, cudaStream_t stream, int* launches);
 typedef int (*qmlp_spec_abi_fn)(void);
 }
-#define QMLP_SPEC_ABI_VERSION 9
+#define QMLP_SPEC_ABI_VERSION 10

@@ -34,7 +34,7 @@ using OptTensor = std::optional<Tensor>;
     X(network_destroy) X(network_set_parameter) X(network_inference) X(network_inference_host) X(network_forward_memory)  \
     X(network_forward) X(network_adjoint_memory) X(network_adjoint) X(network_parameter_count) X(encoding_create)         \
     X(encoding_num_output_channels) X(encoding_has_parameters) X(encoding_set_parameter) X(encoding_forward)              \
-    X(encoding_adjoint) X(activation_create) X(activation_forward) X(activation_adjoint) X(trainer_workspace_bytes)       \
+    X(encoding_adjoint_memory) X(encoding_adjoint_with_memory) X(activation_create) X(activation_forward) X(activation_adjoint) X(trainer_workspace_bytes)       \
     X(trainer_gradients_part) X(trainer_update) X(convert_half)
 
 struct Api {
@@ -339,9 +339,13 @@ std::tuple<Tensor, Tensor> encodingAdjoint(const Tensor& input, const OptTensor&
     Tensor adjParam = param ? zeros(parameters->sizes(), floatLike(*parameters)) : at::empty({0}, input.options());
     const qmlp_tensor_t in = wrap(input), ao = wrap(go), p = parameters.has_value() ? wrap(*parameters) : qmlp_tensor_t{};
     qmlp_tensor_t ai = wantInput ? wrap(adjInput) : qmlp_tensor_t{}, ap = param ? wrap(adjParam) : qmlp_tensor_t{};
+    const int mode = (wantInput ? QMLP_ENCODING_INPUT_GRADIENTS : 0) | (param ? QMLP_ENCODING_PARAM_GRADIENTS : 0);
+    size_t bytes = 0;
+    check(api.encoding_adjoint_memory(e.handle, input.size(0), mode, &bytes));
+    const Tensor tmp = bytes > 0 ? at::empty({static_cast<int64_t>(bytes)}, floatLike(input).dtype(torch::kUInt8)) : Tensor();
     std::lock_guard<std::mutex> lock(e.mutex);
-    check(api.encoding_adjoint(e.handle, &in, &ao, &ai, currentStream(), parameters.has_value() ? &p : nullptr, param ? &ap : nullptr,
-                               (wantInput ? QMLP_ENCODING_INPUT_GRADIENTS : 0) | (param ? QMLP_ENCODING_PARAM_GRADIENTS : 0)));
+    check(api.encoding_adjoint_with_memory(e.handle, &in, &ao, &ai, currentStream(), parameters.has_value() ? &p : nullptr, param ? &ap : nullptr, mode,
+                                           bytes > 0 ? tmp.data_ptr() : nullptr, bytes));
     return {adjInput, adjParam};
 }
 Tensor activationForward(const Tensor& input, std::string_view cfg)

@@ -208,8 +208,12 @@ class Encoding:
         mode = (1 if want_input else 0) | (2 if adj_param is not None else 0)
         p = wrap(parameters) if parameters is not None else None
         g = wrap(adj_param) if adj_param is not None else None
-        check(lib().qmlp_encoding_adjoint(self._h, wrap(input), wrap(adj_output.contiguous()), wrap(adj_input), current_stream(),
-                                          C.byref(p) if p is not None else None, C.byref(g) if g is not None else None, mode))
+        b = C.c_size_t()
+        check(lib().qmlp_encoding_adjoint_memory(self._h, input.shape[0], mode, C.byref(b)))
+        tmp = torch.empty((b.value,), dtype=torch.uint8, device=input.device) if b.value else None
+        check(lib().qmlp_encoding_adjoint_with_memory(self._h, wrap(input), wrap(adj_output.contiguous()), wrap(adj_input), current_stream(),
+                                                      C.byref(p) if p is not None else None, C.byref(g) if g is not None else None, mode,
+                                                      tmp.data_ptr() if tmp is not None else None, b.value))
         return adj_input, adj_param
 
     def adjoint(self, input, adj_output):

@@ -185,3 +185,34 @@ def test_encoding_errors():
     cfg, e, oe = _enc("dense2d")
     with pytest.raises(QmlpError):
         e.inference_with_parameter(torch.zeros((4, 2), device="cuda"), torch.zeros((3,), device="cuda"))  # wrong size
+
+
+@pytest.mark.parametrize("name,n", [("dense2d_multires", 32769), ("dense2d_multires", 70001), ("hash3d_f2", 30000), ("hash3d_f2", 65),
+                                    ("hash2d_f8", 20001), ("hash3d_f3_add", 30001)])
+def test_adjoint_with_gradient_copies(name, n):
+    """Table and input gradients with scratch memory for copies of the small levels (lengths at which no, some and all levels
+    have copies, odd numbers of points) against the same call without scratch. Both add the same fp32 terms in different
+    orders: a row of k terms of one sign may differ by k * 2^-24 relative, here k <= 2^15 on a level of a few hundred rows."""
+    import ctypes as C
+    import torch
+    from qmlp._capi import check, lib, wrap
+    cfg, e, oe = _enc(name)
+    lo = float(oe.box_min.min())
+    hi = lo + float((1.0 / oe.box_inv_size).max())
+    x = torch.from_numpy(helpers.uniform(9, 1, (n, oe.start_in + oe.n_in), lo, hi)).cuda()
+    adj = torch.from_numpy(helpers.uniform(9, 2, (n, oe.num_outputs), 0.0, 1.0)).cuda()
+    table = torch.from_numpy(helpers.uniform(9, 3, (oe.num_parameters,), -1.0, 1.0)).cuda()
+    need = C.c_size_t()
+    check(lib().qmlp_encoding_adjoint_memory(e._h, n, 3, C.byref(need)))
+    assert (need.value > 0) == (n != 65)
+    results = []
+    for tmp in (None, torch.full((max(need.value, 16),), 0x7e, dtype=torch.uint8, device="cuda")):
+        gx, gt = torch.zeros_like(x), torch.zeros_like(table)
+        p, g, ai = wrap(table), wrap(gt), wrap(gx)
+        check(lib().qmlp_encoding_adjoint_with_memory(e._h, wrap(x), wrap(adj), ai, None, C.byref(p), C.byref(g), 3,
+                                                      tmp.data_ptr() if tmp is not None else None, need.value if tmp is not None else 0))
+        torch.cuda.synchronize()
+        results.append((gx, gt))
+    (gx0, gt0), (gx1, gt1) = results
+    assert torch.equal(gx0, gx1)
+    helpers.assert_close(gt1.cpu().numpy(), gt0.cpu().numpy(), f"{name} n={n}", rtol=2.0 ** -9, atol=1e-5 * float(gt0.abs().max()))
