@@ -1146,6 +1146,34 @@ int qmlp_trainer_gradients_part(qmlp_trainer_t* tr, const qmlp_tensor_t* input, 
             a.tS1 = 1;
         }
     }
+    // The layers' forward, loss, backward and weight gradients in one kernel on the planes (kernels/fused_train_tc.cuh),
+    // for every network and batch it is instantiated for; the separate kernels below remain for wider networks, line
+    // integration, the sorted step, the mma.sync-only path and bounds-checking instantiations (which test the stash).
+    if (!sorted && (path == 0 || path == 2) && !lib.boundsCheck && lib.splitScatter != 0 && numel > 0) {
+        auto m = n.module(n.currentHalfMask());
+        if (n.trainKernel < 0) {
+            kernel::LaunchArgs none = a;
+            none.numel = 0;
+            n.trainKernel = m->launch(kernel::KERNEL_TRAIN, &none, static_cast<cudaStream_t>(stream), nullptr) == 0 ? 1 : 0;
+        }
+        if (n.trainKernel == 1) {
+            a.planes = planes;
+            a.planeStride = n32;
+            a.flags = kernel::FLAG_GRAD_WEIGHTS | (anyGrid ? kernel::FLAG_GRAD_ENCODINGS : 0);
+            if (what == 4 && !anyGrid) throw std::runtime_error("this network has no grid levels to scatter: use parts = 1");
+            if (what & 5) {
+                if (anyGrid) launchModule(n, *m, kernel::KERNEL_ENCODE_PLANES, a, stream);
+                launchModule(n, *m, kernel::KERNEL_TRAIN, a, stream);
+            }
+            if (what == 8) {
+                if (levelEnd <= levelBegin) throw std::runtime_error("empty range of grid levels");
+                a.scatterLevelBegin = levelBegin;
+                a.scatterLevelEnd = levelEnd;
+            }
+            if (anyGrid && (what == 1 || what == 3 || what == 8)) launchModule(n, *m, kernel::KERNEL_SCATTER_PLANES, a, stream);
+            return QMLP_OK;
+        }
+    }
     if (what & 5) {
         bool done = false;
         if (wantPlanes) {

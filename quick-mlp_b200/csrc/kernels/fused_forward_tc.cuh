@@ -541,14 +541,10 @@ struct TcLaunchers {
         constexpr int threads = TL::warpgroups() * 128;
         static DeviceOnce once;   // function attributes are per device
         auto k = fused_forward_tc_kernel<Spec, PLANES>;
-        // the maps depend on the address of the parameter vector alone: the ones of this thread's last call usually serve
-        static thread_local TcWeightMaps<Spec> maps;
-        static thread_local const __half* mapsOf = nullptr;
-        if (mapsOf != a.weights) {
-            mapsOf = nullptr;
-            const cudaError_t e = encodeWeightMaps(a.weights, maps);
+        const TcWeightMaps<Spec>* maps = nullptr;
+        {
+            const cudaError_t e = weightMaps(a.weights, maps);
             if (e != cudaSuccess) return e;
-            mapsOf = a.weights;
         }
         {
             const cudaError_t e = once.run([&] { return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); });
@@ -557,8 +553,22 @@ struct TcLaunchers {
         const long long tiles = (a.numel + TC_TILE - 1) / TC_TILE;
         long long blocks = tiles < a.numSMs ? tiles : a.numSMs;
         if (blocks < 1) blocks = 1;
-        k<<<static_cast<unsigned>(blocks), threads, smem, s>>>(a, maps);
+        k<<<static_cast<unsigned>(blocks), threads, smem, s>>>(a, *maps);
         return cudaGetLastError();
+    }
+    // The maps depend on the address of the parameter vector alone: the ones of this thread's last call usually serve.
+    static cudaError_t weightMaps(const __half* weights, const TcWeightMaps<Spec>*& out)
+    {
+        static thread_local TcWeightMaps<Spec> maps;
+        static thread_local const __half* mapsOf = nullptr;
+        if (mapsOf != weights) {
+            mapsOf = nullptr;
+            const cudaError_t e = encodeWeightMaps(weights, maps);
+            if (e != cudaSuccess) return e;
+            mapsOf = weights;
+        }
+        out = &maps;
+        return cudaSuccess;
     }
     // Tensor maps over the weight matrices of the bound parameter vector. Encoding is host arithmetic (no driver call
     // touches the device), a microsecond per matrix; the maps travel as a kernel parameter.

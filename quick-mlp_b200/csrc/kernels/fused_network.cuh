@@ -1080,6 +1080,8 @@ struct PerDevice {
 };
 
 template <class Spec> struct TcLaunchers;
+template <class Spec> struct TrainLayout;  // fused_train_tc.cuh
+template <class Spec> struct TrainLaunchers;
 template <class Spec> struct PlaneLaunchers;
 template <class Spec> struct SortLaunchers;
 
@@ -1212,6 +1214,11 @@ struct NetworkLaunchers {
         case KERNEL_BACKWARD: e = backward(a, s); n = (a.flags & 7) ? 1 : 0; break;
         case KERNEL_WGRAD: e = wgrad(a, s); break;
         case KERNEL_SCATTER_PLANES: e = PlaneLaunchers<Spec>::scatter(a, s); break;
+        case KERNEL_TRAIN:
+            if constexpr (TrainLayout<Spec>::eligible()) e = TrainLaunchers<Spec>::run(a, s);
+            else e = cudaErrorNotSupported;
+            if (a.numel == 0) n = 0;
+            break;
         case KERNEL_SORT_POINTS: e = SortLaunchers<Spec>::sort(a, s, &n); break;
         case KERNEL_SCATTER_SORTED: e = SortLaunchers<Spec>::scatter(a, s); break;
         default: break;

@@ -122,6 +122,7 @@ enum KernelId {
     KERNEL_SCATTER_PLANES = 11,    // adjoint feature planes -> grid table gradients, one grid level at a time
     KERNEL_FORWARD_LOSS_PLANES = 12, // KERNEL_FORWARD_LOSS with layer 0 fed from the planes of KERNEL_ENCODE_PLANES
     KERNEL_SORT_POINTS = 13,         // points (and targets) -> Morton-bin order: count, scan, reorder
+    KERNEL_TRAIN = 14,               // layers of a training step on the planes: forward, loss, backward, weight gradients; adjoints back to the planes
     KERNEL_SCATTER_SORTED = 15       // KERNEL_SCATTER_PLANES for sorted points: coarse levels summed in shared memory first
 };
 

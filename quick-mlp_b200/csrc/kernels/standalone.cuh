@@ -5,6 +5,7 @@
 #pragma once
 #include "fused_network.cuh"
 #include "fused_forward_tc.cuh"
+#include "fused_train_tc.cuh"
 
 namespace qmlp {
 namespace kernel {

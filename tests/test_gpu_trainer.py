@@ -244,3 +244,45 @@ def test_step_from_host_memory_with_prefetch():
     diff = np.abs(m_host - m_dev)
     assert float((diff > 2e-4 + 1e-3 * np.abs(m_dev)).mean()) < 0.01 and float(diff.max()) <= 4.1e-2
     assert bindings.QuickMLP.device_status() == 0
+
+
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 148 * 128 + 1, 2 * 148 * 128 + 77])
+@pytest.mark.parametrize("name", ["config1", "config2", "ref_widths", "uneven", "per_channel", "config3_small", "config4_small", "config5_small",
+                                  "grid2d_add_plus_identity"])
+def test_train_kernel_matches_separate_kernels(name, n):
+    """Gradients and loss of one step from the fused layer kernel against the forward / backward / weight-gradient kernels
+    (kernel path 1): batches that end inside a tile, fill one tile, and give a CTA one, two and three tiles; widths with
+    and without the bias MMA, one and two blocks of 64 channels, kept and recomputed accumulators. Both round the same
+    values to fp16; fp32 sums in another order move a rounding by 2^-11 now and then, and a pre-activation within that of
+    zero may flip a relu: 1e-2 of the norm of each segment."""
+    import torch
+    from qmlp import bindings
+    from qmlp.trainer import FusedTrainer
+    from test_gpu_network import network_cases
+    cfg, rng, _ = network_cases()[name]
+    spec = oracle.parse_spec(cfg)
+    x = torch.from_numpy(helpers.uniform(31, 1, (n, spec.num_inputs), *rng)).cuda()
+    t = torch.from_numpy(helpers.uniform(31, 2, (n, spec.num_outputs), -1.0, 1.0)).cuda()
+    params = torch.from_numpy(helpers.xavier_parameters(spec, cfg, bias_scale=0.1).astype(np.float32)).cuda()
+    tables = [torch.from_numpy(tb).cuda() if tb is not None else None for tb in helpers.grid_tables(spec, scale=0.5)]
+    results = []
+    try:
+        for path in (0, 1):
+            bindings.QuickMLP.set_kernel_path(path)
+            net = bindings.Network(json.dumps(cfg))
+            tr = FusedTrainer(net, grid_half_copy=False)
+            tr.set_parameters(params, tables)
+            tr.backend.gradients(x, t, n, tr.loss_sum)
+            torch.cuda.synchronize()
+            results.append((tr, net.launch_count()))
+    finally:
+        bindings.QuickMLP.set_kernel_path(0)
+    (a, launches), (b, launches_separate) = results
+    assert launches < launches_separate + (1 if spec.encodings[0].num_parameters else 0)     # the fused kernel ran
+    assert abs(a.loss_sum.item() - b.loss_sum.item()) <= 1e-2 * abs(b.loss_sum.item())
+    for i in range(1 + len(spec.encodings)):
+        ga, gb = a.segment(a.gradient, i), b.segment(b.gradient, i)
+        if gb is None:
+            continue
+        norm = float(gb.norm())
+        assert norm > 0 and float((ga - gb).norm()) <= 1e-2 * norm, f"{name} n={n} segment {i}: {float((ga - gb).norm()) / norm}"
