@@ -436,15 +436,22 @@ static void inferenceLocked(Network& n, const qmlp_tensor_t* input, qmlp_tensor_
     a.output = static_cast<float*>(output->data);
     a.outS0 = output->strides[0];
     a.outS1 = output->strides[1];
-    // Encode level by level into planes, chunk by chunk, then run the layer chain on the planes
-    // (kernels/grid_planes.cuh): when the tables are much larger than L2 (the level in work stays L2-resident), and when
-    // the gather dominates a large batch (96 or more table rows per point: the dedicated pass keeps four light CTAs per
-    // SM on nothing but gathers and runs at the SM's L2-request rate; config 3 at 2^20 points 0.40 -> 0.34 ms, while
-    // config 4 with 72 rows per point and a heavier layer chain is level). kernelPath 2 forces this path.
+    // Encode level by level into planes, chunk by chunk, then run the layer chain on the planes (kernels/grid_planes.cuh), or
+    // gather inside the layer kernel (fused_forward_kernel). Since both gather with lane pairs the fused kernel wins wherever
+    // the level being gathered does not become resident any closer by going level by level: 3-D grid, 16 levels of 2^19
+    // rows, 2^20 points 272 against 281 us. The pass wins with
+    //  - tables larger than L2 (one level at a time stays in it): 4-D grid of 2^20 rows, 2^20 points 689 against 1178 us;
+    //  - levels of up to 384 KB on average (one level at a time stays largely in L1), from 2^19 points on: 3-D grid of 2^15
+    //    fp16 rows, 2^20 points 192 against 257 us;
+    //  - 192 or more rows per point (the fused kernel's 16 warps per SM keep too few of them in flight), from 2^17 points on
+    //    with fp16 tables, 2^19 with fp32: 4-D grid of 2^18 fp16 rows, 2^20 points 635 against 711 us.
+    // kernelPath 2 forces this path.
     const int path = Library::instance().kernelPath;
-    const bool gatherBound = n.gathersPerPoint() >= 96 && a.numel >= (1 << 18);
-    const bool wantPlanes = !n.planesUnsupported && a.numGrids > 0 && a.numel > 0 &&
-                            (path == 2 || (path == 0 && (n.gridTableBytes() > (96ll << 20) || gatherBound)));
+    const int64_t tableBytes = n.gridTableBytes();
+    const bool halfTables = n.currentHalfMask() != 0;
+    const bool chosen = tableBytes > (96ll << 20) || (a.numel >= (1 << 19) && tableBytes <= (384ll << 10) * n.gridLevels()) ||
+                        (n.gathersPerPoint() >= 192 && a.numel >= (halfTables ? 1 << 17 : 1 << 19));
+    const bool wantPlanes = !n.planesUnsupported && a.numGrids > 0 && a.numel > 0 && (path == 2 || (path == 0 && chosen));
     if (wantPlanes) {
         // Chunk: as many points as fit in 512 MB of planes, at most 2^22. A level's table is fetched from HBM once per
         // chunk, so large chunks amortise it; the planes themselves are streamed (written once, read once).

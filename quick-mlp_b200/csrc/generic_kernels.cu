@@ -35,7 +35,8 @@ __global__ void __launch_bounds__(256) adam_kernel(float4* __restrict__ master, 
         master[i] = p;
         m[i] = mm;
         v[i] = vv;
-        grad[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        // a gradient that is zero already (rows no point of the batch touched) is not written back
+        if (gp[0] != 0.f || gp[1] != 0.f || gp[2] != 0.f || gp[3] != 0.f) grad[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         __half2 h0 = __floats2half2_rn(pp[0], pp[1]), h1 = __floats2half2_rn(pp[2], pp[3]);
         uint2 u;
         u.x = *reinterpret_cast<unsigned int*>(&h0);

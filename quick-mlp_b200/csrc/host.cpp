@@ -622,6 +622,14 @@ int Network::gathersPerPoint() const
     return g;
 }
 
+int Network::gridLevels() const
+{
+    int l = 0;
+    for (const auto& e : encodings_)
+        if (auto* h = dynamic_cast<const EncodingHashGrid*>(e.get())) l += static_cast<int>(h->levelTable().size());
+    return l;
+}
+
 int Network::sortDimensions() const
 {
     for (const auto& e : encodings_)

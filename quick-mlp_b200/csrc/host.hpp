@@ -254,6 +254,7 @@ public:
     ~Network();
     int64_t gridTableBytes() const;   // bytes of all bound grid tables (what the gather walks through)
     int gathersPerPoint() const;      // table rows fetched per point by all plain grid encodings: sum of levels * 2^D
+    int gridLevels() const;           // levels of all grid encodings
     int sortDimensions() const;       // dimension of the grid whose bounding box bins the points of a training step (0: none)
     // level-major encoding pass (inference of networks with tables larger than L2): chunk buffer, allocated at the
     // first such call and kept until the network is destroyed

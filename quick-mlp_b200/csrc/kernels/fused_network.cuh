@@ -135,6 +135,9 @@ __host__ __device__ constexpr int resident_ctas()
 #endif
 }
 
+// Weights and biases -> shared memory, all layers in flight at once (asynchronous 16-byte copies; the caller waits with
+// cp_async_wait<0>() and __syncthreads()). A loop of loads and stores per layer waited out one memory latency per pass:
+// 1000 points through the 64-wide network 8.4 -> 3.7 us (the first tile is encoded meanwhile). Offsets of weights and biases in the vector are multiples of 16 halfs.
 template <class Spec, int L>
 __device__ __forceinline__ void stage_layer(const LaunchArgs& p, __half* sW, __half* sB)
 {
@@ -144,14 +147,14 @@ __device__ __forceinline__ void stage_layer(const LaunchArgs& p, __half* sW, __h
         constexpr int CHUNKS = CIN / 8; // 16-byte chunks per row
         const __half* gW = p.weights + Spec::WOFF[L];
         __half* dW = sW + SL::wOffsetHalfs(L);
-        for (int i = threadIdx.x; i < COUT * CHUNKS; i += blockDim.x) {
+#pragma unroll
+        for (int i = threadIdx.x; i < COUT * CHUNKS; i += Spec::WARPS * 32) {
             const int r = i / CHUNKS, c = i % CHUNKS;
-            const uint4 v = *reinterpret_cast<const uint4*>(gW + r * CIN + c * 8);
-            *reinterpret_cast<uint4*>(dW + r * SL::wStride(L) + c * 8) = v;
+            cp_async16(smem_u32(dW + r * SL::wStride(L) + c * 8), gW + r * CIN + c * 8, true);
         }
-        __half* dB = sB + SL::biasOffset(L);
-        for (int i = threadIdx.x; i < COUT; i += blockDim.x)
-            dB[i] = Spec::BOFF[L] >= 0 ? p.weights[(Spec::BOFF[L] >= 0 ? Spec::BOFF[L] : 0) + i] : __ushort_as_half(0);
+        constexpr bool BIAS = Spec::BOFF[L] >= 0;
+        for (int i = threadIdx.x; i < COUT / 8; i += Spec::WARPS * 32)
+            cp_async16(smem_u32(sB + SL::biasOffset(L) + i * 8), p.weights + (BIAS ? Spec::BOFF[L] : 0) + i * 8, BIAS);
         stage_layer<Spec, L + 1>(p, sW, sB);
     }
 }
@@ -312,6 +315,56 @@ __device__ __forceinline__ void encode_point(const LaunchArgs& p, const RowReade
             }
         }
         encode_point<Spec, E + 1, Out>(p, in, out);
+    }
+}
+
+// The same for the 32 points of a warp, lanes in pairs (see grid.cuh): both lanes gather half of the corners of the even
+// lane's point, then of the odd lane's, and each ends up with the features of its own point. `in0` / `in1`: input rows of
+// the pair's two points (inside the batch); all lanes of the warp take part.
+template <class Spec, int E, class Out>
+__device__ __forceinline__ void encode_pair(const LaunchArgs& p, const RowReader& in0, const RowReader& in1, const Out& out)
+{
+    if constexpr (E < Spec::NUM_ENCODINGS) {
+        using Enc = typename Spec::template Enc<E>;
+        const int side = threadIdx.x & 1;
+        if constexpr (Enc::IS_LINE) {
+            line_forward<Enc>(p.grids[Enc::SLOT], side ? in1 : in0, out);
+        } else if constexpr (!Enc::IS_GRID) {
+            const RowReader& in = side ? in1 : in0;
+#pragma unroll
+            for (int i = 0; i < Enc::N; ++i) out(Enc::OUT_OFF + i, in(i + Enc::START));
+        } else {
+            constexpr int D = Enc::D, F = Enc::F;
+            const GridP& g = p.grids[Enc::SLOT];
+            float pos0[D], pos1[D], sum[F];
+            grid_position<D, Enc::START>(g, in0, pos0);
+            grid_position<D, Enc::START>(g, in1, pos1);
+#pragma unroll
+            for (int i = 0; i < F; ++i) sum[i] = 0.f;
+#pragma unroll 2
+            for (int l = 0; l < Enc::L; ++l) {
+                const GridLevelP& lv = g.levels[l];
+                float f0[F], f1[F];
+                if (lv.hashed) {
+                    grid_half_forward<D, F, Enc::HALF_TABLE, 0>(g, lv, pos0, side, f0);
+                    grid_half_forward<D, F, Enc::HALF_TABLE, 0>(g, lv, pos1, side, f1);
+                } else {
+                    grid_half_forward<D, F, Enc::HALF_TABLE, D - 1>(g, lv, pos0, side, f0);
+                    grid_half_forward<D, F, Enc::HALF_TABLE, D - 1>(g, lv, pos1, side, f1);
+                }
+#pragma unroll
+                for (int i = 0; i < F; ++i) {
+                    const float v = (side ? f1[i] : f0[i]) + __shfl_xor_sync(0xffffffffu, side ? f0[i] : f1[i], 1);
+                    if constexpr (Enc::CONCAT) out(Enc::OUT_OFF + l * F + i, v);
+                    else sum[i] += v;
+                }
+            }
+            if constexpr (!Enc::CONCAT) {
+#pragma unroll
+                for (int i = 0; i < F; ++i) out(Enc::OUT_OFF + i, sum[i]);
+            }
+        }
+        encode_pair<Spec, E + 1, Out>(p, in0, in1, out);
     }
 }
 
@@ -512,7 +565,7 @@ fused_forward_kernel(const __grid_constant__ LaunchArgs p)
     __half* sW = reinterpret_cast<__half*>(smem);
     __half* sB = reinterpret_cast<__half*>(smem + SL::biasStartBytes());
     stage_layer<Spec, 0>(p, sW, sB);
-    __syncthreads();
+    cp_async_commit();
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     __half* tile = reinterpret_cast<__half*>(smem + SL::tileStartBytes() + warp * SL::tileBytesPerWarp());
@@ -522,19 +575,19 @@ fused_forward_kernel(const __grid_constant__ LaunchArgs p)
     const long long numTiles = n32 / TILE_POINTS;
     float lossAcc = 0.f;
 
-    for (long long t = static_cast<long long>(blockIdx.x) * Spec::WARPS + warp; t < numTiles;
-         t += static_cast<long long>(gridDim.x) * Spec::WARPS) {
+    // encodings of tile t -> this warp's tile in shared memory (and the stash)
+    auto encode = [&](long long t) {
         const long long rowBase = t * TILE_POINTS;
         const long long myRow = rowBase + lane;
         __half* row = tile + lane * TS;
         // encodings; padding channels and invalid tail points are zero (kernels/network_forward.cuh:67-89)
+        if constexpr (!FROM_PLANES) {
+            const long long last = p.numel - 1, i0 = myRow & ~1ll;   // (a lane past the end repeats the last point)
+            const RowReader in0{p.input + (i0 < last ? i0 : last) * p.inS0, p.inS1}, in1{p.input + (i0 + 1 < last ? i0 + 1 : last) * p.inS0, p.inS1};
+            encode_pair<Spec, 0>(p, in0, in1, HalfRowWriter{row});
+        }
         if (myRow < p.numel) {
-            if constexpr (FROM_PLANES) {
-                read_planes_point<Spec, 0>(p, myRow, HalfRowPlaneWriter{row});
-            } else {
-                RowReader in{p.input + myRow * p.inS0, p.inS1};
-                encode_point<Spec, 0>(p, in, HalfRowWriter{row});
-            }
+            if constexpr (FROM_PLANES) read_planes_point<Spec, 0>(p, myRow, HalfRowPlaneWriter{row});
 #pragma unroll
             for (int c = Spec::ENC_CHANNELS; c < CIN0; ++c) row[c] = __ushort_as_half(0);
         } else {
@@ -552,6 +605,20 @@ fused_forward_kernel(const __grid_constant__ LaunchArgs p)
                     *reinterpret_cast<uint4*>(st + (rowBase + rr) * CIN0 + cc * 8) = *reinterpret_cast<const uint4*>(tile + rr * TS + cc * 8);
             }
         }
+    };
+    // Tiles go round the CTAs first, so that a batch of fewer tiles than warps is spread over all SMs. The first tile is
+    // encoded while the weights are on their way.
+    const long long step = static_cast<long long>(gridDim.x) * Spec::WARPS;
+    bool staged = false;
+    for (long long t = blockIdx.x + static_cast<long long>(warp) * gridDim.x;; t += step) {
+        if (t < numTiles) encode(t);
+        if (!staged) {
+            cp_async_wait<0>();
+            __syncthreads();
+            staged = true;
+        }
+        if (t >= numTiles) break;
+        const long long rowBase = t * TILE_POINTS;
         uint32_t a0[MT][CIN0 / 16][4];
 #pragma unroll
         for (int m = 0; m < MT; ++m)
@@ -608,6 +675,70 @@ __device__ __forceinline__ void encode_adjoint_point(const LaunchArgs& p, const 
             }
         }
         encode_adjoint_point<Spec, E + 1, INPUT_GRAD, PARAM_GRAD, AdjOut>(p, in, adjOut, adjInRow, aiS1);
+    }
+}
+
+// The same for the 32 points of a warp, lanes in pairs. `tile`: adjoint features of the warp's points, row by row; `row0`: its
+// first point; all lanes of the warp take part.
+template <class Spec, int E, bool INPUT_GRAD, bool PARAM_GRAD>
+__device__ __forceinline__ void encode_adjoint_pair(const LaunchArgs& p, long long row0, const __half* tile, int tileStride)
+{
+    if constexpr (E < Spec::NUM_ENCODINGS) {
+        using Enc = typename Spec::template Enc<E>;
+        const int lane = threadIdx.x & 31, side = lane & 1;
+        const long long mine = row0 + lane, last = p.numel - 1;
+        if constexpr (!Enc::IS_GRID) {
+            if (mine <= last) {
+                const RowReader in{p.input + mine * p.inS0, p.inS1};
+                const HalfRowReader adj{tile + lane * tileStride};
+                float* adjInRow = INPUT_GRAD ? p.adjInput + mine * p.aiS0 : nullptr;
+                if constexpr (Enc::IS_LINE) {
+                    line_adjoint<Enc, INPUT_GRAD, PARAM_GRAD>(p.grids[Enc::SLOT], in, adj, adjInRow, p.aiS1);
+                } else if constexpr (INPUT_GRAD) {
+#pragma unroll
+                    for (int i = 0; i < Enc::N; ++i) adjInRow[(i + Enc::START) * p.aiS1] += adj(Enc::OUT_OFF + i);
+                }
+            }
+        } else {
+            constexpr int D = Enc::D, F = Enc::F;
+            const GridP& g = p.grids[Enc::SLOT];
+            const bool paramGrad = PARAM_GRAD && g.grad != nullptr;
+            const long long i0 = mine & ~1ll;
+            float pos[2][D], adjPos[2][D];
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+                grid_position<D, Enc::START>(g, RowReader{p.input + (i0 + s < last ? i0 + s : last) * p.inS0, p.inS1}, pos[s]);
+#pragma unroll
+                for (int k = 0; k < D; ++k) adjPos[s][k] = 0.f;
+            }
+            for (int l = 0; l < Enc::L; ++l) {
+                const GridLevelP& lv = g.levels[l];
+#pragma unroll
+                for (int s = 0; s < 2; ++s) {
+                    if (i0 + s > last) continue;
+                    const HalfRowReader adj{tile + ((lane & ~1) + s) * tileStride};
+                    float adjF[F];
+#pragma unroll
+                    for (int i = 0; i < F; ++i) adjF[i] = adj(Enc::OUT_OFF + (Enc::CONCAT ? l * F : 0) + i);
+                    if (paramGrad) {
+                        if (lv.hashed) grid_half_adjoint<D, F, Enc::HALF_TABLE, true, INPUT_GRAD, 0>(g, g.grad, lv, pos[s], side, adjF, adjPos[s]);
+                        else grid_half_adjoint<D, F, Enc::HALF_TABLE, true, INPUT_GRAD, D - 1>(g, g.grad, lv, pos[s], side, adjF, adjPos[s]);
+                    } else if constexpr (INPUT_GRAD) {
+                        if (lv.hashed) grid_half_adjoint<D, F, Enc::HALF_TABLE, false, true, 0>(g, g.grad, lv, pos[s], side, adjF, adjPos[s]);
+                        else grid_half_adjoint<D, F, Enc::HALF_TABLE, false, true, D - 1>(g, g.grad, lv, pos[s], side, adjF, adjPos[s]);
+                    }
+                }
+            }
+            if constexpr (INPUT_GRAD) {
+                // encoding_hashgrid.cuh:414-421
+#pragma unroll
+                for (int k = 0; k < D; ++k) {
+                    const float v = (side ? adjPos[1][k] : adjPos[0][k]) + __shfl_xor_sync(0xffffffffu, side ? adjPos[0][k] : adjPos[1][k], 1);
+                    if (mine <= last) p.adjInput[mine * p.aiS0 + (k + Enc::START) * p.aiS1] += v * g.boxInvSize[k];
+                }
+            }
+        }
+        encode_adjoint_pair<Spec, E + 1, INPUT_GRAD, PARAM_GRAD>(p, row0, tile, tileStride);
     }
 }
 
@@ -748,15 +879,10 @@ __device__ __forceinline__ void backward_layers(const LaunchArgs& p, const __hal
                     }
             __syncwarp();
             const long long myRow = rowBase + lane;
-            if (myRow < p.numel) {
-                if constexpr ((FLAGS & FLAG_SPLIT_SCATTER) != 0) {
-                    write_adjoint_planes<Spec, 0>(p, myRow, tile + lane * TS);
-                } else {
-                    RowReader in{p.input + myRow * p.inS0, p.inS1};
-                    float* adjInRow = (FLAGS & FLAG_GRAD_INPUT) ? p.adjInput + myRow * p.aiS0 : nullptr;
-                    encode_adjoint_point<Spec, 0, (FLAGS & FLAG_GRAD_INPUT) != 0, (FLAGS & FLAG_GRAD_ENCODINGS) != 0>(
-                        p, in, HalfRowReader{tile + lane * TS}, adjInRow, p.aiS1);
-                }
+            if constexpr ((FLAGS & FLAG_SPLIT_SCATTER) != 0) {
+                if (myRow < p.numel) write_adjoint_planes<Spec, 0>(p, myRow, tile + lane * TS);
+            } else {
+                encode_adjoint_pair<Spec, 0, (FLAGS & FLAG_GRAD_INPUT) != 0, (FLAGS & FLAG_GRAD_ENCODINGS) != 0>(p, rowBase, tile, TS);
             }
             __syncwarp();
         }
@@ -772,6 +898,8 @@ fused_backward_kernel(const __grid_constant__ LaunchArgs p)
     __half* sW = reinterpret_cast<__half*>(smem);
     __half* sB = reinterpret_cast<__half*>(smem + SL::biasStartBytes());
     stage_layer<Spec, 0>(p, sW, sB);
+    cp_async_commit();
+    cp_async_wait<0>();
     __syncthreads();
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -782,8 +910,7 @@ fused_backward_kernel(const __grid_constant__ LaunchArgs p)
     const long long n32 = (p.numel + 31) / 32 * 32;
     const long long numTiles = n32 / TILE_POINTS;
 
-    for (long long t = static_cast<long long>(blockIdx.x) * Spec::WARPS + warp; t < numTiles;
-         t += static_cast<long long>(gridDim.x) * Spec::WARPS) {
+    for (long long t = blockIdx.x + static_cast<long long>(warp) * gridDim.x; t < numTiles; t += static_cast<long long>(gridDim.x) * Spec::WARPS) {
         const long long rowBase = t * TILE_POINTS;
         // dL/dout (fp32, N x NUM_OUTPUTS) -> half fragments, zero padded (kernels/network_backward.cuh:67-80)
         uint32_t adj[MT][KT][4];
@@ -1041,6 +1168,20 @@ wgrad_kernel(const __grid_constant__ LaunchArgs p)
     wgrad_dispatch<Spec, 0>(p, smem);
 }
 
+// table rows fetched per point by all plain grids of a network
+template <class Spec, int E = 0>
+__host__ __device__ constexpr int table_rows_per_point()
+{
+    if constexpr (E >= Spec::NUM_ENCODINGS) {
+        return 0;
+    } else {
+        using Enc = typename Spec::template Enc<E>;
+        int own = 0;
+        if constexpr (Enc::IS_GRID) own = Enc::L << Enc::D;
+        return own + table_rows_per_point<Spec, E + 1>();
+    }
+}
+
 // ---- host-side launchers (compiled into each instantiation) -------------------------------------------------------
 template <class Spec> struct TcLayout;     // fused_forward_tc.cuh
 // Per-device latch for kernel attributes (a process may drive several GPUs): `run` performs `set` once per device and
@@ -1115,7 +1256,7 @@ struct NetworkLaunchers {
             if (e != cudaSuccess) return e;
         }
         const long long tiles = (a.numel + TILE_POINTS - 1) / TILE_POINTS;
-        long long blocks = (tiles + Spec::WARPS - 1) / Spec::WARPS;
+        long long blocks = tiles;
         const long long cap = static_cast<long long>(a.numSMs) * perSM;
         if (blocks > cap) blocks = cap;
         if (blocks < 1) blocks = 1;
@@ -1135,7 +1276,7 @@ struct NetworkLaunchers {
             if (e != cudaSuccess) return e;
         }
         const long long tiles = (a.numel + TILE_POINTS - 1) / TILE_POINTS;
-        long long blocks = (tiles + Spec::WARPS - 1) / Spec::WARPS;
+        long long blocks = tiles;
         const long long cap = static_cast<long long>(a.numSMs) * perSM;
         if (blocks > cap) blocks = cap;
         if (blocks < 1) blocks = 1;
@@ -1191,8 +1332,10 @@ struct NetworkLaunchers {
                 // The tcgen05 kernel pays a fixed price per launch (tensor-memory allocation, operand staging for 148
                 // large CTAs) and needs at least one 128-point tile per slot to use what it sets up; below that the
                 // mma.sync kernel is quicker (config 1 at 2^16 points: 2.7 us against 4.7 us; config 2 at 2^16: 11.5
-                // against 12.9 us, at 2^20: 89 against 62 us).
-                const bool enough = a.numel >= TcLayout<Spec>::pointsPerCta() * a.numSMs;
+                // against 12.9 us, at 2^20: 89 against 62 us). With a grid in front the gather decides, and the mma.sync
+                // kernel gathers with lane pairs and 16 warps (128 rows per point, 2^20 points: 272 against 364 us); few rows
+                // leave the layers in charge.
+                const bool enough = a.numel >= TcLayout<Spec>::pointsPerCta() * a.numSMs && table_rows_per_point<Spec>() < 32;
                 if (a.forcePath == 3 || (a.forcePath != 1 && enough)) { e = TcLaunchers<Spec>::inference(a, s); break; }
             }
             e = forward<0>(a, s);
@@ -1202,8 +1345,10 @@ struct NetworkLaunchers {
             else e = cudaErrorNotSupported;   // the caller falls back to the fused gather
             break;
         case KERNEL_INFERENCE_PLANES:
-            if constexpr (TcLayout<Spec>::eligible()) e = TcLaunchers<Spec>::inferencePlanes(a, s);
-            else e = cudaErrorNotSupported;
+            if constexpr (TcLayout<Spec>::eligible()) {
+                const bool enough = a.numel >= TcLayout<Spec>::pointsPerCta() * a.numSMs;   // as above
+                e = enough ? TcLaunchers<Spec>::inferencePlanes(a, s) : forward<4>(a, s);
+            } else e = cudaErrorNotSupported;
             break;
         case KERNEL_FORWARD: e = forward<1>(a, s); break;
         case KERNEL_FORWARD_LOSS: e = forward<2>(a, s); break;

@@ -43,18 +43,11 @@ namespace kernel {
 constexpr int TRAIN_WARPGROUPS = 4, TRAIN_THREADS = TRAIN_WARPGROUPS * 128 + 32;   // the last warp issues the MMAs
 constexpr int TRAIN_BLOCK = TC_TILE * 128;   // bytes of a block: 128 points x 64 channels
 
-template <class Spec, int E = 0>
-__host__ __device__ constexpr bool any_grid()
-{
-    if constexpr (E >= Spec::NUM_ENCODINGS) return false;
-    else return Spec::template Enc<E>::IS_GRID || any_grid<Spec, E + 1>();
-}
-
 template <class Spec>
 struct TrainLayout {
     using TL = TcLayout<Spec>;
     static constexpr int NL = Spec::NUM_LAYERS;
-    static constexpr bool GRID = any_grid<Spec>();   // the adjoint of the features is wanted
+    static constexpr bool GRID = table_rows_per_point<Spec>() > 0;   // the adjoint of the features is wanted
     __host__ __device__ static constexpr int blocks(int channels) { return (channels + 63) / 64; }
     __host__ __device__ static constexpr bool bias(int l) { return Spec::BOFF[l] >= 0; }
     // buffer l < NL: input of layer l (later delta of layer l - 1); buffer NL: delta of the last layer. A narrow last delta
