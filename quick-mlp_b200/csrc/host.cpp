@@ -201,7 +201,7 @@ std::shared_ptr<KernelModule> Encoding::standaloneModule(bool halfTable)
     auto& m = standalone_[(halfTable ? 1 : 0) + (Library::instance().boundsCheck ? 2 : 0)];
     if (m) return m;
     std::ostringstream s;
-    s << "// stand-alone encoding kernels: " << toJson().dump() << "\n#include \"standalone.cuh\"\nusing namespace qmlp::kernel;\n"
+    s << "// stand-alone encoding kernels: " << toJson().dump() << "\n#define QMLP_GRIDS " << (isGrid() ? 1 : 0) << "\n#include \"standalone.cuh\"\nusing namespace qmlp::kernel;\n"
       << "namespace {\nstruct EncSpec {\n    static constexpr int NUM_ENCODINGS = 1;\n    template <int E> struct Enc;\n};\n"
       << "template <> struct EncSpec::Enc<0> : " << deviceType(0, 0, halfTable) << " {};\n}\n"
       << "extern \"C\" int qmlp_spec_abi() { return QMLP_SPEC_ABI_VERSION; }\n"
@@ -734,7 +734,9 @@ std::string Network::generateSource(unsigned halfMask) const
     for (const auto& l : layers_)
         s << " " << l.channelsIn << "->" << l.channelsOut << (l.useBias ? "+b" : "") << ":"
           << (l.perChannel.empty() ? l.activation->id() : std::string("per-channel"));
-    s << "\n#include \"standalone.cuh\"\nusing namespace qmlp::kernel;\nnamespace {\nnamespace activations {\n";
+    int gridSlots = 0;
+    for (const auto& e : encodings_) gridSlots += e->isGrid() ? 1 : 0;
+    s << "\n#define QMLP_GRIDS " << gridSlots << "\n#include \"standalone.cuh\"\nusing namespace qmlp::kernel;\nnamespace {\nnamespace activations {\n";
     std::set<std::string> seen;
     for (const auto& l : layers_) {
         if (!l.activation->isBuiltin() && seen.insert(l.activation->id()).second) s << l.activation->functorDefinition();

@@ -12,6 +12,14 @@ namespace kernel {
 
 constexpr int MAX_GRID_LEVELS = 32;
 constexpr int MAX_GRIDS = 4;
+// Grid slots of the launch arguments as this translation unit sees them. The generated source of a network defines how many
+// it uses, so that a launch copies no more: the slots are the last member, and an instantiation reads a prefix of what the
+// library passes.
+#ifdef QMLP_GRIDS
+constexpr int GRID_SLOTS = QMLP_GRIDS;
+#else
+constexpr int GRID_SLOTS = MAX_GRIDS;
+#endif
 constexpr int MAX_GRID_DIMS = 6;
 
 struct GridLevelP {
@@ -95,7 +103,7 @@ struct LaunchArgs {
     int scatterLevelBegin, scatterLevelEnd;        // KERNEL_SCATTER_PLANES: grid levels (counted over all grids) to scatter; 0, 0 = all
     int runAggregation;                            // 0: every point of every level scatters straight to the gradient table
     GradReplicas replicas;                         // KERNEL_ENCODING_ADJOINT
-    GridP grids[MAX_GRIDS];
+    GridP grids[GRID_SLOTS];                       // the last member (GRID_SLOTS)
 };
 
 // Bins of the point sort: a regular grid of 2^sort_bin_bits(D) cells per dimension over the bounding box of the first

@@ -262,7 +262,8 @@ class Network:
         check(lib().qmlp_network_create(cfg.encode(), parent.encode(), C.byref(h)))
         self._h = h
         # owns the handle and serialises the calls (the bound parameter pointers are state of the network, bind_network.h:20)
-        self._calls = _capi.calls().NetworkCalls(h.value)
+        self._native = _capi.calls()
+        self._calls = self._native.NetworkCalls(h.value)
         self._channels = (lib().qmlp_network_channels_in(h), lib().qmlp_network_channels_out(h))
 
     def cfg(self) -> str:
@@ -340,11 +341,11 @@ class Network:
 
     # -- launches ----------------------------------------------------------------------------------------------------
     def _bind(self, network_parameters, encoding_parameters: Sequence[Optional[torch.Tensor]]):
-        _capi.calls().network_bind(self._calls, network_parameters, list(encoding_parameters))
+        self._native.network_bind(self._calls, network_parameters, list(encoding_parameters))
 
     def inference(self, input: torch.Tensor, network_parameters: torch.Tensor,
                   encoding_parameters: Sequence[Optional[torch.Tensor]] = ()) -> torch.Tensor:
-        return _capi.calls().network_inference(self._calls, input, network_parameters, encoding_parameters)
+        return self._native.network_inference(self._calls, input, network_parameters, encoding_parameters)
 
     def inference_host(self, input: torch.Tensor, network_parameters: torch.Tensor,
                        encoding_parameters: Sequence[Optional[torch.Tensor]] = (),
@@ -359,14 +360,14 @@ class Network:
             output = torch.empty((n, self.channels_out()), dtype=torch.float32, pin_memory=True)
         assert output.device.type == "cpu" and output.dtype == torch.float32 and output.is_contiguous()
         assert tuple(output.shape) == (n, self.channels_out()) and input.shape[1] == self.channels_in()
-        _capi.calls().network_inference_host(self._calls, input, network_parameters, encoding_parameters, output, int(chunk_points))
+        self._native.network_inference_host(self._calls, input, network_parameters, encoding_parameters, output, int(chunk_points))
         return output
 
     def forward(self, input: torch.Tensor, network_parameters: torch.Tensor,
                 encoding_parameters: Sequence[Optional[torch.Tensor]] = ()) -> torch.Tensor:
         """Inference, or - when gradients are enabled and one of the tensors requires them - an autograd node
         (csrc/torch/calls.cpp)."""
-        return _capi.calls().network_forward(self._calls, input, network_parameters, encoding_parameters)
+        return self._native.network_forward(self._calls, input, network_parameters, encoding_parameters)
 
     def forward_memory(self, n: int, flags: int = 7) -> int:
         b = C.c_size_t()

@@ -17,6 +17,7 @@ class FusedNetwork(torch.nn.Module):
         self._cfg, self._parent = cfg, parent
         self._network = Network(cfg, parent)
         self._num_output_channels = self._network.channels_out()
+        self._num_input_channels = self._network.channels_in()
         self._num_layers = self._network.num_layers()
 
         weights = self._network.create_inference_parameters(device)
@@ -30,6 +31,7 @@ class FusedNetwork(torch.nn.Module):
         assert self._num_encodings > 0
         self._encodings = [self._network.encoding(i) for i in range(self._num_encodings)]
         self._encoding_has_parameters = [e.has_parameters() for e in self._encodings]
+        self._no_encoding_parameters = not any(self._encoding_has_parameters)
         params = []
         for e in self._encodings:
             if e.has_parameters():
@@ -88,13 +90,19 @@ class FusedNetwork(torch.nn.Module):
         t.copy_(value)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        assert len(x.shape) == 2
-        assert x.shape[1] == self.channels_in()
-        if self.weights.requires_grad and self.weights.dtype == torch.float16 and torch.is_grad_enabled():
+        shape = x.shape
+        assert len(shape) == 2
+        assert shape[1] == self._num_input_channels
+        weights = self._parameters["weights"]     # (the attribute lookup of a module is a good part of a small call)
+        if weights.dtype == torch.float16 and torch.is_grad_enabled() and weights.requires_grad:
             warnings.warn("Attempt to train network with 16-bit weights: the gradient tensor will also have 16-bit "
                           "precision. Consider weight_dtype=torch.float32.")
-        enc = [self.encoding_parameters[i] if has else None for i, has in enumerate(self._encoding_has_parameters)]
-        return self._network.forward(x, self.weights, enc)
+        if self._no_encoding_parameters:
+            enc = ()
+        else:
+            params = self.encoding_parameters
+            enc = [params[i] if has else None for i, has in enumerate(self._encoding_has_parameters)]
+        return self._network.forward(x, weights, enc)
 
     def __repr__(self):
         return f"FusedNetwork(\"{self._cfg}\")"
