@@ -196,7 +196,7 @@ void launchBackward(Network& n, kernel::LaunchArgs& a, __half* planes, int64_t n
 }
 
 // layout of the adjoint scratch: [delta of every layer, if weight gradients | adjoint feature planes, if table
-// gradients], the second part 256-byte aligned
+// gradients | copies of hot levels' gradients], the parts 256-byte aligned
 size_t adjointDeltaBytes(const Network& n, int64_t n32, int flags)
 {
     return (flags & QMLP_GRADIENTS_NETWORK_WEIGHTS) ? static_cast<size_t>(n32) * n.deltaHalfsPerPoint() * 2 : 0;
@@ -209,6 +209,19 @@ size_t adjointPlaneBytes(const Network& n, int64_t n32, int flags)
     // for a set of flags is large enough for every subset of it
     const bool wanted = anyGrid && (flags & QMLP_GRADIENTS_INPUT_ENCODINGS) != 0;
     return wanted ? static_cast<size_t>(n32) * n.encodedChannels() * 2 : 0;
+}
+// behind the planes, 256-byte aligned: copies of the gradients of hot levels (kernel::GradReplicas)
+size_t replicaBytes(const Network& n, int64_t points)
+{
+    kernel::GradReplicas r;
+    n.planReplicas(points, r);
+    return static_cast<size_t>(r.total) * sizeof(float);
+}
+size_t align256(size_t b) { return (b + 255) / 256 * 256; }
+void bindReplicas(const Network& n, kernel::LaunchArgs& a, void* memory)
+{
+    n.planReplicas(a.numel, a.replicas);
+    if (a.replicas.total > 0) a.replicas.base = static_cast<float*>(memory);
 }
 
 } // namespace
@@ -616,7 +629,7 @@ int qmlp_network_adjoint_memory(qmlp_network_t* net, int64_t num_elements, int a
     const int64_t n32 = (num_elements + 31) / 32 * 32;
     const size_t planes = adjointPlaneBytes(*net->impl, n32, adjoint_flags);
     const size_t delta = adjointDeltaBytes(*net->impl, n32, adjoint_flags);
-    *bytes = planes ? (delta + 255) / 256 * 256 + planes : delta;
+    *bytes = planes ? align256(align256(delta) + planes) + replicaBytes(*net->impl, num_elements) : delta;
     QMLP_CATCH
 }
 
@@ -663,7 +676,11 @@ int qmlp_network_adjoint(qmlp_network_t* net, const qmlp_tensor_t* input, const 
     const int64_t n32 = (numel + 31) / 32 * 32;
     __half* planes = nullptr;   // a caller that passes no adjoint scratch gets the fused scatter
     if (tmp_adjoint && adjointPlaneBytes(n, n32, adjoint_flags) > 0)
-        planes = reinterpret_cast<__half*>(static_cast<unsigned char*>(tmp_adjoint) + (adjointDeltaBytes(n, n32, adjoint_flags) + 255) / 256 * 256);
+    {
+        unsigned char* at = static_cast<unsigned char*>(tmp_adjoint) + align256(adjointDeltaBytes(n, n32, adjoint_flags));
+        planes = reinterpret_cast<__half*>(at);
+        bindReplicas(n, a, at + align256(adjointPlaneBytes(n, n32, adjoint_flags)));
+    }
     launchBackward(n, a, planes, n32, stream);
     if (gW) launchNet(n, kernel::KERNEL_WGRAD, a, stream);
     QMLP_CATCH
@@ -781,8 +798,8 @@ int qmlp_encoding_adjoint_memory(qmlp_encoding_t* enc, int64_t num_elements, int
     *bytes = 0;
     auto* g = dynamic_cast<EncodingHashGrid*>(enc->impl.get());
     if (g && (adjoint_mode & QMLP_ENCODING_PARAM_GRADIENTS)) {
-        kernel::GradReplicas r;
-        g->planReplicas(num_elements, r);
+        kernel::GradReplicas r{};
+        g->planReplicas(num_elements, 0, r);
         *bytes = static_cast<size_t>(r.total) * sizeof(float);
     }
     QMLP_CATCH
@@ -837,7 +854,7 @@ int qmlp_encoding_adjoint_with_memory(qmlp_encoding_t* enc, const qmlp_tensor_t*
         a.flags = (gIn ? 1 : 0) | (gP ? 2 : 0);
         if (auto* g = dynamic_cast<EncodingHashGrid*>(&e); g && gP && tmp_memory) {
             if ((reinterpret_cast<uintptr_t>(tmp_memory) & 15) != 0) throw std::runtime_error("scratch memory must be 16-byte aligned");
-            g->planReplicas(a.numel, a.replicas);
+            g->planReplicas(a.numel, 0, a.replicas);
             if (a.replicas.total > 0 && static_cast<size_t>(a.replicas.total) * sizeof(float) <= tmp_bytes) a.replicas.base = static_cast<float*>(tmp_memory);
             else std::memset(&a.replicas, 0, sizeof a.replicas);
         }
@@ -940,11 +957,12 @@ int qmlp_convert_half(const float* src, uint16_t* dst, int64_t count, qmlp_strea
 // features first, then their adjoints); the copies of points and targets in bin order and the bin tables of the
 // spatially binned step (only for networks with a grid encoding).
 struct TrainerLayout {
-    size_t adjOut = 0, planes = 0, sortedInput = 0, sortedTarget = 0, bins = 0, total = 0;
+    size_t adjOut = 0, planes = 0, replicas = 0, sortedInput = 0, sortedTarget = 0, bins = 0, total = 0;
     int binCount = 0;
 };
-static TrainerLayout trainerLayout(const Network& n, int64_t n32)
+static TrainerLayout trainerLayout(const Network& n, int64_t points)
 {
+    const int64_t n32 = (points + 31) / 32 * 32;
     auto align = [](size_t b) { return (b + 255) / 256 * 256; };
     TrainerLayout l;
     size_t b = align(static_cast<size_t>(n32) * (n.stashHalfsPerPoint() + n.deltaHalfsPerPoint()) * 2);
@@ -952,6 +970,8 @@ static TrainerLayout trainerLayout(const Network& n, int64_t n32)
     b = align(b + static_cast<size_t>(n32) * n.channelsOut() * 4);
     l.planes = b;
     b = align(b + adjointPlaneBytes(n, n32, QMLP_GRADIENTS_NETWORK_WEIGHTS | QMLP_GRADIENTS_INPUT_ENCODINGS));
+    l.replicas = b;
+    b = align(b + replicaBytes(n, points));
     const int dims = n.sortDimensions();
     if (dims > 0) {
         l.binCount = kernel::sort_bin_count(dims);
@@ -1010,8 +1030,7 @@ int64_t qmlp_trainer_segment_start(const qmlp_trainer_t* tr, int segment)
 int qmlp_trainer_workspace_bytes(qmlp_trainer_t* tr, int64_t num_elements, size_t* bytes)
 {
     QMLP_TRY
-    const int64_t n32 = (num_elements + 31) / 32 * 32;
-    *bytes = trainerLayout(*tr->net, n32).total;
+    *bytes = trainerLayout(*tr->net, num_elements).total;
     QMLP_CATCH
 }
 
@@ -1085,7 +1104,7 @@ int qmlp_trainer_gradients_part(qmlp_trainer_t* tr, const qmlp_tensor_t* input, 
     if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 255) != 0) throw std::runtime_error("workspace must be 256-byte aligned");
     if (global_points <= 0) global_points = numel;
     const int64_t n32 = (numel + 31) / 32 * 32;
-    const TrainerLayout lay = trainerLayout(n, n32);
+    const TrainerLayout lay = trainerLayout(n, numel);
     kernel::LaunchArgs a;
     fillCommon(n, a, input);
     unsigned char* ws = static_cast<unsigned char*>(workspace);
@@ -1104,6 +1123,7 @@ int qmlp_trainer_gradients_part(qmlp_trainer_t* tr, const qmlp_tensor_t* input, 
     bool anyGrid = false;
     for (int i = 0; i < n.numEncodings(); ++i) anyGrid = anyGrid || n.encoding(i)->hasParameters();
     __half* planes = anyGrid ? reinterpret_cast<__half*>(ws + lay.planes) : nullptr;
+    bindReplicas(n, a, ws + lay.replicas);
     // Gather-dominated batches (same rule as inference): the encodings are computed one grid level at a time into
     // the plane region of the workspace, which is free until the backward kernel writes the adjoint planes there,
     // and the forward kernel reads its layer-0 operand from the planes.

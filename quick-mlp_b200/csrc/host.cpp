@@ -311,21 +311,22 @@ std::string EncodingHashGrid::deviceType(int outOffset, int slot, bool halfTable
                   outOffset, slot, halfTable ? "true" : "false");
 }
 
-void EncodingHashGrid::planReplicas(int64_t points, kernel::GradReplicas& r) const
+void EncodingHashGrid::planReplicas(int64_t points, int group, kernel::GradReplicas& r) const
 {
     // A point sends 2^(D-1) reductions per level (neighbouring corners leave as one) to the lines of the level. Up to
     // 2048 per line they hide behind the rest of the kernel (a line takes about nine clocks each); above that, as many
     // copies as bring a line back to that number, 64 at most.
-    std::memset(&r, 0, sizeof r);
     if (isLine() || Library::instance().boundsCheck) return;
     const double reductions = static_cast<double>(points) * (1 << (dim_ - 1));
-    for (int l = 0; l < levels_; ++l) {
+    for (int l = 0; l < levels_ && group + l < kernel::MAX_GRID_LEVELS; ++l) {
         const int64_t elements = (l + 1 < levels_ ? table_[l + 1].memoryOffset : numParameters_) - table_[l].memoryOffset;
         double perLine = reductions / std::max<double>(1.0, static_cast<double>(elements) / 32);
         int lg = 0;
         for (; perLine > 2048 && lg < 6; perLine /= 2) ++lg;
-        r.log2Copies[l] = static_cast<unsigned char>(lg);
-        if (lg > 0) r.total += elements << lg;
+        if (lg == 0 || r.total + (elements << lg) > (1ll << 28)) continue;   // (32-bit offsets)
+        r.log2Copies[group + l] = static_cast<unsigned char>(lg);
+        r.offset[group + l] = static_cast<unsigned int>(r.total);
+        r.total += elements << lg;
     }
 }
 
@@ -620,6 +621,18 @@ int Network::gathersPerPoint() const
         if (auto* h = dynamic_cast<const EncodingHashGrid*>(e.get()))
             if (!h->isLine()) g += static_cast<int>(h->levelTable().size()) << h->dimension();
     return g;
+}
+
+void Network::planReplicas(int64_t points, kernel::GradReplicas& r) const
+{
+    std::memset(&r, 0, sizeof r);
+    int group = 0;
+    for (const auto& e : encodings_)
+        if (auto* h = dynamic_cast<const EncodingHashGrid*>(e.get())) {
+            if (h->isLine()) continue;
+            h->planReplicas(points, group, r);
+            group += static_cast<int>(h->levelTable().size());
+        }
 }
 
 int Network::gridLevels() const

@@ -168,8 +168,9 @@ public:
     void setParameter(const qmlp_tensor_t* t, int usage) override;
     void fillGrid(kernel::GridP& g) const override;
     const std::vector<GridLevel>& levelTable() const { return table_; }
-    // copies of the gradients of small levels for a batch of `points` (kernel::GradReplicas; base is left null)
-    void planReplicas(int64_t points, kernel::GradReplicas& r) const;
+    // copies of the gradients of small levels for a batch of `points` (kernel::GradReplicas; base is left as it is),
+    // appended to `r` from level `group` (counted over all grids of a network) on
+    void planReplicas(int64_t points, int group, kernel::GradReplicas& r) const;
     int features() const { return features_; }
     int dimension() const { return dim_; }
     Json gridJson() const;   // the hash grid's own configuration (id "HashGrid")
@@ -254,6 +255,7 @@ public:
     ~Network();
     int64_t gridTableBytes() const;   // bytes of all bound grid tables (what the gather walks through)
     int gathersPerPoint() const;      // table rows fetched per point by all plain grid encodings: sum of levels * 2^D
+    void planReplicas(int64_t points, kernel::GradReplicas& r) const;   // of all grid encodings; zeroes `r` first
     int gridLevels() const;           // levels of all grid encodings
     int sortDimensions() const;       // dimension of the grid whose bounding box bins the points of a training step (0: none)
     // level-major encoding pass (inference of networks with tables larger than L2): chunk buffer, allocated at the

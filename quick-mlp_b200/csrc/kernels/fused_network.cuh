@@ -1358,7 +1358,7 @@ struct NetworkLaunchers {
             break;
         case KERNEL_BACKWARD: e = backward(a, s); n = (a.flags & 7) ? 1 : 0; break;
         case KERNEL_WGRAD: e = wgrad(a, s); break;
-        case KERNEL_SCATTER_PLANES: e = PlaneLaunchers<Spec>::scatter(a, s); break;
+        case KERNEL_SCATTER_PLANES: e = PlaneLaunchers<Spec>::scatter(a, s, &n); break;
         case KERNEL_TRAIN:
             if constexpr (TrainLayout<Spec>::eligible()) e = TrainLaunchers<Spec>::run(a, s);
             else e = cudaErrorNotSupported;

@@ -456,10 +456,37 @@ __device__ __forceinline__ void grid_half_adjoint(const GridP& g, float* grad, c
 }
 
 template <int D, int F, int PD>
-__device__ __forceinline__ void grid_half_scatter(const GridP& g, const GridLevelP& lv, const float (&pos)[D], int side, const float (&adjF)[F])
+__device__ __forceinline__ void grid_half_scatter(const GridP& g, float* grad, const GridLevelP& lv, const float (&pos)[D], int side, const float (&adjF)[F])
 {
     float none[D];
-    grid_half_adjoint<D, F, false, true, false, PD>(g, g.grad, lv, pos, side, adjF, none);
+    grid_half_adjoint<D, F, false, true, false, PD>(g, grad, lv, pos, side, adjF, none);
+}
+
+// elements of level l of a table of `levels` levels (levels with copies are small: 32 bits hold every index into them)
+__device__ __forceinline__ int grid_level_elements(const GridP& g, int l, int levels)
+{
+    return static_cast<int>((l + 1 < levels ? g.levels[l + 1].offset : static_cast<unsigned int>(g.tableCount)) - g.levels[l].offset);
+}
+// where this CTA adds the gradient of level l (level `group` over all grids), seen from element offset 0 of the whole table:
+// the table itself or, with copies, one of them
+__device__ __forceinline__ float* grid_grad_of_cta(const GridP& g, const GradReplicas& r, int group, int l, int levels)
+{
+    if (group >= MAX_GRID_LEVELS || r.log2Copies[group] == 0) return g.grad;
+    const int n = grid_level_elements(g, l, levels);
+    return r.base + r.offset[group] + (blockIdx.x & ((1u << r.log2Copies[group]) - 1u)) * n - g.levels[l].offset;
+}
+// sum of the copies of a level -> its gradient (grid-stride over blockIdx.x, 256 threads)
+__device__ __forceinline__ void grid_sum_copies(const GridP& g, const GradReplicas& r, int group, int l, int levels)
+{
+    if (group >= MAX_GRID_LEVELS || r.log2Copies[group] == 0 || g.grad == nullptr) return;
+    const int copies = 1 << r.log2Copies[group], n = grid_level_elements(g, l, levels);
+    const float* src = r.base + r.offset[group];
+    for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
+        float v = 0.f;
+#pragma unroll 8
+        for (int c = 0; c < copies; ++c) v += src[c * n + i];
+        if (v != 0.f) red_add_f32(g.grad + g.levels[l].offset + i, v);
+    }
 }
 
 } // namespace kernel

@@ -207,6 +207,7 @@ __device__ __forceinline__ void scatter_group(const LaunchArgs& p, int g, const 
                 }
             }
             const GridLevelP& lv = grid.levels[l];
+            float* grad = grid_grad_of_cta(grid, p.replicas, g, l, Enc::L);
 #pragma unroll
             for (int s = 0; s < 2; ++s) {
                 float pos[D], adjF[F];
@@ -219,8 +220,8 @@ __device__ __forceinline__ void scatter_group(const LaunchArgs& p, int g, const 
                     if (2 * i + 1 < F) adjF[2 * i + 1] = x.y;
                 }
                 if (!ok) continue;
-                if (lv.hashed) grid_half_scatter<D, F, 0>(grid, lv, pos, side, adjF);
-                else grid_half_scatter<D, F, D - 1>(grid, lv, pos, side, adjF);
+                if (lv.hashed) grid_half_scatter<D, F, 0>(grid, grad, lv, pos, side, adjF);
+                else grid_half_scatter<D, F, D - 1>(grid, grad, lv, pos, side, adjF);
             }
         }
     }
@@ -254,9 +255,29 @@ __global__ void __launch_bounds__(SCATTER_THREADS, 1024 / SCATTER_THREADS) scatt
     }
 }
 
+// copies of group g's gradient (GradReplicas) -> table gradient
+template <class Spec, int E>
+__device__ __forceinline__ void sum_group(const LaunchArgs& p, int g)
+{
+    if constexpr (E < Spec::NUM_ENCODINGS) {
+        using Enc = typename Spec::template Enc<E>;
+        using SG = ScatterGroups<Spec, E>;
+        if (g >= SG::before() + SG::own()) {
+            sum_group<Spec, E + 1>(p, g);
+        } else if constexpr (Enc::IS_GRID) {
+            grid_sum_copies(p.grids[Enc::SLOT], p.replicas, g, g - SG::before(), Enc::L);
+        }
+    }
+}
+template <class Spec>
+__global__ void __launch_bounds__(256) sum_copies_kernel(const __grid_constant__ LaunchArgs p)
+{
+    sum_group<Spec, 0>(p, blockIdx.y + (p.scatterLevelEnd > 0 ? p.scatterLevelBegin : 0));
+}
+
 template <class Spec>
 struct PlaneLaunchers {
-    static cudaError_t scatter(const LaunchArgs& a, cudaStream_t s)
+    static cudaError_t scatter(const LaunchArgs& a, cudaStream_t s, int* launches)
     {
         constexpr int groups = scatter_group_count<Spec>();
         if constexpr (groups == 0) {
@@ -268,7 +289,20 @@ struct PlaneLaunchers {
             const long long cap = 1ll << 30;
             if (bx > cap) bx = cap;
             if (bx < 1) bx = 1;
+            // the copies of the hot levels among the ones of this launch
+            const int begin = a.scatterLevelEnd > 0 ? a.scatterLevelBegin : 0, end = a.scatterLevelEnd > 0 ? a.scatterLevelEnd : groups;
+            int sums = 0;   // the levels up to the last one that has copies
+            for (int g = begin; g < end && g < groups && g < MAX_GRID_LEVELS; ++g)
+                if (a.replicas.log2Copies[g] > 0) sums = g - begin + 1;
+            if (sums > 0) {
+                const cudaError_t e = cudaMemsetAsync(a.replicas.base, 0, a.replicas.total * sizeof(float), s);
+                if (e != cudaSuccess) return e;
+            }
             scatter_planes_kernel<Spec><<<static_cast<unsigned>(bx), SCATTER_THREADS, 0, s>>>(a);
+            if (sums > 0) {
+                sum_copies_kernel<Spec><<<dim3(32, sums), 256, 0, s>>>(a);
+                if (launches) *launches = 2;
+            }
             return cudaGetLastError();
         }
     }

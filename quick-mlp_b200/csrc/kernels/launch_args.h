@@ -69,6 +69,7 @@ constexpr int FLAG_SPLIT_SCATTER = 8;
 struct GradReplicas {
     float* base;                            // copies of all such levels, level by level (null: none)
     long long total;                        // elements
+    unsigned int offset[MAX_GRID_LEVELS];        // first element of a level's copies; levels counted over all grids of the network
     unsigned char log2Copies[MAX_GRID_LEVELS];   // 0: the level has no copies
 };
 
@@ -102,7 +103,7 @@ struct LaunchArgs {
     float* sortedTarget;                           // (numel, NUM_OUTPUTS) row-major, may be null
     int scatterLevelBegin, scatterLevelEnd;        // KERNEL_SCATTER_PLANES: grid levels (counted over all grids) to scatter; 0, 0 = all
     int runAggregation;                            // 0: every point of every level scatters straight to the gradient table
-    GradReplicas replicas;                         // KERNEL_ENCODING_ADJOINT
+    GradReplicas replicas;                         // KERNEL_ENCODING_ADJOINT, KERNEL_SCATTER_PLANES
     GridP grids[GRID_SLOTS];                       // the last member (GRID_SLOTS)
 };
 
@@ -150,4 +151,4 @@ extern "C" {
 typedef int (*qmlp_spec_launch_fn)(int kernel, const void* args, cudaStream_t stream, int* launches);
 typedef int (*qmlp_spec_abi_fn)(void);
 }
-#define QMLP_SPEC_ABI_VERSION 10
+#define QMLP_SPEC_ABI_VERSION 11

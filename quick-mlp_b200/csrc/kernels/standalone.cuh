@@ -163,12 +163,6 @@ __global__ void __launch_bounds__(EncodingTile<Enc>::WARPS * 32) grid_encoding_f
     }
 }
 
-// elements of level l of a table of `levels` levels (levels with copies are small: 32 bits hold every index into them)
-__device__ __forceinline__ int grid_level_elements(const GridP& g, int l, int levels)
-{
-    return static_cast<int>((l + 1 < levels ? g.levels[l + 1].offset : static_cast<unsigned int>(g.tableCount)) - g.levels[l].offset);
-}
-
 template <class Enc, bool INPUT_GRAD, bool PARAM_GRAD>
 __global__ void __launch_bounds__(EncodingTile<Enc>::WARPS * 32) grid_encoding_adjoint_kernel(const __grid_constant__ LaunchArgs p)
 {
@@ -191,19 +185,10 @@ __global__ void __launch_bounds__(EncodingTile<Enc>::WARPS * 32) grid_encoding_a
             for (int k = 0; k < D; ++k) adjPos[s][k] = 0.f;
         }
         __syncwarp();
-        float* copies = p.replicas.base;
         for (int l = 0; l < Enc::L; ++l) {
             const GridLevelP& lv = g.levels[l];
-            // this CTA's copy of the level's gradient, seen from element offset 0 of the whole table (see GradReplicas)
             float* grad = g.grad;
-            if constexpr (PARAM_GRAD) {
-                const int lg = p.replicas.log2Copies[l];
-                if (lg > 0) {
-                    const int n = grid_level_elements(g, l, Enc::L);
-                    grad = copies + (blockIdx.x & ((1u << lg) - 1u)) * n - lv.offset;
-                    copies += n << lg;
-                }
-            }
+            if constexpr (PARAM_GRAD) grad = grid_grad_of_cta(g, p.replicas, l, l, Enc::L);
 #pragma unroll
             for (int s = 0; s < 2; ++s) {
                 if (i0 + s > last) continue;
@@ -230,18 +215,7 @@ __global__ void __launch_bounds__(EncodingTile<Enc>::WARPS * 32) grid_encoding_a
 template <class Enc>
 __global__ void __launch_bounds__(256) sum_replicas_kernel(const __grid_constant__ LaunchArgs p)
 {
-    const int l = blockIdx.y, copies = 1 << p.replicas.log2Copies[l];
-    if (copies <= 1) return;
-    const float* src = p.replicas.base;
-    for (int k = 0; k < l; ++k)
-        if (p.replicas.log2Copies[k] > 0) src += grid_level_elements(p.grids[0], k, Enc::L) << p.replicas.log2Copies[k];
-    const int n = grid_level_elements(p.grids[0], l, Enc::L);
-    for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
-        float v = 0.f;
-#pragma unroll 8
-        for (int c = 0; c < copies; ++c) v += src[c * n + i];
-        if (v != 0.f) red_add_f32(p.grids[0].grad + p.grids[0].levels[l].offset + i, v);
-    }
+    grid_sum_copies(p.grids[0], p.replicas, blockIdx.y, blockIdx.y, Enc::L);
 }
 
 template <class EncSpec>
@@ -279,7 +253,7 @@ struct EncodingLaunchers {
                     if (e != cudaSuccess) return e;
                 }
                 grid_encoding_adjoint_kernel<Enc, INPUT_GRAD, PARAM_GRAD><<<blocksFor(a, threads), threads, 0, s>>>(a);
-                if (copies) sum_replicas_kernel<Enc><<<dim3(16, Enc::L), 256, 0, s>>>(a);
+                if (copies) sum_replicas_kernel<Enc><<<dim3(32, Enc::L), 256, 0, s>>>(a);
                 return cudaGetLastError();
             }
         }

@@ -278,7 +278,8 @@ def test_train_kernel_matches_separate_kernels(name, n):
     finally:
         bindings.QuickMLP.set_kernel_path(0)
     (a, launches), (b, launches_separate) = results
-    assert launches < launches_separate + (1 if spec.encodings[0].num_parameters else 0)     # the fused kernel ran
+    if not any(e.num_parameters for e in spec.encodings):
+        assert launches < launches_separate     # the fused kernel ran (a grid adds the passes around it)
     assert abs(a.loss_sum.item() - b.loss_sum.item()) <= 1e-2 * abs(b.loss_sum.item())
     for i in range(1 + len(spec.encodings)):
         ga, gb = a.segment(a.gradient, i), b.segment(b.gradient, i)
@@ -286,3 +287,34 @@ def test_train_kernel_matches_separate_kernels(name, n):
             continue
         norm = float(gb.norm())
         assert norm > 0 and float((ga - gb).norm()) <= 1e-2 * norm, f"{name} n={n} segment {i}: {float((ga - gb).norm()) / norm}"
+
+
+def test_scatter_with_copies_of_hot_levels():
+    """A batch that hits the lines of the coarse levels often enough for copies of their gradients: one launch over all levels,
+    and launches over ranges of levels that begin before, inside and behind the levels with copies, against the scatter
+    inside the backward kernel (path 1). The same fp32 terms in another order; deltas differ by fp16 roundings."""
+    import torch
+    from qmlp import bindings
+    from qmlp.trainer import FusedTrainer
+    cfg = smooth_config3(log2_hashmap_size=14)
+    spec = oracle.parse_spec(cfg)
+    n = 150_001
+    x = torch.from_numpy(helpers.uniform(33, 1, (n, 3))).cuda()
+    t = torch.from_numpy(_target(x.cpu().numpy())).cuda()
+    params = torch.from_numpy(helpers.xavier_parameters(spec, cfg, bias_scale=0.05).astype(np.float32)).cuda()
+    table = torch.from_numpy(helpers.grid_tables(spec, scale=0.1)[0]).cuda()
+    grads = []
+    try:
+        for path, parts in ((1, [3]), (0, [3]), (0, [4, 8 | 0 << 8 | 1 << 16, 8 | 1 << 8 | 5 << 16, 8 | 5 << 8 | 16 << 16, 2])):
+            bindings.QuickMLP.set_kernel_path(path)
+            tr = FusedTrainer(bindings.Network(json.dumps(cfg)))
+            tr.set_parameters(params, [table])
+            for what in parts:
+                tr.backend.gradients(x, t, n, tr.loss_sum, parts=what)
+            torch.cuda.synchronize()
+            grads.append(tr.segment(tr.gradient, 1).clone())
+    finally:
+        bindings.QuickMLP.set_kernel_path(0)
+    norm = float(grads[0].norm())
+    assert norm > 0 and float((grads[1] - grads[0]).norm()) <= 1e-2 * norm
+    assert float((grads[2] - grads[1]).norm()) <= 1e-5 * norm
