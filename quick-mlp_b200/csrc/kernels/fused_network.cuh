@@ -1223,6 +1223,8 @@ struct PerDevice {
 template <class Spec> struct TcLaunchers;
 template <class Spec> struct TrainLayout;  // fused_train_tc.cuh
 template <class Spec> struct TrainLaunchers;
+template <class Spec> struct TsLayout;     // fused_forward_ts.cuh
+template <class Spec> struct TsLaunchers;
 template <class Spec> struct PlaneLaunchers;
 template <class Spec> struct SortLaunchers;
 
@@ -1336,7 +1338,11 @@ struct NetworkLaunchers {
                 // kernel gathers with lane pairs and 16 warps (128 rows per point, 2^20 points: 272 against 364 us); few rows
                 // leave the layers in charge.
                 const bool enough = a.numel >= TcLayout<Spec>::pointsPerCta() * a.numSMs && table_rows_per_point<Spec>() < 32;
-                if (a.forcePath == 3 || (a.forcePath != 1 && enough)) { e = TcLaunchers<Spec>::inference(a, s); break; }
+                if (a.forcePath == 3 || (a.forcePath != 1 && enough)) {
+                    if constexpr (TsLayout<Spec>::eligible() && table_rows_per_point<Spec>() == 0) e = TsLaunchers<Spec>::run(a, s);
+                    else e = TcLaunchers<Spec>::inference(a, s);
+                    break;
+                }
             }
             e = forward<0>(a, s);
             break;
@@ -1347,7 +1353,9 @@ struct NetworkLaunchers {
         case KERNEL_INFERENCE_PLANES:
             if constexpr (TcLayout<Spec>::eligible()) {
                 const bool enough = a.numel >= TcLayout<Spec>::pointsPerCta() * a.numSMs;   // as above
-                e = enough ? TcLaunchers<Spec>::inferencePlanes(a, s) : forward<4>(a, s);
+                if (!enough) e = forward<4>(a, s);
+                else if constexpr (TsLayout<Spec>::eligible()) e = TsLaunchers<Spec>::run(a, s);
+                else e = TcLaunchers<Spec>::inferencePlanes(a, s);
             } else e = cudaErrorNotSupported;
             break;
         case KERNEL_FORWARD: e = forward<1>(a, s); break;

@@ -6,6 +6,7 @@
 #include "fused_network.cuh"
 #include "fused_forward_tc.cuh"
 #include "fused_train_tc.cuh"
+#include "fused_forward_ts.cuh"
 
 namespace qmlp {
 namespace kernel {
