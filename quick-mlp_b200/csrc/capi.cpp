@@ -533,48 +533,74 @@ int qmlp_network_inference_host(qmlp_network_t* net, const float* host_input, fl
     if (num_points == 0) return QMLP_OK;
     if (!host_input || !host_output) throw std::runtime_error("null host buffer");
     const int cin = n.channelsIn(), cout = n.channelsOut();
-    // default chunk: an eighth of the batch, between 2^16 and 2^20 points (measured best on a PCIe 5 x16 host link:
-    // 8 chunks of 2^19 points). Smaller chunks pay more per-copy overhead, larger ones a longer pipeline fill (first
-    // upload) and drain (last kernel + download).
+    // A page-locked result of one channel is written by the kernels themselves (a warp's results are one 128-byte line): no
+    // download behind the last kernel, and nothing beside the uploads on the copy engines.
+    float* mapped = nullptr;
+    if (cout == 1) {
+        cudaPointerAttributes attr;
+        if (cudaPointerGetAttributes(&attr, host_output) == cudaSuccess && attr.type == cudaMemoryTypeHost)
+            mapped = static_cast<float*>(attr.devicePointer);
+        else
+            (void)cudaGetLastError();
+    }
+    // Default chunk: an eighth of the batch, with the results written in place between 2^18 and 2^20 points (a chunk costs the
+    // host about 10 us of calls and is worth them only for the overlap of its kernel: 2^20 points in 8 / 4 / 2 chunks 372 / 289 /
+    // 298 us, 2^18 points in 2 / 1 chunks 152 / 133 us), otherwise between 2^16 and 2^20 points (smaller chunks pay more per-copy
+    // overhead, larger ones a longer pipeline fill and drain).
     int64_t chunk = chunk_points;
     if (chunk == 0) {
-        chunk = 1 << 16;
+        chunk = mapped ? 1 << 18 : 1 << 16;
         while (chunk < (1 << 20) && chunk * 8 < num_points) chunk *= 2;
     }
     chunk = std::min(chunk, num_points);
     n.claimDevice();
     HostPipeline& hp = n.hostPipeline;
-    hp.reserve(chunk, cin, cout);
+    hp.reserve(chunk, cin, mapped ? 0 : cout);
     const cudaStream_t user = static_cast<cudaStream_t>(stream);
+    if (chunk == num_points) {   // nothing to overlap: in order on the caller's stream
+        qmlp_tensor_t ti{hp.in[0], QMLP_FLOAT, 2, {num_points, cin}, {cin, 1}};
+        qmlp_tensor_t to{mapped ? mapped : hp.out[0], QMLP_FLOAT, 2, {num_points, cout}, {cout, 1}};
+        checkCuda(cudaStreamWaitEvent(user, hp.computed[0], 0), "cudaStreamWaitEvent");   // an earlier call, on whatever stream
+        checkCuda(cudaStreamWaitEvent(user, hp.downloaded[0], 0), "cudaStreamWaitEvent");
+        checkCuda(cudaMemcpyAsync(hp.in[0], host_input, static_cast<size_t>(num_points) * cin * 4, cudaMemcpyHostToDevice, user), "cudaMemcpyAsync(host to device)");
+        inferenceLocked(n, &ti, &to, stream);
+        checkCuda(cudaEventRecord(hp.computed[0], user), "cudaEventRecord");
+        if (!mapped)
+            checkCuda(cudaMemcpyAsync(host_output, hp.out[0], static_cast<size_t>(num_points) * cout * 4, cudaMemcpyDeviceToHost, user),
+                      "cudaMemcpyAsync(device to host)");
+        if (!mapped) checkCuda(cudaEventRecord(hp.downloaded[0], user), "cudaEventRecord");
+        return QMLP_OK;
+    }
     // uploads start after the work already queued on the caller's stream (e.g. a parameter update)
     checkCuda(cudaEventRecord(hp.start, user), "cudaEventRecord");
     checkCuda(cudaStreamWaitEvent(hp.copyIn, hp.start, 0), "cudaStreamWaitEvent");
-    checkCuda(cudaStreamWaitEvent(hp.copyOut, hp.start, 0), "cudaStreamWaitEvent");
+    if (!mapped) checkCuda(cudaStreamWaitEvent(hp.copyOut, hp.start, 0), "cudaStreamWaitEvent");
     int64_t k = 0;
     for (int64_t p0 = 0; p0 < num_points; p0 += chunk, ++k) {
         const int s = static_cast<int>(k % HostPipeline::SLOTS);
         const int64_t m = std::min(chunk, num_points - p0);
-        if (k >= HostPipeline::SLOTS) {
-            // the slot's previous kernel has consumed its input; its previous download has left its output
-            checkCuda(cudaStreamWaitEvent(hp.copyIn, hp.computed[s], 0), "cudaStreamWaitEvent");
-            checkCuda(cudaStreamWaitEvent(user, hp.downloaded[s], 0), "cudaStreamWaitEvent");
-        }
+        // the slot's previous kernel (of this call or an earlier one) has consumed its input; its previous download has left its
+        // output
+        checkCuda(cudaStreamWaitEvent(hp.copyIn, hp.computed[s], 0), "cudaStreamWaitEvent");
+        if (!mapped) checkCuda(cudaStreamWaitEvent(user, hp.downloaded[s], 0), "cudaStreamWaitEvent");
         checkCuda(cudaMemcpyAsync(hp.in[s], host_input + p0 * cin, static_cast<size_t>(m) * cin * 4, cudaMemcpyHostToDevice, hp.copyIn),
                   "cudaMemcpyAsync(host to device)");
         checkCuda(cudaEventRecord(hp.uploaded[s], hp.copyIn), "cudaEventRecord");
         checkCuda(cudaStreamWaitEvent(user, hp.uploaded[s], 0), "cudaStreamWaitEvent");
         qmlp_tensor_t ti{hp.in[s], QMLP_FLOAT, 2, {m, cin}, {cin, 1}};
-        qmlp_tensor_t to{hp.out[s], QMLP_FLOAT, 2, {m, cout}, {cout, 1}};
+        qmlp_tensor_t to{mapped ? mapped + p0 : hp.out[s], QMLP_FLOAT, 2, {m, cout}, {cout, 1}};
         inferenceLocked(n, &ti, &to, stream);
         checkCuda(cudaEventRecord(hp.computed[s], user), "cudaEventRecord");
+        if (mapped) continue;
         checkCuda(cudaStreamWaitEvent(hp.copyOut, hp.computed[s], 0), "cudaStreamWaitEvent");
         checkCuda(cudaMemcpyAsync(host_output + p0 * cout, hp.out[s], static_cast<size_t>(m) * cout * 4, cudaMemcpyDeviceToHost, hp.copyOut),
                   "cudaMemcpyAsync(device to host)");
         checkCuda(cudaEventRecord(hp.downloaded[s], hp.copyOut), "cudaEventRecord");
     }
     // the caller's stream completes when the last downloads have landed
-    for (int s = 0; s < HostPipeline::SLOTS && s < k; ++s)
-        checkCuda(cudaStreamWaitEvent(user, hp.downloaded[s], 0), "cudaStreamWaitEvent");
+    if (!mapped)
+        for (int s = 0; s < HostPipeline::SLOTS && s < k; ++s)
+            checkCuda(cudaStreamWaitEvent(user, hp.downloaded[s], 0), "cudaStreamWaitEvent");
     QMLP_CATCH
 }
 

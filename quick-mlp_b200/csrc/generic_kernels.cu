@@ -16,8 +16,8 @@ __global__ void __launch_bounds__(256) adam_kernel(float4* __restrict__ master, 
                                                    uint2* __restrict__ halfCopy, long long count4, float gradScale,
                                                    float beta1, float beta2, float stepSize, float invSqrtBc2, float eps)
 {
-    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < count4;
-         i += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+    if (i < count4) {
         float4 g = grad[i];
         float4 p = master[i], mm = m[i], vv = v[i];
         float* gp = reinterpret_cast<float*>(&g);
@@ -77,8 +77,11 @@ cudaError_t launchAdam(float* master, float* grad, float* m, float* v, uint16_t*
                        float gradScale, float beta1, float beta2, float stepSize, float invSqrtBc2, float eps,
                        int numSMs, cudaStream_t stream)
 {
+    // One CTA per 256 vectors, refilled by the hardware as they retire: 13 M parameters 65 us (5.2 TB/s), with 8 looping CTAs per
+    // SM 72 us, with two vectors per thread in flight 72 us. (Streaming hints on the vectors: no change.)
     const long long count4 = count / 4;
-    adam_kernel<<<gridFor(count4, numSMs), 256, 0, stream>>>(
+    (void)numSMs;
+    adam_kernel<<<static_cast<unsigned>((count4 + 255) / 256), 256, 0, stream>>>(
         reinterpret_cast<float4*>(master), reinterpret_cast<float4*>(grad), reinterpret_cast<float4*>(m),
         reinterpret_cast<float4*>(v), reinterpret_cast<uint2*>(halfCopy), count4, gradScale, beta1, beta2, stepSize,
         invSqrtBc2, eps);

@@ -570,32 +570,32 @@ void HostPipeline::reserve(int64_t points, int channelsIn, int channelsOut)
             pipelineCheck(cudaEventCreateWithFlags(&downloaded[s], cudaEventDisableTiming), "cudaEventCreate");
         }
     }
-    if (points <= capacity) return;
-    // cudaFree waits for the device, so no earlier call still uses the old slots
-    for (int s = 0; s < SLOTS; ++s) {
-        if (in[s]) cudaFree(in[s]);
-        if (out[s]) cudaFree(out[s]);
-        in[s] = out[s] = nullptr;
+    const int64_t need = SLOTS * points * (channelsIn + channelsOut);
+    if (need > capacity) {
+        // cudaFree waits for the device, so no earlier call still uses the old slots
+        if (block) cudaFree(block);
+        block = nullptr;
+        capacity = 0;
+        pipelineCheck(cudaMalloc(&block, static_cast<size_t>(need) * sizeof(float)), "cudaMalloc(staging slots)");
+        capacity = need;
     }
-    capacity = 0;
     for (int s = 0; s < SLOTS; ++s) {
-        pipelineCheck(cudaMalloc(&in[s], static_cast<size_t>(points) * channelsIn * sizeof(float)), "cudaMalloc(upload slot)");
-        pipelineCheck(cudaMalloc(&out[s], static_cast<size_t>(points) * channelsOut * sizeof(float)), "cudaMalloc(download slot)");
+        in[s] = block + s * points * channelsIn;
+        out[s] = channelsOut > 0 ? block + SLOTS * points * channelsIn + s * points * channelsOut : nullptr;
     }
-    capacity = points;
 }
 
 void HostPipeline::release()
 {
     for (int s = 0; s < SLOTS; ++s) {
-        if (in[s]) cudaFree(in[s]);
-        if (out[s]) cudaFree(out[s]);
         if (uploaded[s]) cudaEventDestroy(uploaded[s]);
         if (computed[s]) cudaEventDestroy(computed[s]);
         if (downloaded[s]) cudaEventDestroy(downloaded[s]);
         in[s] = out[s] = nullptr;
         uploaded[s] = computed[s] = downloaded[s] = nullptr;
     }
+    if (block) cudaFree(block);
+    block = nullptr;
     if (start) cudaEventDestroy(start);
     if (copyIn) cudaStreamDestroy(copyIn);
     if (copyOut) cudaStreamDestroy(copyOut);

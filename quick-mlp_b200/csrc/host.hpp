@@ -223,10 +223,11 @@ struct HostPipeline {
     cudaStream_t copyIn = nullptr, copyOut = nullptr;
     cudaEvent_t start = nullptr;
     cudaEvent_t uploaded[SLOTS] = {}, computed[SLOTS] = {}, downloaded[SLOTS] = {};
+    float* block = nullptr;  // one allocation: the slots' inputs, then their outputs
     float* in[SLOTS] = {};
     float* out[SLOTS] = {};
-    int64_t capacity = 0;   // points per slot
-    void reserve(int64_t points, int channelsIn, int channelsOut);
+    int64_t capacity = 0;    // floats in the block
+    void reserve(int64_t points, int channelsIn, int channelsOut);   // channelsOut 0: no output slots
     void release();
 };
 

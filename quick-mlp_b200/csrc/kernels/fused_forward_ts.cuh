@@ -15,6 +15,9 @@
 //     warp of the slot issues the K/16 MMAs, the bias MMA (operand [1, 0, ...] x block with the bias in its first K column) and
 //     the commit. The issuing warps of the slots sit on different SM sub-partitions.
 //   * The features of the slot's next tile are fetched under the layers of the current one.
+// Measured, 64-wide network of five layers (relu, celu, sine, relu), 2^22 points: 204 -> 186 us; without its special-function
+// operations it would take 122 us, without its MMAs 152: bound by the special-function unit (128 operations per point, 71 %
+// busy) with five warps per scheduler to cover the rest. Two warpgroups per slot on four slots: 217 us.
 // Every wait is bounded; on a timeout the CTA runs through without waiting and the status word is set.
 #pragma once
 #include "fused_train_tc.cuh"

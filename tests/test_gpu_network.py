@@ -465,6 +465,47 @@ def test_argument_errors():
     assert out.shape == (0, 1)
 
 
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 148 * 128 + 1, 148 * 128 * 6 + 33])
+@pytest.mark.parametrize("name,path", [("config1", 3), ("config2", 3), ("uneven", 3), ("per_channel", 3), ("config3_small", 2)])
+def test_activations_in_tensor_memory(name, path, n):
+    """The kernel that keeps the activations in tensor memory (identity inputs, and feature planes): batches that end inside a
+    tile, fill one, and give a slot its second tile; 16, 32 and 64 channels, with and without bias. Against the mma.sync
+    kernel: both round every layer to fp16 (2^-11), the fp32 sums differ in order."""
+    import torch
+    from qmlp import bindings
+    cfg, rng, spec, net, params, tables, acts, t_params, t_tables = _setup(name)
+    x = torch.from_numpy(helpers.uniform(46, 1, (n, spec.num_inputs), *rng)).cuda()
+    out = []
+    try:
+        for p in (path, 1):
+            bindings.QuickMLP.set_kernel_path(p)
+            out.append(net.inference(x, t_params, t_tables).cpu().numpy())
+    finally:
+        bindings.QuickMLP.set_kernel_path(0)
+    helpers.assert_close(out[0], out[1], f"{name} n={n}", rtol=5e-3, atol=2e-3, max_violations=0.005)
+
+
+@pytest.mark.parametrize("n,chunk", [(1, 0), (129, 0), (5000, 1024), ((1 << 18) + 33, 0)])
+@pytest.mark.parametrize("pinned", [True, False], ids=["pinned", "pageable"])
+def test_inference_from_host_memory_in_place(n, chunk, pinned):
+    """One output channel: a page-locked result is written by the kernels, a pageable one goes through the download slots; one
+    chunk, several chunks, a ragged last one, a result that starts inside its allocation, and calls on two streams in turn.
+    Each chunk runs the kernel that its own size picks: compared chunk by chunk with the device call."""
+    import torch
+    cfg, rng, spec, net, params, tables, acts, t_params, t_tables = _setup("config2")
+    x = torch.from_numpy(helpers.uniform(45, 1, (n, spec.num_inputs), *rng))
+    step = chunk if chunk else ((1 << 18) if pinned else (1 << 16))
+    ref = torch.cat([net.inference(x[i:i + step].cuda(), t_params, t_tables).cpu() for i in range(0, n, step)])
+    hx = x.pin_memory()
+    buf = torch.full((n + 2, 1), 7.0, pin_memory=pinned)
+    for stream in (torch.cuda.current_stream(), torch.cuda.Stream()):
+        with torch.cuda.stream(stream):
+            out = net.inference_host(hx, t_params, t_tables, output=buf[1:n + 1], chunk_points=chunk)
+        stream.synchronize()
+        assert torch.equal(out, ref) and float(buf[0]) == 7.0 and float(buf[n + 1]) == 7.0
+        out.zero_()
+
+
 @pytest.mark.parametrize("n,offset", [(1, 0), (3, 0), (4, 0), (1024, 0), (1023, 0), (1024, 1), (4097, 2)])
 def test_convert_half(n, offset):
     """fp32 -> fp16 copy of a parameter vector: vector and scalar kernels, lengths and alignments either side of the rule."""
