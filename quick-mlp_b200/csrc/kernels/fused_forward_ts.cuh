@@ -1,16 +1,17 @@
-// Fused inference with the activations in tensor memory, for networks up to 64 channels wide whose layer-0 input is at hand
+// Fused inference with the activations in tensor memory, for networks up to 128 channels wide whose layer-0 input is at hand
 // (identity encodings, or the feature planes of encode_planes_kernel).
 //
 // Same contract as fused_forward_tc_kernel (replaces NetworkKernelInferenceAndForward,
-// src_cpp/include/qmlp/kernels/network_forward.cuh:34-114). That kernel is bound by shared memory at these widths: an MMA
+// src_cpp/include/qmlp/kernels/network_forward.cuh:34-114). That kernel is bound by shared memory up to 64 channels: an MMA
 // of 128 x 64 x 16 reads 4 KB of activations and 2 KB of weights at 128 bytes per clock, 48 clocks for an operation that the
 // tensor core does in 32, and the epilogues write every activation there first (64-wide network of five layers: about 1570
 // of the 1780 clocks a tile took). Here the epilogue writes the next operand to tensor memory (tcgen05.st), the MMA
 // takes it from there, and shared memory only delivers weights.
 //
-//   * One persistent CTA per SM, one warpgroup per tile slot. A slot is 128 points in flight: an fp32 accumulator of 64 (32)
-//     columns and the fp16 operand of the next layer in 32 (16) columns, two channels per column. 512 columns hold five
-//     (eight) slots and the constant operand of the bias MMA. Thread = point row = TMEM lane.
+//   * One persistent CTA per SM, one warpgroup per tile slot (three for wide networks, which take the blocks of 16 channels in
+//     turn). A slot is 128 points in flight: an fp32 accumulator of 64 (32, 128) columns and the fp16 operand of the next
+//     layer in 32 (16, 64) columns, two channels per column. 512 columns hold five (eight, two) slots and the constant
+//     operand of the bias MMA. Lane = point row = TMEM lane.
 //   * Per layer: wait for the accumulator, read it, activate, write the operand, meet on the slot's named barrier; then one
 //     warp of the slot issues the K/16 MMAs, the bias MMA (operand [1, 0, ...] x block with the bias in its first K column) and
 //     the commit. The issuing warps of the slots sit on different SM sub-partitions.
@@ -29,10 +30,14 @@ template <class Spec>
 struct TsLayout {
     using TL = TcLayout<Spec>;
     static constexpr int NL = Spec::NUM_LAYERS;
-    static constexpr int ACC = TL::maxCout() <= 32 ? 32 : 64, OPERAND = TL::maxCin() <= 32 ? 16 : 32, ONES = 8;   // columns
-    static constexpr int SLOTS = (512 - ONES) / (ACC + OPERAND) > 8 ? 8 : (512 - ONES) / (ACC + OPERAND);
-    static constexpr int THREADS = SLOTS * 128;
-    __host__ __device__ static constexpr bool eligible() { return TL::eligible() && TL::maxCout() <= 64 && TL::maxCin() <= 64; }
+    static constexpr int ACC = TL::maxCout() <= 32 ? 32 : TL::maxCout() <= 64 ? 64 : 128,
+                         OPERAND = TL::maxCin() <= 32 ? 16 : TL::maxCin() <= 64 ? 32 : 64, ONES = 8;   // columns
+    // warpgroups of a slot: 128 channels fit two slots only (192 columns each); with three warpgroups per slot (two / four) the
+    // 64 -> 128 -> 128 -> 128 -> 4 layers of 2^22 points take 309 us (320 / 324; 406 with the operands in shared memory)
+    static constexpr int WG = ACC == 128 ? 3 : 1;
+    static constexpr int FIT = (512 - ONES) / (ACC + OPERAND), SLOTS = FIT < 8 ? FIT : 8;
+    static constexpr int THREADS = SLOTS * WG * 128;
+    __host__ __device__ static constexpr bool eligible() { return TL::eligible() && TL::maxCout() <= 128 && TL::maxCin() <= 128; }
     // bias block of layer l: COUT rows of 16 halfs, un-swizzled (bias_block_offset)
     __host__ __device__ static constexpr int biasOffset(int l)
     {
@@ -61,19 +66,23 @@ __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.
 
 template <class Spec>
 struct TsSlot {
-    static constexpr int PIECES = Spec::CIN[0] / 8;
+    static constexpr int WG = TsLayout<Spec>::WG, STEPS = (Spec::CIN[0] / 16 + WG - 1) / WG;   // 16-channel steps this thread writes
     uint32_t tmem;          // accumulator, lane field of this warp included; the operand follows
     uint32_t full, parity;  // mbarrier the MMAs commit to
     long long point;
-    uint32_t features[PIECES][4];   // of the next tile
+    uint32_t features[STEPS][2][4];   // of the next tile
 };
 
 template <class Spec, int K>
-__device__ __forceinline__ void ts_fetch(const LaunchArgs& p, TsSlot<Spec>& sl, long long point)
+__device__ __forceinline__ void ts_fetch(const LaunchArgs& p, TsSlot<Spec>& sl, int wg, long long point)
 {
-    if constexpr (K < TsSlot<Spec>::PIECES) {
-        fetch_piece<Spec, K * 8, K * 8 + 8>(p, point, sl.features[K]);
-        ts_fetch<Spec, K + 1>(p, sl, point);
+    constexpr int WG = TsSlot<Spec>::WG;
+    if constexpr (K * 16 < Spec::CIN[0]) {
+        if (wg == K % WG) {
+            fetch_piece<Spec, K * 16, K * 16 + 8>(p, point, sl.features[K / WG][0]);
+            fetch_piece<Spec, K * 16 + 8, K * 16 + 16>(p, point, sl.features[K / WG][1]);
+        }
+        ts_fetch<Spec, K + 1>(p, sl, wg, point);
     }
 }
 
@@ -85,7 +94,7 @@ __device__ __forceinline__ void ts_issue(uint32_t lead, uint32_t smem, uint32_t 
     constexpr uint32_t idesc = umma_idesc_f16(TC_TILE, COUT);
     const uint64_t b = umma_desc_sw128(smem + TcLayout<Spec>::wOffset(L));
 #pragma unroll
-    for (int k = 0; k < CIN / 16; ++k) umma_f16_ts_elected(lead, slotTmem, slotTmem + TS::ACC + k * 8, b + ((k * 32) >> 4), idesc, k > 0 ? 1u : 0u);
+    for (int k = 0; k < CIN / 16; ++k) umma_f16_ts_elected(lead, slotTmem, slotTmem + TS::ACC + k * 8, b + (((k >> 2) * (COUT * 128) + (k & 3) * 32) >> 4), idesc, k > 0 ? 1u : 0u);
     if constexpr (Spec::BOFF[L] >= 0) umma_f16_ts_elected(lead, slotTmem, onesTmem, umma_desc_k16_noswizzle(smem + TS::biasOffset(L)), idesc, 1u);
     umma_commit_elected(lead, full);
 }
@@ -93,19 +102,23 @@ __device__ __forceinline__ void ts_issue(uint32_t lead, uint32_t smem, uint32_t 
 // Stage 0: features -> operand of layer 0. Stage L + 1: epilogue of layer L. Every stage but the last ends with the MMAs of the
 // next layer.
 template <class Spec, int ST>
-__device__ __forceinline__ void ts_stages(const LaunchArgs& p, TsSlot<Spec>& sl, uint32_t smem, uint32_t onesTmem, int barrierId, bool issuer, uint32_t lead,
+__device__ __forceinline__ void ts_stages(const LaunchArgs& p, TsSlot<Spec>& sl, uint32_t smem, uint32_t onesTmem, int wg, int barrierId, bool issuer, uint32_t lead,
                                           long long next, volatile int* abortFlag, bool& dead)
 {
     using TS = TsLayout<Spec>;
     constexpr int NL = Spec::NUM_LAYERS;
+    constexpr int WG = TS::WG;
     if constexpr (ST == 0) {
+        constexpr int CIN0 = Spec::CIN[0];
 #pragma unroll
-        for (int k = 0; k < Spec::CIN[0] / 16; ++k) {
-            const uint32_t (&a)[4] = sl.features[2 * k], (&b)[4] = sl.features[2 * k + 1];
+        for (int k = 0; k < TsSlot<Spec>::STEPS; ++k) {
+            const int step = wg + k * WG;
+            if (step * 16 >= CIN0) continue;
+            const uint32_t (&a)[4] = sl.features[k][0], (&b)[4] = sl.features[k][1];
             const uint32_t v[8] = {a[0], a[1], a[2], a[3], b[0], b[1], b[2], b[3]};
-            tmem_st8(sl.tmem + TS::ACC + k * 8, v);
+            tmem_st8(sl.tmem + TS::ACC + step * 8, v);
         }
-        if (next < p.numel) ts_fetch<Spec, 0>(p, sl, next);
+        if (next < p.numel) ts_fetch<Spec, 0>(p, sl, wg, next);
     } else {
         constexpr int L = ST - 1, COUT = Spec::COUT[L];
         using Act = typename Spec::template Act<L>;
@@ -114,19 +127,25 @@ __device__ __forceinline__ void ts_stages(const LaunchArgs& p, TsSlot<Spec>& sl,
         __syncwarp();   // tcgen05.ld is warp-collective
         tc_fence_after();
         if constexpr (ST < NL) {
-            constexpr int W = COUT < 32 ? COUT : 32;   // columns per wait
+            // the warpgroups take the blocks of 16 columns in turn; two blocks per wait
+            constexpr int BLOCKS = (COUT / 16 + WG - 1) / WG;
 #pragma unroll
-            for (int c0 = 0; c0 < COUT; c0 += W) {
-                float v[W];
+            for (int b0 = 0; b0 < BLOCKS; b0 += 2) {
+                float v[2][16];
 #pragma unroll
-                for (int g = 0; g < W / 16; ++g) tmem_ld16(sl.tmem + c0 + g * 16, *reinterpret_cast<float (*)[16]>(&v[g * 16]));
+                for (int b = 0; b < 2; ++b) {
+                    const int col = (wg + (b0 + b) * WG) * 16;
+                    if (b0 + b < BLOCKS && col < COUT) tmem_ld16(sl.tmem + col, v[b]);
+                }
                 tmem_wait_ld();
 #pragma unroll
-                for (int g = 0; g < W / 16; ++g) {
+                for (int b = 0; b < 2; ++b) {
+                    const int col = (wg + (b0 + b) * WG) * 16;
+                    if (b0 + b >= BLOCKS || col >= COUT) continue;
                     uint32_t w[8];
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) w[i] = h2_as_u32(act_forward_f32x2<Act>(v[g * 16 + 2 * i], v[g * 16 + 2 * i + 1], c0 + g * 16 + 2 * i));
-                    tmem_st8(sl.tmem + TS::ACC + (c0 + g * 16) / 2, w);
+                    for (int i = 0; i < 8; ++i) w[i] = h2_as_u32(act_forward_f32x2<Act>(v[b][2 * i], v[b][2 * i + 1], col + 2 * i));
+                    tmem_st8(sl.tmem + TS::ACC + col / 2, w);
                 }
             }
         } else {
@@ -134,6 +153,7 @@ __device__ __forceinline__ void ts_stages(const LaunchArgs& p, TsSlot<Spec>& sl,
             constexpr int OUT = Spec::NUM_OUTPUTS;
 #pragma unroll
             for (int c0 = 0; c0 < OUT; c0 += 8) {
+                if (c0 / 8 % WG != wg) continue;
                 float v[8];
                 tmem_ld8(sl.tmem + c0, v);
                 tmem_wait_ld();
@@ -152,12 +172,12 @@ __device__ __forceinline__ void ts_stages(const LaunchArgs& p, TsSlot<Spec>& sl,
     if constexpr (ST < NL) {
         tmem_wait_st();
         tc_fence_before();
-        asm volatile("bar.sync %0, 128;" ::"r"(barrierId) : "memory");
+        asm volatile("bar.sync %0, %1;" ::"r"(barrierId), "n"(WG * 128) : "memory");
         if (issuer && !dead) {
             tc_fence_after();
             ts_issue<Spec, ST>(lead, smem, sl.tmem & 0x0000ffffu, onesTmem, sl.full);
         }
-        ts_stages<Spec, ST + 1>(p, sl, smem, onesTmem, barrierId, issuer, lead, next, abortFlag, dead);
+        ts_stages<Spec, ST + 1>(p, sl, smem, onesTmem, wg, barrierId, issuer, lead, next, abortFlag, dead);
     }
 }
 
@@ -190,7 +210,7 @@ fused_forward_ts_kernel(const __grid_constant__ LaunchArgs p, const __grid_const
     uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(weightBar + 1);
     volatile int* abortFlag = reinterpret_cast<int*>(tmemSlot + 1);
     const uint32_t smemBase = smem_u32(smem);
-    const int warp = threadIdx.x >> 5, slot = warp >> 2, row = threadIdx.x & 127;
+    const int warp = threadIdx.x >> 5, slot = (warp >> 2) / TS::WG, wg = (warp >> 2) % TS::WG, row = threadIdx.x & 127;
 
     if (threadIdx.x == 0) {
         mbar_init(smem_u32(weightBar), 1);
@@ -208,8 +228,10 @@ fused_forward_ts_kernel(const __grid_constant__ LaunchArgs p, const __grid_const
     TsSlot<Spec> sl;
     sl.point = pointOf(slot);
 #pragma unroll
-    for (int k = 0; k < TsSlot<Spec>::PIECES; ++k) sl.features[k][0] = sl.features[k][1] = sl.features[k][2] = sl.features[k][3] = 0u;
-    if (sl.point < p.numel) ts_fetch<Spec, 0>(p, sl, sl.point);
+    for (int k = 0; k < TsSlot<Spec>::STEPS; ++k)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sl.features[k][i / 4][i % 4] = 0u;
+    if (sl.point < p.numel) ts_fetch<Spec, 0>(p, sl, wg, sl.point);
     ts_stage_bias<Spec, 0>(p, smem);
     if (warp == 0) {
         tmem_alloc(smem_u32(tmemSlot), 512);
@@ -222,7 +244,7 @@ fused_forward_ts_kernel(const __grid_constant__ LaunchArgs p, const __grid_const
     const uint32_t tmemBase = *tmemSlot;
     const uint32_t laneField = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const uint32_t onesTmem = tmemBase + TS::SLOTS * (TS::ACC + TS::OPERAND);
-    if (slot == 0) {   // constant operand of the bias MMA: every row = [1, 0, ..., 0]
+    if (warp < 4) {   // constant operand of the bias MMA: every row = [1, 0, ..., 0]
         const uint32_t one[8] = {0x3C00u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
         tmem_st8(onesTmem + laneField, one);
         tmem_wait_st();
@@ -235,13 +257,13 @@ fused_forward_ts_kernel(const __grid_constant__ LaunchArgs p, const __grid_const
     sl.tmem = tmemBase + slot * (TS::ACC + TS::OPERAND) + laneField;
     sl.full = smem_u32(bars + 2 * slot);
     sl.parity = 0;
-    const bool issuer = (warp & 3) == (slot & 3);
+    const bool issuer = wg == 0 && (warp & 3) == (slot & 3);
     const uint32_t lead = elect_one();
     train_wait(smem_u32(weightBar), 0, abortFlag, dead);
     __syncwarp();
     for (int i = slot; i < myTiles; i += TS::SLOTS) {
         const long long next = pointOf(i + TS::SLOTS);
-        ts_stages<Spec, 0>(p, sl, smemBase, onesTmem, 1 + slot, issuer, lead, next, abortFlag, dead);
+        ts_stages<Spec, 0>(p, sl, smemBase, onesTmem, wg, 1 + slot, issuer, lead, next, abortFlag, dead);
         sl.point = next;
     }
     if (issuer && __any_sync(0xffffffffu, dead)) {   // gave up: let the MMAs in flight finish

@@ -466,10 +466,11 @@ def test_argument_errors():
 
 
 @pytest.mark.parametrize("n", [1, 127, 128, 129, 148 * 128 + 1, 148 * 128 * 6 + 33])
-@pytest.mark.parametrize("name,path", [("config1", 3), ("config2", 3), ("uneven", 3), ("per_channel", 3), ("config3_small", 2)])
+@pytest.mark.parametrize("name,path", [("config1", 3), ("config2", 3), ("uneven", 3), ("per_channel", 3), ("config3_small", 2),
+                                       ("config4_small", 2), ("config5_small", 2)])
 def test_activations_in_tensor_memory(name, path, n):
     """The kernel that keeps the activations in tensor memory (identity inputs, and feature planes): batches that end inside a
-    tile, fill one, and give a slot its second tile; 16, 32 and 64 channels, with and without bias. Against the mma.sync
+    tile, fill one, and give a slot its second tile; 16 to 128 channels, with and without bias. Against the mma.sync
     kernel: both round every layer to fp16 (2^-11), the fp32 sums differ in order."""
     import torch
     from qmlp import bindings
