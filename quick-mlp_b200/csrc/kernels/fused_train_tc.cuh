@@ -10,7 +10,7 @@
 //
 //   * One persistent CTA of 16 + 1 warps per SM. A tile is 128 points; the CTA has two tile slots of two warpgroups each, or
 //     one of four where shared or tensor memory is short. The slots run independently: the MMAs of one run under the epilogue
-//     of the other. Thread = (point row, column share): the warpgroups of a slot take the blocks of 16 columns of an
+//     of the other. Thread = (point row, column share): the warpgroups of a slot take the blocks of 8 columns of an
 //     accumulator row in turn.
 //   * Shared memory, all in the 128-byte swizzled layout (rows = points, 64 channels per block): the weights (staged by
 //     TMA), per slot one buffer per layer input and one for the last delta. The delta of layer l - 1 overwrites the input
@@ -24,13 +24,15 @@
 //     delta^T * input (M = outputs) or input^T * delta (M = inputs), whichever needs fewer columns. The bias gradient is one
 //     more column (or row) of the same MMA: a channel of ones in the padding of the input's block, or a constant block of
 //     ones behind it.
-//   * One warp issues all MMAs, in whatever order the slots get ready, so MMAs of the two slots into the shared accumulators
-//     stay in order. The adjoint MMAs of a layer are committed before its weight gradient, which only has to be done when the
-//     input buffer is overwritten.
-// Measured, step of 32 -> 64 -> 64 -> 1 on 2^20 points: 94 (forward) + 123 (backward) + 127 us (weight gradients) -> 136 us;
-// 48 -> 128 -> 64 -> 16 -> 4 on 2^21 points: 709 (with the gather) + 1022 (with the scatter) + 473 -> 660 us. Bound by
-// the tensor core: an MMA of K = 16 takes 48 clocks up to N = 64 however few columns it has, and a stage's round trip
-// (barrier, issue, MMAs, commit) takes several hundred that one other slot cannot cover.
+//   * The warp of a slot that finishes a stage last issues the MMAs that the next stage waits for (a warp of its own polling both
+//     slots took several hundred clocks to notice: 606 -> 577 us in the second example below). The weight gradients of
+//     all slots go to the same accumulators, so one warp issues all of them, in order; they only have to be done when the
+//     next stage of the slot overwrites their operands.
+// Measured, step of 32 -> 64 -> 64 -> 1 on 2^20 points: 94 (forward) + 123 (backward) + 127 us (weight gradients) -> 137 us;
+// 48 -> 128 -> 64 -> 16 -> 4 on 2^21 points: 709 (with the gather) + 1022 (with the scatter) + 473 -> 577 us (655 with 16
+// columns per block instead of 8: the narrow layers then leave a warpgroup idle). Bound by the latency of the stages: an MMA of
+// K = 16 takes 48 clocks up to N = 64 from shared memory however few columns it has, and the round trip of a stage (arrival,
+// issue, MMAs, commit, accumulator load) takes about a thousand clocks that one other slot cannot cover.
 // Every wait is bounded; on a timeout the CTA runs through without waiting and the status word is set.
 //
 // Same roundings as the separate kernels: fp16 activations, deltas and pre-activations (bias added in half), fp32 sums.
@@ -40,7 +42,7 @@
 namespace qmlp {
 namespace kernel {
 
-constexpr int TRAIN_WARPGROUPS = 4, TRAIN_THREADS = TRAIN_WARPGROUPS * 128 + 32;   // the last warp issues the MMAs
+constexpr int TRAIN_WARPGROUPS = 4, TRAIN_THREADS = TRAIN_WARPGROUPS * 128 + 32;   // the last warp issues the weight gradients
 constexpr int TRAIN_BLOCK = TC_TILE * 128;   // bytes of a block: 128 points x 64 channels
 
 template <class Spec>
@@ -96,7 +98,8 @@ struct TrainLayout {
     __host__ __device__ static constexpr int onesStart(int slots) { return slotStart() + slots * slotBytes(); }
     __host__ __device__ static constexpr int biasStart(int slots) { return onesStart(slots) + TRAIN_BLOCK; }
     __host__ __device__ static constexpr int barStart(int slots) { return biasStart(slots) + (dBefore(NL) * 2 + 127) / 128 * 128; }
-    __host__ __device__ static constexpr int bytes(int slots) { return barStart(slots) + 128 + 1024; }
+    // barriers, arrival counters and flags (fused_train_tc_kernel)
+    __host__ __device__ static constexpr int bytes(int slots) { return barStart(slots) + 384 + 1024; }
     __host__ __device__ static constexpr bool fits(int slots, bool recompute)
     {
         return slots * (recompute ? 128 : keptCols()) + wgCol(NL) <= 512 && bytes(slots) <= 227 * 1024;
@@ -279,7 +282,7 @@ __device__ __forceinline__ void store_piece(const LaunchArgs& p, long long point
     }
 }
 
-// ---- MMAs (issued by one warp) --------------------------------------------------------------------------------------------
+// ---- MMAs (issued by one elected lane of a whole warp) --------------------------------------------------------------------------------------------
 template <class Spec, int SLOTS>
 struct TrainIssue {
     using TL = TcLayout<Spec>;
@@ -331,31 +334,44 @@ struct TrainIssue {
                                  umma_idesc_f16(TC_TILE, 16) | UMMA_A_MN | UMMA_B_MN, k == 0 ? accumulate : 1u);
         }
     }
-    // everything that follows stage ST. `started`: layers whose weight-gradient accumulator holds sums already
+    // what the next stage of the slot waits for after stage ST
     template <int ST>
-    static __device__ __forceinline__ void after(uint32_t lead, uint32_t smem, uint32_t slotSmem, uint32_t slotTmem, uint32_t wgTmem, uint32_t& started, uint32_t bars)
+    static __device__ __forceinline__ void critical(uint32_t lead, uint32_t smem, uint32_t slotSmem, uint32_t slotTmem, uint32_t bars)
     {
-        constexpr int NL = Spec::NUM_LAYERS;
+        constexpr int NL = Spec::NUM_LAYERS, NEXT = ST + 1;
         if constexpr (ST < NL) {
             forward<ST, 0, Spec::COUT[ST]>(lead, smem, slotSmem, slotTmem + TR::dCol(ST));
             umma_commit_elected(lead, bars);
-        } else {
-            // operands of the next step, committed first; then the weight gradient of the layer whose delta is complete
-            constexpr int NEXT = ST + 1;
-            if constexpr (NEXT < TR::lastStage()) {
-                constexpr int L = TR::stepLayer(NEXT), FIRST = 64 * TR::stepIndex(NEXT), LEFT = Spec::COUT[L] - FIRST;
-                constexpr int N = TR::RECOMPUTE && LEFT > 64 ? 64 : LEFT;
-                if constexpr (TR::RECOMPUTE) forward<L, FIRST, N>(lead, smem, slotSmem, slotTmem);
-                adjoint<L + 1, FIRST, N>(lead, smem, slotSmem, slotTmem + TR::adjCol());
-                umma_commit_elected(lead, bars);
-            } else if constexpr (TR::GRID) {
-                adjoint<0, 0, Spec::CIN[0]>(lead, smem, slotSmem, slotTmem + TR::featureAdjCol());
-                umma_commit_elected(lead, bars);
-            }
-            constexpr int DONE = ST == NL ? NL - 1 : TR::stepLayer(ST == NL ? NL + 1 : ST);
-            if constexpr (ST == NL || TR::stepIndex(ST == NL ? NL + 1 : ST) == TR::steps(DONE) - 1) {
-                gradient<DONE>(lead, smem, slotSmem, wgTmem, (started >> DONE) & 1u);
-                started |= 1u << DONE;
+        } else if constexpr (NEXT < TR::lastStage()) {
+            constexpr int L = TR::stepLayer(NEXT), FIRST = 64 * TR::stepIndex(NEXT), LEFT = Spec::COUT[L] - FIRST;
+            constexpr int N = TR::RECOMPUTE && LEFT > 64 ? 64 : LEFT;
+            if constexpr (TR::RECOMPUTE) forward<L, FIRST, N>(lead, smem, slotSmem, slotTmem);
+            adjoint<L + 1, FIRST, N>(lead, smem, slotSmem, slotTmem + TR::adjCol());
+            umma_commit_elected(lead, bars);
+        } else if constexpr (TR::GRID) {
+            adjoint<0, 0, Spec::CIN[0]>(lead, smem, slotSmem, slotTmem + TR::featureAdjCol());
+            umma_commit_elected(lead, bars);
+        }
+    }
+    // layer whose delta is complete after stage ST (-1: none)
+    template <int ST>
+    __host__ __device__ static constexpr int graded()
+    {
+        constexpr int NL = Spec::NUM_LAYERS;
+        if constexpr (ST < NL) return -1;
+        else if constexpr (ST == NL) return NL - 1;
+        else return TR::stepIndex(ST) == TR::steps(TR::stepLayer(ST)) - 1 ? TR::stepLayer(ST) : -1;
+    }
+    // weight gradient of layer `layer`. `started`: layers whose accumulator holds sums already
+    template <int L>
+    static __device__ __forceinline__ void weights(uint32_t lead, int layer, uint32_t smem, uint32_t slotSmem, uint32_t wgTmem, uint32_t& started, uint32_t bars)
+    {
+        if constexpr (L < Spec::NUM_LAYERS) {
+            if (layer != L) {
+                weights<L + 1>(lead, layer, smem, slotSmem, wgTmem, started, bars);
+            } else {
+                gradient<L>(lead, smem, slotSmem, wgTmem, (started >> L) & 1u);
+                started |= 1u << L;
                 umma_commit_elected(lead, bars + 8);
             }
         }
@@ -370,7 +386,9 @@ struct TrainSlot {
     static constexpr int TARGETS = Spec::NUM_OUTPUTS <= 4 ? Spec::NUM_OUTPUTS : 0;  // prefetched by the warpgroup that takes the loss
     uint32_t row;          // shared address of this thread's row in buffer 0
     uint32_t tmem;         // base column, lane field of this warp included
-    uint32_t bars;         // full: accumulator done; graded: weight gradient done; ready: operands written (one arrival per warp)
+    uint32_t bars;         // full: accumulator done; graded: weight gradient done; ready: a delta is complete
+    uint32_t counter;      // arrivals of the slot's warps
+    uint32_t smem, slotSmem, slotTmem, lead;   // what the MMAs of the slot are issued from
     uint32_t full, graded; // parities
     long long point;
     bool valid;
@@ -410,30 +428,28 @@ __device__ __forceinline__ void train_store_adjoint(const LaunchArgs& p, const T
     }
 }
 
-// pre-activations of 16 accumulator columns: rounded to half, then the half bias is added
+// pre-activations of 8 accumulator columns: rounded to half, then the half bias is added
 template <class Spec, int L>
-__device__ __forceinline__ void train_pre(const float (&v)[16], const __half* bias, int col, __half2 (&pre)[8])
+__device__ __forceinline__ void train_pre(const float (&v)[8], const __half* bias, int col, __half2 (&pre)[4])
 {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) pre[i] = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
+    for (int i = 0; i < 4; ++i) pre[i] = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
     if constexpr (Spec::BOFF[L] >= 0) {
-        const uint4* b = reinterpret_cast<const uint4*>(bias + TrainLayout<Spec>::dBefore(L) + col);
-        const uint4 b0 = b[0], b1 = b[1];
-        const uint32_t w[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+        const uint4 b0 = *reinterpret_cast<const uint4*>(bias + TrainLayout<Spec>::dBefore(L) + col);
+        const uint32_t w[4] = {b0.x, b0.y, b0.z, b0.w};
 #pragma unroll
-        for (int i = 0; i < 8; ++i) pre[i] = __hadd2(pre[i], u32_as_h2(w[i]));
+        for (int i = 0; i < 4; ++i) pre[i] = __hadd2(pre[i], u32_as_h2(w[i]));
     }
 }
-// 16 channels starting at chunk CHUNK (8 channels each) + `col` of this thread's row of a buffer
+// 8 channels at chunk CHUNK (8 channels each) + `col` / 8 of this thread's row of a buffer
 template <int CHUNK = 0>
-__device__ __forceinline__ void train_put(uint32_t rowAddr, int row, int col, const uint32_t (&w)[8])
+__device__ __forceinline__ void train_put(uint32_t rowAddr, int row, int col, const uint32_t (&w)[4])
 {
     sts128(rowAddr + sw128_row_offset(row, CHUNK + col / 8), w[0], w[1], w[2], w[3]);
-    sts128(rowAddr + sw128_row_offset(row, CHUNK + col / 8 + 1), w[4], w[5], w[6], w[7]);
 }
 
 // One stage of a slot's tile (TrainLayout::lastStage). Every stage but the last is followed by the MMAs of the next one: the
-// warps arrive on the slot's `ready` barrier, the issuing warp waits for all of them.
+// warps count their arrivals, and the last one issues.
 template <class Spec, int ST>
 __device__ __forceinline__ void train_stage(const LaunchArgs& p, TrainSlot<Spec>& sl, const __half* bias, int wg, int row, long long nextPoint,
                                             float& lossAcc, volatile int* abortFlag, bool& dead)
@@ -467,34 +483,34 @@ __device__ __forceinline__ void train_stage(const LaunchArgs& p, TrainSlot<Spec>
             constexpr int L = ST - 1, COUT = Spec::COUT[L];
             using Act = typename Spec::template Act<L>;
 #pragma unroll
-            for (int k = 0; k < (COUT / 16 + WG - 1) / WG; ++k) {
-                const int col = (wg + k * WG) * 16;
+            for (int k = 0; k < (COUT / 8 + WG - 1) / WG; ++k) {
+                const int col = (wg + k * WG) * 8;
                 if (col >= COUT) continue;
-                float v[16];
-                __half2 pre[8];
-                uint32_t w[8];
-                tmem_ld16(sl.tmem + TR::dCol(L) + col, v);
+                float v[8];
+                __half2 pre[4];
+                uint32_t w[4];
+                tmem_ld8(sl.tmem + TR::dCol(L) + col, v);
                 tmem_wait_ld();
                 train_pre<Spec, L>(v, bias, col, pre);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) w[i] = h2_as_u32(act_forward2<Act>(pre[i], col + 2 * i));
+                for (int i = 0; i < 4; ++i) w[i] = h2_as_u32(act_forward2<Act>(pre[i], col + 2 * i));
                 train_put(sl.row + TR::bufOffset(L + 1), row, col, w);
             }
         } else if constexpr (ST == NL) {
             constexpr int L = NL - 1, COUT = Spec::COUT[L];
             using Act = typename Spec::template Act<L>;
 #pragma unroll
-            for (int k = 0; k < (COUT / 16 + WG - 1) / WG; ++k) {
-                const int col = (wg + k * WG) * 16;
+            for (int k = 0; k < (COUT / 8 + WG - 1) / WG; ++k) {
+                const int col = (wg + k * WG) * 8;
                 if (col >= COUT) continue;
-                float v[16];
-                __half2 pre[8];
-                uint32_t w[8];
-                tmem_ld16(sl.tmem + TR::dCol(L) + col, v);
+                float v[8];
+                __half2 pre[4];
+                uint32_t w[4];
+                tmem_ld8(sl.tmem + TR::dCol(L) + col, v);
                 tmem_wait_ld();
                 train_pre<Spec, L>(v, bias, col, pre);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
+                for (int i = 0; i < 4; ++i) {
                     float adj[2] = {0.f, 0.f};
                     if (col + 2 * i < Spec::NUM_OUTPUTS && sl.valid) {
                         const float2 out = __half22float2(act_forward2<Act>(pre[i], col + 2 * i));
@@ -526,18 +542,18 @@ __device__ __forceinline__ void train_stage(const LaunchArgs& p, TrainSlot<Spec>
             using Act = typename Spec::template Act<L>;
             bool graded = H > 0;
 #pragma unroll
-            for (int k = 0; k < (N / 16 + WG - 1) / WG; ++k) {
-                const int col = (wg + k * WG) * 16;
+            for (int k = 0; k < (N / 8 + WG - 1) / WG; ++k) {
+                const int col = (wg + k * WG) * 8;
                 if (col >= N) continue;
-                float v[16], x[16];
-                __half2 pre[8];
-                uint32_t w[8];
-                tmem_ld16(sl.tmem + TR::dCol(L) + col, v);
-                tmem_ld16(sl.tmem + TR::adjCol() + col, x);
+                float v[8], x[8];
+                __half2 pre[4];
+                uint32_t w[4];
+                tmem_ld8(sl.tmem + TR::dCol(L) + col, v);
+                tmem_ld8(sl.tmem + TR::adjCol() + col, x);
                 tmem_wait_ld();
                 train_pre<Spec, L>(v, bias, FIRST + col, pre);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
+                for (int i = 0; i < 4; ++i) {
                     const __half2 d = act_adjoint2<Act>(pre[i], __floats2half2_rn(x[2 * i], x[2 * i + 1]), FIRST + col + 2 * i);
                     w[i] = sl.valid ? h2_as_u32(d) : 0u;
                 }
@@ -554,10 +570,20 @@ __device__ __forceinline__ void train_stage(const LaunchArgs& p, TrainSlot<Spec>
         }
     }
     if constexpr (ST < TR::lastStage()) {
+        using Issue = TrainIssue<Spec, TR::SLOTS>;
         tc_fence_before();
         fence_proxy_async();   // generic-proxy writes of the operands become visible to the tensor core
         __syncwarp();
-        if ((threadIdx.x & 31) == 0) mbar_arrive(sl.bars + 16);
+        uint32_t before = 0;
+        if ((threadIdx.x & 31) == 0)
+            asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;" : "=r"(before) : "r"(sl.counter) : "memory");
+        before = __shfl_sync(0xffffffffu, before, 0);
+        if ((before & (WG * 4 - 1)) == WG * 4 - 1) {
+            tc_fence_after();
+            if (!__any_sync(0xffffffffu, dead)) Issue::template critical<ST>(sl.lead, sl.smem, sl.slotSmem, sl.slotTmem, sl.bars);
+            if constexpr (Issue::template graded<ST>() >= 0)
+                if ((threadIdx.x & 31) == 0) mbar_arrive(sl.bars + 16);
+        }
     }
 }
 
@@ -571,27 +597,19 @@ __device__ __forceinline__ void train_stages(const LaunchArgs& p, TrainSlot<Spec
     }
 }
 
-template <class Spec, int ST, int SLOTS>
-__device__ __forceinline__ void train_issue_stage(uint32_t lead, int stage, uint32_t smem, uint32_t slotSmem, uint32_t slotTmem, uint32_t wgTmem, uint32_t& started,
-                                                  uint32_t bars)
-{
-    if constexpr (ST < TrainLayout<Spec>::lastStage()) {
-        if (stage == ST) TrainIssue<Spec, SLOTS>::template after<ST>(lead, smem, slotSmem, slotTmem, wgTmem, started, bars);
-        else train_issue_stage<Spec, ST + 1, SLOTS>(lead, stage, smem, slotSmem, slotTmem, wgTmem, started, bars);
-    }
-}
-// the issuing warp: whenever a slot's operands are written, the MMAs that follow
+// The weight-gradient warp: whenever a slot's delta is complete, the MMAs of that layer's gradient. All slots add to the same
+// accumulators, so one thread issues them; nobody waits for them before the slot's next stage has computed its results.
 template <class Spec, int SLOTS>
-__device__ __forceinline__ void train_issue(uint32_t smem, uint32_t tmemBase, uint32_t bars, int myTiles, volatile int* abortFlag)
+__device__ __forceinline__ void train_gradients(uint32_t lead, uint32_t smem, uint32_t tmemBase, uint32_t bars, int myTiles, volatile int* abortFlag, bool& dead)
 {
     using TR = TrainLayout<Spec>;
-    const uint32_t lead = elect_one();
-    int stage[SLOTS], left[SLOTS], open = 0;   // left: stages the slot still has to run
+    constexpr int NL = Spec::NUM_LAYERS;
+    int layer[SLOTS], left[SLOTS], open = 0;
     uint32_t parity = 0, started = 0, idle = 0;
 #pragma unroll
     for (int j = 0; j < SLOTS; ++j) {
-        stage[j] = 0;
-        left[j] = myTiles > j ? (myTiles - j + SLOTS - 1) / SLOTS * TR::lastStage() : 0;
+        layer[j] = NL - 1;
+        left[j] = myTiles > j ? (myTiles - j + SLOTS - 1) / SLOTS * NL : 0;
         open += left[j] > 0;
     }
     while (open > 0) {
@@ -603,18 +621,16 @@ __device__ __forceinline__ void train_issue(uint32_t smem, uint32_t tmemBase, ui
             // (opaque copies: the descriptors of all MMAs would be computed ahead of the loop and spilled)
             uint32_t base = smem, tmem = tmemBase;
             asm volatile("" : "+r"(base), "+r"(tmem));
-            train_issue_stage<Spec, 0, SLOTS>(lead, stage[j], base, base + TR::slotStart() + j * TR::slotBytes(), tmem + j * TR::slotCols(),
-                                              tmem + SLOTS * TR::slotCols(), started, bars + j * 24);
+            TrainIssue<Spec, SLOTS>::template weights<0>(lead, layer[j], base, base + TR::slotStart() + j * TR::slotBytes(), tmem + SLOTS * TR::slotCols(), started,
+                                                         bars + j * 24);
             parity ^= 1u << j;
-            stage[j] = stage[j] == TR::lastStage() - 1 ? 0 : stage[j] + 1;
+            layer[j] = layer[j] == 0 ? NL - 1 : layer[j] - 1;
             if (--left[j] == 0) --open;
             idle = 0;
         }
         if (idle > 4 * TC_SPIN_LIMIT || ((idle & 1023u) == 1023u && __any_sync(0xffffffffu, *abortFlag != 0))) {
-            // gave up: let the MMAs in flight finish before the CTA goes on to its end
             *abortFlag = 1;
-            umma_commit_elected(lead, bars + 24 * SLOTS + 8);
-            mbar_wait(bars + 24 * SLOTS + 8, 0);
+            dead = true;
             return;
         }
     }
@@ -691,21 +707,25 @@ fused_train_tc_kernel(const __grid_constant__ LaunchArgs p, const __grid_constan
     extern __shared__ unsigned char smemRaw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~static_cast<uintptr_t>(1023));
     __half* sBias = reinterpret_cast<__half*>(smem + TR::biasStart(SLOTS));
-    // full, graded and ready of every slot, the weight staging, the drain after a timeout
+    // full, graded and ready of every slot, the weight staging, the drain of every warp after a timeout; arrival counters
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + TR::barStart(SLOTS));
     uint64_t* weightBar = bars + 3 * SLOTS;
-    uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(weightBar + 2);
+    uint64_t* drainBar = weightBar + 1;
+    uint32_t* counters = reinterpret_cast<uint32_t*>(drainBar + TRAIN_THREADS / 32);
+    uint32_t* tmemSlot = counters + SLOTS;
     volatile int* abortFlag = reinterpret_cast<int*>(tmemSlot + 1);
+    static_assert(8 * (3 * SLOTS + 1 + TRAIN_THREADS / 32) + 4 * (SLOTS + 2) <= 384, "barrier area");
     const uint32_t smemBase = smem_u32(smem);
     const int warp = threadIdx.x >> 5, warpgroup = warp >> 2, row = threadIdx.x & 127;
 
     if (threadIdx.x == 0) {
         mbar_init(smem_u32(weightBar), 1);
-        mbar_init(smem_u32(weightBar + 1), 1);
+        for (int w = 0; w < TRAIN_THREADS / 32; ++w) mbar_init(smem_u32(drainBar + w), 1);
         for (int s = 0; s < SLOTS; ++s) {
             mbar_init(smem_u32(bars + 3 * s), 1);                                // one tcgen05.commit per phase
             mbar_init(smem_u32(bars + 3 * s + 1), 1);
-            mbar_init(smem_u32(bars + 3 * s + 2), TrainSlot<Spec>::WG * 4);      // one arrival per warp
+            mbar_init(smem_u32(bars + 3 * s + 2), 1);                            // the last warp of a stage that completes a delta
+            counters[s] = 0;
         }
         *abortFlag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -737,11 +757,12 @@ fused_train_tc_kernel(const __grid_constant__ LaunchArgs p, const __grid_constan
     const int stride = gridDim.x;
     const int myTiles = static_cast<int>(blockIdx.x) < numTiles ? (numTiles - static_cast<int>(blockIdx.x) + stride - 1) / stride : 0;
     bool dead = false;
+    const uint32_t lead = elect_one();
+    train_wait(smem_u32(weightBar), 0, abortFlag, dead);
+    __syncwarp();
     if (warpgroup == TRAIN_WARPGROUPS) {
-        train_wait(smem_u32(weightBar), 0, abortFlag, dead);   // only the MMAs read the weights
-        __syncwarp();
         const uint32_t smemU = __shfl_sync(0xffffffffu, smemBase, 0), tmemU = __shfl_sync(0xffffffffu, tmemBase, 0);
-        if (!__any_sync(0xffffffffu, dead)) train_issue<Spec, SLOTS>(smemU, tmemU, smemU + TR::barStart(SLOTS), myTiles, abortFlag);
+        if (!__any_sync(0xffffffffu, dead)) train_gradients<Spec, SLOTS>(lead, smemU, tmemU, smemU + TR::barStart(SLOTS), myTiles, abortFlag, dead);
     } else {
         // tile i of this CTA's sequence belongs to slot i % SLOTS
         const int slot = warpgroup / TrainSlot<Spec>::WG, wg = warpgroup % TrainSlot<Spec>::WG;
@@ -750,6 +771,11 @@ fused_train_tc_kernel(const __grid_constant__ LaunchArgs p, const __grid_constan
         sl.row = smemBase + TR::slotStart() + slot * TR::slotBytes() + row * 128;
         sl.tmem = tmemBase + slot * TR::slotCols() + laneField;
         sl.bars = smem_u32(bars + 3 * slot);
+        sl.counter = smem_u32(counters + slot);
+        sl.smem = smemBase;
+        sl.slotSmem = smemBase + TR::slotStart() + slot * TR::slotBytes();
+        sl.slotTmem = tmemBase + slot * TR::slotCols();
+        sl.lead = lead;
         sl.full = sl.graded = 0;
         sl.point = pointOf(slot);
         train_fetch<Spec, 0>(p, sl, wg, sl.point);
@@ -762,7 +788,7 @@ fused_train_tc_kernel(const __grid_constant__ LaunchArgs p, const __grid_constan
         }
         tc_fence_before();
         asm volatile("bar.sync 1, %0;" ::"n"(TRAIN_WARPGROUPS * 128) : "memory");   // every slot's weight gradients are in
-        if (myTiles > 0 && *abortFlag == 0) {
+        if (myTiles > 0 && !__any_sync(0xffffffffu, *abortFlag != 0)) {
             tc_fence_after();
             train_flush<Spec, 0>(p, wgTmem + laneField, warpgroup, row);
             if (p.lossSum != nullptr) {
@@ -771,6 +797,12 @@ fused_train_tc_kernel(const __grid_constant__ LaunchArgs p, const __grid_constan
                 if ((threadIdx.x & 31) == 0 && lossAcc != 0.f) atomicAdd(p.lossSum, lossAcc);
             }
         }
+    }
+    __syncthreads();         // (nobody raises the flag any more)
+    if (*abortFlag != 0) {   // gave up: let this warp's MMAs in flight finish
+        umma_commit_elected(lead, smem_u32(drainBar + warp));
+        mbar_wait(smem_u32(drainBar + warp), 0);
+        __syncwarp();
     }
     tc_fence_before();
     __syncthreads();
