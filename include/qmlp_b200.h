@@ -144,6 +144,12 @@ QMLP_API int qmlp_network_initialize_parameters_host(qmlp_network_t* net, uint64
 /* FusedNetwork::inference, src_cpp/src/fused_network.cpp:507-551 */
 QMLP_API int qmlp_network_inference(qmlp_network_t* net, const qmlp_tensor_t* input, qmlp_tensor_t* output,
                                     qmlp_stream_t stream);
+/* The same with scratch memory from the caller (qmlp_network_inference_memory() bytes with the parameters bound as for the
+ * call, 0 if none is needed; 256-byte aligned, contents irrelevant). Without it, or with less, the network allocates a
+ * buffer of its own at the first call that needs one and keeps it. */
+QMLP_API int qmlp_network_inference_memory(qmlp_network_t* net, int64_t num_elements, size_t* bytes);
+QMLP_API int qmlp_network_inference_with_memory(qmlp_network_t* net, const qmlp_tensor_t* input, qmlp_tensor_t* output,
+                                                qmlp_stream_t stream, void* tmp_memory, size_t tmp_bytes);
 /* Inference from and to HOST memory. The reference has no such call: a host caller of it uploads the whole batch,
  * runs FusedNetwork::inference (src_cpp/src/fused_network.cpp:507-551) and downloads the whole result, three serial
  * steps. Here the batch is cut into chunks that move through upload -> kernel -> download on three streams, so the two

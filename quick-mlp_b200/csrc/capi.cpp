@@ -440,8 +440,37 @@ int qmlp_network_clear_cached_kernels(qmlp_network_t* net)
     QMLP_CATCH
 }
 
-// inference on device tensors; the caller holds the network's mutex
-static void inferenceLocked(Network& n, const qmlp_tensor_t* input, qmlp_tensor_t* output, qmlp_stream_t stream)
+// Points per chunk of the level-major pass for a batch of `points`, 0: the fused gather.
+// Encode level by level into planes, chunk by chunk, then run the layer chain on the planes (kernels/grid_planes.cuh), or
+// gather inside the layer kernel (fused_forward_kernel). Since both gather with lane pairs the fused kernel wins wherever
+// the level being gathered does not become resident any closer by going level by level: 3-D grid, 16 levels of 2^19
+// rows, 2^20 points 272 against 281 us. The pass wins with
+//  - tables larger than L2 (one level at a time stays in it): 4-D grid of 2^20 rows, 2^20 points 689 against 1178 us;
+//  - levels of up to 384 KB on average (one level at a time stays largely in L1), from 2^19 points on: 3-D grid of 2^15
+//    fp16 rows, 2^20 points 192 against 257 us;
+//  - 192 or more rows per point (the fused kernel's 16 warps per SM keep too few of them in flight), from 2^17 points on
+//    with fp16 tables, 2^19 with fp32: 4-D grid of 2^18 fp16 rows, 2^20 points 635 against 711 us.
+// kernelPath 2 forces this path.
+static int64_t planeChunk(const Network& n, int64_t points)
+{
+    if (n.planesUnsupported || n.gridLevels() == 0 || points <= 0) return 0;
+    const int path = Library::instance().kernelPath;
+    const int64_t tableBytes = n.gridTableBytes();
+    const bool halfTables = n.currentHalfMask() != 0;
+    const bool chosen = tableBytes > (96ll << 20) || (points >= (1 << 19) && tableBytes <= (384ll << 10) * n.gridLevels()) ||
+                        (n.gathersPerPoint() >= 192 && points >= (halfTables ? 1 << 17 : 1 << 19));
+    if (!(path == 2 || (path == 0 && chosen))) return 0;
+    // Chunk: as many points as fit in 512 MB of planes, at most 2^22. A level's table is fetched from HBM once per chunk, so
+    // large chunks amortise it; the planes themselves are streamed (written once, read once).
+    const int64_t rowBytes = static_cast<int64_t>(n.encodedChannels()) * 2;
+    int64_t cap = 1 << 16;
+    while (cap < (1 << 22) && cap * 2 * rowBytes <= (512ll << 20)) cap *= 2;
+    return std::min<int64_t>(cap, (points + 65535) / 65536 * 65536);
+}
+
+// inference on device tensors; the caller holds the network's mutex. `memory`: planes from the caller (else the network's own)
+static void inferenceLocked(Network& n, const qmlp_tensor_t* input, qmlp_tensor_t* output, qmlp_stream_t stream, void* memory = nullptr,
+                            size_t memoryBytes = 0)
 {
     checkIO(n, input, output, "output");
     kernel::LaunchArgs a;
@@ -449,51 +478,36 @@ static void inferenceLocked(Network& n, const qmlp_tensor_t* input, qmlp_tensor_
     a.output = static_cast<float*>(output->data);
     a.outS0 = output->strides[0];
     a.outS1 = output->strides[1];
-    // Encode level by level into planes, chunk by chunk, then run the layer chain on the planes (kernels/grid_planes.cuh), or
-    // gather inside the layer kernel (fused_forward_kernel). Since both gather with lane pairs the fused kernel wins wherever
-    // the level being gathered does not become resident any closer by going level by level: 3-D grid, 16 levels of 2^19
-    // rows, 2^20 points 272 against 281 us. The pass wins with
-    //  - tables larger than L2 (one level at a time stays in it): 4-D grid of 2^20 rows, 2^20 points 689 against 1178 us;
-    //  - levels of up to 384 KB on average (one level at a time stays largely in L1), from 2^19 points on: 3-D grid of 2^15
-    //    fp16 rows, 2^20 points 192 against 257 us;
-    //  - 192 or more rows per point (the fused kernel's 16 warps per SM keep too few of them in flight), from 2^17 points on
-    //    with fp16 tables, 2^19 with fp32: 4-D grid of 2^18 fp16 rows, 2^20 points 635 against 711 us.
-    // kernelPath 2 forces this path.
-    const int path = Library::instance().kernelPath;
-    const int64_t tableBytes = n.gridTableBytes();
-    const bool halfTables = n.currentHalfMask() != 0;
-    const bool chosen = tableBytes > (96ll << 20) || (a.numel >= (1 << 19) && tableBytes <= (384ll << 10) * n.gridLevels()) ||
-                        (n.gathersPerPoint() >= 192 && a.numel >= (halfTables ? 1 << 17 : 1 << 19));
-    const bool wantPlanes = !n.planesUnsupported && a.numGrids > 0 && a.numel > 0 && (path == 2 || (path == 0 && chosen));
-    if (wantPlanes) {
-        // Chunk: as many points as fit in 512 MB of planes, at most 2^22. A level's table is fetched from HBM once per
-        // chunk, so large chunks amortise it; the planes themselves are streamed (written once, read once).
+    int64_t need = a.numGrids > 0 ? planeChunk(n, a.numel) : 0;
+    if (need > 0) {
         const int64_t rowBytes = static_cast<int64_t>(n.encodedChannels()) * 2;
-        int64_t cap = 1 << 16;
-        while (cap < (1 << 22) && cap * 2 * rowBytes <= (512ll << 20)) cap *= 2;
-        const int64_t need = std::min<int64_t>(cap, (a.numel + 65535) / 65536 * 65536);
-        n.claimDevice();
-        if (n.planeCapacity < need) {
-            if (n.planes) {
-                checkCuda(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)), "cudaStreamSynchronize");
-                checkCuda(cudaFree(n.planes), "cudaFree(feature planes)");
-                n.planes = nullptr;
-                n.planeCapacity = 0;
+        __half* planes = static_cast<__half*>(memory);
+        if (memory == nullptr || memoryBytes < static_cast<size_t>(need * rowBytes)) {
+            n.claimDevice();
+            if (n.planeCapacity < need) {
+                if (n.planes) {
+                    checkCuda(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)), "cudaStreamSynchronize");
+                    checkCuda(cudaFree(n.planes), "cudaFree(feature planes)");
+                    n.planes = nullptr;
+                    n.planeCapacity = 0;
+                }
+                checkCuda(cudaMalloc(&n.planes, static_cast<size_t>(need * rowBytes)), "cudaMalloc(feature planes)");
+                n.planeCapacity = need;
             }
-            checkCuda(cudaMalloc(&n.planes, static_cast<size_t>(need * rowBytes)), "cudaMalloc(feature planes)");
-            n.planeCapacity = need;
+            need = n.planeCapacity;
+            planes = static_cast<__half*>(n.planes);
         }
         auto m = n.module(n.currentHalfMask());
         const long long total = a.numel;
         const float* in0 = a.input;
         float* out0 = a.output;
         bool ok = true;
-        for (long long c0 = 0; c0 < total && ok; c0 += n.planeCapacity) {
-            a.numel = std::min<long long>(n.planeCapacity, total - c0);
+        for (long long c0 = 0; c0 < total && ok; c0 += need) {
+            a.numel = std::min<long long>(need, total - c0);
             a.input = in0 + c0 * a.inS0;
             a.output = out0 + c0 * a.outS0;
-            a.planes = static_cast<__half*>(n.planes);
-            a.planeStride = n.planeCapacity;
+            a.planes = planes;
+            a.planeStride = need;
             int launches = 0;
             int e;
             {
@@ -516,10 +530,27 @@ static void inferenceLocked(Network& n, const qmlp_tensor_t* input, qmlp_tensor_
 
 int qmlp_network_inference(qmlp_network_t* net, const qmlp_tensor_t* input, qmlp_tensor_t* output, qmlp_stream_t stream)
 {
+    return qmlp_network_inference_with_memory(net, input, output, stream, nullptr, 0);
+}
+
+int qmlp_network_inference_memory(qmlp_network_t* net, int64_t num_elements, size_t* bytes)
+{
+    QMLP_TRY
+    if (!bytes) throw std::runtime_error("null argument");
+    Network& n = *net->impl;
+    std::lock_guard<std::mutex> lock(n.mutex);
+    *bytes = static_cast<size_t>(planeChunk(n, num_elements)) * n.encodedChannels() * 2;
+    QMLP_CATCH
+}
+
+int qmlp_network_inference_with_memory(qmlp_network_t* net, const qmlp_tensor_t* input, qmlp_tensor_t* output, qmlp_stream_t stream,
+                                       void* tmp_memory, size_t tmp_bytes)
+{
     QMLP_TRY
     Network& n = *net->impl;
     std::lock_guard<std::mutex> lock(n.mutex);
-    inferenceLocked(n, input, output, stream);
+    if ((reinterpret_cast<uintptr_t>(tmp_memory) & 255) != 0) throw std::runtime_error("scratch memory must be 256-byte aligned");
+    inferenceLocked(n, input, output, stream, tmp_memory, tmp_bytes);
     QMLP_CATCH
 }
 

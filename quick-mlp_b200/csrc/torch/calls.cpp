@@ -31,7 +31,7 @@ using OptTensor = std::optional<Tensor>;
 // ---- the C ABI -------------------------------------------------------------------------------------------------------
 #define QMLP_CALLS(X)                                                                                                     \
     X(last_error) X(network_num_encodings) X(network_channels_in) X(network_channels_out) X(network_encoding)             \
-    X(network_destroy) X(network_set_parameter) X(network_inference) X(network_inference_host) X(network_forward_memory)  \
+    X(network_destroy) X(network_set_parameter) X(network_inference_memory) X(network_inference_with_memory) X(network_inference_host) X(network_forward_memory)  \
     X(network_forward) X(network_adjoint_memory) X(network_adjoint) X(network_parameter_count) X(encoding_create)         \
     X(encoding_num_output_channels) X(encoding_has_parameters) X(encoding_set_parameter) X(encoding_forward)              \
     X(encoding_adjoint_memory) X(encoding_adjoint_with_memory) X(activation_create) X(activation_forward) X(activation_adjoint) X(trainer_workspace_bytes)       \
@@ -171,7 +171,10 @@ Tensor networkInference(const NetworkCalls_ptr& self, const Tensor& input, const
     const Tensor half = toHalf(parameters);
     std::lock_guard<std::mutex> lock(self->mutex);
     self->bind(half, encodingParameters);
-    check(api.network_inference(self->handle, &in, &out, currentStream()));
+    size_t bytes = 0;   // feature planes of large grid batches
+    check(api.network_inference_memory(self->handle, input.size(0), &bytes));
+    const Tensor tmp = bytes > 0 ? at::empty({static_cast<int64_t>(bytes)}, floatLike(input).dtype(torch::kUInt8)) : Tensor();
+    check(api.network_inference_with_memory(self->handle, &in, &out, currentStream(), bytes > 0 ? tmp.data_ptr() : nullptr, bytes));
     return output;
 }
 
