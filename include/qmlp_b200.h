@@ -188,6 +188,18 @@ QMLP_API int qmlp_network_adjoint_memory(qmlp_network_t* net, int64_t num_elemen
 QMLP_API int qmlp_network_adjoint(qmlp_network_t* net, const qmlp_tensor_t* input, const qmlp_tensor_t* adj_output,
                                   int adjoint_flags, qmlp_tensor_t* adj_input, const void* tmp_forward,
                                   void* tmp_adjoint, qmlp_stream_t stream);
+/* Forward and adjoint that keep the encoded features only (not the pre-activations) and compute the layers a second time on
+ * the tensor core in the backward pass. qmlp_network_recompute_memory: bytes of the two scratch memories, with the
+ * parameters bound as for the call; forward_bytes is 0 where the pair does not apply (weight gradients not wanted, position
+ * gradients of a grid wanted, widths the kernel has no room for, line integration). Arguments otherwise as for
+ * qmlp_network_forward / qmlp_network_adjoint, with the same flags in both calls. */
+QMLP_API int qmlp_network_recompute_memory(qmlp_network_t* net, int64_t num_elements, int adjoint_flags, size_t* forward_bytes,
+                                           size_t* adjoint_bytes);
+QMLP_API int qmlp_network_forward_recompute(qmlp_network_t* net, const qmlp_tensor_t* input, qmlp_tensor_t* output, void* tmp_memory,
+                                            qmlp_stream_t stream);
+QMLP_API int qmlp_network_adjoint_recompute(qmlp_network_t* net, const qmlp_tensor_t* input, const qmlp_tensor_t* adj_output,
+                                            int adjoint_flags, qmlp_tensor_t* adj_input, const void* tmp_forward, void* tmp_adjoint,
+                                            qmlp_stream_t stream);
 /* FusedNetwork::clearCachedKernels, src_cpp/src/fused_network.cpp:1147-1153 */
 QMLP_API int qmlp_network_clear_cached_kernels(qmlp_network_t* net);
 /* Replaces the lazy compile*Kernel calls (src_cpp/src/fused_network.cpp:392-505, 553-672, 746-995): instantiate the

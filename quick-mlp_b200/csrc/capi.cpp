@@ -743,6 +743,103 @@ int qmlp_network_adjoint(qmlp_network_t* net, const qmlp_tensor_t* input, const 
     QMLP_CATCH
 }
 
+// Forward and backward with the layers computed a second time (kernels/fused_train_tc.cuh): which calls can take them
+static bool recomputes(Network& n, int64_t points, int flags)
+{
+    bool grid = false, line = false;
+    for (int i = 0; i < n.numEncodings(); ++i) {
+        grid = grid || n.encoding(i)->hasParameters();
+        line = line || n.encoding(i)->isLine();
+    }
+    const Library& lib = Library::instance();
+    // (the weight gradients come with the pass; the position gradient of a grid has no pass of its own)
+    if (points <= 0 || line || !(flags & QMLP_GRADIENTS_NETWORK_WEIGHTS) || ((flags & QMLP_GRADIENTS_INPUT) && grid) || lib.kernelPath == 1 ||
+        lib.boundsCheck || lib.splitScatter == 0)
+        return false;
+    if (n.recomputeKernel < 0) {
+        kernel::LaunchArgs none;
+        std::memset(&none, 0, sizeof none);
+        n.recomputeKernel = n.module(n.currentHalfMask())->launch(kernel::KERNEL_BACKWARD_FEATURES, &none, nullptr, nullptr) == 0 ? 1 : 0;
+    }
+    return n.recomputeKernel == 1;
+}
+
+int qmlp_network_recompute_memory(qmlp_network_t* net, int64_t num_elements, int adjoint_flags, size_t* forward_bytes, size_t* adjoint_bytes)
+{
+    QMLP_TRY
+    if (!forward_bytes || !adjoint_bytes) throw std::runtime_error("null argument");
+    Network& n = *net->impl;
+    std::lock_guard<std::mutex> lock(n.mutex);
+    *forward_bytes = *adjoint_bytes = 0;
+    if (!recomputes(n, num_elements, adjoint_flags)) return QMLP_OK;
+    const int64_t n32 = (num_elements + 31) / 32 * 32;
+    *forward_bytes = static_cast<size_t>(n32) * n.layer(0).channelsIn * 2;
+    const size_t planes = adjointPlaneBytes(n, n32, adjoint_flags);
+    *adjoint_bytes = planes ? align256(planes) + replicaBytes(n, num_elements) : 0;
+    QMLP_CATCH
+}
+
+int qmlp_network_forward_recompute(qmlp_network_t* net, const qmlp_tensor_t* input, qmlp_tensor_t* output, void* tmp_memory, qmlp_stream_t stream)
+{
+    QMLP_TRY
+    Network& n = *net->impl;
+    std::lock_guard<std::mutex> lock(n.mutex);
+    checkIO(n, input, output, "output");
+    if (!tmp_memory && input->sizes[0] > 0) throw std::runtime_error("tmpMemory is null");
+    if ((reinterpret_cast<uintptr_t>(tmp_memory) & 15) != 0) throw std::runtime_error("tmpMemory must be 16-byte aligned");
+    kernel::LaunchArgs a;
+    fillCommon(n, a, input);
+    a.output = static_cast<float*>(output->data);
+    a.outS0 = output->strides[0];
+    a.outS1 = output->strides[1];
+    a.fwdTmp = static_cast<__half*>(tmp_memory);
+    launchNet(n, kernel::KERNEL_FORWARD_FEATURES, a, stream);
+    QMLP_CATCH
+}
+
+int qmlp_network_adjoint_recompute(qmlp_network_t* net, const qmlp_tensor_t* input, const qmlp_tensor_t* adj_output, int adjoint_flags,
+                                   qmlp_tensor_t* adj_input, const void* tmp_forward, void* tmp_adjoint, qmlp_stream_t stream)
+{
+    QMLP_TRY
+    Network& n = *net->impl;
+    std::lock_guard<std::mutex> lock(n.mutex);
+    checkIO(n, input, adj_output, "adjOutput");
+    const int64_t numel = input->sizes[0];
+    if (numel == 0) return QMLP_OK;
+    if (!recomputes(n, numel, adjoint_flags)) throw std::runtime_error("this call has no recomputing backward pass (qmlp_network_recompute_memory returns 0)");
+    if (!n.paramGradients.defined()) throw std::runtime_error("Weight gradients requested, but no gradient tensor is bound (setNetworkParameter(..., GRADIENTS))");
+    if (!tmp_forward) throw std::runtime_error("tmpMemoryForward is null: run forward() first");
+    kernel::LaunchArgs a;
+    fillCommon(n, a, input);
+    a.adjOutput = static_cast<const float*>(adj_output->data);
+    a.aoS0 = adj_output->strides[0];
+    a.aoS1 = adj_output->strides[1];
+    if (adjoint_flags & QMLP_GRADIENTS_INPUT) {
+        if (adj_input == nullptr || adj_input->ndim <= 0 || adj_input->data == nullptr)
+            throw std::runtime_error("Input gradients requested, but adjInput is undefined");
+        checkDim(adj_input, 2, "adjInput");
+        checkSize(adj_input, 1, n.channelsIn(), "adjInput");
+        checkSize(adj_input, 0, numel, "adjInput");
+        checkDtype(adj_input, QMLP_FLOAT, "adjInput");
+        a.adjInput = static_cast<float*>(adj_input->data);
+        a.aiS0 = adj_input->strides[0];
+        a.aiS1 = adj_input->strides[1];
+    }
+    a.fwdTmp = const_cast<__half*>(static_cast<const __half*>(tmp_forward));
+    const int64_t n32 = (numel + 31) / 32 * 32;
+    const size_t planeBytes = adjointPlaneBytes(n, n32, adjoint_flags);
+    if (planeBytes > 0) {
+        if (!tmp_adjoint || (reinterpret_cast<uintptr_t>(tmp_adjoint) & 15) != 0) throw std::runtime_error("tmpMemoryAdjoint is null or not 16-byte aligned");
+        a.planes = static_cast<__half*>(tmp_adjoint);
+        a.planeStride = n32;
+        bindReplicas(n, a, static_cast<unsigned char*>(tmp_adjoint) + align256(planeBytes));
+    }
+    a.flags = kernel::FLAG_GRAD_WEIGHTS | (planeBytes > 0 ? kernel::FLAG_GRAD_ENCODINGS | kernel::FLAG_SPLIT_SCATTER : 0);
+    launchNet(n, kernel::KERNEL_BACKWARD_FEATURES, a, stream);
+    if (planeBytes > 0) launchNet(n, kernel::KERNEL_SCATTER_PLANES, a, stream);
+    QMLP_CATCH
+}
+
 // ---- encodings -----------------------------------------------------------------------------------------------------
 int qmlp_encoding_create(const char* cfg_json, qmlp_encoding_t** out)
 {

@@ -265,6 +265,7 @@ public:
     int64_t planeCapacity = 0;        // points per chunk
     bool planesUnsupported = false;   // the spec has no instantiation of the plane kernels
     int trainKernel = -1;             // KERNEL_TRAIN is instantiated for the spec: 1 yes, 0 no, -1 not asked yet
+    int recomputeKernel = -1;         // the same for KERNEL_BACKWARD_FEATURES
     bool sortUnsupported = false;     // the spec has no instantiation of the point sort
     HostPipeline hostPipeline;
     int ownedDevice = -1;             // device the library-owned buffers above live on (-1: none allocated yet)

@@ -449,7 +449,8 @@ __device__ __forceinline__ void read_planes_point(const LaunchArgs& p, long long
 }
 
 // ---- forward layer chain -------------------------------------------------------------------------------------
-// MODE 0: inference, 1: forward with stash, 2: forward with stash + L2 loss gradient instead of the output
+// MODE 0: inference, 1: forward with stash, 2: forward with stash + L2 loss gradient instead of the output, 3: forward that
+// stashes the encoded input only
 template <class Spec, int L, int MODE>
 __device__ __forceinline__ void forward_layers(const LaunchArgs& p, const __half* sW, const __half* sB,
                                                uint32_t (&aIn)[MT][Spec::CIN[L] / 16][4], long long rowBase, long long n32,
@@ -507,7 +508,7 @@ __device__ __forceinline__ void forward_layers(const LaunchArgs& p, const __half
                 }
             }
             const long long row0 = rowBase + m * 16 + r;
-            if constexpr (MODE >= 1) {
+            if constexpr (MODE == 1 || MODE == 2) {
                 // pre-activation stash (N32, COUT) per layer (reference: kernels/layer.cuh:156-163) in 8 x 8 blocks
                 // (stash_block): a register of the warp is one 128-byte line
                 __half* st = p.fwdTmp + n32 * SL::preOffset(L) + (r * 8 + q * 2);
@@ -1221,7 +1222,7 @@ struct PerDevice {
 };
 
 template <class Spec> struct TcLaunchers;
-template <class Spec> struct TrainLayout;  // fused_train_tc.cuh
+template <class Spec, bool LOSS> struct TrainLayout;  // fused_train_tc.cuh
 template <class Spec> struct TrainLaunchers;
 template <class Spec> struct TsLayout;     // fused_forward_ts.cuh
 template <class Spec> struct TsLaunchers;
@@ -1368,7 +1369,13 @@ struct NetworkLaunchers {
         case KERNEL_WGRAD: e = wgrad(a, s); break;
         case KERNEL_SCATTER_PLANES: e = PlaneLaunchers<Spec>::scatter(a, s, &n); break;
         case KERNEL_TRAIN:
-            if constexpr (TrainLayout<Spec>::eligible()) e = TrainLaunchers<Spec>::run(a, s);
+            if constexpr (TrainLayout<Spec, true>::eligible()) e = TrainLaunchers<Spec>::template run<true>(a, s);
+            else e = cudaErrorNotSupported;
+            if (a.numel == 0) n = 0;
+            break;
+        case KERNEL_FORWARD_FEATURES: e = forward<3>(a, s); break;
+        case KERNEL_BACKWARD_FEATURES:
+            if constexpr (TrainLayout<Spec, false>::eligible()) e = TrainLaunchers<Spec>::template run<false>(a, s);
             else e = cudaErrorNotSupported;
             if (a.numel == 0) n = 0;
             break;

@@ -35,6 +35,10 @@
 // issue, MMAs, commit, accumulator load) takes about a thousand clocks that one other slot cannot cover.
 // Every wait is bounded; on a timeout the CTA runs through without waiting and the status word is set.
 //
+// The second instantiation (LOSS false) is the backward pass of a forward call that stashed the encoded features only: the layers
+// are computed a second time on the tensor core instead of being written by the forward kernel and read twice. 32 -> 64 -> 64 -> 1
+// on 2^18 points: forward 104 -> 93 us, backward and weight gradients 71 -> 42 us.
+//
 // Same roundings as the separate kernels: fp16 activations, deltas and pre-activations (bias added in half), fp32 sums.
 #pragma once
 #include "fused_forward_tc.cuh"
@@ -45,11 +49,13 @@ namespace kernel {
 constexpr int TRAIN_WARPGROUPS = 4, TRAIN_THREADS = TRAIN_WARPGROUPS * 128 + 32;   // the last warp issues the weight gradients
 constexpr int TRAIN_BLOCK = TC_TILE * 128;   // bytes of a block: 128 points x 64 channels
 
-template <class Spec>
+// LOSS: the training step's kernel (features from the planes, L2 loss against targets); else the backward pass of an earlier
+// forward call (features from its stash, the adjoint of the output from the caller)
+template <class Spec, bool LOSS = true>
 struct TrainLayout {
     using TL = TcLayout<Spec>;
     static constexpr int NL = Spec::NUM_LAYERS;
-    static constexpr bool GRID = table_rows_per_point<Spec>() > 0;   // the adjoint of the features is wanted
+    static constexpr bool FEATURE_ADJOINT = !LOSS || table_rows_per_point<Spec>() > 0;   // the adjoint of the features is wanted
     __host__ __device__ static constexpr int blocks(int channels) { return (channels + 63) / 64; }
     __host__ __device__ static constexpr bool bias(int l) { return Spec::BOFF[l] >= 0; }
     // buffer l < NL: input of layer l (later delta of layer l - 1); buffer NL: delta of the last layer. A narrow last delta
@@ -91,7 +97,7 @@ struct TrainLayout {
     __host__ __device__ static constexpr int keptCols()
     {
         int m = Spec::COUT[NL - 1];
-        for (int i = GRID ? 0 : 1; i < NL; ++i) m = Spec::CIN[i] > m ? Spec::CIN[i] : m;
+        for (int i = FEATURE_ADJOINT ? 0 : 1; i < NL; ++i) m = Spec::CIN[i] > m ? Spec::CIN[i] : m;
         return dBefore(NL - 1) + m;
     }
     __host__ __device__ static constexpr int slotStart() { return TL::weightBytes(); }
@@ -258,7 +264,8 @@ __device__ __forceinline__ void fetch_piece(const LaunchArgs& p, long long point
         }
     }
 }
-// adjoints of channels [C, END) -> planes of the grids
+// adjoints of channels [C, END) -> planes of the grids (if any), gradient of the input for identity encodings (if wanted; an
+// input channel may feed several encodings)
 template <class Spec, int C, int END>
 __device__ __forceinline__ void store_piece(const LaunchArgs& p, long long point, const uint32_t (&v)[4])
 {
@@ -267,10 +274,15 @@ __device__ __forceinline__ void store_piece(const LaunchArgs& p, long long point
         constexpr int j = C % 8;
         if constexpr (E >= 0) {
             using Enc = typename Spec::template Enc<E>;
-            if constexpr (Enc::IS_GRID) {
+            if constexpr (!Enc::IS_GRID) {
+                if (p.adjInput != nullptr)
+                    red_add_f32(p.adjInput + point * p.aiS0 + (C - Enc::OUT_OFF + Enc::START) * p.aiS1,
+                                __half2float(__ushort_as_half(static_cast<unsigned short>(j % 2 == 0 ? v[j / 2] & 0xffffu : v[j / 2] >> 16))));
+            } else {
                 constexpr int F = Enc::F, i = (C - Enc::OUT_OFF) % F, W = plane_vector<Enc, C>();
                 __half* at = p.planes + p.planeStride * (C - i) + point * F + i;
-                if constexpr (W == 8) *reinterpret_cast<uint4*>(at) = make_uint4(v[0], v[1], v[2], v[3]);
+                if (p.planes == nullptr) {}
+                else if constexpr (W == 8) *reinterpret_cast<uint4*>(at) = make_uint4(v[0], v[1], v[2], v[3]);
                 else if constexpr (W == 4) *reinterpret_cast<uint2*>(at) = make_uint2(v[j / 2], v[j / 2 + 1]);
                 else if constexpr (W == 2) *reinterpret_cast<uint32_t*>(at) = v[j / 2];
                 else *at = __ushort_as_half(static_cast<unsigned short>(j % 2 == 0 ? v[j / 2] & 0xffffu : v[j / 2] >> 16));
@@ -283,10 +295,10 @@ __device__ __forceinline__ void store_piece(const LaunchArgs& p, long long point
 }
 
 // ---- MMAs (issued by one elected lane of a whole warp) --------------------------------------------------------------------------------------------
-template <class Spec, int SLOTS>
+template <class Spec, bool LOSS, int SLOTS>
 struct TrainIssue {
     using TL = TcLayout<Spec>;
-    using TR = TrainLayout<Spec>;
+    using TR = TrainLayout<Spec, LOSS>;
     // outputs [FIRST, FIRST + N) of layer L = input * W^T, to column `dTmem`
     template <int L, int FIRST, int N>
     static __device__ __forceinline__ void forward(uint32_t lead, uint32_t smem, uint32_t slotSmem, uint32_t dTmem)
@@ -348,7 +360,7 @@ struct TrainIssue {
             if constexpr (TR::RECOMPUTE) forward<L, FIRST, N>(lead, smem, slotSmem, slotTmem);
             adjoint<L + 1, FIRST, N>(lead, smem, slotSmem, slotTmem + TR::adjCol());
             umma_commit_elected(lead, bars);
-        } else if constexpr (TR::GRID) {
+        } else if constexpr (TR::FEATURE_ADJOINT) {
             adjoint<0, 0, Spec::CIN[0]>(lead, smem, slotSmem, slotTmem + TR::featureAdjCol());
             umma_commit_elected(lead, bars);
         }
@@ -379,9 +391,9 @@ struct TrainIssue {
 };
 
 // ---- one tile slot, per thread --------------------------------------------------------------------------------------------
-template <class Spec>
+template <class Spec, bool LOSS>
 struct TrainSlot {
-    static constexpr int WG = TRAIN_WARPGROUPS / TrainLayout<Spec>::SLOTS;          // warpgroups of a slot
+    static constexpr int WG = TRAIN_WARPGROUPS / TrainLayout<Spec, LOSS>::SLOTS;          // warpgroups of a slot
     static constexpr int PIECES = (Spec::CIN[0] / 8 + WG - 1) / WG;                 // 8-channel pieces of the input this thread writes
     static constexpr int TARGETS = Spec::NUM_OUTPUTS <= 4 ? Spec::NUM_OUTPUTS : 0;  // prefetched by the warpgroup that takes the loss
     uint32_t row;          // shared address of this thread's row in buffer 0
@@ -396,35 +408,42 @@ struct TrainSlot {
     float target[TARGETS > 0 ? TARGETS : 1];
 };
 
-template <class Spec, int K>
-__device__ __forceinline__ void train_fetch(const LaunchArgs& p, TrainSlot<Spec>& sl, int wg, long long point)
+template <class Spec, bool LOSS, int K>
+__device__ __forceinline__ void train_fetch(const LaunchArgs& p, TrainSlot<Spec, LOSS>& sl, int wg, long long point)
 {
-    constexpr int WG = TrainSlot<Spec>::WG;
-    if constexpr (K < TrainSlot<Spec>::PIECES * WG) {
+    constexpr int WG = TrainSlot<Spec, LOSS>::WG;
+    if constexpr (K < TrainSlot<Spec, LOSS>::PIECES * WG) {
         if (wg == K % WG) {
             uint32_t (&v)[4] = sl.features[K / WG];
             if constexpr (K * 8 < Spec::CIN[0]) {
-                if (point < p.numel) fetch_piece<Spec, K * 8, K * 8 + 8>(p, point, v);
+                if (point < p.numel) {
+                    if constexpr (LOSS) {
+                        fetch_piece<Spec, K * 8, K * 8 + 8>(p, point, v);
+                    } else {
+                        const uint4 u = *reinterpret_cast<const uint4*>(p.fwdTmp + point * Spec::CIN[0] + K * 8);
+                        v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w;
+                    }
+                }
                 else v[0] = v[1] = v[2] = v[3] = 0u;
             }
         }
-        train_fetch<Spec, K + 1>(p, sl, wg, point);
+        train_fetch<Spec, LOSS, K + 1>(p, sl, wg, point);
     }
 }
-template <class Spec, int K>
-__device__ __forceinline__ void train_store_adjoint(const LaunchArgs& p, const TrainSlot<Spec>& sl, int wg)
+template <class Spec, bool LOSS, int K>
+__device__ __forceinline__ void train_store_adjoint(const LaunchArgs& p, const TrainSlot<Spec, LOSS>& sl, int wg)
 {
     if constexpr (K * 8 < Spec::CIN[0]) {
-        if (wg == K % TrainSlot<Spec>::WG) {
+        if (wg == K % TrainSlot<Spec, LOSS>::WG) {
             float x[8];
-            tmem_ld8(sl.tmem + TrainLayout<Spec>::featureAdjCol() + K * 8, x);
+            tmem_ld8(sl.tmem + TrainLayout<Spec, LOSS>::featureAdjCol() + K * 8, x);
             tmem_wait_ld();
             uint32_t v[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) v[i] = h2_as_u32(__floats2half2_rn(x[2 * i], x[2 * i + 1]));
             if (sl.valid) store_piece<Spec, K * 8, K * 8 + 8>(p, sl.point, v);
         }
-        train_store_adjoint<Spec, K + 1>(p, sl, wg);
+        train_store_adjoint<Spec, LOSS, K + 1>(p, sl, wg);
     }
 }
 
@@ -450,30 +469,31 @@ __device__ __forceinline__ void train_put(uint32_t rowAddr, int row, int col, co
 
 // One stage of a slot's tile (TrainLayout::lastStage). Every stage but the last is followed by the MMAs of the next one: the
 // warps count their arrivals, and the last one issues.
-template <class Spec, int ST>
-__device__ __forceinline__ void train_stage(const LaunchArgs& p, TrainSlot<Spec>& sl, const __half* bias, int wg, int row, long long nextPoint,
+template <class Spec, bool LOSS, int ST>
+__device__ __forceinline__ void train_stage(const LaunchArgs& p, TrainSlot<Spec, LOSS>& sl, const __half* bias, int wg, int row, long long nextPoint,
                                             float& lossAcc, volatile int* abortFlag, bool& dead)
 {
-    using TR = TrainLayout<Spec>;
-    constexpr int NL = Spec::NUM_LAYERS, WG = TrainSlot<Spec>::WG;
+    using TR = TrainLayout<Spec, LOSS>;
+    constexpr int NL = Spec::NUM_LAYERS, WG = TrainSlot<Spec, LOSS>::WG;
     if constexpr (ST == 0) {
         constexpr int CIN0 = Spec::CIN[0];
 #pragma unroll
-        for (int k = 0; k < TrainSlot<Spec>::PIECES; ++k) {
+        for (int k = 0; k < TrainSlot<Spec, LOSS>::PIECES; ++k) {
             const int piece = wg + k * WG;
             if (piece * 8 < CIN0) {
                 const uint32_t(&v)[4] = sl.features[k];
                 sts128(sl.row + sw128_row_offset(row, piece), v[0], v[1], v[2], v[3]);
             }
         }
-        if constexpr (TrainSlot<Spec>::TARGETS > 0) {
+        if constexpr (TrainSlot<Spec, LOSS>::TARGETS > 0) {
             if (wg == 0 && sl.valid) {
 #pragma unroll
-                for (int c = 0; c < Spec::NUM_OUTPUTS; ++c) sl.target[c] = __ldg(p.target + sl.point * p.tS0 + c * p.tS1);
+                for (int c = 0; c < Spec::NUM_OUTPUTS; ++c)
+                    sl.target[c] = LOSS ? __ldg(p.target + sl.point * p.tS0 + c * p.tS1) : __ldg(p.adjOutput + sl.point * p.aoS0 + c * p.aoS1);
             }
         }
     } else {
-        if constexpr (ST < TR::lastStage() || TR::GRID) {
+        if constexpr (ST < TR::lastStage() || TR::FEATURE_ADJOINT) {
             train_wait(sl.bars, sl.full, abortFlag, dead);
             sl.full ^= 1u;
         }
@@ -520,11 +540,15 @@ __device__ __forceinline__ void train_stage(const LaunchArgs& p, TrainSlot<Spec>
                             const int c = col + 2 * i + e;
                             if (c < Spec::NUM_OUTPUTS) {
                                 float t;
-                                if constexpr (TrainSlot<Spec>::TARGETS > 0) t = sl.target[(2 * i + e) % TrainSlot<Spec>::TARGETS];   // (here col == 0)
-                                else t = __ldg(p.target + sl.point * p.tS0 + c * p.tS1);
-                                const float d = o[e] - t;
-                                lossAcc += d * d;
-                                adj[e] = p.lossScale * d;
+                                if constexpr (TrainSlot<Spec, LOSS>::TARGETS > 0) t = sl.target[(2 * i + e) % TrainSlot<Spec, LOSS>::TARGETS];   // (here col == 0)
+                                else t = LOSS ? __ldg(p.target + sl.point * p.tS0 + c * p.tS1) : __ldg(p.adjOutput + sl.point * p.aoS0 + c * p.aoS1);
+                                if constexpr (LOSS) {
+                                    const float d = o[e] - t;
+                                    lossAcc += d * d;
+                                    adj[e] = p.lossScale * d;
+                                } else {
+                                    adj[e] = t;
+                                }
                             }
                         }
                     }
@@ -534,7 +558,7 @@ __device__ __forceinline__ void train_stage(const LaunchArgs& p, TrainSlot<Spec>
                 train_put<TR::SHARED_LAST ? 4 : 0>(sl.row + TR::bufOffset(TR::SHARED_LAST ? NL - 1 : NL), row, col, w);
             }
             // the next tile of this slot: its features are fetched under the backward pass
-            train_fetch<Spec, 0>(p, sl, wg, nextPoint);
+            train_fetch<Spec, LOSS, 0>(p, sl, wg, nextPoint);
         } else if constexpr (ST < TR::lastStage()) {
             // outputs [FIRST, FIRST + N) of the delta of layer L from the adjoint of layer L + 1's input
             constexpr int L = TR::stepLayer(ST), H = TR::stepIndex(ST), FIRST = 64 * H, LEFT = Spec::COUT[L] - FIRST,
@@ -564,13 +588,13 @@ __device__ __forceinline__ void train_stage(const LaunchArgs& p, TrainSlot<Spec>
             if (!graded) train_wait(sl.bars + 8, sl.graded, abortFlag, dead);       // (no columns here: stay in step with the barrier)
             if constexpr (H == 0) sl.graded ^= 1u;
         } else {
-            if constexpr (TR::GRID) train_store_adjoint<Spec, 0>(p, sl, wg);
+            if constexpr (TR::FEATURE_ADJOINT) train_store_adjoint<Spec, LOSS, 0>(p, sl, wg);
             train_wait(sl.bars + 8, sl.graded, abortFlag, dead);   // buffer 0 is written next
             sl.graded ^= 1u;
         }
     }
     if constexpr (ST < TR::lastStage()) {
-        using Issue = TrainIssue<Spec, TR::SLOTS>;
+        using Issue = TrainIssue<Spec, LOSS, TR::SLOTS>;
         tc_fence_before();
         fence_proxy_async();   // generic-proxy writes of the operands become visible to the tensor core
         __syncwarp();
@@ -587,22 +611,22 @@ __device__ __forceinline__ void train_stage(const LaunchArgs& p, TrainSlot<Spec>
     }
 }
 
-template <class Spec, int ST>
-__device__ __forceinline__ void train_stages(const LaunchArgs& p, TrainSlot<Spec>& sl, const __half* bias, int wg, int row, long long nextPoint, float& lossAcc,
+template <class Spec, bool LOSS, int ST>
+__device__ __forceinline__ void train_stages(const LaunchArgs& p, TrainSlot<Spec, LOSS>& sl, const __half* bias, int wg, int row, long long nextPoint, float& lossAcc,
                                              volatile int* abortFlag, bool& dead)
 {
-    if constexpr (ST <= TrainLayout<Spec>::lastStage()) {
-        train_stage<Spec, ST>(p, sl, bias, wg, row, nextPoint, lossAcc, abortFlag, dead);
-        train_stages<Spec, ST + 1>(p, sl, bias, wg, row, nextPoint, lossAcc, abortFlag, dead);
+    if constexpr (ST <= TrainLayout<Spec, LOSS>::lastStage()) {
+        train_stage<Spec, LOSS, ST>(p, sl, bias, wg, row, nextPoint, lossAcc, abortFlag, dead);
+        train_stages<Spec, LOSS, ST + 1>(p, sl, bias, wg, row, nextPoint, lossAcc, abortFlag, dead);
     }
 }
 
 // The weight-gradient warp: whenever a slot's delta is complete, the MMAs of that layer's gradient. All slots add to the same
 // accumulators, so one thread issues them; nobody waits for them before the slot's next stage has computed its results.
-template <class Spec, int SLOTS>
+template <class Spec, bool LOSS, int SLOTS>
 __device__ __forceinline__ void train_gradients(uint32_t lead, uint32_t smem, uint32_t tmemBase, uint32_t bars, int myTiles, volatile int* abortFlag, bool& dead)
 {
-    using TR = TrainLayout<Spec>;
+    using TR = TrainLayout<Spec, LOSS>;
     constexpr int NL = Spec::NUM_LAYERS;
     int layer[SLOTS], left[SLOTS], open = 0;
     uint32_t parity = 0, started = 0, idle = 0;
@@ -621,7 +645,7 @@ __device__ __forceinline__ void train_gradients(uint32_t lead, uint32_t smem, ui
             // (opaque copies: the descriptors of all MMAs would be computed ahead of the loop and spilled)
             uint32_t base = smem, tmem = tmemBase;
             asm volatile("" : "+r"(base), "+r"(tmem));
-            TrainIssue<Spec, SLOTS>::template weights<0>(lead, layer[j], base, base + TR::slotStart() + j * TR::slotBytes(), tmem + SLOTS * TR::slotCols(), started,
+            TrainIssue<Spec, LOSS, SLOTS>::template weights<0>(lead, layer[j], base, base + TR::slotStart() + j * TR::slotBytes(), tmem + SLOTS * TR::slotCols(), started,
                                                          bars + j * 24);
             parity ^= 1u << j;
             layer[j] = layer[j] == 0 ? NL - 1 : layer[j] - 1;
@@ -637,11 +661,11 @@ __device__ __forceinline__ void train_gradients(uint32_t lead, uint32_t smem, ui
 }
 
 // weight-gradient accumulators of this CTA -> fp32 gradient vector
-template <class Spec, int L>
+template <class Spec, bool LOSS, int L>
 __device__ __forceinline__ void train_flush(const LaunchArgs& p, uint32_t wgTmem, int warpgroup, int lane)
 {
     if constexpr (L < Spec::NUM_LAYERS) {
-        using TR = TrainLayout<Spec>;
+        using TR = TrainLayout<Spec, LOSS>;
         constexpr int CIN = Spec::CIN[L], COUT = Spec::COUT[L];
         constexpr bool OUT = TR::mIsOut(L), BIAS = TR::bias(L);
         constexpr int CHUNKS = TR::wgCols(L) / 16;
@@ -675,16 +699,16 @@ __device__ __forceinline__ void train_flush(const LaunchArgs& p, uint32_t wgTmem
                 }
             }
         }
-        train_flush<Spec, L + 1>(p, wgTmem, warpgroup, lane);
+        train_flush<Spec, LOSS, L + 1>(p, wgTmem, warpgroup, lane);
     }
 }
 
 // biases of all layers -> shared memory (whole CTA), or the channel of ones of every input buffer (one warpgroup)
-template <class Spec, int L, int SLOTS, bool ONES>
+template <class Spec, bool LOSS, int L, int SLOTS, bool ONES>
 __device__ __forceinline__ void train_init(const LaunchArgs& p, uint32_t smemBase, __half* sBias, int row)
 {
     if constexpr (L < Spec::NUM_LAYERS) {
-        using TR = TrainLayout<Spec>;
+        using TR = TrainLayout<Spec, LOSS>;
         constexpr int CIN = Spec::CIN[L], COUT = Spec::COUT[L];
         if constexpr (!ONES) {
             if constexpr (Spec::BOFF[L] >= 0)
@@ -694,16 +718,16 @@ __device__ __forceinline__ void train_init(const LaunchArgs& p, uint32_t smemBas
             for (int s = 0; s < SLOTS; ++s)
                 sts16(smemBase + TR::slotStart() + s * TR::slotBytes() + TR::bufOffset(L) + row * 128 + sw128_row_offset(row, CIN / 8), __ushort_as_half(0x3C00));
         }
-        train_init<Spec, L + 1, SLOTS, ONES>(p, smemBase, sBias, row);
+        train_init<Spec, LOSS, L + 1, SLOTS, ONES>(p, smemBase, sBias, row);
     }
 }
 
-template <class Spec, int SLOTS>
+template <class Spec, bool LOSS, int SLOTS>
 __global__ void __launch_bounds__(TRAIN_THREADS, 1)
 fused_train_tc_kernel(const __grid_constant__ LaunchArgs p, const __grid_constant__ TcWeightMaps<Spec> weightMaps)
 {
     using TL = TcLayout<Spec>;
-    using TR = TrainLayout<Spec>;
+    using TR = TrainLayout<Spec, LOSS>;
     extern __shared__ unsigned char smemRaw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~static_cast<uintptr_t>(1023));
     __half* sBias = reinterpret_cast<__half*>(smem + TR::biasStart(SLOTS));
@@ -736,11 +760,11 @@ fused_train_tc_kernel(const __grid_constant__ LaunchArgs p, const __grid_constan
     // channel of the input (stages write the channels before it only), in the last block channel 0.
     for (int i = threadIdx.x; i < (TR::onesStart(SLOTS) + TRAIN_BLOCK - TR::slotStart()) / 16; i += TRAIN_THREADS)
         reinterpret_cast<uint4*>(smem + TR::slotStart())[i] = make_uint4(0, 0, 0, 0);
-    train_init<Spec, 0, SLOTS, false>(p, smemBase, sBias, row);
+    train_init<Spec, LOSS, 0, SLOTS, false>(p, smemBase, sBias, row);
     __syncthreads();
     if (warpgroup == 0) {
         sts16(smemBase + TR::onesStart(SLOTS) + row * 128 + sw128_row_offset(row, 0), __ushort_as_half(0x3C00));
-        train_init<Spec, 0, SLOTS, true>(p, smemBase, sBias, row);
+        train_init<Spec, LOSS, 0, SLOTS, true>(p, smemBase, sBias, row);
     }
     if (warp == 0) {
         tmem_alloc(smem_u32(tmemSlot), 512);
@@ -762,12 +786,12 @@ fused_train_tc_kernel(const __grid_constant__ LaunchArgs p, const __grid_constan
     __syncwarp();
     if (warpgroup == TRAIN_WARPGROUPS) {
         const uint32_t smemU = __shfl_sync(0xffffffffu, smemBase, 0), tmemU = __shfl_sync(0xffffffffu, tmemBase, 0);
-        if (!__any_sync(0xffffffffu, dead)) train_gradients<Spec, SLOTS>(lead, smemU, tmemU, smemU + TR::barStart(SLOTS), myTiles, abortFlag, dead);
+        if (!__any_sync(0xffffffffu, dead)) train_gradients<Spec, LOSS, SLOTS>(lead, smemU, tmemU, smemU + TR::barStart(SLOTS), myTiles, abortFlag, dead);
     } else {
         // tile i of this CTA's sequence belongs to slot i % SLOTS
-        const int slot = warpgroup / TrainSlot<Spec>::WG, wg = warpgroup % TrainSlot<Spec>::WG;
+        const int slot = warpgroup / TrainSlot<Spec, LOSS>::WG, wg = warpgroup % TrainSlot<Spec, LOSS>::WG;
         auto pointOf = [&](int i) { return i < myTiles ? (blockIdx.x + static_cast<long long>(i) * stride) * TC_TILE + row : p.numel; };
-        TrainSlot<Spec> sl;
+        TrainSlot<Spec, LOSS> sl;
         sl.row = smemBase + TR::slotStart() + slot * TR::slotBytes() + row * 128;
         sl.tmem = tmemBase + slot * TR::slotCols() + laneField;
         sl.bars = smem_u32(bars + 3 * slot);
@@ -778,20 +802,20 @@ fused_train_tc_kernel(const __grid_constant__ LaunchArgs p, const __grid_constan
         sl.lead = lead;
         sl.full = sl.graded = 0;
         sl.point = pointOf(slot);
-        train_fetch<Spec, 0>(p, sl, wg, sl.point);
+        train_fetch<Spec, LOSS, 0>(p, sl, wg, sl.point);
         float lossAcc = 0.f;
         for (int i = slot; i < myTiles; i += SLOTS) {
             sl.valid = sl.point < p.numel;
             const long long next = pointOf(i + SLOTS);
-            train_stages<Spec, 0>(p, sl, sBias, wg, row, next, lossAcc, abortFlag, dead);
+            train_stages<Spec, LOSS, 0>(p, sl, sBias, wg, row, next, lossAcc, abortFlag, dead);
             sl.point = next;
         }
         tc_fence_before();
         asm volatile("bar.sync 1, %0;" ::"n"(TRAIN_WARPGROUPS * 128) : "memory");   // every slot's weight gradients are in
         if (myTiles > 0 && !__any_sync(0xffffffffu, *abortFlag != 0)) {
             tc_fence_after();
-            train_flush<Spec, 0>(p, wgTmem + laneField, warpgroup, row);
-            if (p.lossSum != nullptr) {
+            train_flush<Spec, LOSS, 0>(p, wgTmem + laneField, warpgroup, row);
+            if (LOSS && p.lossSum != nullptr) {
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) lossAcc += __shfl_xor_sync(0xffffffffu, lossAcc, o);
                 if ((threadIdx.x & 31) == 0 && lossAcc != 0.f) atomicAdd(p.lossSum, lossAcc);
@@ -816,13 +840,14 @@ fused_train_tc_kernel(const __grid_constant__ LaunchArgs p, const __grid_constan
 template <class Spec>
 struct TrainLaunchers {
     // a.numel == 0 asks whether the kernel exists for this network
+    template <bool LOSS>
     static cudaError_t run(const LaunchArgs& a, cudaStream_t s)
     {
-        using TR = TrainLayout<Spec>;
+        using TR = TrainLayout<Spec, LOSS>;
         constexpr int smem = TR::bytes(TR::SLOTS);
         if (a.numel == 0) return cudaSuccess;
         static DeviceOnce once;
-        auto k = fused_train_tc_kernel<Spec, TR::SLOTS>;
+        auto k = fused_train_tc_kernel<Spec, LOSS, TR::SLOTS>;
         const cudaError_t e = once.run([&] { return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); });
         if (e != cudaSuccess) return e;
         const TcWeightMaps<Spec>* maps = nullptr;

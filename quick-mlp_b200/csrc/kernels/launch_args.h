@@ -132,6 +132,8 @@ enum KernelId {
     KERNEL_FORWARD_LOSS_PLANES = 12, // KERNEL_FORWARD_LOSS with layer 0 fed from the planes of KERNEL_ENCODE_PLANES
     KERNEL_SORT_POINTS = 13,         // points (and targets) -> Morton-bin order: count, scan, reorder
     KERNEL_TRAIN = 14,               // layers of a training step on the planes: forward, loss, backward, weight gradients; adjoints back to the planes
+    KERNEL_FORWARD_FEATURES = 16,    // forward that stashes the encoded input only
+    KERNEL_BACKWARD_FEATURES = 17,   // its backward pass: layers computed again, weight gradients, adjoints to the planes / the input
     KERNEL_SCATTER_SORTED = 15       // KERNEL_SCATTER_PLANES for sorted points: coarse levels summed in shared memory first
 };
 

@@ -32,7 +32,7 @@ using OptTensor = std::optional<Tensor>;
 #define QMLP_CALLS(X)                                                                                                     \
     X(last_error) X(network_num_encodings) X(network_channels_in) X(network_channels_out) X(network_encoding)             \
     X(network_destroy) X(network_set_parameter) X(network_inference_memory) X(network_inference_with_memory) X(network_inference_host) X(network_forward_memory)  \
-    X(network_forward) X(network_adjoint_memory) X(network_adjoint) X(network_parameter_count) X(encoding_create)         \
+    X(network_forward) X(network_adjoint_memory) X(network_adjoint) X(network_recompute_memory) X(network_forward_recompute) X(network_adjoint_recompute) X(network_parameter_count) X(encoding_create)         \
     X(encoding_num_output_channels) X(encoding_has_parameters) X(encoding_set_parameter) X(encoding_forward)              \
     X(encoding_adjoint_memory) X(encoding_adjoint_with_memory) X(activation_create) X(activation_forward) X(activation_adjoint) X(trainer_workspace_bytes)       \
     X(trainer_gradients_part) X(trainer_update) X(convert_half)
@@ -202,16 +202,25 @@ struct NetworkFunction : torch::autograd::Function<NetworkFunction> {
     {
         const qmlp_tensor_t in = wrap(input);
         const Tensor half = toHalf(parameters);
-        size_t bytes = 0;
-        check(api.network_forward_memory(self->handle, input.size(0), static_cast<int>(flags), &bytes));
-        Tensor tmp = at::empty({static_cast<int64_t>(std::max<size_t>(bytes, 16))}, floatLike(input).dtype(torch::kUInt8));
         Tensor output = at::empty({input.size(0), self->channelsOut}, floatLike(input));
         qmlp_tensor_t out = wrap(output);
+        Tensor tmp;
+        size_t bytes = 0, adjointBytes = 0;
+        bool recompute;
         {
             std::lock_guard<std::mutex> lock(self->mutex);
             self->bind(half, bySlot(*self, slots, encodingList));
-            check(api.network_forward(self->handle, &in, &out, tmp.data_ptr(), currentStream()));
+            check(api.network_recompute_memory(self->handle, input.size(0), static_cast<int>(flags), &bytes, &adjointBytes));
+            recompute = bytes > 0;
+            if (!recompute) {
+                check(api.network_forward_memory(self->handle, input.size(0), static_cast<int>(flags), &bytes));
+                check(api.network_adjoint_memory(self->handle, input.size(0), static_cast<int>(flags), &adjointBytes));
+            }
+            tmp = at::empty({static_cast<int64_t>(std::max<size_t>(bytes, 16))}, floatLike(input).dtype(torch::kUInt8));
+            check((recompute ? api.network_forward_recompute : api.network_forward)(self->handle, &in, &out, tmp.data_ptr(), currentStream()));
         }
+        ctx->saved_data["recompute"] = recompute;
+        ctx->saved_data["adjoint_bytes"] = static_cast<int64_t>(adjointBytes);
         ctx->saved_data["self"] = c10::IValue::make_capsule(self);
         ctx->saved_data["flags"] = flags;
         ctx->saved_data["slots"] = slots;
@@ -234,9 +243,8 @@ struct NetworkFunction : torch::autograd::Function<NetworkFunction> {
         Tensor adjInput = (flags & QMLP_GRADIENTS_INPUT) ? zerosLike(input) : Tensor();
         Tensor adjParams = (flags & QMLP_GRADIENTS_NETWORK_WEIGHTS) ? zeros(half.sizes(), floatLike(half)) : Tensor();
         std::vector<Tensor> adjEncodings(slots.size());
-        size_t bytes = 0;
-        check(api.network_adjoint_memory(self->handle, input.size(0), flags, &bytes));
-        Tensor adjTmp = at::empty({static_cast<int64_t>(std::max<size_t>(bytes, 16))}, floatLike(input).dtype(torch::kUInt8));
+        const bool recompute = ctx->saved_data["recompute"].toBool();
+        Tensor adjTmp = at::empty({std::max<int64_t>(ctx->saved_data["adjoint_bytes"].toInt(), 16)}, floatLike(input).dtype(torch::kUInt8));
         {
             std::lock_guard<std::mutex> lock(self->mutex);
             self->bind(half, bySlot(*self, slots, at::ArrayRef<Tensor>(saved).slice(3)));
@@ -256,7 +264,8 @@ struct NetworkFunction : torch::autograd::Function<NetworkFunction> {
                     if (self->hasParameters[i]) check(api.encoding_set_parameter(self->encodings[i], &bound[i], QMLP_GRADIENTS));
             }
             qmlp_tensor_t ai = wrap(adjInput);
-            check(api.network_adjoint(self->handle, &in, &go, flags, &ai, tmp.data_ptr(), adjTmp.data_ptr(), currentStream()));
+            check((recompute ? api.network_adjoint_recompute : api.network_adjoint)(self->handle, &in, &go, flags, &ai, tmp.data_ptr(), adjTmp.data_ptr(),
+                                                                                   currentStream()));
         }
         if (adjParams.defined()) adjParams = adjParams.to(static_cast<c10::ScalarType>(ctx->saved_data["param_dtype"].toInt()));
         variable_list out = {Tensor(), Tensor(), Tensor(), adjInput, adjParams};

@@ -83,6 +83,9 @@ SIGNATURES = {
     "qmlp_network_zero_gradients": (C.c_int, [_P, _P]),
     "qmlp_network_adjoint_memory": (C.c_int, [_P, C.c_int64, C.c_int, C.POINTER(C.c_size_t)]),
     "qmlp_network_adjoint": (C.c_int, [_P, _TP, _TP, C.c_int, _TP, _P, _P, _P]),
+    "qmlp_network_recompute_memory": (C.c_int, [_P, C.c_int64, C.c_int, C.POINTER(C.c_size_t), C.POINTER(C.c_size_t)]),
+    "qmlp_network_forward_recompute": (C.c_int, [_P, _TP, _TP, _P, _P]),
+    "qmlp_network_adjoint_recompute": (C.c_int, [_P, _TP, _TP, C.c_int, _TP, _P, _P, _P]),
     "qmlp_network_clear_cached_kernels": (C.c_int, [_P]),
     "qmlp_network_compile": (C.c_int, [_P, C.c_int]),
     "qmlp_network_launch_count": (C.c_int64, [_P]),

@@ -517,3 +517,41 @@ def test_convert_half(n, offset):
     check(lib().qmlp_convert_half(src.data_ptr(), dst[offset:].data_ptr(), n, None))
     torch.cuda.synchronize()
     assert torch.equal(dst[offset:offset + n], src.half()) and float(dst[offset + n]) == 0.0
+
+
+@pytest.mark.parametrize("n", [1, 128, 129, 40_001])
+@pytest.mark.parametrize("name", ["config1", "config2", "ref_widths", "uneven", "per_channel", "config3_small", "config4_small", "config5_small",
+                                  "grid2d_add_plus_identity", "line_net"])
+def test_recomputing_backward_pass(name, n):
+    """Autograd through the pair that keeps the encoded features only and computes the layers a second time, against the pair that
+    stashes the pre-activations (kernel path 1): output, weight gradient, table gradients, and the input gradient where no
+    grid asks for its own. Batches that end inside a tile, fill one, and give a CTA three. Both round the same values to
+    fp16; fp32 sums in another order move a rounding by 2^-11 now and then, and a pre-activation within that of zero may
+    flip a relu: 1e-2 of each gradient's norm. (line_net has no such pair: the call falls back.)"""
+    import torch
+    from qmlp import bindings
+    cfg, rng, spec, net, params, tables, acts, t_params, t_tables = _setup(name)
+    grid = any(e.num_parameters for e in spec.encodings)
+    x0 = torch.from_numpy(helpers.uniform(47, 1, (n, spec.num_inputs), *rng)).cuda()
+    adj = torch.from_numpy(helpers.uniform(47, 2, (n, spec.num_outputs), -1.0, 1.0)).cuda()
+    results = []
+    try:
+        for path in (0, 1):
+            bindings.QuickMLP.set_kernel_path(path)
+            x = x0.clone().requires_grad_(not grid)
+            w = t_params.float().requires_grad_(True)
+            tabs = [t.clone().requires_grad_(True) if t is not None else None for t in t_tables]
+            before = net.launch_count()
+            out = net.forward(x, w, tabs)
+            out.backward(adj)
+            torch.cuda.synchronize()
+            results.append(([out.detach(), w.grad] + [t.grad for t in tabs if t is not None] + ([x.grad] if not grid else []), net.launch_count() - before))
+    finally:
+        bindings.QuickMLP.set_kernel_path(0)
+    (a, launches), (b, launches_stash) = results
+    if not grid:
+        assert launches < launches_stash     # no weight-gradient kernel of its own
+    for i, (ga, gb) in enumerate(zip(a, b)):
+        norm = float(gb.norm())
+        assert norm > 0 or n == 1     # (a single point may sit where a relu output is zero)
+        assert float((ga - gb).norm()) <= 1e-2 * norm, f"{name} n={n} result {i}: {float((ga - gb).norm())} of {norm}"
