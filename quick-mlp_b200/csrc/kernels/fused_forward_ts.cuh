@@ -37,7 +37,18 @@ struct TsLayout {
     static constexpr int WG = ACC == 128 ? 3 : 1;
     static constexpr int FIT = (512 - ONES) / (ACC + OPERAND), SLOTS = FIT < 8 ? FIT : 8;
     static constexpr int THREADS = SLOTS * WG * 128;
-    __host__ __device__ static constexpr bool eligible() { return TL::eligible() && TL::maxCout() <= 128 && TL::maxCin() <= 128; }
+    __host__ __device__ static constexpr bool wideThroughout()
+    {
+        for (int i = 0; i + 1 < NL; ++i)
+            if (Spec::COUT[i] <= 64) return false;
+        return true;
+    }
+    // Two slots of three warpgroups pay only where every hidden layer keeps them busy: 48 -> 128 -> 64 -> 16 -> 4 with its encode pass,
+    // 2^20 points, 287 us against 253 us with the operands in shared memory.
+    __host__ __device__ static constexpr bool eligible() { return TL::eligible() && (ACC <= 64 || wideThroughout()); }
+    // Points per SM from which the kernel is quicker than the mma.sync one: two tiles, four for networks up to 32 wide (64-wide
+    // network 47360 points 7.9 against 9.0 us, 32768 points 7.1 against 6.4; 16-wide 80000 points 4.0 against 5.0, 65536 4.0 / 3.9)
+    __host__ __device__ static constexpr long long pointsPerSM() { return ACC == 32 ? 4 * TC_TILE : 2 * TC_TILE; }
     // bias block of layer l: COUT rows of 16 halfs, un-swizzled (bias_block_offset)
     __host__ __device__ static constexpr int biasOffset(int l)
     {

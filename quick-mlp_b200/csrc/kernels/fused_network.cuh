@@ -1247,6 +1247,16 @@ struct NetworkLaunchers {
         return o;
     }
 
+    // As few CTAs as give every warp a tile (each stages the weights), in whole rounds of one per SM so that the tiles spread
+    // evenly, but no more than there are tiles.
+    static long long ctasFor(long long tiles, int numSMs, int perSM)
+    {
+        const long long full = (tiles + Spec::WARPS - 1) / Spec::WARPS, rounds = (full + numSMs - 1) / numSMs;
+        long long blocks = (rounds < perSM ? rounds : perSM) * numSMs;
+        if (blocks > tiles) blocks = tiles;
+        return blocks < 1 ? 1 : blocks;
+    }
+
     template <int MODE>
     static cudaError_t forward(const LaunchArgs& a, cudaStream_t s)
     {
@@ -1259,10 +1269,7 @@ struct NetworkLaunchers {
             if (e != cudaSuccess) return e;
         }
         const long long tiles = (a.numel + TILE_POINTS - 1) / TILE_POINTS;
-        long long blocks = tiles;
-        const long long cap = static_cast<long long>(a.numSMs) * perSM;
-        if (blocks > cap) blocks = cap;
-        if (blocks < 1) blocks = 1;
+        const long long blocks = ctasFor(tiles, a.numSMs, perSM);
         k<<<static_cast<unsigned>(blocks), Spec::WARPS * 32, smem, s>>>(a);
         return cudaGetLastError();
     }
@@ -1279,10 +1286,7 @@ struct NetworkLaunchers {
             if (e != cudaSuccess) return e;
         }
         const long long tiles = (a.numel + TILE_POINTS - 1) / TILE_POINTS;
-        long long blocks = tiles;
-        const long long cap = static_cast<long long>(a.numSMs) * perSM;
-        if (blocks > cap) blocks = cap;
-        if (blocks < 1) blocks = 1;
+        const long long blocks = ctasFor(tiles, a.numSMs, perSM);
         k<<<static_cast<unsigned>(blocks), Spec::WARPS * 32, smem, s>>>(a);
         return cudaGetLastError();
     }
@@ -1331,19 +1335,16 @@ struct NetworkLaunchers {
         int n = 1;
         switch (kernel) {
         case KERNEL_INFERENCE:
-            if constexpr (TcLayout<Spec>::eligible()) {
-                // The tcgen05 kernel pays a fixed price per launch (tensor-memory allocation, operand staging for 148
-                // large CTAs) and needs at least one 128-point tile per slot to use what it sets up; below that the
-                // mma.sync kernel is quicker (config 1 at 2^16 points: 2.7 us against 4.7 us; config 2 at 2^16: 11.5
-                // against 12.9 us, at 2^20: 89 against 62 us). With a grid in front the gather decides, and the mma.sync
-                // kernel gathers with lane pairs and 16 warps (128 rows per point, 2^20 points: 272 against 364 us); few rows
-                // leave the layers in charge.
+            // The tcgen05 kernels pay a fixed price per launch (tensor-memory allocation, operand staging for 148 large CTAs); below
+            // a number of points the mma.sync kernel is quicker. With a grid in front the gather decides, and the mma.sync
+            // kernel gathers with lane pairs and 16 warps (128 rows per point, 2^20 points: 272 against 364 us); few rows leave the
+            // layers in charge.
+            if constexpr (TsLayout<Spec>::eligible() && table_rows_per_point<Spec>() == 0) {
+                if (a.forcePath == 3 || (a.forcePath != 1 && a.numel >= TsLayout<Spec>::pointsPerSM() * a.numSMs)) { e = TsLaunchers<Spec>::run(a, s); break; }
+            } else if constexpr (TcLayout<Spec>::eligible()) {
+                // (at least one tile per slot: 2^20 points through the 64-wide network 62 against 89 us, 2^16 points 12.9 / 11.5)
                 const bool enough = a.numel >= TcLayout<Spec>::pointsPerCta() * a.numSMs && table_rows_per_point<Spec>() < 32;
-                if (a.forcePath == 3 || (a.forcePath != 1 && enough)) {
-                    if constexpr (TsLayout<Spec>::eligible() && table_rows_per_point<Spec>() == 0) e = TsLaunchers<Spec>::run(a, s);
-                    else e = TcLaunchers<Spec>::inference(a, s);
-                    break;
-                }
+                if (a.forcePath == 3 || (a.forcePath != 1 && enough)) { e = TcLaunchers<Spec>::inference(a, s); break; }
             }
             e = forward<0>(a, s);
             break;
@@ -1353,10 +1354,12 @@ struct NetworkLaunchers {
             break;
         case KERNEL_INFERENCE_PLANES:
             if constexpr (TcLayout<Spec>::eligible()) {
-                const bool enough = a.numel >= TcLayout<Spec>::pointsPerCta() * a.numSMs;   // as above
-                if (!enough) e = forward<4>(a, s);
-                else if constexpr (TsLayout<Spec>::eligible()) e = TsLaunchers<Spec>::run(a, s);
-                else e = TcLaunchers<Spec>::inferencePlanes(a, s);
+                if constexpr (TsLayout<Spec>::eligible()) {
+                    if (a.numel >= TsLayout<Spec>::pointsPerSM() * a.numSMs) { e = TsLaunchers<Spec>::run(a, s); break; }
+                } else {
+                    if (a.numel >= TcLayout<Spec>::pointsPerCta() * a.numSMs) { e = TcLaunchers<Spec>::inferencePlanes(a, s); break; }
+                }
+                e = forward<4>(a, s);
             } else e = cudaErrorNotSupported;
             break;
         case KERNEL_FORWARD: e = forward<1>(a, s); break;
