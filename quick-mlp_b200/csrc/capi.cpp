@@ -508,6 +508,7 @@ static void inferenceLocked(Network& n, const qmlp_tensor_t* input, qmlp_tensor_
             a.output = out0 + c0 * a.outS0;
             a.planes = planes;
             a.planeStride = need;
+            a.flags = kernel::FLAG_HALF_SUMS;
             int launches = 0;
             int e;
             {

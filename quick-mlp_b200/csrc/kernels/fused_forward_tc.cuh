@@ -608,7 +608,9 @@ struct TcLaunchers {
         const long long cap = static_cast<long long>(a.numSMs) * 8;
         if (bx > cap) bx = cap;
         if (bx < 1) bx = 1;
-        encode_planes_kernel<Spec><<<dim3(static_cast<unsigned>(bx), groups), 256, 0, s>>>(a);
+        const dim3 grid(static_cast<unsigned>(bx), groups);
+        if (a.flags & FLAG_HALF_SUMS) encode_planes_kernel<Spec, false><<<grid, 256, 0, s>>>(a);
+        else encode_planes_kernel<Spec, true><<<grid, 256, 0, s>>>(a);
         return cudaGetLastError();
     }
 };

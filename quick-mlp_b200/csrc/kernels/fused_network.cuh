@@ -320,8 +320,8 @@ __device__ __forceinline__ void encode_point(const LaunchArgs& p, const RowReade
 
 // The same for the 32 points of a warp, lanes in pairs (see grid.cuh): both lanes gather half of the corners of the even
 // lane's point, then of the odd lane's, and each ends up with the features of its own point. `in0` / `in1`: input rows of
-// the pair's two points (inside the batch); all lanes of the warp take part.
-template <class Spec, int E, class Out>
+// the pair's two points (inside the batch); all lanes of the warp take part. EXACT: see grid_pair_forward.
+template <class Spec, int E, bool EXACT, class Out>
 __device__ __forceinline__ void encode_pair(const LaunchArgs& p, const RowReader& in0, const RowReader& in1, const Out& out)
 {
     if constexpr (E < Spec::NUM_ENCODINGS) {
@@ -344,19 +344,12 @@ __device__ __forceinline__ void encode_pair(const LaunchArgs& p, const RowReader
 #pragma unroll 2
             for (int l = 0; l < Enc::L; ++l) {
                 const GridLevelP& lv = g.levels[l];
-                float f0[F], f1[F];
-                if (lv.hashed) {
-                    grid_half_forward<D, F, Enc::HALF_TABLE, 0>(g, lv, pos0, side, f0);
-                    grid_half_forward<D, F, Enc::HALF_TABLE, 0>(g, lv, pos1, side, f1);
-                } else {
-                    grid_half_forward<D, F, Enc::HALF_TABLE, D - 1>(g, lv, pos0, side, f0);
-                    grid_half_forward<D, F, Enc::HALF_TABLE, D - 1>(g, lv, pos1, side, f1);
-                }
+                float feat[F];
+                grid_pair_forward<D, F, Enc::HALF_TABLE, EXACT>(g, lv, pos0, pos1, side, feat);
 #pragma unroll
                 for (int i = 0; i < F; ++i) {
-                    const float v = (side ? f1[i] : f0[i]) + __shfl_xor_sync(0xffffffffu, side ? f0[i] : f1[i], 1);
-                    if constexpr (Enc::CONCAT) out(Enc::OUT_OFF + l * F + i, v);
-                    else sum[i] += v;
+                    if constexpr (Enc::CONCAT) out(Enc::OUT_OFF + l * F + i, feat[i]);
+                    else sum[i] += feat[i];
                 }
             }
             if constexpr (!Enc::CONCAT) {
@@ -364,7 +357,7 @@ __device__ __forceinline__ void encode_pair(const LaunchArgs& p, const RowReader
                 for (int i = 0; i < F; ++i) out(Enc::OUT_OFF + i, sum[i]);
             }
         }
-        encode_pair<Spec, E + 1, Out>(p, in0, in1, out);
+        encode_pair<Spec, E + 1, EXACT, Out>(p, in0, in1, out);
     }
 }
 
@@ -585,7 +578,7 @@ fused_forward_kernel(const __grid_constant__ LaunchArgs p)
         if constexpr (!FROM_PLANES) {
             const long long last = p.numel - 1, i0 = myRow & ~1ll;   // (a lane past the end repeats the last point)
             const RowReader in0{p.input + (i0 < last ? i0 : last) * p.inS0, p.inS1}, in1{p.input + (i0 + 1 < last ? i0 + 1 : last) * p.inS0, p.inS1};
-            encode_pair<Spec, 0>(p, in0, in1, HalfRowWriter{row});
+            encode_pair<Spec, 0, MODE != 0>(p, in0, in1, HalfRowWriter{row});
         }
         if (myRow < p.numel) {
             if constexpr (FROM_PLANES) read_planes_point<Spec, 0>(p, myRow, HalfRowPlaneWriter{row});

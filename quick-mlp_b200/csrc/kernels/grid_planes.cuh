@@ -64,14 +64,14 @@ __device__ __forceinline__ void store_halfs(const LaunchArgs& p, __half* dst, co
 // Features of group `g` (relative to all groups) for the points `i` of a warp -> their planes. Lanes work in pairs (see
 // grid.cuh): both lanes gather half of the corners of the even lane's point, then of the odd lane's, and each ends up
 // with the sum for its own point. `in0` / `in1`: input rows of the pair's two points; all lanes of the warp take part.
-template <class Spec, int E>
+template <class Spec, int E, bool EXACT>
 __device__ __forceinline__ void encode_group(const LaunchArgs& p, int g, const RowReader& in0, const RowReader& in1, long long local, bool valid)
 {
     if constexpr (E < Spec::NUM_ENCODINGS) {
         using Enc = typename Spec::template Enc<E>;
         using PG = PlaneGroups<Spec, E>;
         if (g >= PG::before() + PG::own()) {
-            encode_group<Spec, E + 1>(p, g, in0, in1, local, valid);
+            encode_group<Spec, E + 1, EXACT>(p, g, in0, in1, local, valid);
             return;
         }
         const int side = threadIdx.x & 1;
@@ -93,16 +93,10 @@ __device__ __forceinline__ void encode_group(const LaunchArgs& p, int g, const R
             const int first = Enc::CONCAT ? g - PG::before() : 0, end = Enc::CONCAT ? first + 1 : Enc::L;
             for (int l = first; l < end; ++l) {
                 const GridLevelP& lv = grid.levels[l];
-                float f0[F], f1[F];
-                if (lv.hashed) {
-                    grid_half_forward<D, F, Enc::HALF_TABLE, 0>(grid, lv, pos0, side, f0);
-                    grid_half_forward<D, F, Enc::HALF_TABLE, 0>(grid, lv, pos1, side, f1);
-                } else {
-                    grid_half_forward<D, F, Enc::HALF_TABLE, D - 1>(grid, lv, pos0, side, f0);
-                    grid_half_forward<D, F, Enc::HALF_TABLE, D - 1>(grid, lv, pos1, side, f1);
-                }
+                float f[F];
+                grid_pair_forward<D, F, Enc::HALF_TABLE, EXACT>(grid, lv, pos0, pos1, side, f);
 #pragma unroll
-                for (int i = 0; i < F; ++i) feat[i] += (side ? f1[i] : f0[i]) + __shfl_xor_sync(0xffffffffu, side ? f0[i] : f1[i], 1);
+                for (int i = 0; i < F; ++i) feat[i] += f[i];
             }
             if (valid) store_halfs<F>(p, p.planes + p.planeStride * (Enc::OUT_OFF + (Enc::CONCAT ? first * F : 0)) + local * F, feat);
         }
@@ -133,7 +127,8 @@ __host__ __device__ constexpr int plane_min_blocks()
 #endif
 }
 
-template <class Spec>
+// EXACT: see grid_pair_forward
+template <class Spec, bool EXACT>
 __global__ void __launch_bounds__(256, plane_min_blocks<Spec>()) encode_planes_kernel(const __grid_constant__ LaunchArgs p)
 {
     const int g = blockIdx.y;
@@ -143,7 +138,7 @@ __global__ void __launch_bounds__(256, plane_min_blocks<Spec>()) encode_planes_k
         const long long i = base + (threadIdx.x & 31), last = p.numel - 1;
         const long long i0 = i & ~1ll;
         const RowReader in0{p.input + (i0 < last ? i0 : last) * p.inS0, p.inS1}, in1{p.input + (i0 + 1 < last ? i0 + 1 : last) * p.inS0, p.inS1};
-        encode_group<Spec, 0>(p, g, in0, in1, i, i < p.numel);
+        encode_group<Spec, 0, EXACT>(p, g, in0, in1, i, i < p.numel);
     }
 }
 

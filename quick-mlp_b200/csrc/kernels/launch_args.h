@@ -62,6 +62,8 @@ constexpr int FLAG_GRAD_ENCODINGS = 4;
 // table gradients are scattered from there by KERNEL_SCATTER_PLANES. Only with FLAG_GRAD_ENCODINGS and without
 // FLAG_GRAD_INPUT.
 constexpr int FLAG_SPLIT_SCATTER = 8;
+// KERNEL_ENCODE_PLANES for a pass without gradients: see grid_pair_forward
+constexpr int FLAG_HALF_SUMS = 16;
 
 // Copies of the gradients of small grid levels. Reductions to one 128-byte line execute one after the other in its L2 slice
 // (about nine clocks each): a level of a few lines that a large batch keeps hitting holds the whole kernel up. Such
@@ -153,4 +155,4 @@ extern "C" {
 typedef int (*qmlp_spec_launch_fn)(int kernel, const void* args, cudaStream_t stream, int* launches);
 typedef int (*qmlp_spec_abi_fn)(void);
 }
-#define QMLP_SPEC_ABI_VERSION 11
+#define QMLP_SPEC_ABI_VERSION 12

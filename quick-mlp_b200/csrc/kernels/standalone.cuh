@@ -142,19 +142,10 @@ __global__ void __launch_bounds__(EncodingTile<Enc>::WARPS * 32) grid_encoding_f
         for (int i = 0; i < F; ++i) sum[i] = 0.f;
         for (int l = 0; l < Enc::L; ++l) {
             const GridLevelP& lv = g.levels[l];
-            float f0[F], f1[F];
-            if (lv.hashed) {
-                grid_half_forward<D, F, Enc::HALF_TABLE, 0>(g, lv, pos0, side, f0);
-                grid_half_forward<D, F, Enc::HALF_TABLE, 0>(g, lv, pos1, side, f1);
-            } else {
-                grid_half_forward<D, F, Enc::HALF_TABLE, D - 1>(g, lv, pos0, side, f0);
-                grid_half_forward<D, F, Enc::HALF_TABLE, D - 1>(g, lv, pos1, side, f1);
-            }
+            float feat[F];
+            grid_pair_forward<D, F, Enc::HALF_TABLE, false>(g, lv, pos0, pos1, side, feat);
 #pragma unroll
-            for (int i = 0; i < F; ++i) {
-                const float v = (side ? f1[i] : f0[i]) + __shfl_xor_sync(0xffffffffu, side ? f0[i] : f1[i], 1);
-                sum[i] = Enc::CONCAT ? v : sum[i] + v;
-            }
+            for (int i = 0; i < F; ++i) sum[i] = Enc::CONCAT ? feat[i] : sum[i] + feat[i];
             if constexpr (Enc::CONCAT) T::put(tile + lane * T::STRIDE, l * F, sum);
         }
         if constexpr (!Enc::CONCAT) T::put(tile + lane * T::STRIDE, 0, sum);

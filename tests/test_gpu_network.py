@@ -206,6 +206,32 @@ def test_lane_pairs_of_the_plane_kernels(name, n):
                                  atol=1e-5 * float(b.abs().max()))
 
 
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 257])
+@pytest.mark.parametrize("half_tables", [False, True])
+@pytest.mark.parametrize("name", ["config3_small", "config4_small", "config5_small", "grid2d_add_plus_identity"])
+def test_features_of_a_pass_with_gradients(name, half_tables, n):
+    """The forward pass that a backward pass follows exchanges the rows of a lane pair instead of half sums: its encoded input
+    (the first rows of the stash) against the oracle. One fp16 rounding; a coordinate rounded differently by half an ulp
+    moves the fraction of a cell by resolution * 2^-24 per dimension, between rows that are at most 2 apart."""
+    import torch
+    from qmlp._capi import check, lib, wrap
+    cfg, rng, spec, net, params, tables, acts, t_params, t_tables = _setup(name)
+    x = helpers.uniform(43, 3, (n, spec.num_inputs), *rng)
+    tx = torch.from_numpy(x).cuda()
+    out = torch.empty((n, spec.num_outputs), device="cuda")
+    fwd = torch.empty((net.forward_memory(n),), dtype=torch.uint8, device="cuda")
+    net._bind(t_params, [t.half() if (t is not None and half_tables) else t for t in t_tables])
+    check(lib().qmlp_network_forward(net._h, wrap(tx), wrap(out), fwd.data_ptr(), None))
+    torch.cuda.synchronize()
+    tabs = [t.astype(np.float16).astype(np.float32) if (t is not None and half_tables) else t for t in tables]
+    expected = oracle.encode(spec, x, tabs)
+    width = spec.layers[0].channels_in
+    got = fwd.view(torch.float16)[:n * width].view(n, width).float().cpu().numpy()
+    grids = [e for e in spec.encodings if e.levels]
+    atol = max(2 * len(e.levels) * 4 * max(lv.resolution for lv in e.levels) for e in grids) * 2.0 ** -24
+    helpers.assert_close(got, expected, f"{name} n={n}", rtol=2.0 ** -10, atol=atol)
+
+
 @pytest.mark.parametrize("name,n,chunk", [("config2", 100_003, 0), ("config2", 5000, 1024), ("config3_small", 70_001, 4096),
                                           ("config1", 17, 0), ("config1", 0, 0)])
 def test_inference_from_host_memory(name, n, chunk):
