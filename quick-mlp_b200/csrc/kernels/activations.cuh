@@ -145,6 +145,14 @@ __device__ __forceinline__ __half2 act_forward_f32x2(float a, float b, int chann
     else return A::forward_f32x2(a, b);
 }
 
+// the same with the comparison form's answer to NaN (relu: 0)
+template <class A>
+__device__ __forceinline__ __half2 act_forward_f32x2_nan(float a, float b, int channel)
+{
+    if constexpr (std::is_base_of<BuiltinRelu, A>::value) return A::forward2(__floats2half2_rn(a, b));   // (rounding and clamping commute)
+    else return act_forward_f32x2<A>(a, b, channel);
+}
+
 // both values belong to the same channel (fragments that pair two points of one channel)
 template <class A>
 __device__ __forceinline__ __half2 act_forward2_same_channel(__half2 x, int channel)

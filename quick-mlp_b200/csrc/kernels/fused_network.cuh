@@ -443,7 +443,10 @@ __device__ __forceinline__ void read_planes_point(const LaunchArgs& p, long long
 
 // ---- forward layer chain -------------------------------------------------------------------------------------
 // MODE 0: inference, 1: forward with stash, 2: forward with stash + L2 loss gradient instead of the output, 3: forward that
-// stashes the encoded input only
+// stashes the encoded input only.
+// Inference rounds a layer once: the accumulators start from the bias and the activation takes fp32, as in the tcgen05
+// kernels, so that a batch gives the same results whichever kernel its size picks. Where a backward pass follows the
+// pre-activation is rounded to half and the half bias is added: the value whose derivative that pass takes.
 template <class Spec, int L, int MODE>
 __device__ __forceinline__ void forward_layers(const LaunchArgs& p, const __half* sW, const __half* sB,
                                                uint32_t (&aIn)[MT][Spec::CIN[L] / 16][4], long long rowBase, long long n32,
@@ -470,12 +473,17 @@ __device__ __forceinline__ void forward_layers(const LaunchArgs& p, const __half
             if (j * 16 >= Spec::NUM_OUTPUTS) continue; // padded output channels are never read
         }
         float acc[MT][2][4];
+        float2 start[2] = {{0.f, 0.f}, {0.f, 0.f}};
+        if constexpr (MODE == 0 && BIAS) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) start[h] = __half22float2(*reinterpret_cast<const __half2*>(bias + j * 16 + h * 8 + q * 2));
+        }
 #pragma unroll
         for (int m = 0; m < MT; ++m)
 #pragma unroll
             for (int h = 0; h < 2; ++h)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) acc[m][h][e] = 0.f;
+                for (int e = 0; e < 4; ++e) acc[m][h][e] = (e & 1) ? start[h].y : start[h].x;
 #pragma unroll
         for (int k = 0; k < KT; ++k) {
             uint32_t b[4];
@@ -490,7 +498,7 @@ __device__ __forceinline__ void forward_layers(const LaunchArgs& p, const __half
         for (int m = 0; m < MT; ++m) {
             __half2 pre[2][2]; // [h][row r | row r + 8]
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
+            for (int h = 0; h < (MODE == 0 ? 0 : 2); ++h) {
                 pre[h][0] = __floats2half2_rn(acc[m][h][0], acc[m][h][1]);
                 pre[h][1] = __floats2half2_rn(acc[m][h][2], acc[m][h][3]);
                 if constexpr (BIAS) {
@@ -517,8 +525,14 @@ __device__ __forceinline__ void forward_layers(const LaunchArgs& p, const __half
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int col = j * 16 + h * 8 + q * 2;
-                const __half2 lo = pre[h][0], hi = pre[h][1];
-                const __half2 zlo = act_forward2<Act>(lo, col), zhi = act_forward2<Act>(hi, col);
+                __half2 zlo, zhi;
+                if constexpr (MODE == 0) {
+                    zlo = act_forward_f32x2_nan<Act>(acc[m][h][0], acc[m][h][1], col);
+                    zhi = act_forward_f32x2_nan<Act>(acc[m][h][2], acc[m][h][3], col);
+                } else {
+                    zlo = act_forward2<Act>(pre[h][0], col);
+                    zhi = act_forward2<Act>(pre[h][1], col);
+                }
                 if constexpr (!LAST) {
                     aOut[m][j][h * 2 + 0] = h2_as_u32(zlo);
                     aOut[m][j][h * 2 + 1] = h2_as_u32(zhi);

@@ -512,6 +512,63 @@ def test_activations_in_tensor_memory(name, path, n):
     helpers.assert_close(out[0], out[1], f"{name} n={n}", rtol=5e-3, atol=2e-3, max_violations=0.005)
 
 
+def _rounded_chain(spec, params, feat, acts, roundings):
+    """Layer chain in 64 bits with fp16 inputs: one rounding per layer (bias and activation before it), or two (the
+    accumulator, then the sum with the bias, and the activation of that)."""
+    def half(a):
+        return a.astype(np.float16).astype(np.float64)
+    w = params.astype(np.float64)
+    h = half(feat)
+    for i, l in enumerate(spec.layers):
+        pre = h @ oracle.weight_view(spec, w, i).T
+        b = oracle.bias_view(spec, w, i)
+        bias = 0.0 if b is None else b[None, :]
+        pre = half(half(pre) + bias) if roundings == 2 else pre + bias
+        h = half(oracle._act_forward(acts, l.activation, pre))
+    return h[:, :spec.num_outputs]
+
+
+@pytest.mark.parametrize("name,path", [("config2", 1), ("config2", 3), ("uneven", 1), ("uneven", 3), ("config3_small", 1), ("config3_small", 2),
+                                       ("config5_small", 2)])
+def test_inference_rounds_a_layer_once(name, path):
+    """Every inference kernel (mma.sync: path 1, and on a few points from the planes: path 2; tcgen05: path 3) adds the
+    bias and applies the activation in fp32. Against the chain in 64 bits with one rounding per layer; how far the chain
+    with two roundings is from that is the scale (fp32 sums and the special-function unit flip a rounding now and then)."""
+    import torch
+    from qmlp import bindings
+    cfg, rng, spec, net, params, tables, acts, t_params, t_tables = _setup(name)
+    params = helpers.xavier_parameters(spec, cfg, bias_scale=0.5)
+    x = helpers.uniform(61, 1, (3000, spec.num_inputs), *rng)
+    feat = oracle.encode(spec, x, tables)
+    once, twice = (_rounded_chain(spec, params, feat, acts, r) for r in (1, 2))
+    try:
+        bindings.QuickMLP.set_kernel_path(path)
+        out = net.inference(torch.from_numpy(x).cuda(), torch.from_numpy(params).cuda(), t_tables).cpu().numpy().astype(np.float64)
+    finally:
+        bindings.QuickMLP.set_kernel_path(0)
+    assert np.linalg.norm(out - once) < 0.5 * np.linalg.norm(twice - once)
+
+
+@pytest.mark.parametrize("path", [0, 1])
+def test_relu_of_nan(path):
+    """"z = __hgt(x, hZERO()) ? x : hZERO()" is 0 for NaN in the mma.sync kernel: a NaN coordinate ends in the first layer's
+    relu and the outputs are those of zero activations behind it; other rows of its tile are not touched."""
+    import torch
+    from qmlp import bindings
+    cfg, rng, spec, net, params, tables, acts, t_params, t_tables = _setup("config2")
+    x = helpers.uniform(61, 1, (300, spec.num_inputs), *rng)
+    x[5, 1] = np.nan
+    ref = oracle.network_forward(spec, params, x, tables, half=True)
+    assert np.isfinite(ref).all()
+    try:
+        bindings.QuickMLP.set_kernel_path(path)
+        out = net.inference(torch.from_numpy(x).cuda(), t_params).cpu().numpy()
+    finally:
+        bindings.QuickMLP.set_kernel_path(0)
+    helpers.assert_close(out, ref, f"path {path}", max_violations=0.01)
+    helpers.assert_close(out[5], ref[5], f"path {path}, row with a NaN")
+
+
 @pytest.mark.parametrize("n,chunk", [(1, 0), (129, 0), (5000, 1024), ((1 << 18) + 33, 0)])
 @pytest.mark.parametrize("pinned", [True, False], ids=["pinned", "pageable"])
 def test_inference_from_host_memory_in_place(n, chunk, pinned):
