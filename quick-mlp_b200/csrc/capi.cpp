@@ -589,18 +589,22 @@ int qmlp_network_inference_host(qmlp_network_t* net, const float* host_input, fl
     HostPipeline& hp = n.hostPipeline;
     hp.reserve(chunk, cin, mapped ? 0 : cout);
     const cudaStream_t user = static_cast<cudaStream_t>(stream);
+    // The slots are cut by the chunk size of the call, so slot s of one call overlaps other slots of another: a call starts after
+    // the last one, on whatever stream that was. Under capture it does not (a graph cannot wait for work outside of
+    // it); replays share the slots with other calls and are ordered by the caller.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    checkCuda(cudaStreamIsCapturing(user, &capture), "cudaStreamIsCapturing");
+    const bool ordered = capture == cudaStreamCaptureStatusNone;
+    if (ordered) checkCuda(cudaStreamWaitEvent(user, hp.finished, 0), "cudaStreamWaitEvent");
     if (chunk == num_points) {   // nothing to overlap: in order on the caller's stream
         qmlp_tensor_t ti{hp.in[0], QMLP_FLOAT, 2, {num_points, cin}, {cin, 1}};
         qmlp_tensor_t to{mapped ? mapped : hp.out[0], QMLP_FLOAT, 2, {num_points, cout}, {cout, 1}};
-        checkCuda(cudaStreamWaitEvent(user, hp.computed[0], 0), "cudaStreamWaitEvent");   // an earlier call, on whatever stream
-        checkCuda(cudaStreamWaitEvent(user, hp.downloaded[0], 0), "cudaStreamWaitEvent");
         checkCuda(cudaMemcpyAsync(hp.in[0], host_input, static_cast<size_t>(num_points) * cin * 4, cudaMemcpyHostToDevice, user), "cudaMemcpyAsync(host to device)");
         inferenceLocked(n, &ti, &to, stream);
-        checkCuda(cudaEventRecord(hp.computed[0], user), "cudaEventRecord");
         if (!mapped)
             checkCuda(cudaMemcpyAsync(host_output, hp.out[0], static_cast<size_t>(num_points) * cout * 4, cudaMemcpyDeviceToHost, user),
                       "cudaMemcpyAsync(device to host)");
-        if (!mapped) checkCuda(cudaEventRecord(hp.downloaded[0], user), "cudaEventRecord");
+        if (ordered) checkCuda(cudaEventRecord(hp.finished, user), "cudaEventRecord");
         return QMLP_OK;
     }
     // uploads start after the work already queued on the caller's stream (e.g. a parameter update)
@@ -611,10 +615,11 @@ int qmlp_network_inference_host(qmlp_network_t* net, const float* host_input, fl
     for (int64_t p0 = 0; p0 < num_points; p0 += chunk, ++k) {
         const int s = static_cast<int>(k % HostPipeline::SLOTS);
         const int64_t m = std::min(chunk, num_points - p0);
-        // the slot's previous kernel (of this call or an earlier one) has consumed its input; its previous download has left its
-        // output
-        checkCuda(cudaStreamWaitEvent(hp.copyIn, hp.computed[s], 0), "cudaStreamWaitEvent");
-        if (!mapped) checkCuda(cudaStreamWaitEvent(user, hp.downloaded[s], 0), "cudaStreamWaitEvent");
+        if (k >= HostPipeline::SLOTS) {
+            // the slot's previous kernel has consumed its input; its previous download has left its output
+            checkCuda(cudaStreamWaitEvent(hp.copyIn, hp.computed[s], 0), "cudaStreamWaitEvent");
+            if (!mapped) checkCuda(cudaStreamWaitEvent(user, hp.downloaded[s], 0), "cudaStreamWaitEvent");
+        }
         checkCuda(cudaMemcpyAsync(hp.in[s], host_input + p0 * cin, static_cast<size_t>(m) * cin * 4, cudaMemcpyHostToDevice, hp.copyIn),
                   "cudaMemcpyAsync(host to device)");
         checkCuda(cudaEventRecord(hp.uploaded[s], hp.copyIn), "cudaEventRecord");
@@ -633,6 +638,7 @@ int qmlp_network_inference_host(qmlp_network_t* net, const float* host_input, fl
     if (!mapped)
         for (int s = 0; s < HostPipeline::SLOTS && s < k; ++s)
             checkCuda(cudaStreamWaitEvent(user, hp.downloaded[s], 0), "cudaStreamWaitEvent");
+    if (ordered) checkCuda(cudaEventRecord(hp.finished, user), "cudaEventRecord");
     QMLP_CATCH
 }
 

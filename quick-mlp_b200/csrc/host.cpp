@@ -564,6 +564,7 @@ void HostPipeline::reserve(int64_t points, int channelsIn, int channelsOut)
         pipelineCheck(cudaStreamCreateWithFlags(&copyIn, cudaStreamNonBlocking), "cudaStreamCreate");
         pipelineCheck(cudaStreamCreateWithFlags(&copyOut, cudaStreamNonBlocking), "cudaStreamCreate");
         pipelineCheck(cudaEventCreateWithFlags(&start, cudaEventDisableTiming), "cudaEventCreate");
+        pipelineCheck(cudaEventCreateWithFlags(&finished, cudaEventDisableTiming), "cudaEventCreate");
         for (int s = 0; s < SLOTS; ++s) {
             pipelineCheck(cudaEventCreateWithFlags(&uploaded[s], cudaEventDisableTiming), "cudaEventCreate");
             pipelineCheck(cudaEventCreateWithFlags(&computed[s], cudaEventDisableTiming), "cudaEventCreate");
@@ -597,9 +598,10 @@ void HostPipeline::release()
     if (block) cudaFree(block);
     block = nullptr;
     if (start) cudaEventDestroy(start);
+    if (finished) cudaEventDestroy(finished);
     if (copyIn) cudaStreamDestroy(copyIn);
     if (copyOut) cudaStreamDestroy(copyOut);
-    start = nullptr;
+    start = finished = nullptr;
     copyIn = copyOut = nullptr;
     capacity = 0;
 }

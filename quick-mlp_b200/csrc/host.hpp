@@ -222,6 +222,7 @@ struct HostPipeline {
     static constexpr int SLOTS = 3;
     cudaStream_t copyIn = nullptr, copyOut = nullptr;
     cudaEvent_t start = nullptr;
+    cudaEvent_t finished = nullptr;   // end of the last call outside of a capture: the next one waits for it
     cudaEvent_t uploaded[SLOTS] = {}, computed[SLOTS] = {}, downloaded[SLOTS] = {};
     float* block = nullptr;  // one allocation: the slots' inputs, then their outputs
     float* in[SLOTS] = {};

@@ -590,6 +590,64 @@ def test_inference_from_host_memory_in_place(n, chunk, pinned):
         out.zero_()
 
 
+@pytest.mark.parametrize("name", ["config2", "uneven"])
+def test_inference_from_host_memory_on_two_streams(name):
+    """Calls on two streams with nothing between them: chunks of 2^15 points, one chunk of 300 001, and a pageable result
+    after a page-locked one. Each call cuts the staging memory its own way, so a slot of one covers several of another."""
+    import torch
+    cfg, rng, spec, net, params, tables, acts, t_params, t_tables = _setup(name)
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    jobs = []
+    for i, (n, chunk, pinned) in enumerate([(1 << 20, 1 << 15, True), (300_001, 300_001, True), (1 << 19, 1 << 14, False),
+                                            (300_001, 300_001, True), (1 << 20, 1 << 15, True), (100_003, 0, False)]):
+        x = torch.from_numpy(helpers.uniform(62, i, (n, spec.num_inputs), *rng)).pin_memory()
+        out = torch.empty((n, spec.num_outputs), pin_memory=pinned)
+        ref = net.inference_host(x, t_params, t_tables, output=torch.empty_like(out, pin_memory=pinned), chunk_points=chunk)
+        torch.cuda.synchronize()
+        jobs.append((x, out, ref, chunk))
+    for _ in range(5):
+        for i, (x, out, ref, chunk) in enumerate(jobs):
+            out.zero_()
+        for i, (x, out, ref, chunk) in enumerate(jobs):
+            with torch.cuda.stream(streams[i & 1]):
+                net.inference_host(x, t_params, t_tables, output=out, chunk_points=chunk)
+        torch.cuda.synchronize()
+        for i, (x, out, ref, chunk) in enumerate(jobs):
+            assert torch.equal(out, ref), i
+
+
+@pytest.mark.parametrize("chunk", [0, 1024])
+@pytest.mark.parametrize("name", ["config2", "uneven"])
+def test_inference_from_host_memory_under_capture(name, chunk):
+    """A call that is captured after one that was not, its replay, and a call that is not captured after it."""
+    import torch
+    cfg, rng, spec, net, params, tables, acts, t_params, t_tables = _setup(name)
+    n = 5000
+    x = torch.from_numpy(helpers.uniform(45, 1, (n, spec.num_inputs), *rng)).pin_memory()
+    out = torch.zeros((n, spec.num_outputs), pin_memory=True)
+    stream = torch.cuda.Stream()
+
+    def call():
+        net.inference_host(x, t_params, t_tables, output=out, chunk_points=chunk)
+
+    def result():
+        torch.cuda.synchronize()
+        r = out.clone()
+        out.zero_()
+        return r
+    with torch.cuda.stream(stream):
+        call()
+    ref = result()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        call()
+    graph.replay()
+    assert torch.equal(result(), ref)
+    with torch.cuda.stream(stream):
+        call()
+    assert torch.equal(result(), ref)
+
+
 @pytest.mark.parametrize("n,offset", [(1, 0), (3, 0), (4, 0), (1024, 0), (1023, 0), (1024, 1), (4097, 2)])
 def test_convert_half(n, offset):
     """fp32 -> fp16 copy of a parameter vector: vector and scalar kernels, lengths and alignments either side of the rule."""
