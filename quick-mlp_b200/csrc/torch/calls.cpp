@@ -414,11 +414,48 @@ struct ActivationFunction : torch::autograd::Function<ActivationFunction> {
         return {op.call(ctx->get_saved_variables()[0], grad[0].contiguous(), ctx->saved_data["cfg"].toStringRef()), Tensor()};
     }
 };
+// The kernels write into fresh tensors: without a node of their own the results of the adjoint operators would count as
+// constants in a second differentiation (create_graph), and a gradient term of a loss would drop out unnoticed.
+[[noreturn]] void raiseNotTwice(const char* op)
+{
+    throw std::runtime_error(std::string("qmlp_b200::") + op + " is not differentiable: the operators can be differentiated once only");
+}
+struct EncodingAdjointFunction : torch::autograd::Function<EncodingAdjointFunction> {
+    static variable_list forward(AutogradContext* ctx, const Tensor& input, const OptTensor& parameters, const Tensor& adjOutput, bool wantInput,
+                                 bool wantParameters, const std::string& cfg)
+    {
+        at::AutoDispatchBelowADInplaceOrView below;
+        static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("qmlp_b200::encoding_adjoint", "").typed<decltype(encodingAdjoint)>();
+        auto g = op.call(input, parameters, adjOutput, wantInput, wantParameters, cfg);
+        return {std::get<0>(g), std::get<1>(g)};
+    }
+    static variable_list backward(AutogradContext*, variable_list) { raiseNotTwice("encoding_adjoint"); }
+};
+struct ActivationAdjointFunction : torch::autograd::Function<ActivationAdjointFunction> {
+    static Tensor forward(AutogradContext*, const Tensor& input, const Tensor& adjOutput, const std::string& cfg)
+    {
+        at::AutoDispatchBelowADInplaceOrView below;
+        static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("qmlp_b200::activation_adjoint", "").typed<decltype(activationAdjoint)>();
+        return op.call(input, adjOutput, cfg);
+    }
+    static variable_list backward(AutogradContext*, variable_list) { raiseNotTwice("activation_adjoint"); }
+};
+
 Tensor encodingForwardAutograd(const Tensor& input, const OptTensor& parameters, std::string_view cfg)
 {
     return EncodingFunction::apply(input, parameters, std::string(cfg));
 }
 Tensor activationForwardAutograd(const Tensor& input, std::string_view cfg) { return ActivationFunction::apply(input, std::string(cfg)); }
+std::tuple<Tensor, Tensor> encodingAdjointAutograd(const Tensor& input, const OptTensor& parameters, const Tensor& adjOutput, bool wantInput,
+                                                   bool wantParameters, std::string_view cfg)
+{
+    auto g = EncodingAdjointFunction::apply(input, parameters, adjOutput, wantInput, wantParameters, std::string(cfg));
+    return {g[0], g[1]};
+}
+Tensor activationAdjointAutograd(const Tensor& input, const Tensor& adjOutput, std::string_view cfg)
+{
+    return ActivationAdjointFunction::apply(input, adjOutput, std::string(cfg));
+}
 
 Tensor encodingForwardMeta(const Tensor& input, const OptTensor&, std::string_view cfg)
 {
@@ -480,8 +517,8 @@ TORCH_LIBRARY_IMPL(qmlp_b200, Autograd, m)
 {
     m.impl("encoding_forward", encodingForwardAutograd);
     m.impl("activation_forward", activationForwardAutograd);
-    m.impl("encoding_adjoint", torch::CppFunction::makeFallthrough());
-    m.impl("activation_adjoint", torch::CppFunction::makeFallthrough());
+    m.impl("encoding_adjoint", encodingAdjointAutograd);
+    m.impl("activation_adjoint", activationAdjointAutograd);
 }
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m)
