@@ -441,20 +441,44 @@ struct ActivationAdjointFunction : torch::autograd::Function<ActivationAdjointFu
     static variable_list backward(AutogradContext*, variable_list) { raiseNotTwice("activation_adjoint"); }
 };
 
+// Nodes are made only where a gradient can be asked for. Otherwise the operator runs below autograd, as operators without a
+// forward-mode formula do: a dual tensor that requires no gradient is taken for its primal value.
+bool differentiable(const Tensor& t) { return t.defined() && t.requires_grad(); }
+bool differentiable(const OptTensor& t) { return t.has_value() && differentiable(*t); }
+template <class... T>
+bool wantsNode(const T&... tensors) { return torch::GradMode::is_enabled() && (differentiable(tensors) || ...); }
+
 Tensor encodingForwardAutograd(const Tensor& input, const OptTensor& parameters, std::string_view cfg)
 {
-    return EncodingFunction::apply(input, parameters, std::string(cfg));
+    if (wantsNode(input, parameters)) return EncodingFunction::apply(input, parameters, std::string(cfg));
+    at::AutoDispatchBelowADInplaceOrView below;
+    static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("qmlp_b200::encoding_forward", "").typed<decltype(encodingForward)>();
+    return op.call(input, parameters, cfg);
 }
-Tensor activationForwardAutograd(const Tensor& input, std::string_view cfg) { return ActivationFunction::apply(input, std::string(cfg)); }
+Tensor activationForwardAutograd(const Tensor& input, std::string_view cfg)
+{
+    if (wantsNode(input)) return ActivationFunction::apply(input, std::string(cfg));
+    at::AutoDispatchBelowADInplaceOrView below;
+    static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("qmlp_b200::activation_forward", "").typed<decltype(activationForward)>();
+    return op.call(input, cfg);
+}
 std::tuple<Tensor, Tensor> encodingAdjointAutograd(const Tensor& input, const OptTensor& parameters, const Tensor& adjOutput, bool wantInput,
                                                    bool wantParameters, std::string_view cfg)
 {
-    auto g = EncodingAdjointFunction::apply(input, parameters, adjOutput, wantInput, wantParameters, std::string(cfg));
-    return {g[0], g[1]};
+    if (wantsNode(input, parameters, adjOutput)) {
+        auto g = EncodingAdjointFunction::apply(input, parameters, adjOutput, wantInput, wantParameters, std::string(cfg));
+        return {g[0], g[1]};
+    }
+    at::AutoDispatchBelowADInplaceOrView below;
+    static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("qmlp_b200::encoding_adjoint", "").typed<decltype(encodingAdjoint)>();
+    return op.call(input, parameters, adjOutput, wantInput, wantParameters, cfg);
 }
 Tensor activationAdjointAutograd(const Tensor& input, const Tensor& adjOutput, std::string_view cfg)
 {
-    return ActivationAdjointFunction::apply(input, adjOutput, std::string(cfg));
+    if (wantsNode(input, adjOutput)) return ActivationAdjointFunction::apply(input, adjOutput, std::string(cfg));
+    at::AutoDispatchBelowADInplaceOrView below;
+    static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("qmlp_b200::activation_adjoint", "").typed<decltype(activationAdjoint)>();
+    return op.call(input, adjOutput, cfg);
 }
 
 Tensor encodingForwardMeta(const Tensor& input, const OptTensor&, std::string_view cfg)

@@ -36,3 +36,21 @@ def test_second_backward_raises():
     # once, and without a graph of the gradient
     torch.ops.qmlp_b200.encoding_forward(x, table, cfg).backward(grad)
     assert x.grad.shape == x.shape and table.grad.shape == table.shape and not x.grad.requires_grad
+
+
+def test_forward_mode_without_a_gradient():
+    """The operators have no forward-mode formula: a dual tensor that requires no gradient is taken for its primal value
+    (torch.func.jvp too), one that does is refused."""
+    import torch
+    import torch.autograd.forward_ad as fwad
+    import qmlp  # noqa: F401
+    cfg, x, table, grad = _operands(requires_grad=False)
+
+    def call(a):
+        return torch.ops.qmlp_b200.encoding_forward(a, table, cfg)
+    with fwad.dual_level():
+        out = fwad.unpack_dual(call(fwad.make_dual(x, torch.empty_like(x))))
+        assert out.primal.shape == grad.shape and out.tangent is None
+        with pytest.raises(RuntimeError):
+            call(fwad.make_dual(x.clone().requires_grad_(True), torch.empty_like(x)))
+    assert torch.func.jvp(call, (x,), (torch.empty_like(x),))[0].shape == grad.shape
