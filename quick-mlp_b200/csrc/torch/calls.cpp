@@ -46,19 +46,6 @@ struct Api {
 PyObject* errorType = nullptr;          // qmlp._capi.QmlpError
 PyObject* configurationErrorType = nullptr;
 
-void load(const std::string& path, py::object error, py::object configurationError)
-{
-    void* h = ::dlopen(path.c_str(), RTLD_NOW | RTLD_LOCAL);
-    if (!h) throw std::runtime_error(std::string("dlopen: ") + ::dlerror());
-#define QMLP_RESOLVE(name)                                                                                                \
-    api.name = reinterpret_cast<decltype(&qmlp_##name)>(::dlsym(h, "qmlp_" #name));                                       \
-    if (!api.name) throw std::runtime_error("qmlp_" #name " not found in " + path);
-    QMLP_CALLS(QMLP_RESOLVE)
-#undef QMLP_RESOLVE
-    errorType = error.release().ptr();
-    configurationErrorType = configurationError.release().ptr();
-}
-
 // raises a Python exception from any thread, with or without the interpreter lock
 [[noreturn]] void raise(PyObject* type, const std::string& message)
 {
@@ -514,36 +501,37 @@ void trainerUpdate(intptr_t trainer, int64_t step, double gradScale)
     check(api.trainer_update(reinterpret_cast<qmlp_trainer_t*>(trainer), step, static_cast<float>(gradScale), currentStream()));
 }
 
-} // namespace
+// Resolves the C ABI, then registers the kernels of the operators that qmlp/ops.py defines (in this order: another thread may
+// call an operator as soon as it is registered). The devices' own autograd keys are used: the alias key holds the entry that
+// loads this module.
+void load(const std::string& path, py::object error, py::object configurationError)
+{
+    void* h = ::dlopen(path.c_str(), RTLD_NOW | RTLD_LOCAL);
+    if (!h) throw std::runtime_error(std::string("dlopen: ") + ::dlerror());
+#define QMLP_RESOLVE(name)                                                                                                \
+    api.name = reinterpret_cast<decltype(&qmlp_##name)>(::dlsym(h, "qmlp_" #name));                                       \
+    if (!api.name) throw std::runtime_error("qmlp_" #name " not found in " + path);
+    QMLP_CALLS(QMLP_RESOLVE)
+#undef QMLP_RESOLVE
+    errorType = error.release().ptr();
+    configurationErrorType = configurationError.release().ptr();
+    auto kernels = [](c10::DispatchKey key, auto encodingForwardK, auto encodingAdjointK, auto activationForwardK, auto activationAdjointK) {
+        auto* m = new torch::Library(torch::Library::IMPL, "qmlp_b200", key, __FILE__, __LINE__);   // (lives as long as the process)
+        m->impl("encoding_forward", encodingForwardK);
+        m->impl("encoding_adjoint", encodingAdjointK);
+        m->impl("activation_forward", activationForwardK);
+        m->impl("activation_adjoint", activationAdjointK);
+    };
+    static bool registered = false;
+    if (registered) return;
+    registered = true;
+    kernels(c10::DispatchKey::CUDA, encodingForward, encodingAdjoint, activationForward, activationAdjoint);
+    kernels(c10::DispatchKey::Meta, encodingForwardMeta, encodingAdjointMeta, activationForwardMeta, activationAdjointMeta);
+    for (auto key : {c10::DispatchKey::AutogradCUDA, c10::DispatchKey::AutogradMeta, c10::DispatchKey::AutogradOther})   // (Other: functorch)
+        kernels(key, encodingForwardAutograd, encodingAdjointAutograd, activationForwardAutograd, activationAdjointAutograd);
+}
 
-TORCH_LIBRARY(qmlp_b200, m)
-{
-    m.def("encoding_forward(Tensor input, Tensor? parameters, str cfg) -> Tensor");
-    m.def("encoding_adjoint(Tensor input, Tensor? parameters, Tensor adj_output, bool want_input, bool want_parameters, str cfg) -> (Tensor, Tensor)");
-    m.def("activation_forward(Tensor input, str cfg) -> Tensor");
-    m.def("activation_adjoint(Tensor input, Tensor adj_output, str cfg) -> Tensor");
-}
-TORCH_LIBRARY_IMPL(qmlp_b200, CUDA, m)
-{
-    m.impl("encoding_forward", encodingForward);
-    m.impl("encoding_adjoint", encodingAdjoint);
-    m.impl("activation_forward", activationForward);
-    m.impl("activation_adjoint", activationAdjoint);
-}
-TORCH_LIBRARY_IMPL(qmlp_b200, Meta, m)
-{
-    m.impl("encoding_forward", encodingForwardMeta);
-    m.impl("encoding_adjoint", encodingAdjointMeta);
-    m.impl("activation_forward", activationForwardMeta);
-    m.impl("activation_adjoint", activationAdjointMeta);
-}
-TORCH_LIBRARY_IMPL(qmlp_b200, Autograd, m)
-{
-    m.impl("encoding_forward", encodingForwardAutograd);
-    m.impl("activation_forward", activationForwardAutograd);
-    m.impl("encoding_adjoint", encodingAdjointAutograd);
-    m.impl("activation_adjoint", activationAdjointAutograd);
-}
+} // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m)
 {

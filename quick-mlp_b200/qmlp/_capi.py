@@ -7,6 +7,7 @@ The library must be present: there is no fallback path.
 import ctypes as C
 import importlib.util
 import os
+import threading
 
 import torch
 
@@ -147,6 +148,7 @@ def lib():
 
 
 _calls = None
+_calls_lock = threading.Lock()
 
 
 def calls():
@@ -154,15 +156,17 @@ def calls():
     (python quick-mlp_b200/build_torch_ext.py)."""
     global _calls
     if _calls is None:
-        path = os.path.abspath(os.path.join(_HERE, "..", "lib", "torch_ext", "qmlp_calls.so"))
-        if not os.path.exists(path):
-            raise ImportError(f"{path} not found: build it with `python quick-mlp_b200/build_torch_ext.py`")
-        lib()
-        spec = importlib.util.spec_from_file_location("qmlp_calls", path)
-        module = importlib.util.module_from_spec(spec)
-        spec.loader.exec_module(module)
-        module.load(os.path.abspath(os.environ.get("QMLP_B200_LIBRARY", LIB_PATH)), QmlpError, ConfigurationError)
-        _calls = module
+        with _calls_lock:
+            if _calls is None:
+                path = os.path.abspath(os.path.join(_HERE, "..", "lib", "torch_ext", "qmlp_calls.so"))
+                if not os.path.exists(path):
+                    raise ImportError(f"{path} not found: build it with `python quick-mlp_b200/build_torch_ext.py`")
+                lib()
+                spec = importlib.util.spec_from_file_location("qmlp_calls", path)
+                module = importlib.util.module_from_spec(spec)
+                spec.loader.exec_module(module)
+                module.load(os.path.abspath(os.environ.get("QMLP_B200_LIBRARY", LIB_PATH)), QmlpError, ConfigurationError)
+                _calls = module
     return _calls
 
 

@@ -1,6 +1,7 @@
 """qmlp.FusedActivation, API of src_py/qmlp/activation.py:8-79."""
 import torch
 
+from . import _capi
 from . import ops  # noqa: F401  (registers torch.ops.qmlp_b200.*)
 from .bindings import Activation
 
@@ -28,6 +29,7 @@ class FusedActivation(torch.nn.Module):
         """``cfg`` is a built-in id (relu, celu, sine, identity) or an inline JSON object
         {"id": ..., "forward": "z = ...", "adjoint": "adjx = ..."} with CUDA statements over half."""
         super().__init__()
+        _capi.calls()     # the kernels behind the operator
         self._cfg = cfg
         self._activation = Activation(cfg)
 

@@ -1,6 +1,7 @@
 """qmlp.FusedEncoding, API of src_py/qmlp/encoding.py:9-122."""
 import torch
 
+from . import _capi
 from . import ops  # noqa: F401  (registers torch.ops.qmlp_b200.*)
 from .bindings import Encoding
 
@@ -10,6 +11,7 @@ class FusedEncoding(torch.nn.Module):
 
     def __init__(self, cfg_or_impl):
         super().__init__()
+        _capi.calls()     # the kernels behind the operator
         if isinstance(cfg_or_impl, str):
             self._encoding = Encoding(cfg_or_impl)
         elif isinstance(cfg_or_impl, Encoding):

@@ -1,6 +1,9 @@
 """The Python surface as far as it goes without a GPU: the registered operators on meta tensors (shapes, autograd graph), the
 modules' handling of parameters, and what importing the package loads."""
 import json
+import os
+import subprocess
+import sys
 
 import pytest
 
@@ -54,3 +57,54 @@ def test_forward_mode_without_a_gradient():
         with pytest.raises(RuntimeError):
             call(fwad.make_dual(x.clone().requires_grad_(True), torch.empty_like(x)))
     assert torch.func.jvp(call, (x,), (torch.empty_like(x),))[0].shape == grad.shape
+
+
+def _in_fresh_process(code, *args):
+    root = os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "quick-mlp_b200")
+    run = subprocess.run([sys.executable, "-c", f"import sys; sys.path.insert(0, {root!r})\n" + code, *args], capture_output=True, text=True)
+    assert run.returncode == 0, run.stderr[-2000:]
+
+
+def test_import_loads_no_native_library():
+    """Importing the package (its configurations, the stock PyTorch modules) needs none of the native libraries."""
+    _in_fresh_process("""
+import qmlp
+from qmlp import configs
+qmlp.SimulatedNetwork(configs.dumps(configs.config2()))
+maps = open("/proc/self/maps").read()
+assert "qmlp_calls" not in maps and "libqmlp_b200" not in maps
+""")
+
+
+def test_saved_graph_runs_before_any_object_exists(tmp_path):
+    """A traced graph that is loaded in a process which has only imported the package: the first call of the operator loads
+    its kernels, on the way to a gradient too."""
+    import torch
+    cfg, x, table, grad = _operands(requires_grad=False)
+
+    class Module(torch.nn.Module):
+        def forward(self, x, table):
+            return torch.ops.qmlp_b200.encoding_forward(x, table, cfg)
+    path = str(tmp_path / "graph.pt")
+    torch.jit.save(torch.jit.trace(Module(), (x, table), check_trace=False), path)
+    _in_fresh_process(f"""
+import torch, qmlp
+graph = torch.jit.load(sys.argv[1])
+x, table = torch.empty((10, 2), device="meta", requires_grad=True), torch.empty(({table.numel()},), device="meta", requires_grad=True)
+out = graph(x, table)
+out.sum().backward()
+assert tuple(out.shape) == {tuple(grad.shape)} and x.grad.shape == x.shape and table.grad.shape == table.shape
+""", path)
+
+
+def test_operators_of_other_devices_and_their_names():
+    import torch
+    import qmlp
+    from qmlp._capi import QmlpError
+    cfg, x, table, grad = _operands()
+    with pytest.raises(QmlpError, match="CUDA device"):
+        torch.ops.qmlp_b200.encoding_forward(torch.zeros(x.shape), torch.zeros(table.shape), cfg)
+    with pytest.raises(QmlpError, match="CUDA device"):
+        qmlp.ops.activation_adjoint(torch.zeros((4, 16)), torch.zeros((4, 16)), "relu")
+    assert qmlp.ops.encoding_forward(x, table, cfg).shape == grad.shape
+    assert torch.Tag.pt2_compliant_tag in torch.ops.qmlp_b200.encoding_forward.default.tags
