@@ -93,7 +93,11 @@ class FusedNetwork(torch.nn.Module):
         shape = x.shape
         assert len(shape) == 2
         assert shape[1] == self._num_input_channels
-        weights = self._parameters["weights"]     # (the attribute lookup of a module is a good part of a small call)
+        # the attribute lookup of a module is a good part of a small call; a parametrised or pruned weight, or that of a
+        # data-parallel replica, is an attribute only
+        weights = self._parameters.get("weights")
+        if weights is None:
+            weights = self.weights
         if weights.dtype == torch.float16 and torch.is_grad_enabled() and weights.requires_grad:
             warnings.warn("Attempt to train network with 16-bit weights: the gradient tensor will also have 16-bit "
                           "precision. Consider weight_dtype=torch.float32.")

@@ -108,3 +108,44 @@ def test_operators_of_other_devices_and_their_names():
         qmlp.ops.activation_adjoint(torch.zeros((4, 16)), torch.zeros((4, 16)), "relu")
     assert qmlp.ops.encoding_forward(x, table, cfg).shape == grad.shape
     assert torch.Tag.pt2_compliant_tag in torch.ops.qmlp_b200.encoding_forward.default.tags
+
+
+class _Doubled:
+    """Stands for the native network: what forward() passes on."""
+    def forward(self, x, weights, encoding_parameters):
+        return x, weights, encoding_parameters
+
+
+def _cpu_network(cfg):
+    import qmlp
+    net = qmlp.FusedNetwork(specs.dumps(cfg), weight_dtype=__import__("torch").float32, device="cpu")
+    native, net._network = net._network, _Doubled()
+    net._keep = native
+    return net
+
+
+def test_forward_takes_weights_that_are_no_parameter():
+    """Parametrised and pruned weights, and those of a DataParallel replica, are attributes of the module but not in its
+    parameter dictionary."""
+    import torch
+    from torch.nn.utils import parametrize, prune
+
+    class Twice(torch.nn.Module):
+        def forward(self, w):
+            return 2 * w
+    cfg = specs.config1()
+    x = torch.zeros((4, 3))
+    net = _cpu_network(cfg)
+    before = net.weights.detach().clone()
+    parametrize.register_parametrization(net, "weights", Twice())
+    assert torch.equal(net(x)[1], 2 * before)
+    net = _cpu_network(cfg)
+    prune.random_unstructured(net, "weights", 0.5)
+    assert torch.equal(net(x)[1], net.weights_orig * net.weights_mask)
+    net = _cpu_network(cfg)
+    replica = net._replicate_for_data_parallel()
+    replica.weights = before
+    assert replica(x)[1] is before
+    net = _cpu_network(cfg)
+    other = torch.zeros_like(net.weights)
+    assert torch.func.functional_call(net, {"weights": other}, (x,))[1] is other
