@@ -17,7 +17,6 @@ class FusedNetwork(torch.nn.Module):
         self._cfg, self._parent = cfg, parent
         self._network = Network(cfg, parent)
         self._num_output_channels = self._network.channels_out()
-        self._num_input_channels = self._network.channels_in()
         self._num_layers = self._network.num_layers()
 
         weights = self._network.create_inference_parameters(device)
@@ -30,8 +29,6 @@ class FusedNetwork(torch.nn.Module):
         self._num_encodings = self._network.num_encodings()
         assert self._num_encodings > 0
         self._encodings = [self._network.encoding(i) for i in range(self._num_encodings)]
-        self._encoding_has_parameters = [e.has_parameters() for e in self._encodings]
-        self._no_encoding_parameters = not any(self._encoding_has_parameters)
         params = []
         for e in self._encodings:
             if e.has_parameters():
@@ -39,8 +36,19 @@ class FusedNetwork(torch.nn.Module):
             else:
                 params.append(torch.nn.Parameter(torch.zeros((1,), device=device), requires_grad=False))
         self.encoding_parameters = torch.nn.ParameterList(params)
+        self._remember_shape()
         if verbose:
             print("Number of trainable network parameters:", weights.shape)
+
+    def _remember_shape(self):
+        """What forward() needs to know of the network, without a call into the library."""
+        self._num_input_channels = self._network.channels_in()
+        self._encoding_has_parameters = [e.has_parameters() for e in self._encodings]
+        self._no_encoding_parameters = not any(self._encoding_has_parameters)
+
+    def __setstate__(self, state):
+        super().__setstate__(state)
+        self._remember_shape()     # (modules saved without it)
 
     @staticmethod
     def MatrixSize() -> int:

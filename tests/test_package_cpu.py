@@ -149,3 +149,18 @@ def test_forward_takes_weights_that_are_no_parameter():
     net = _cpu_network(cfg)
     other = torch.zeros_like(net.weights)
     assert torch.func.functional_call(net, {"weights": other}, (x,))[1] is other
+
+
+def test_module_saved_without_the_cached_shape():
+    """A whole module pickled when it did not keep what forward() needs of the network."""
+    import pickle
+    import torch
+    import qmlp
+    net = qmlp.FusedNetwork(specs.dumps(specs.config3(log2_hashmap_size=12)), device="cpu")
+    for name in ("_num_input_channels", "_encoding_has_parameters", "_no_encoding_parameters"):
+        del net.__dict__[name]
+    loaded = pickle.loads(pickle.dumps(net))
+    loaded._network = _Doubled()
+    x = torch.zeros((4, 3))
+    _, weights, encodings = loaded(x)
+    assert torch.equal(weights, net.weights) and len(encodings) == 1 and torch.equal(encodings[0], net.encoding_parameters[0])
