@@ -316,7 +316,9 @@ void EncodingHashGrid::planReplicas(int64_t points, int group, kernel::GradRepli
     // A point sends 2^(D-1) reductions per level (neighbouring corners leave as one) to the lines of the level. Up to
     // 2048 per line they hide behind the rest of the kernel (a line takes about nine clocks each); above that, as many
     // copies as bring a line back to that number, 64 at most.
-    if (isLine() || Library::instance().boundsCheck) return;
+    // The plan, and with it the size of the scratch memory, depends on the grid and the number of points alone: memory sized
+    // under one set of tuning switches serves a call under another.
+    if (isLine()) return;
     const double reductions = static_cast<double>(points) * (1 << (dim_ - 1));
     for (int l = 0; l < levels_ && group + l < kernel::MAX_GRID_LEVELS; ++l) {
         const int64_t elements = (l + 1 < levels_ ? table_[l + 1].memoryOffset : numParameters_) - table_[l].memoryOffset;

@@ -58,23 +58,37 @@ __device__ __forceinline__ unsigned int grid_vertex_index(const unsigned int (&v
     return idx * F + lv.offset;
 }
 
-// Element index of corner `bits` of a cell (bit k set -> high corner in dimension k). Every table access of every kernel
-// takes its index from here, so this is where a QMLP_BOUNDS_CHECK build tests it: a row that does not lie inside the
-// table is reported through the status word and replaced by row 0 of the table, and the kernel carries on.
+// Every table access of every kernel passes its element index through here, so this is where a QMLP_BOUNDS_CHECK build tests
+// it: a row that does not lie inside its level is reported through the status word and replaced by the level's first row
+// (which the copies of a level's gradient hold too), and the kernel carries on.
+template <int D, int F>
+__device__ __forceinline__ unsigned int grid_checked_index(const GridP& g, const GridLevelP& lv, unsigned int e)
+{
+    if constexpr (BOUNDS_CHECK) {
+        unsigned long long rows = lv.hashGridSize;
+        if (!lv.hashed) {
+            rows = 1;
+#pragma unroll
+            for (int k = 0; k < D; ++k) rows *= static_cast<unsigned long long>(lv.resolution);
+        }
+        const unsigned long long last = lv.offset + rows * F, end = last < g.tableCount ? last : g.tableCount;
+        if (e < lv.offset || static_cast<unsigned long long>(e) + F > end) {
+            if (g.status != nullptr) atomicOr(g.status, STATUS_TABLE_ROW);
+            return lv.offset;
+        }
+    }
+    (void)g; (void)lv;
+    return e;
+}
+
+// element index of corner `bits` of a cell (bit k set -> high corner in dimension k)
 template <int D, int F>
 __device__ __forceinline__ unsigned int grid_corner_index(const GridP& g, const GridCell<D>& c, const GridLevelP& lv, int bits)
 {
     unsigned int v[D];
 #pragma unroll
     for (int k = 0; k < D; ++k) v[k] = ((bits >> k) & 1) ? c.hi[k] : c.lo[k];
-    const unsigned int e = grid_vertex_index<D, F>(v, lv);
-    if constexpr (BOUNDS_CHECK) {
-        if (static_cast<unsigned long long>(e) + F > g.tableCount) {
-            if (g.status != nullptr) atomicOr(g.status, STATUS_TABLE_ROW);
-            return 0u;
-        }
-    }
-    return e;
+    return grid_checked_index<D, F>(g, lv, grid_vertex_index<D, F>(v, lv));
 }
 
 // encoding_hashgrid.cuh:177-185,209-215: product taken from dimension D-1 down to 0
@@ -348,14 +362,7 @@ struct GridHalfCell {
 #pragma unroll
             for (int k = 1; k < D; ++k) idx = v[k] + idx * static_cast<unsigned int>(lv.resolution);
         }
-        const unsigned int e = idx * F + lv.offset;
-        if constexpr (BOUNDS_CHECK) {
-            if (static_cast<unsigned long long>(e) + F > g.tableCount) {
-                if (g.status != nullptr) atomicOr(g.status, STATUS_TABLE_ROW);
-                return 0u;
-            }
-        }
-        return e;
+        return grid_checked_index<D, F>(g, lv, idx * F + lv.offset);
     }
     __device__ __forceinline__ float weight(int h) const
     {
@@ -578,6 +585,7 @@ __device__ __forceinline__ float* grid_grad_of_cta(const GridP& g, const GradRep
 {
     if (group >= MAX_GRID_LEVELS || r.log2Copies[group] == 0) return g.grad;
     const int n = grid_level_elements(g, l, levels);
+    if (BOUNDS_CHECK && n <= 0) return g.grad;   // (a table declared shorter than it is)
     return r.base + r.offset[group] + (blockIdx.x & ((1u << r.log2Copies[group]) - 1u)) * n - g.levels[l].offset;
 }
 // sum of the copies of a level -> its gradient (grid-stride over blockIdx.x, 256 threads)

@@ -335,3 +335,49 @@ def test_bounds_check_reports_instead_of_faulting(bounds_check):
     assert not (status & 1)
     assert bool(torch.isfinite(tr.gradient).all())
     assert bindings.QuickMLP.device_status() == 0                          # reading the word cleared it
+
+
+def test_scratch_memory_does_not_depend_on_the_switches():
+    """Scratch sized with bounds_check on serves a call with it off: the workspace a trainer keeps for a number of points, and
+    the adjoint scratch an autograd node asked for in its forward call. 2^18 points: the coarse levels have copies."""
+    import torch
+    from qmlp import bindings
+    from qmlp.trainer import FusedTrainer
+    cfg = specs.config3(log2_hashmap_size=12)
+    spec = oracle.parse_spec(cfg)
+    n = 1 << 18
+    x = torch.from_numpy(helpers.uniform(84, 1, (n, 3))).cuda()
+    t = torch.from_numpy(helpers.uniform(84, 2, (n, 1), -1.0, 1.0)).cuda()
+    params = torch.from_numpy(helpers.xavier_parameters(spec, cfg, bias_scale=0.05)).cuda()
+    table = torch.from_numpy(helpers.grid_tables(spec, scale=0.5)[0]).cuda()
+
+    def switch(value):
+        bindings.QuickMLP.set_tuning("bounds_check", value)
+    trained, differentiated = [], []
+    net = bindings.Network(json.dumps(cfg))
+    tr = FusedTrainer(bindings.Network(json.dumps(cfg)))
+    tr.set_parameters(params, [table])
+    try:
+        for before, after in ((1, 0), (0, 0)):
+            switch(before)
+            tr.backend.gradients(x, t, n, tr.loss_sum)
+            switch(after)
+            tr.gradient.zero_()
+            tr.backend.gradients(x, t, n, tr.loss_sum)
+            trained.append(tr.gradient.clone())
+            tr.gradient.zero_()
+        for before, after in ((1, 0), (0, 0)):
+            switch(before)
+            w, tb = params.float().requires_grad_(True), table.half().requires_grad_(True)
+            out = net.forward(x, w, [tb])
+            switch(after)
+            out.backward(t)
+            torch.cuda.synchronize()
+            differentiated.append((w.grad, tb.grad.float()))
+    finally:
+        switch(0)
+    assert bindings.QuickMLP.device_status() == 0
+    # fp32 sums in another order; a rounding to fp16 that flips moves a relu now and then
+    assert float((trained[0] - trained[1]).norm()) <= 1e-2 * float(trained[1].norm()) > 0
+    for a, b in zip(*differentiated):
+        assert float((a - b).norm()) <= 1e-2 * float(b.norm()) > 0
