@@ -750,25 +750,29 @@ int qmlp_network_adjoint(qmlp_network_t* net, const qmlp_tensor_t* input, const 
     QMLP_CATCH
 }
 
-// Forward and backward with the layers computed a second time (kernels/fused_train_tc.cuh): which calls can take them
-static bool recomputes(Network& n, int64_t points, int flags)
+// Forward and backward with the layers computed a second time (kernels/fused_train_tc.cuh). canRecompute: whether the network and
+// the gradients asked for have the pair; recomputes: whether a forward call takes it. The backward call of a forward call that
+// did must not depend on the switches in between.
+static bool canRecompute(Network& n, int64_t points, int flags)
 {
     bool grid = false, line = false;
     for (int i = 0; i < n.numEncodings(); ++i) {
         grid = grid || n.encoding(i)->hasParameters();
         line = line || n.encoding(i)->isLine();
     }
-    const Library& lib = Library::instance();
     // (the weight gradients come with the pass; the position gradient of a grid has no pass of its own)
-    if (points <= 0 || line || !(flags & QMLP_GRADIENTS_NETWORK_WEIGHTS) || ((flags & QMLP_GRADIENTS_INPUT) && grid) || lib.kernelPath == 1 ||
-        lib.boundsCheck || lib.splitScatter == 0)
-        return false;
+    if (points <= 0 || line || !(flags & QMLP_GRADIENTS_NETWORK_WEIGHTS) || ((flags & QMLP_GRADIENTS_INPUT) && grid)) return false;
     if (n.recomputeKernel < 0) {
         kernel::LaunchArgs none;
         std::memset(&none, 0, sizeof none);
         n.recomputeKernel = n.module(n.currentHalfMask())->launch(kernel::KERNEL_BACKWARD_FEATURES, &none, nullptr, nullptr) == 0 ? 1 : 0;
     }
     return n.recomputeKernel == 1;
+}
+static bool recomputes(Network& n, int64_t points, int flags)
+{
+    const Library& lib = Library::instance();
+    return lib.kernelPath != 1 && !lib.boundsCheck && lib.splitScatter != 0 && canRecompute(n, points, flags);
 }
 
 int qmlp_network_recompute_memory(qmlp_network_t* net, int64_t num_elements, int adjoint_flags, size_t* forward_bytes, size_t* adjoint_bytes)
@@ -813,7 +817,7 @@ int qmlp_network_adjoint_recompute(qmlp_network_t* net, const qmlp_tensor_t* inp
     checkIO(n, input, adj_output, "adjOutput");
     const int64_t numel = input->sizes[0];
     if (numel == 0) return QMLP_OK;
-    if (!recomputes(n, numel, adjoint_flags)) throw std::runtime_error("this call has no recomputing backward pass (qmlp_network_recompute_memory returns 0)");
+    if (!canRecompute(n, numel, adjoint_flags)) throw std::runtime_error("this call has no recomputing backward pass (qmlp_network_recompute_memory returns 0)");
     if (!n.paramGradients.defined()) throw std::runtime_error("Weight gradients requested, but no gradient tensor is bound (setNetworkParameter(..., GRADIENTS))");
     if (!tmp_forward) throw std::runtime_error("tmpMemoryForward is null: run forward() first");
     kernel::LaunchArgs a;

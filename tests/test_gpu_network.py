@@ -696,3 +696,30 @@ def test_recomputing_backward_pass(name, n):
         norm = float(gb.norm())
         assert norm > 0 or n == 1     # (a single point may sit where a relu output is zero)
         assert float((ga - gb).norm()) <= 1e-2 * norm, f"{name} n={n} result {i}: {float((ga - gb).norm())} of {norm}"
+
+
+@pytest.mark.parametrize("switch", ["kernel_path", "split_scatter"])
+def test_backward_after_a_switch(switch):
+    """The backward pass of a forward call that keeps the encoded features only does not depend on the switches that forward
+    calls choose by."""
+    import torch
+    from qmlp import bindings
+    cfg, rng, spec, net, params, tables, acts, t_params, t_tables = _setup("config3_small")
+    x = torch.from_numpy(helpers.uniform(63, 1, (3000, 3), *rng)).cuda()
+    adj = torch.from_numpy(helpers.uniform(63, 2, (3000, 1), -1.0, 1.0)).cuda()
+    grads = []
+    for switched in (False, True):
+        w, tb = t_params.float().requires_grad_(True), t_tables[0].clone().requires_grad_(True)
+        out = net.forward(x, w, [tb])
+        try:
+            if switched and switch == "kernel_path":
+                bindings.QuickMLP.set_kernel_path(1)
+            elif switched:
+                bindings.QuickMLP.set_tuning(switch, 0)
+            out.backward(adj)
+        finally:
+            bindings.QuickMLP.set_kernel_path(0)
+            bindings.QuickMLP.set_tuning("split_scatter", -1)
+        grads.append((w.grad, tb.grad))
+    for a, b in zip(*grads):   # the same kernels: fp32 sums in another order
+        assert float((a - b).norm()) <= 1e-5 * float(a.norm()) > 0
