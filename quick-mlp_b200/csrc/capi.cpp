@@ -132,13 +132,16 @@ struct TimedLaunch {
 };
 
 // The launch arguments with the sizes of the scratch buffers they point to, for bounds-checking instantiations: the stash
-// and the delta stash hold n32 rows of the network's widths, the planes planeStride points of the encoded channels.
-kernel::LaunchArgs withScratchSizes(const Network& n, const kernel::LaunchArgs& a)
+// (of the encoded input alone, for the recomputing pair) and the delta stash hold n32 rows of the network's widths, the planes
+// planeStride points of the encoded channels.
+kernel::LaunchArgs withScratchSizes(const Network& n, int kernelId, const kernel::LaunchArgs& a)
 {
     kernel::LaunchArgs b = a;
     const long long n32 = (a.numel + 31) / 32 * 32;
+    const bool features = kernelId == kernel::KERNEL_FORWARD_FEATURES || kernelId == kernel::KERNEL_BACKWARD_FEATURES;
+    const long long stashHalfs = features ? n.layer(0).channelsIn : n.stashHalfsPerPoint();
     const long long shrink = Library::instance().boundsShrink;
-    b.fwdTmpHalfs = a.fwdTmp ? std::max<long long>(1, n32 * n.stashHalfsPerPoint() - shrink) : 0;
+    b.fwdTmpHalfs = a.fwdTmp ? std::max<long long>(1, n32 * stashHalfs - shrink) : 0;
     b.adjTmpHalfs = a.adjTmp ? std::max<long long>(1, n32 * n.deltaHalfsPerPoint() - shrink) : 0;
     b.planeHalfs = a.planes ? std::max<long long>(1, a.planeStride * n.encodedChannels() - shrink) : 0;
     return b;
@@ -148,7 +151,7 @@ void launchModule(Network& n, KernelModule& m, int kernelId, const kernel::Launc
 {
     TimedLaunch timed(kernelId, static_cast<cudaStream_t>(stream));
     int launches = 0;
-    const kernel::LaunchArgs b = withScratchSizes(n, a);
+    const kernel::LaunchArgs b = withScratchSizes(n, kernelId, a);
     checkLaunch(m.launch(kernelId, &b, static_cast<cudaStream_t>(stream), &launches), "kernel launch failed");
     n.launchCount += launches;
 }
@@ -513,7 +516,7 @@ static void inferenceLocked(Network& n, const qmlp_tensor_t* input, qmlp_tensor_
             int e;
             {
                 TimedLaunch timed(kernel::KERNEL_ENCODE_PLANES, static_cast<cudaStream_t>(stream));
-                const kernel::LaunchArgs sized = withScratchSizes(n, a);
+                const kernel::LaunchArgs sized = withScratchSizes(n, kernel::KERNEL_ENCODE_PLANES, a);
                 e = m->launch(kernel::KERNEL_ENCODE_PLANES, &sized, static_cast<cudaStream_t>(stream), &launches);
             }
             if (e == static_cast<int>(cudaErrorNotSupported) && c0 == 0) { n.planesUnsupported = true; ok = false; break; }
@@ -772,7 +775,7 @@ static bool canRecompute(Network& n, int64_t points, int flags)
 static bool recomputes(Network& n, int64_t points, int flags)
 {
     const Library& lib = Library::instance();
-    return lib.kernelPath != 1 && !lib.boundsCheck && lib.splitScatter != 0 && canRecompute(n, points, flags);
+    return lib.kernelPath != 1 && lib.splitScatter != 0 && canRecompute(n, points, flags);
 }
 
 int qmlp_network_recompute_memory(qmlp_network_t* net, int64_t num_elements, int adjoint_flags, size_t* forward_bytes, size_t* adjoint_bytes)
@@ -1340,8 +1343,9 @@ int qmlp_trainer_gradients_part(qmlp_trainer_t* tr, const qmlp_tensor_t* input, 
     }
     // The layers' forward, loss, backward and weight gradients in one kernel on the planes (kernels/fused_train_tc.cuh),
     // for every network and batch it is instantiated for; the separate kernels below remain for wider networks, line
-    // integration, the sorted step, the mma.sync-only path and bounds-checking instantiations (which test the stash).
-    if (!sorted && (path == 0 || path == 2) && !lib.boundsCheck && lib.splitScatter != 0 && numel > 0) {
+    // integration, the sorted step, the mma.sync-only path and, on kernel path 2, the bounds-checking instantiations (so that
+    // both forms of the step can be checked).
+    if (!sorted && (path == 0 || (path == 2 && !lib.boundsCheck)) && lib.splitScatter != 0 && numel > 0) {
         auto m = n.module(n.currentHalfMask());
         if (n.trainKernel < 0) {
             kernel::LaunchArgs none = a;
@@ -1376,7 +1380,7 @@ int qmlp_trainer_gradients_part(qmlp_trainer_t* tr, const qmlp_tensor_t* input, 
             int e;
             {
                 TimedLaunch timed(kernel::KERNEL_ENCODE_PLANES, static_cast<cudaStream_t>(stream));
-                const kernel::LaunchArgs sized = withScratchSizes(n, a);
+                const kernel::LaunchArgs sized = withScratchSizes(n, kernel::KERNEL_ENCODE_PLANES, a);
                 e = m->launch(kernel::KERNEL_ENCODE_PLANES, &sized, static_cast<cudaStream_t>(stream), &launches);
             }
             if (e == static_cast<int>(cudaErrorNotSupported)) {

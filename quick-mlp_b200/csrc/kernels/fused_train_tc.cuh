@@ -247,7 +247,11 @@ __device__ __forceinline__ void fetch_piece(const LaunchArgs& p, long long point
             } else {
                 constexpr int F = Enc::F, i = (C - Enc::OUT_OFF) % F, W = plane_vector<Enc, C>();
                 const __half* at = p.planes + p.planeStride * (C - i) + point * F + i;
-                if constexpr (W == 8) {
+                if (!scratch_ok(p, at - p.planes, W, p.planeHalfs, STATUS_PLANES)) {
+#pragma unroll
+                    for (int w = j; w < j + W; w += 2)
+                        if (w % 2 == 0) v[w / 2] = 0u;
+                } else if constexpr (W == 8) {
                     const uint4 u = *reinterpret_cast<const uint4*>(at);
                     v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w;
                 } else if constexpr (W == 4) {
@@ -281,7 +285,7 @@ __device__ __forceinline__ void store_piece(const LaunchArgs& p, long long point
             } else {
                 constexpr int F = Enc::F, i = (C - Enc::OUT_OFF) % F, W = plane_vector<Enc, C>();
                 __half* at = p.planes + p.planeStride * (C - i) + point * F + i;
-                if (p.planes == nullptr) {}
+                if (p.planes == nullptr || !scratch_ok(p, at - p.planes, W, p.planeHalfs, STATUS_PLANES)) {}
                 else if constexpr (W == 8) *reinterpret_cast<uint4*>(at) = make_uint4(v[0], v[1], v[2], v[3]);
                 else if constexpr (W == 4) *reinterpret_cast<uint2*>(at) = make_uint2(v[j / 2], v[j / 2 + 1]);
                 else if constexpr (W == 2) *reinterpret_cast<uint32_t*>(at) = v[j / 2];
@@ -411,17 +415,19 @@ struct TrainSlot {
 template <class Spec, bool LOSS, int K>
 __device__ __forceinline__ void train_fetch(const LaunchArgs& p, TrainSlot<Spec, LOSS>& sl, int wg, long long point)
 {
-    constexpr int WG = TrainSlot<Spec, LOSS>::WG;
+    constexpr int WG = TrainSlot<Spec, LOSS>::WG, CIN0 = Spec::CIN[0];
     if constexpr (K < TrainSlot<Spec, LOSS>::PIECES * WG) {
         if (wg == K % WG) {
             uint32_t (&v)[4] = sl.features[K / WG];
-            if constexpr (K * 8 < Spec::CIN[0]) {
+            if constexpr (K * 8 < CIN0) {
                 if (point < p.numel) {
                     if constexpr (LOSS) {
                         fetch_piece<Spec, K * 8, K * 8 + 8>(p, point, v);
-                    } else {
-                        const uint4 u = *reinterpret_cast<const uint4*>(p.fwdTmp + point * Spec::CIN[0] + K * 8);
+                    } else if (const long long at = point * CIN0 + K * 8; scratch_ok(p, at, 8, p.fwdTmpHalfs, STATUS_STASH)) {
+                        const uint4 u = *reinterpret_cast<const uint4*>(p.fwdTmp + at);
                         v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w;
+                    } else {
+                        v[0] = v[1] = v[2] = v[3] = 0u;
                     }
                 }
                 else v[0] = v[1] = v[2] = v[3] = 0u;

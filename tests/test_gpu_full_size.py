@@ -337,6 +337,55 @@ def test_bounds_check_reports_instead_of_faulting(bounds_check):
     assert bindings.QuickMLP.device_status() == 0                          # reading the word cleared it
 
 
+def test_bounds_check_reaches_the_step_and_the_recomputing_pair(bounds_check):
+    """With bounds_check on, the training step and an autograd call run the kernels that they run without it, in instantiations
+    that test the planes and the stash of features: silent with honest sizes, reported and skipped with sizes declared
+    3000 elements smaller."""
+    import ctypes as C
+    import torch
+    from qmlp import bindings
+    from qmlp._capi import check, lib
+    from qmlp.trainer import FusedTrainer
+    cfg = specs.config3(log2_hashmap_size=12)
+    spec = oracle.parse_spec(cfg)
+    n = 5000
+    x = torch.from_numpy(helpers.uniform(85, 1, (n, 3))).cuda()
+    t = torch.from_numpy(helpers.uniform(85, 2, (n, 1), -1.0, 1.0)).cuda()
+    params = torch.from_numpy(helpers.xavier_parameters(spec, cfg, bias_scale=0.05)).cuda()
+    table = torch.from_numpy(helpers.grid_tables(spec, scale=0.5)[0]).cuda()
+    tr = FusedTrainer(bindings.Network(json.dumps(cfg)))
+    tr.set_parameters(params, [table])
+    net = bindings.Network(json.dumps(cfg))
+
+    def step():
+        tr.gradient.zero_()
+        tr.backend.gradients(x, t, n, tr.loss_sum)
+        return [tr.gradient.clone()]
+
+    def autograd():
+        w, tb = params.float().requires_grad_(True), table.half().requires_grad_(True)
+        net.forward(x, w, [tb]).backward(t)
+        return [w.grad, tb.grad]
+    for call, kernel in ((step, 14), (autograd, 17)):
+        ids, ms, launches = (C.c_int * 64)(), (C.c_float * 64)(), (C.c_int * 64)()
+        check(lib().qmlp_set_kernel_timing(1))
+        try:
+            call()
+            torch.cuda.synchronize()
+            count = lib().qmlp_read_kernel_timing(64, ids, ms, launches)
+        finally:
+            check(lib().qmlp_set_kernel_timing(0))
+        assert kernel in ids[:count]
+        assert bindings.QuickMLP.device_status() == 0
+        bindings.QuickMLP.set_tuning("bounds_shrink", 3000)
+        result = call()
+        status = bindings.QuickMLP.device_status()
+        bindings.QuickMLP.set_tuning("bounds_shrink", 0)
+        assert status & 8 and not status & 1
+        assert (status & 4) or kernel == 14          # the step keeps no stash
+        assert all(bool(torch.isfinite(r).all()) for r in result)
+
+
 def test_scratch_memory_does_not_depend_on_the_switches():
     """Scratch sized with bounds_check on serves a call with it off: the workspace a trainer keeps for a number of points, and
     the adjoint scratch an autograd node asked for in its forward call. 2^18 points: the coarse levels have copies."""
