@@ -822,7 +822,8 @@ int qmlp_network_adjoint_recompute(qmlp_network_t* net, const qmlp_tensor_t* inp
     if (numel == 0) return QMLP_OK;
     if (!canRecompute(n, numel, adjoint_flags)) throw std::runtime_error("this call has no recomputing backward pass (qmlp_network_recompute_memory returns 0)");
     if (!n.paramGradients.defined()) throw std::runtime_error("Weight gradients requested, but no gradient tensor is bound (setNetworkParameter(..., GRADIENTS))");
-    if (!tmp_forward) throw std::runtime_error("tmpMemoryForward is null: run forward() first");
+    if (!tmp_forward || (reinterpret_cast<uintptr_t>(tmp_forward) & 15) != 0)
+        throw std::runtime_error("tmpMemoryForward is null or not 16-byte aligned: run forward() first");
     kernel::LaunchArgs a;
     fillCommon(n, a, input);
     a.adjOutput = static_cast<const float*>(adj_output->data);

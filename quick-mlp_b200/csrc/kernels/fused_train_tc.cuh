@@ -677,6 +677,7 @@ __device__ __forceinline__ void train_flush(const LaunchArgs& p, uint32_t wgTmem
         constexpr int CHUNKS = TR::wgCols(L) / 16;
         float* gw = p.gradWeights + Spec::WOFF[L];
         float* gb = p.gradWeights + (BIAS ? Spec::BOFF[L] : 0);
+        const bool vec = (reinterpret_cast<uintptr_t>(gw) & 15) == 0;   // (a caller's gradient vector may start anywhere)
         for (int c = warpgroup; c < CHUNKS; c += TRAIN_WARPGROUPS) {
             const int col = c * 16;
             float v[16];
@@ -686,7 +687,14 @@ __device__ __forceinline__ void train_flush(const LaunchArgs& p, uint32_t wgTmem
                 if (lane < COUT) {
                     if (col < CIN) {
 #pragma unroll
-                        for (int i = 0; i < 16; i += 4) red_add_v4_f32(gw + lane * CIN + col + i, v[i], v[i + 1], v[i + 2], v[i + 3]);
+                        for (int i = 0; i < 16; i += 4) {
+                            float* at = gw + lane * CIN + col + i;
+                            if (vec) red_add_v4_f32(at, v[i], v[i + 1], v[i + 2], v[i + 3]);
+                            else {
+#pragma unroll
+                                for (int e = 0; e < 4; ++e) red_add_f32(at + e, v[i + e]);
+                            }
+                        }
                     } else if constexpr (BIAS) {
                         red_add_f32(gb + lane, v[0]);
                     }

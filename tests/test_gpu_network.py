@@ -723,3 +723,39 @@ def test_backward_after_a_switch(switch):
         grads.append((w.grad, tb.grad))
     for a, b in zip(*grads):   # the same kernels: fp32 sums in another order
         assert float((a - b).norm()) <= 1e-5 * float(a.norm()) > 0
+
+
+@pytest.mark.parametrize("offset", [0, 1, 2, 3])
+@pytest.mark.parametrize("name", ["config2", "config4_small"])
+def test_recomputing_pair_with_a_gradient_vector_at_any_offset(name, offset):
+    """A caller of the C entry points may bind a gradient vector that starts at any element (16-byte reductions where they are
+    aligned, scalar ones elsewhere), with weight gradients taken as delta^T * input and as input^T * delta."""
+    import torch
+    from qmlp import _capi
+    from qmlp._capi import check, lib, wrap
+    cfg, rng, spec, net, params, tables, acts, t_params, t_tables = _setup(name)
+    n = 3000
+    x = torch.from_numpy(helpers.uniform(64, 1, (n, spec.num_inputs), *rng)).cuda()
+    adj = torch.from_numpy(helpers.uniform(64, 2, (n, spec.num_outputs), -1.0, 1.0)).cuda()
+    out = torch.empty_like(adj)
+    check(lib().qmlp_network_set_parameter(net._h, wrap(t_params), _capi.QMLP_INFERENCE))
+    for i, t in enumerate(t_tables):
+        if t is not None:
+            net.encoding(i).set_parameter(t, _capi.QMLP_INFERENCE)
+    forward, adjoint = C.c_size_t(), C.c_size_t()
+    check(lib().qmlp_network_recompute_memory(net._h, n, 2, C.byref(forward), C.byref(adjoint)))
+    assert forward.value > 0
+    tmp = torch.empty((forward.value + 16,), dtype=torch.uint8, device="cuda")
+    check(lib().qmlp_network_forward_recompute(net._h, wrap(x), wrap(out), tmp.data_ptr(), None))
+    grads = []
+    for off in (0, offset):
+        buf = torch.zeros((spec.num_parameters + 4,), device="cuda")
+        g = buf[off:off + spec.num_parameters]
+        check(lib().qmlp_network_set_parameter(net._h, wrap(g), _capi.QMLP_GRADIENTS))
+        check(lib().qmlp_network_adjoint_recompute(net._h, wrap(x), wrap(adj), 2, None, tmp.data_ptr(), None, None))
+        torch.cuda.synchronize()
+        assert float(buf[:off].abs().sum()) == 0.0 and float(buf[off + spec.num_parameters:].abs().sum()) == 0.0
+        grads.append(g.clone())
+    assert float((grads[0] - grads[1]).norm()) <= 1e-5 * float(grads[0].norm()) > 0      # fp32 sums in another order
+    with pytest.raises(_capi.QmlpError):
+        check(lib().qmlp_network_adjoint_recompute(net._h, wrap(x), wrap(adj), 2, None, tmp.data_ptr() + 2, None, None))
