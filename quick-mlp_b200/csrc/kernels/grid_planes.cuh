@@ -284,13 +284,23 @@ struct PlaneLaunchers {
             const long long cap = 1ll << 30;
             if (bx > cap) bx = cap;
             if (bx < 1) bx = 1;
-            // the copies of the hot levels among the ones of this launch
+            // The copies of the hot levels among the ones of this launch. Only these are cleared: the copies lie level by level, and
+            // launches of other ranges may run at the same time.
             const int begin = a.scatterLevelEnd > 0 ? a.scatterLevelBegin : 0, end = a.scatterLevelEnd > 0 ? a.scatterLevelEnd : groups;
             int sums = 0;   // the levels up to the last one that has copies
-            for (int g = begin; g < end && g < groups && g < MAX_GRID_LEVELS; ++g)
-                if (a.replicas.log2Copies[g] > 0) sums = g - begin + 1;
+            long long from = a.replicas.total, to = a.replicas.total;
+            for (int g = 0; g < groups && g < MAX_GRID_LEVELS; ++g) {
+                if (a.replicas.log2Copies[g] == 0) continue;
+                if (g >= begin && g < end) {
+                    if (sums == 0) from = a.replicas.offset[g];
+                    sums = g - begin + 1;
+                } else if (g >= end) {
+                    to = a.replicas.offset[g];
+                    break;
+                }
+            }
             if (sums > 0) {
-                const cudaError_t e = cudaMemsetAsync(a.replicas.base, 0, a.replicas.total * sizeof(float), s);
+                const cudaError_t e = cudaMemsetAsync(a.replicas.base + from, 0, (to - from) * sizeof(float), s);
                 if (e != cudaSuccess) return e;
             }
             scatter_planes_kernel<Spec><<<static_cast<unsigned>(bx), SCATTER_THREADS, 0, s>>>(a);

@@ -318,3 +318,35 @@ def test_scatter_with_copies_of_hot_levels():
     norm = float(grads[0].norm())
     assert norm > 0 and float((grads[1] - grads[0]).norm()) <= 1e-2 * norm
     assert float((grads[2] - grads[1]).norm()) <= 1e-5 * norm
+
+
+def test_level_ranges_on_two_streams():
+    """The level ranges of a step may be scattered on different streams: each launch clears and sums the copies of its own
+    levels only. 2^18 points: the coarse levels have copies."""
+    import torch
+    from qmlp import bindings
+    from qmlp.trainer import FusedTrainer
+    cfg = specs.config3(log2_hashmap_size=14)
+    spec = oracle.parse_spec(cfg)
+    tr = FusedTrainer(bindings.Network(json.dumps(cfg)))
+    tr.set_parameters(torch.from_numpy(helpers.xavier_parameters(spec, cfg, bias_scale=0.05)).cuda(),
+                      [torch.from_numpy(t).cuda() for t in helpers.grid_tables(spec, scale=0.5)])
+    n = 1 << 18
+    x = torch.from_numpy(helpers.uniform(86, 1, (n, 3))).cuda()
+    t = torch.from_numpy(helpers.uniform(86, 2, (n, 1), -1.0, 1.0)).cuda()
+    tr.backend.gradients(x, t, n, tr.loss_sum)
+    whole = tr.gradient.clone()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    for cuts in ([0, 2, 4, 16], [0, 1, 2, 3, 4, 5, 6, 16], [0, 16]):
+        tr.gradient.zero_()
+        tr.backend.gradients(x, t, n, tr.loss_sum, parts=4)
+        torch.cuda.synchronize()
+        for i, (begin, end) in enumerate(zip(cuts, cuts[1:])):
+            with torch.cuda.stream(streams[i & 1]):
+                tr.backend.gradients(x, t, n, tr.loss_sum, parts=8 | (begin << 8) | (end << 16))
+        torch.cuda.synchronize()
+        tr.backend.gradients(x, t, n, tr.loss_sum, parts=2)
+        # fp32 sums in another order
+        assert float((tr.gradient - whole).norm()) <= 1e-5 * float(whole.norm()) > 0
+        for begin, end in tr.backend.scatter_levels():
+            assert float((tr.gradient[begin:end] - whole[begin:end]).norm()) <= 1e-5 * float(whole[begin:end].norm()) > 0
