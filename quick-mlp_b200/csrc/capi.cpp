@@ -7,6 +7,7 @@
 #include <cmath>
 #include <cstring>
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 using namespace qmlp;
@@ -558,6 +559,29 @@ int qmlp_network_inference_with_memory(qmlp_network_t* net, const qmlp_tensor_t*
     QMLP_CATCH
 }
 
+// Device address of `bytes` bytes of host memory, or null unless all of them are page-locked as one piece (a caller may have
+// registered the beginning of a buffer only; a copy to such a buffer is an error, a kernel's write a fault).
+static float* mappedAddress(float* host, size_t bytes)
+{
+    using Query = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+    static const Query query = [] {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+        const bool ok = cudaGetDriverEntryPoint("cuPointerGetAttributes", &fn, cudaEnableDefault, &found) == cudaSuccess && found == cudaDriverEntryPointSuccess;
+        return ok ? reinterpret_cast<Query>(fn) : nullptr;
+    }();
+    if (query == nullptr) return nullptr;
+    unsigned type = 0;
+    CUdeviceptr device = 0, begin = 0;
+    size_t size = 0;
+    CUpointer_attribute which[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                   CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void* values[] = {&type, &device, &begin, &size};
+    // (attributes of memory the driver does not know are left at zero)
+    if (query(4, which, values, reinterpret_cast<CUdeviceptr>(host)) != CUDA_SUCCESS || type != CU_MEMORYTYPE_HOST || device == 0) return nullptr;
+    return device >= begin && device + bytes <= begin + size ? reinterpret_cast<float*>(device) : nullptr;
+}
+
 int qmlp_network_inference_host(qmlp_network_t* net, const float* host_input, float* host_output, int64_t num_points,
                                 int64_t chunk_points, qmlp_stream_t stream)
 {
@@ -570,14 +594,7 @@ int qmlp_network_inference_host(qmlp_network_t* net, const float* host_input, fl
     const int cin = n.channelsIn(), cout = n.channelsOut();
     // A page-locked result of one channel is written by the kernels themselves (a warp's results are one 128-byte line): no
     // download behind the last kernel, and nothing beside the uploads on the copy engines.
-    float* mapped = nullptr;
-    if (cout == 1) {
-        cudaPointerAttributes attr;
-        if (cudaPointerGetAttributes(&attr, host_output) == cudaSuccess && attr.type == cudaMemoryTypeHost)
-            mapped = static_cast<float*>(attr.devicePointer);
-        else
-            (void)cudaGetLastError();
-    }
+    float* mapped = cout == 1 ? mappedAddress(host_output, static_cast<size_t>(num_points) * sizeof(float)) : nullptr;
     // Default chunk: an eighth of the batch, with the results written in place between 2^18 and 2^20 points (a chunk costs the
     // host about 10 us of calls and is worth them only for the overlap of its kernel: 2^20 points in 8 / 4 / 2 chunks 372 / 289 /
     // 298 us, 2^18 points in 2 / 1 chunks 152 / 133 us), otherwise between 2^16 and 2^20 points (smaller chunks pay more per-copy

@@ -648,6 +648,35 @@ def test_inference_from_host_memory_under_capture(name, chunk):
     assert torch.equal(result(), ref)
 
 
+@pytest.mark.parametrize("registered", [0, 4096, 8192, 16384])
+def test_inference_from_host_memory_with_a_result_registered_in_part(registered):
+    """A result buffer whose first pages only are page-locked: nothing is written through the mapping. The copy either refuses it
+    or brings the whole result; a buffer registered to its end gets it in any case."""
+    import torch
+    from qmlp._capi import QmlpError
+    cfg, rng, spec, net, params, tables, acts, t_params, t_tables = _setup("config2")
+    n = 4096
+    x = torch.from_numpy(helpers.uniform(65, 1, (n, spec.num_inputs), *rng)).pin_memory()
+    ref = net.inference(x.cuda(), t_params).cpu()
+    raw = np.zeros(n + 1024, dtype=np.float32)
+    first = (-raw.ctypes.data) % 4096 // 4                   # a page boundary
+    out = torch.from_numpy(raw[first:first + n]).view(n, 1)
+    out.fill_(7.0)
+    rt = torch.cuda.cudart()
+    if registered:
+        assert int(rt.cudaHostRegister(out.data_ptr(), registered, 0)) == 0
+    try:
+        net.inference_host(x, t_params, output=out)
+        torch.cuda.synchronize()
+        assert torch.equal(out, ref)
+    except QmlpError:
+        assert registered in (4096, 8192)
+    finally:
+        torch.cuda.synchronize()
+        if registered:
+            assert int(rt.cudaHostUnregister(out.data_ptr())) == 0
+
+
 @pytest.mark.parametrize("n,offset", [(1, 0), (3, 0), (4, 0), (1024, 0), (1023, 0), (1024, 1), (4097, 2)])
 def test_convert_half(n, offset):
     """fp32 -> fp16 copy of a parameter vector: vector and scalar kernels, lengths and alignments either side of the rule."""
