@@ -1140,10 +1140,11 @@ int qmlp_convert_half(const float* src, uint16_t* dst, int64_t count, qmlp_strea
 
 // ---- fused training step -------------------------------------------------------------------------------------------
 // Workspace of one step, every part 256-byte aligned: forward stash and delta stash; dLoss/dOut; feature planes (forward
-// features first, then their adjoints); the copies of points and targets in bin order and the bin tables of the
+// features first, then their adjoints); copies of hot levels' gradients; weight gradients between the first and the second part
+// of a split step; the copies of points and targets in bin order and the bin tables of the
 // spatially binned step (only for networks with a grid encoding).
 struct TrainerLayout {
-    size_t adjOut = 0, planes = 0, replicas = 0, sortedInput = 0, sortedTarget = 0, bins = 0, total = 0;
+    size_t adjOut = 0, planes = 0, replicas = 0, weightSums = 0, sortedInput = 0, sortedTarget = 0, bins = 0, total = 0;
     int binCount = 0;
 };
 static TrainerLayout trainerLayout(const Network& n, int64_t points)
@@ -1158,6 +1159,8 @@ static TrainerLayout trainerLayout(const Network& n, int64_t points)
     b = align(b + adjointPlaneBytes(n, n32, QMLP_GRADIENTS_NETWORK_WEIGHTS | QMLP_GRADIENTS_INPUT_ENCODINGS));
     l.replicas = b;
     b = align(b + replicaBytes(n, points));
+    l.weightSums = b;
+    b = align(b + static_cast<size_t>(n.parameterCount()) * sizeof(float));
     const int dims = n.sortDimensions();
     if (dims > 0) {
         l.binCount = kernel::sort_bin_count(dims);
@@ -1375,9 +1378,21 @@ int qmlp_trainer_gradients_part(qmlp_trainer_t* tr, const qmlp_tensor_t* input, 
             a.planeStride = n32;
             a.flags = kernel::FLAG_GRAD_WEIGHTS | (anyGrid ? kernel::FLAG_GRAD_ENCODINGS : 0);
             if (what == 4 && !anyGrid) throw std::runtime_error("this network has no grid levels to scatter: use parts = 1");
+            // The weight gradients come with the layers, but belong to part 2 of a split step: until then they wait in the
+            // workspace.
+            float* sums = reinterpret_cast<float*>(ws + lay.weightSums);
+            if (what == 1 || what == 4) {
+                checkCuda(cudaMemsetAsync(sums, 0, static_cast<size_t>(n.parameterCount()) * sizeof(float), static_cast<cudaStream_t>(stream)), "cudaMemsetAsync");
+                a.gradWeights = sums;
+            }
             if (what & 5) {
                 if (anyGrid) launchModule(n, *m, kernel::KERNEL_ENCODE_PLANES, a, stream);
                 launchModule(n, *m, kernel::KERNEL_TRAIN, a, stream);
+            }
+            if (what == 2) {
+                checkCuda(kernel::launchAccumulate(sums, static_cast<float*>(n.paramGradients.data), n.parameterCount(), a.numSMs, static_cast<cudaStream_t>(stream)),
+                          "accumulate");
+                n.launchCount += 1;
             }
             if (what == 8) {
                 if (levelEnd <= levelBegin) throw std::runtime_error("empty range of grid levels");

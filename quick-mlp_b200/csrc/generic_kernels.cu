@@ -95,6 +95,19 @@ __global__ void __launch_bounds__(256) convert_half_kernel(const float* __restri
         dst[i] = __float2half(src[i]);
 }
 
+__global__ void __launch_bounds__(256) accumulate_kernel(const float* __restrict__ src, float* __restrict__ dst, long long count)
+{
+    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < count;
+         i += static_cast<long long>(gridDim.x) * blockDim.x)
+        dst[i] += src[i];
+}
+
+cudaError_t launchAccumulate(const float* src, float* dst, long long count, int numSMs, cudaStream_t stream)
+{
+    accumulate_kernel<<<gridFor(count, numSMs), 256, 0, stream>>>(src, dst, count);
+    return cudaGetLastError();
+}
+
 cudaError_t launchRefreshHalf(const float* master, uint16_t* halfCopy, long long count, int numSMs, cudaStream_t stream)
 {
     const long long count4 = count / 4;

@@ -12,6 +12,8 @@ cudaError_t launchAdam(float* master, float* grad, float* m, float* v, uint16_t*
                        int numSMs, cudaStream_t stream);
 // Address, on the current device, of the library's kernel status word (a __device__ variable).
 cudaError_t statusWordAddress(int** out);
+// dst += src
+cudaError_t launchAccumulate(const float* src, float* dst, long long count, int numSMs, cudaStream_t stream);
 cudaError_t launchRefreshHalf(const float* master, uint16_t* halfCopy, long long count, int numSMs, cudaStream_t stream);
 
 } // namespace kernel

@@ -350,3 +350,32 @@ def test_level_ranges_on_two_streams():
         assert float((tr.gradient - whole).norm()) <= 1e-5 * float(whole.norm()) > 0
         for begin, end in tr.backend.scatter_levels():
             assert float((tr.gradient[begin:end] - whole[begin:end]).norm()) <= 1e-5 * float(whole[begin:end].norm()) > 0
+
+
+@pytest.mark.parametrize("name", ["config3", "two_grids"])
+def test_first_part_leaves_the_weight_gradients(name):
+    """Part 1 of a split step makes the table gradients final and leaves the network segment alone; part 2 adds the weight
+    gradients of the same batch."""
+    import torch
+    from qmlp import bindings
+    from qmlp.trainer import FusedTrainer
+    cfg = specs.config3(log2_hashmap_size=14) if name == "config3" else two_grid_config()
+    spec = oracle.parse_spec(cfg)
+    tr = FusedTrainer(bindings.Network(json.dumps(cfg)))
+    tr.set_parameters(torch.from_numpy(helpers.xavier_parameters(spec, cfg, bias_scale=0.05)).cuda(),
+                      [torch.from_numpy(t).cuda() for t in helpers.grid_tables(spec, scale=0.5)])
+    n, first = 5000, tr.backend.segments[1]
+    x = torch.from_numpy(helpers.uniform(87, 1, (n, 3))).cuda()
+    t = torch.from_numpy(helpers.uniform(87, 2, (n, spec.num_outputs), -1.0, 1.0)).cuda()
+    tr.backend.gradients(x, t, n, tr.loss_sum)
+    whole = tr.gradient.clone()
+    tr.gradient.zero_()
+    tr.gradient[:first] = 1.0
+    tr.backend.gradients(x, t, n, tr.loss_sum, parts=1)
+    torch.cuda.synchronize()
+    assert bool((tr.gradient[:first] == 1.0).all())
+    # fp32 sums in another order
+    assert float((tr.gradient[first:] - whole[first:]).norm()) <= 1e-5 * float(whole[first:].norm()) > 0
+    tr.gradient[:first] = 0.0
+    tr.backend.gradients(x, t, n, tr.loss_sum, parts=2)
+    assert float((tr.gradient[:first] - whole[:first]).norm()) <= 1e-5 * float(whole[:first].norm()) > 0
