@@ -1377,7 +1377,8 @@ int qmlp_trainer_gradients_part(qmlp_trainer_t* tr, const qmlp_tensor_t* input, 
             a.planes = planes;
             a.planeStride = n32;
             a.flags = kernel::FLAG_GRAD_WEIGHTS | (anyGrid ? kernel::FLAG_GRAD_ENCODINGS : 0);
-            if (what == 4 && !anyGrid) throw std::runtime_error("this network has no grid levels to scatter: use parts = 1");
+            if ((what == 4 || what == 8) && !splitScatterChosen(n, a, planes != nullptr, sorted))
+                throw std::runtime_error("the scatter of this network does not go level by level (qmlp_trainer_scatter_levels returns 0): use parts = 1");
             // The weight gradients come with the layers, but belong to part 2 of a split step: until then they wait in the
             // workspace.
             float* sums = reinterpret_cast<float*>(ws + lay.weightSums);

@@ -379,3 +379,18 @@ def test_first_part_leaves_the_weight_gradients(name):
     tr.gradient[:first] = 0.0
     tr.backend.gradients(x, t, n, tr.loss_sum, parts=2)
     assert float((tr.gradient[:first] - whole[:first]).norm()) <= 1e-5 * float(whole[:first].norm()) > 0
+
+
+def test_level_ranges_are_refused_where_there_are_none():
+    """Networks without scatter levels (rows of four features) take parts 1, 2 and 3 only."""
+    import torch
+    from qmlp import bindings
+    from qmlp._capi import QmlpError
+    from qmlp.trainer import FusedTrainer
+    tr = FusedTrainer(bindings.Network(json.dumps(two_grid_config())))
+    assert tr.backend.scatter_levels() == []
+    x, t = torch.rand((100, 3), device="cuda"), torch.rand((100, 4), device="cuda")
+    for parts in (4, 8 | (0 << 8) | (1 << 16)):
+        with pytest.raises(QmlpError):
+            tr.backend.gradients(x, t, 100, tr.loss_sum, parts=parts)
+    assert float(tr.gradient.abs().max()) == 0.0
