@@ -34,7 +34,9 @@ int fail(int code, const std::string& msg)
 
 void checkCuda(cudaError_t e, const char* what)
 {
-    if (e != cudaSuccess) throw cuda_error(std::string(what) + ": " + cudaGetErrorString(e));
+    if (e == cudaSuccess) return;
+    (void)cudaGetLastError();   // reported here: the check after the next launch must not find it again
+    throw cuda_error(std::string(what) + ": " + cudaGetErrorString(e));
 }
 void checkLaunch(int e, const char* what)
 {

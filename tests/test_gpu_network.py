@@ -671,6 +671,7 @@ def test_inference_from_host_memory_with_a_result_registered_in_part(registered)
         assert torch.equal(out, ref)
     except QmlpError:
         assert registered in (4096, 8192)
+        assert torch.equal(net.inference(x.cuda(), t_params).cpu(), ref)     # an error is reported once
     finally:
         torch.cuda.synchronize()
         if registered:
