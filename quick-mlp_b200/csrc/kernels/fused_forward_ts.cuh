@@ -35,8 +35,10 @@ struct TsLayout {
     // warpgroups of a slot: 128 channels fit two slots only (192 columns each); with three warpgroups per slot (two / four) the
     // 64 -> 128 -> 128 -> 128 -> 4 layers of 2^22 points take 309 us (320 / 324; 406 with the operands in shared memory)
     static constexpr int WG = ACC == 128 ? 3 : 1;
-    static constexpr int FIT = (512 - ONES) / (ACC + OPERAND), SLOTS = FIT < 8 ? FIT : 8;
+    // slots that tensor memory and 1024 threads have room for (one layer of more than 64 outputs on few inputs: three by columns)
+    static constexpr int FIT = (512 - ONES) / (ACC + OPERAND), MOST = 8 / WG, SLOTS = FIT < MOST ? FIT : MOST;
     static constexpr int THREADS = SLOTS * WG * 128;
+    static_assert(SLOTS >= 1 && THREADS <= 1024, "slots of a CTA");
     __host__ __device__ static constexpr bool wideThroughout()
     {
         for (int i = 0; i + 1 < NL; ++i)

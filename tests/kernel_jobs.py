@@ -21,6 +21,8 @@ def jobs():
         out.append(("net", json.dumps(cfg), 0))
     for name, mask in (("config3_small", 1), ("config4_small", 3), ("config5_small", 1), ("grid2d_add_plus_identity", 1)):
         out.append(("net", json.dumps(tn.network_cases()[name][0]), mask))   # fp16 table variants
+    for cfg in tn.one_layer_configs().values():
+        out.append(("net", json.dumps(cfg), 0))
     for cfg in (tt.smooth_config3(), specs.config3(log2_hashmap_size=14)):
         out.append(("net", json.dumps(cfg), 0))
         out.append(("net", json.dumps(cfg), 1))

@@ -789,3 +789,48 @@ def test_recomputing_pair_with_a_gradient_vector_at_any_offset(name, offset):
     assert float((grads[0] - grads[1]).norm()) <= 1e-5 * float(grads[0].norm()) > 0      # fp32 sums in another order
     with pytest.raises(_capi.QmlpError):
         check(lib().qmlp_network_adjoint_recompute(net._h, wrap(x), wrap(adj), 2, None, tmp.data_ptr() + 2, None, None))
+
+
+def one_layer_configs():
+    """name -> network of one layer: few inputs and many outputs (three slots by tensor memory, two by threads), and the other way
+    round, with and without a grid and a bias"""
+    return {"16_to_128": specs.identity_net(16, [128], ["relu"]),
+            "40_to_100": specs.identity_net(40, [100], ["celu"], bias=False),
+            "100_to_7": specs.identity_net(100, [7], ["sine"]),
+            "grid_to_72": specs.grid_net(3, [specs.hashgrid(3, 4, 2, 10, 4, 48)], [72], ["identity"])}
+
+
+@pytest.mark.parametrize("n", [1, 129, 148 * 256 + 1])
+@pytest.mark.parametrize("name", ["16_to_128", "40_to_100", "100_to_7", "grid_to_72"])
+def test_one_layer(name, n):
+    """Networks of a single layer through the kernels picked for them and through the mma.sync ones (kernel path 1): inference,
+    the recomputing pair, and the kernel of a training step. Roundings to fp16 (2^-11) in the same places."""
+    import torch
+    from qmlp import bindings
+    from qmlp.trainer import FusedTrainer
+    cfg = one_layer_configs()[name]
+    spec, net = oracle.parse_spec(cfg), bindings.Network(json.dumps(cfg))
+    params = torch.from_numpy(helpers.xavier_parameters(spec, cfg, bias_scale=0.2)).cuda()
+    tables = [torch.from_numpy(t).cuda() if t is not None else None for t in helpers.grid_tables(spec, scale=0.7)]
+    grid = any(t is not None for t in tables)
+    x = torch.from_numpy(helpers.uniform(66, 1, (n, spec.num_inputs))).cuda()
+    adj = torch.from_numpy(helpers.uniform(66, 2, (n, spec.num_outputs), -1.0, 1.0)).cuda()
+    results = []
+    try:
+        for path in (1, 0, 2, 3):
+            bindings.QuickMLP.set_kernel_path(path)
+            r = [net.inference(x, params, tables)]
+            xx, w = x.clone().requires_grad_(not grid), params.float().requires_grad_(True)
+            tt = [t.clone().requires_grad_(True) if t is not None else None for t in tables]
+            net.forward(xx, w, tt).backward(adj)
+            r += [w.grad] + [t.grad for t in tt if t is not None] + ([] if grid else [xx.grad])
+            tr = FusedTrainer(net, grid_half_copy=False)
+            tr.set_parameters(params, tables)
+            tr.backend.gradients(x, adj, n, tr.loss_sum)
+            results.append(r + [tr.gradient, tr.loss_sum])
+            torch.cuda.synchronize()
+    finally:
+        bindings.QuickMLP.set_kernel_path(0)
+    for r in results[1:]:
+        for a, b in zip(r, results[0]):
+            assert float((a - b).norm()) <= 5e-3 * float(b.norm())
