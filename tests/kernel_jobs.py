@@ -23,6 +23,7 @@ def jobs():
         out.append(("net", json.dumps(tn.network_cases()[name][0]), mask))   # fp16 table variants
     for cfg in tn.one_layer_configs().values():
         out.append(("net", json.dumps(cfg), 0))
+    out.append(("net", json.dumps(tn.wide_grid_config()), 0))
     for cfg in (tt.smooth_config3(), specs.config3(log2_hashmap_size=14)):
         out.append(("net", json.dumps(cfg), 0))
         out.append(("net", json.dumps(cfg), 1))

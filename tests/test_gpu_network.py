@@ -491,16 +491,32 @@ def test_argument_errors():
     assert out.shape == (0, 1)
 
 
-@pytest.mark.parametrize("n", [1, 127, 128, 129, 148 * 128 + 1, 148 * 128 * 6 + 33])
-@pytest.mark.parametrize("name,path", [("config1", 3), ("config2", 3), ("uneven", 3), ("per_channel", 3), ("config3_small", 2),
-                                       ("config4_small", 2), ("config5_small", 2)])
+def wide_grid_config():
+    """A grid in front of hidden layers that are all wider than 64 channels: activations in tensor memory, two tiles in flight"""
+    return specs.grid_net(3, [specs.hashgrid(3, 8, 4, 10, 4, 48)], [128, 96, 128, 4], ["relu", "celu", "relu", "identity"])
+
+
+# Path 3 runs the kernel on identity inputs at any number of points. From feature planes (path 2) it runs from two tiles per SM
+# on (fewer points of a chunk go to the mma.sync kernel): 37 888 on 148 SMs. 16 tiles per SM give each of eight slots
+# its second tile.
+@pytest.mark.parametrize("name,path,n", [(name, 3, n) for name in ("config1", "config2", "uneven", "per_channel")
+                                         for n in (1, 127, 128, 129, 148 * 128 + 1, 148 * 128 * 6 + 33, 148 * 128 * 16 + 33)] +
+                                        [(name, 2, n) for name in ("config3_small", "config5_small", "wide_grid")
+                                         for n in (148 * 256 - 1, 148 * 256, 148 * 256 + 1, 148 * 256 + 127, 148 * 256 + 128, 148 * 256 + 129,
+                                                   148 * 128 * 16 + 33)])
 def test_activations_in_tensor_memory(name, path, n):
     """The kernel that keeps the activations in tensor memory (identity inputs, and feature planes): batches that end inside a
-    tile, fill one, and give a slot its second tile; 16 to 128 channels, with and without bias. Against the mma.sync
-    kernel: both round every layer to fp16 (2^-11), the fp32 sums differ in order."""
+    tile, fill one, and give a slot its second and third; 16 to 128 channels, with and without bias. Against the mma.sync
+    kernel: both round every layer to fp16 once (2^-11), the fp32 sums differ in order."""
     import torch
     from qmlp import bindings
-    cfg, rng, spec, net, params, tables, acts, t_params, t_tables = _setup(name)
+    if name == "wide_grid":
+        cfg, rng = wide_grid_config(), (0.0, 1.0)
+        spec, net = oracle.parse_spec(cfg), bindings.Network(json.dumps(cfg))
+        t_params = torch.from_numpy(helpers.xavier_parameters(spec, cfg, bias_scale=0.1)).cuda()
+        t_tables = [torch.from_numpy(t).cuda() for t in helpers.grid_tables(spec)]
+    else:
+        cfg, rng, spec, net, params, tables, acts, t_params, t_tables = _setup(name)
     x = torch.from_numpy(helpers.uniform(46, 1, (n, spec.num_inputs), *rng)).cuda()
     out = []
     try:
