@@ -1497,8 +1497,7 @@ int qmlp_trainer_update(qmlp_trainer_t* tr, int64_t step, float grad_scale, qmlp
         TimedLaunch timed(KERNEL_ID_ADAM, static_cast<cudaStream_t>(stream));
         checkCuda(kernel::launchAdam(tr->master, tr->grad, tr->m, tr->v, tr->half, tr->fusedCount, grad_scale, tr->cfg.beta1,
                                      tr->cfg.beta2, static_cast<float>(tr->cfg.learning_rate / bc1),
-                                     static_cast<float>(1.0 / std::sqrt(bc2)), tr->cfg.epsilon, Library::instance().smCount(),
-                                     static_cast<cudaStream_t>(stream)), "adam");
+                                     static_cast<float>(1.0 / std::sqrt(bc2)), tr->cfg.epsilon, static_cast<cudaStream_t>(stream)), "adam");
     }
     tr->net->launchCount += 1;
     QMLP_CATCH

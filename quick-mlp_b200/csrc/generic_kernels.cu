@@ -75,12 +75,11 @@ static unsigned gridFor(long long work, int numSMs)
 
 cudaError_t launchAdam(float* master, float* grad, float* m, float* v, uint16_t* halfCopy, long long count,
                        float gradScale, float beta1, float beta2, float stepSize, float invSqrtBc2, float eps,
-                       int numSMs, cudaStream_t stream)
+                       cudaStream_t stream)
 {
     // One CTA per 256 vectors, refilled by the hardware as they retire: 13 M parameters 65 us (5.2 TB/s), with 8 looping CTAs per
     // SM 72 us, with two vectors per thread in flight 72 us. (Streaming hints on the vectors: no change.)
     const long long count4 = count / 4;
-    (void)numSMs;
     adam_kernel<<<static_cast<unsigned>((count4 + 255) / 256), 256, 0, stream>>>(
         reinterpret_cast<float4*>(master), reinterpret_cast<float4*>(grad), reinterpret_cast<float4*>(m),
         reinterpret_cast<float4*>(v), reinterpret_cast<uint2*>(halfCopy), count4, gradScale, beta1, beta2, stepSize,

@@ -234,7 +234,7 @@ struct EncodingLaunchers {
         return cudaGetLastError();
     }
     template <bool INPUT_GRAD, bool PARAM_GRAD>
-    static cudaError_t adjoint(const LaunchArgs& a, cudaStream_t s)
+    static cudaError_t adjoint(const LaunchArgs& a, cudaStream_t s, int& count)
     {
         if constexpr (Enc::IS_GRID) {
             if constexpr (EncodingTile<Enc>::USED) {
@@ -246,6 +246,7 @@ struct EncodingLaunchers {
                 }
                 grid_encoding_adjoint_kernel<Enc, INPUT_GRAD, PARAM_GRAD><<<blocksFor(a, threads), threads, 0, s>>>(a);
                 if (copies) sum_replicas_kernel<Enc><<<dim3(32, Enc::L), 256, 0, s>>>(a);
+                count = copies ? 2 : 1;
                 return cudaGetLastError();
             }
         }
@@ -256,17 +257,17 @@ struct EncodingLaunchers {
     {
         const LaunchArgs& a = *static_cast<const LaunchArgs*>(args);
         cudaError_t e = cudaErrorInvalidValue;
-        bool none = false;
+        int count = 1;
         if (kernel == KERNEL_ENCODING_FORWARD) {
             e = forward(a, s);
         } else if (kernel == KERNEL_ENCODING_ADJOINT) {
             const bool ig = (a.flags & 1) != 0, pg = (a.flags & 2) != 0;
-            if (ig && pg) e = adjoint<true, true>(a, s);
-            else if (ig) e = adjoint<true, false>(a, s);
-            else if (pg) e = adjoint<false, true>(a, s);
-            else { e = cudaSuccess; none = true; }
+            if (ig && pg) e = adjoint<true, true>(a, s, count);
+            else if (ig) e = adjoint<true, false>(a, s, count);
+            else if (pg) e = adjoint<false, true>(a, s, count);
+            else { e = cudaSuccess; count = 0; }
         }
-        if (launches) *launches = e == cudaSuccess && !none ? 1 : 0;
+        if (launches) *launches = e == cudaSuccess ? count : 0;
         return static_cast<int>(e);
     }
 };
