@@ -1,4 +1,4 @@
-// Level-major encoding pass for networks whose grid tables do not fit in L2.
+// Level-major encoding pass, and the scatter of table gradients from planes.
 //
 // When the gather runs inside the fused kernel, every warp walks through all levels of its own points, so at any moment
 // the SMs touch all tables at once: with tables far larger than the 126 MB L2 (a 4-D grid of 16 levels of which 12 are hashed
@@ -6,8 +6,9 @@
 // of the data: the encodings of a chunk of points are computed one level at a time by the whole GPU (blockIdx.y =
 // level, the slow grid dimension), so the table of the level being processed (32 MB in fp16) stays resident in L2 and
 // corner fetches hit it there. The features go to level-major planes ([level][point][F] halfs, coalesced 4/8/16-byte
-// stores); the layer-chain kernel then reads its layer-0 operand from the planes (coalesced) instead of gathering.
-// The chunk is sized so that planes and one table level together stay inside L2.
+// stores); the layer kernel then reads its layer-0 operand from the planes (coalesced) instead of gathering. Inference takes
+// the pass where that pays (planeChunk, capi.cpp) in chunks of up to 512 MB of planes; a training step always does, because
+// its layer kernel reads features from, and leaves their adjoints in, the planes.
 //
 // Same arithmetic as the fused gather (grid.cuh; reference: src_cpp/include/qmlp/kernels/encoding_hashgrid.cuh:267-336).
 #pragma once
