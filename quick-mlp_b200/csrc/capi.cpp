@@ -565,6 +565,14 @@ int qmlp_network_inference_with_memory(qmlp_network_t* net, const qmlp_tensor_t*
 // registered the beginning of a buffer only; a copy to such a buffer is an error, a kernel's write a fault).
 static float* mappedAddress(float* host, size_t bytes)
 {
+    // (a thread that has made no call yet has no current context, and the runtime then knows no page-locked memory)
+    int dev = 0;
+    cudaPointerAttributes attr;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess || cudaPointerGetAttributes(&attr, host) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return nullptr;
+    }
+    if (attr.type != cudaMemoryTypeHost || attr.devicePointer == nullptr) return nullptr;
     using Query = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
     static const Query query = [] {
         void* fn = nullptr;
@@ -573,15 +581,13 @@ static float* mappedAddress(float* host, size_t bytes)
         return ok ? reinterpret_cast<Query>(fn) : nullptr;
     }();
     if (query == nullptr) return nullptr;
-    unsigned type = 0;
-    CUdeviceptr device = 0, begin = 0;
+    CUdeviceptr begin = 0;
     size_t size = 0;
-    CUpointer_attribute which[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
-                                   CU_POINTER_ATTRIBUTE_RANGE_SIZE};
-    void* values[] = {&type, &device, &begin, &size};
-    // (attributes of memory the driver does not know are left at zero)
-    if (query(4, which, values, reinterpret_cast<CUdeviceptr>(host)) != CUDA_SUCCESS || type != CU_MEMORYTYPE_HOST || device == 0) return nullptr;
-    return device >= begin && device + bytes <= begin + size ? reinterpret_cast<float*>(device) : nullptr;
+    CUpointer_attribute which[] = {CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void* values[] = {&begin, &size};
+    const CUdeviceptr device = reinterpret_cast<CUdeviceptr>(attr.devicePointer);
+    if (query(2, which, values, device) != CUDA_SUCCESS) return nullptr;
+    return device >= begin && device + bytes <= begin + size ? static_cast<float*>(attr.devicePointer) : nullptr;
 }
 
 int qmlp_network_inference_host(qmlp_network_t* net, const float* host_input, float* host_output, int64_t num_points,

@@ -664,6 +664,32 @@ def test_inference_from_host_memory_under_capture(name, chunk):
     assert torch.equal(result(), ref)
 
 
+@pytest.mark.parametrize("fresh", [False, True], ids=["main", "fresh_thread"])
+def test_inference_from_host_memory_takes_the_result_in_place(fresh):
+    """A page-locked result of one channel: chunks of 2^18 points (2^16 with a download), so two launches for 2^18 + 33 points;
+    the same from a thread that has made no CUDA call before."""
+    import threading
+    import torch
+    cfg, rng, spec, net, params, tables, acts, t_params, t_tables = _setup("config2")
+    n = (1 << 18) + 33
+    x = torch.from_numpy(helpers.uniform(67, 1, (n, spec.num_inputs), *rng)).pin_memory()
+    out = torch.empty((n, 1), pin_memory=True)
+    before = net.launch_count()
+
+    def call():
+        net.inference_host(x, t_params, output=out)
+    if fresh:
+        thread = threading.Thread(target=call)
+        thread.start()
+        thread.join()
+    else:
+        call()
+    torch.cuda.synchronize()
+    assert net.launch_count() - before == 2
+    ref = net.inference(x.cuda(), t_params).cpu()
+    assert float((out - ref).norm()) <= 5e-3 * float(ref.norm())
+
+
 @pytest.mark.parametrize("registered", [0, 4096, 8192, 16384])
 def test_inference_from_host_memory_with_a_result_registered_in_part(registered):
     """A result buffer whose first pages only are page-locked: nothing is written through the mapping. The copy either refuses it
