@@ -1190,6 +1190,7 @@ struct qmlp_trainer {
     int64_t fusedCount = 0;
     float *master = nullptr, *grad = nullptr, *m = nullptr, *v = nullptr;
     uint16_t* half = nullptr;
+    bool weightsWait = false;      // the first part of a split step left the weight gradients in the workspace (else: a stash)
 };
 
 extern "C" {
@@ -1374,7 +1375,16 @@ int qmlp_trainer_gradients_part(qmlp_trainer_t* tr, const qmlp_tensor_t* input, 
     // for every network and batch it is instantiated for; the separate kernels below remain for wider networks, line
     // integration, the sorted step, the mma.sync-only path and, on kernel path 2, the bounds-checking instantiations (so that
     // both forms of the step can be checked).
-    if (!sorted && (path == 0 || (path == 2 && !lib.boundsCheck)) && lib.splitScatter != 0 && numel > 0) {
+    // Part 2 follows the route of its first part, whatever the switches are by then.
+    float* sums = reinterpret_cast<float*>(ws + lay.weightSums);
+    if (what == 2 && tr->weightsWait && numel > 0) {
+        checkCuda(kernel::launchAccumulate(sums, static_cast<float*>(n.paramGradients.data), n.parameterCount(), a.numSMs, static_cast<cudaStream_t>(stream)),
+                  "accumulate");
+        n.launchCount += 1;
+        return QMLP_OK;
+    }
+    if ((what == 1 || what == 4) && numel > 0) tr->weightsWait = false;
+    if (what != 2 && !sorted && (path == 0 || (path == 2 && !lib.boundsCheck)) && lib.splitScatter != 0 && numel > 0) {
         auto m = n.module(n.currentHalfMask());
         if (n.trainKernel < 0) {
             kernel::LaunchArgs none = a;
@@ -1389,19 +1399,14 @@ int qmlp_trainer_gradients_part(qmlp_trainer_t* tr, const qmlp_tensor_t* input, 
                 throw std::runtime_error("the scatter of this network does not go level by level (qmlp_trainer_scatter_levels returns 0): use parts = 1");
             // The weight gradients come with the layers, but belong to part 2 of a split step: until then they wait in the
             // workspace.
-            float* sums = reinterpret_cast<float*>(ws + lay.weightSums);
             if (what == 1 || what == 4) {
                 checkCuda(cudaMemsetAsync(sums, 0, static_cast<size_t>(n.parameterCount()) * sizeof(float), static_cast<cudaStream_t>(stream)), "cudaMemsetAsync");
                 a.gradWeights = sums;
+                tr->weightsWait = true;
             }
             if (what & 5) {
                 if (anyGrid) launchModule(n, *m, kernel::KERNEL_ENCODE_PLANES, a, stream);
                 launchModule(n, *m, kernel::KERNEL_TRAIN, a, stream);
-            }
-            if (what == 2) {
-                checkCuda(kernel::launchAccumulate(sums, static_cast<float*>(n.paramGradients.data), n.parameterCount(), a.numSMs, static_cast<cudaStream_t>(stream)),
-                          "accumulate");
-                n.launchCount += 1;
             }
             if (what == 8) {
                 if (levelEnd <= levelBegin) throw std::runtime_error("empty range of grid levels");

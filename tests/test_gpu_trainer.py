@@ -394,3 +394,32 @@ def test_level_ranges_are_refused_where_there_are_none():
         with pytest.raises(QmlpError):
             tr.backend.gradients(x, t, 100, tr.loss_sum, parts=parts)
     assert float(tr.gradient.abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("first,second", [(0, 1), (1, 0)])
+def test_parts_of_a_step_with_a_switch_in_between(first, second):
+    """Part 2 follows its first part: weight gradients that wait in the workspace, or the stash of the separate kernels."""
+    import torch
+    from qmlp import bindings
+    from qmlp.trainer import FusedTrainer
+    cfg = two_grid_config()
+    spec = oracle.parse_spec(cfg)
+    tr = FusedTrainer(bindings.Network(json.dumps(cfg)))
+    tr.set_parameters(torch.from_numpy(helpers.xavier_parameters(spec, cfg, bias_scale=0.05)).cuda(),
+                      [torch.from_numpy(t).cuda() for t in helpers.grid_tables(spec, scale=0.5)])
+    n = 5000
+    x = torch.from_numpy(helpers.uniform(88, 1, (n, 3))).cuda()
+    t = torch.from_numpy(helpers.uniform(88, 2, (n, spec.num_outputs), -1.0, 1.0)).cuda()
+    tr.backend.gradients(x, t, n, tr.loss_sum)
+    whole = tr.gradient.clone()
+    tr.gradient.zero_()
+    try:
+        for path, part in ((first, 1), (second, 2)):
+            bindings.QuickMLP.set_kernel_path(path)
+            tr.backend.gradients(x, t, n, tr.loss_sum, parts=part)
+    finally:
+        bindings.QuickMLP.set_kernel_path(0)
+    # the same roundings to fp16; celu in place of relu: none of them flips a derivative
+    assert float((tr.gradient - whole).norm()) <= 5e-3 * float(whole.norm()) > 0
+    last = tr.backend.segments[1]
+    assert float((tr.gradient[:last] - whole[:last]).norm()) <= 5e-3 * float(whole[:last].norm()) > 0
