@@ -110,17 +110,17 @@ def test_operators_of_other_devices_and_their_names():
     assert torch.Tag.pt2_compliant_tag in torch.ops.qmlp_b200.encoding_forward.default.tags
 
 
-class _Doubled:
-    """Stands for the native network: what forward() passes on."""
+class _Passed:
+    """Stands for the native network: returns what forward() passes on."""
     def forward(self, x, weights, encoding_parameters):
         return x, weights, encoding_parameters
 
 
 def _cpu_network(cfg):
+    import torch
     import qmlp
-    net = qmlp.FusedNetwork(specs.dumps(cfg), weight_dtype=__import__("torch").float32, device="cpu")
-    native, net._network = net._network, _Doubled()
-    net._keep = native
+    net = qmlp.FusedNetwork(specs.dumps(cfg), weight_dtype=torch.float32, device="cpu")
+    net._network = _Passed()
     return net
 
 
@@ -160,7 +160,7 @@ def test_module_saved_without_the_cached_shape():
     for name in ("_num_input_channels", "_encoding_has_parameters", "_no_encoding_parameters"):
         del net.__dict__[name]
     loaded = pickle.loads(pickle.dumps(net))
-    loaded._network = _Doubled()
+    loaded._network = _Passed()
     x = torch.zeros((4, 3))
     _, weights, encodings = loaded(x)
     assert torch.equal(weights, net.weights) and len(encodings) == 1 and torch.equal(encodings[0], net.encoding_parameters[0])
