@@ -8,31 +8,32 @@
 // reaches global memory: with one kernel per phase the pre-activations and deltas of every layer were written once and read
 // back twice (1.3 KB per point for 32 -> 64 -> 64 -> 1).
 //
-//   * One persistent CTA of 16 + 1 warps per SM. A tile is 128 points; the CTA has two tile slots of two warpgroups each, or
-//     one of four where shared or tensor memory is short. The slots run independently: the MMAs of one run under the epilogue
-//     of the other. Thread = (point row, column share): the warpgroups of a slot take the blocks of 8 columns of an
-//     accumulator row in turn.
+//   * One persistent CTA per SM. A tile is 128 points; the CTA has as many tile slots as shared and tensor memory hold, four of one
+//     warpgroup, three of one, two of two, or one of four, and a warp that issues weight gradients. The slots run independently: the MMAs
+//     of one run under the epilogues of the others. Thread = (point row, column share): the warpgroups of a slot take the
+//     blocks of 8 columns of an accumulator row in turn.
 //   * Shared memory, all in the 128-byte swizzled layout (rows = points, 64 channels per block): the weights (staged by
-//     TMA), per slot one buffer per layer input and one for the last delta. The delta of layer l - 1 overwrites the input
-//     of layer l, which has the same shape and is dead once the weight gradient of layer l is done.
-//   * Tensor memory: the accumulator of every layer of the slot stays until the backward pass has taken the activation
-//     derivative from it, or is computed a second time where the columns are short (pre-activation = round to half, add the
-//     half bias: taken from the fp32 accumulator instead of stored); one region for the adjoint of a layer input; and the
-//     weight-gradient accumulators of all layers, which stay for the whole kernel and are added to the gradient vector
-//     once per CTA.
+//     TMA), per slot one buffer per layer input. The delta of layer l - 1 overwrites the input of layer l, which has the same shape
+//     and is dead once the weight gradient of layer l is done; the last delta lies in channels that an input leaves free.
+//   * Tensor memory: per slot one accumulator for the layers and the adjoints one after the other, and packed pre-activations as far as
+//     columns are left (the others stay in registers); and the weight-gradient accumulators of all layers, which stay for the whole
+//     kernel and are added to the gradient vector once per CTA.
 //   * Weight gradients are MMAs over K = the 128 points of the tile: both operands are the tiles above read MN-major. Either
 //     delta^T * input (M = outputs) or input^T * delta (M = inputs), whichever needs fewer columns. The bias gradient is one
-//     more column (or row) of the same MMA: a channel of ones in the padding of the input's block, or a constant block of
-//     ones behind it.
-//   * The warp of a slot that finishes a stage last issues the MMAs that the next stage waits for (a warp of its own polling both
-//     slots took several hundred clocks to notice: 606 -> 577 us in the second example below). The weight gradients of
-//     all slots go to the same accumulators, so one warp issues all of them, in order; they only have to be done when the
-//     next stage of the slot overwrites their operands.
-// Measured, step of 32 -> 64 -> 64 -> 1 on 2^20 points: 94 (forward) + 123 (backward) + 127 us (weight gradients) -> 137 us;
-// 48 -> 128 -> 64 -> 16 -> 4 on 2^21 points: 709 (with the gather) + 1022 (with the scatter) + 473 -> 577 us (655 with 16
-// columns per block instead of 8: the narrow layers then leave a warpgroup idle). Bound by the latency of the stages: an MMA of
-// K = 16 takes 48 clocks up to N = 64 from shared memory however few columns it has, and the round trip of a stage (arrival,
-// issue, MMAs, commit, accumulator load) takes about a thousand clocks that one other slot cannot cover.
+//     more column (or row) of the same MMA: a channel of ones in the padding of the input's block, or a block of ones behind it
+//     that holds 16 points only, which each of the MMAs reads again.
+//   * A slot's warps meet on a named barrier at the end of a stage, and one of them issues the MMAs of the next. The weight gradients of
+//     all slots go to the same accumulators, so one warp issues all of them, in order: it reads requests from a ring in shared memory
+//     (one word to watch; with a barrier per slot to poll it took 500 clocks to notice). They only have to be done when the next stage of
+//     the slot overwrites their operands, and that stage computes all its deltas before it waits.
+// Measured, step of 32 -> 64 -> 64 -> 1 on 2^20 points: 94 (forward) + 123 (backward) + 127 us (weight gradients) -> 137 us with two slots
+// of two warpgroups -> 111 us with four of one; 48 -> 128 -> 64 -> 16 -> 4 on 2^21 points: 709 (with the gather) + 1022 (with the scatter)
+// + 473 -> 577 us with accumulators computed a second time -> 563 us. What it spends (clocks of the first example, measured in the kernel):
+// a tile's MMAs 1970, 54 % of the time per tile (K = 16 takes 40 to 49 clocks from shared memory however few columns, 33 from tensor
+// memory, for which there are no columns left); a slot's stage 2000: 450 waiting for the accumulator behind other slots' MMAs, 1000
+// of epilogue, 130 fences, 300 to issue. Features fetched before the last stage are spilled, and a spill waits for the load (1500 clocks).
+// Weight gradients issued by the slots' own warps under a lock instead of by a warp of their own (128 instead of 96 registers): waits that ran
+// out and sums that were lost; not to be tried again.
 // Every wait is bounded; on a timeout the CTA runs through without waiting and the status word is set.
 //
 // The second instantiation (LOSS false) is the backward pass of a forward call that stashed the encoded features only: the layers
@@ -46,8 +47,8 @@
 namespace qmlp {
 namespace kernel {
 
-constexpr int TRAIN_WARPGROUPS = 4, TRAIN_THREADS = TRAIN_WARPGROUPS * 128 + 32;   // the last warp issues the weight gradients
 constexpr int TRAIN_BLOCK = TC_TILE * 128;   // bytes of a block: 128 points x 64 channels
+constexpr int TRAIN_ONES = 2048;             // and of the block of ones: 16 points
 
 // LOSS: the training step's kernel (features from the planes, L2 loss against targets); else the backward pass of an earlier
 // forward call (features from its stash, the adjoint of the output from the caller)
@@ -58,9 +59,15 @@ struct TrainLayout {
     static constexpr bool FEATURE_ADJOINT = !LOSS || table_rows_per_point<Spec>() > 0;   // the adjoint of the features is wanted
     __host__ __device__ static constexpr int blocks(int channels) { return (channels + 63) / 64; }
     __host__ __device__ static constexpr bool bias(int l) { return Spec::BOFF[l] >= 0; }
-    // buffer l < NL: input of layer l (later delta of layer l - 1); buffer NL: delta of the last layer. A narrow last delta
-    // lies in the upper half of the block of a narrow last input.
-    static constexpr bool SHARED_LAST = Spec::CIN[NL - 1] <= 16 && Spec::COUT[NL - 1] <= 32;
+    // buffer l < NL: input of layer l (later delta of layer l - 1); buffer NL: delta of the last layer. A narrow last delta lies in the
+    // last channels of the first input's block that has room for it behind the input and the channel of ones.
+    __host__ __device__ static constexpr int lastHost()
+    {
+        for (int i = 0; i < NL; ++i)
+            if (Spec::CIN[i] + 16 + Spec::COUT[NL - 1] <= 64) return i;
+        return -1;
+    }
+    static constexpr int LAST_BUFFER = lastHost() >= 0 ? lastHost() : NL, LAST_CHUNK = lastHost() >= 0 ? 8 - Spec::COUT[NL - 1] / 8 : 0;
     __host__ __device__ static constexpr int bufOffset(int l)
     {
         int o = 0;
@@ -68,8 +75,8 @@ struct TrainLayout {
         return o;   // (l == NL: behind the last input)
     }
     // byte offset of the delta of layer l in the slot (its first channel, row 0)
-    __host__ __device__ static constexpr int deltaOffset(int l) { return l < NL - 1 ? bufOffset(l + 1) : (SHARED_LAST ? bufOffset(NL - 1) + 64 : bufOffset(NL)); }
-    __host__ __device__ static constexpr int slotBytes() { return bufOffset(NL) + (SHARED_LAST ? 0 : blocks(Spec::COUT[NL - 1]) * TRAIN_BLOCK); }
+    __host__ __device__ static constexpr int deltaOffset(int l) { return l < NL - 1 ? bufOffset(l + 1) : bufOffset(LAST_BUFFER) + LAST_CHUNK * 16; }
+    __host__ __device__ static constexpr int slotBytes() { return bufOffset(NL) + (lastHost() >= 0 ? 0 : blocks(Spec::COUT[NL - 1]) * TRAIN_BLOCK); }
 
     // weight gradient of layer l: columns if M = outputs / M = inputs, the bias included where it comes for free
     __host__ __device__ static constexpr int colsOut(int l) { return bias(l) ? Spec::CIN[l] + 16 : Spec::CIN[l]; }
@@ -90,56 +97,56 @@ struct TrainLayout {
         for (int i = 0; i < l; ++i) c += Spec::COUT[i];
         return c;
     }
-    // Accumulator columns of a slot. Kept: every layer's accumulator stays until the backward pass has used it, then comes the
-    // adjoint region, where the last layer starts as well (it is consumed before the first adjoint is computed). Recomputed:
-    // all forward accumulators share 128 columns, and the backward pass runs in steps of 64 outputs, with the
-    // recomputed accumulator in the first and the adjoint in the second half.
-    __host__ __device__ static constexpr int keptCols()
+    // accumulator columns of a slot: one region that the layers' outputs, their adjoints and the adjoint of the features share
+    __host__ __device__ static constexpr int slotCols()
     {
         int m = Spec::COUT[NL - 1];
         for (int i = FEATURE_ADJOINT ? 0 : 1; i < NL; ++i) m = Spec::CIN[i] > m ? Spec::CIN[i] : m;
-        return dBefore(NL - 1) + m;
+        return m;
     }
     __host__ __device__ static constexpr int slotStart() { return TL::weightBytes(); }
     __host__ __device__ static constexpr int onesStart(int slots) { return slotStart() + slots * slotBytes(); }
-    __host__ __device__ static constexpr int biasStart(int slots) { return onesStart(slots) + TRAIN_BLOCK; }
+    __host__ __device__ static constexpr int biasStart(int slots) { return onesStart(slots) + TRAIN_ONES; }
     __host__ __device__ static constexpr int barStart(int slots) { return biasStart(slots) + (dBefore(NL) * 2 + 127) / 128 * 128; }
     // barriers, arrival counters and flags (fused_train_tc_kernel)
     __host__ __device__ static constexpr int bytes(int slots) { return barStart(slots) + 384 + 1024; }
-    __host__ __device__ static constexpr bool fits(int slots, bool recompute)
+    __host__ __device__ static constexpr int queueStart() { return barStart(SLOTS) + 8 * (2 * SLOTS + 1 + THREADS / 32); }
+    __host__ __device__ static constexpr bool fits(int slots) { return slots * slotCols() + wgCol(NL) <= 512 && bytes(slots) <= 227 * 1024; }
+    // The pre-activations of the layers but the last wait for the backward pass as packed halfs: in tensor memory, first layers first, as far
+    // as columns are left, else in registers.
+    __host__ __device__ static constexpr int spareCols(int slots) { return (512 - wgCol(NL) - slots * slotCols()) / slots / 16 * 16; }
+    __host__ __device__ static constexpr int preCol(int l, int slots)   // first column behind the slot's accumulator, -1: registers
     {
-        return slots * (recompute ? 128 : keptCols()) + wgCol(NL) <= 512 && bytes(slots) <= 227 * 1024;
+        int c = 0;
+        for (int i = 0; i < NL - 1; ++i) {
+            const bool room = c + Spec::COUT[i] / 2 <= spareCols(slots);
+            if (i == l) return room ? c : -1;
+            if (room) c += Spec::COUT[i] / 2;
+        }
+        return -1;
     }
-    // Two slots hide the MMA round trips (a few hundred clocks per stage) behind each other and are worth recomputing for.
-    static constexpr int SLOTS = fits(2, false) || fits(2, true) ? 2 : 1;
-    static constexpr bool RECOMPUTE = !fits(SLOTS, false);
-    __host__ __device__ static constexpr int slotCols() { return RECOMPUTE ? 128 : keptCols(); }
-    __host__ __device__ static constexpr int dCol(int l) { return RECOMPUTE ? 0 : dBefore(l); }
-    __host__ __device__ static constexpr int adjCol() { return RECOMPUTE ? 64 : dBefore(NL - 1); }
-    __host__ __device__ static constexpr int featureAdjCol() { return RECOMPUTE ? 0 : dBefore(NL - 1); }
-    // Stages: 0 features, 1 .. NL - 1 activations, NL loss, then the backward steps of the layers NL - 2 .. 0 (their deltas; 64
-    // outputs each when recomputing), then the adjoint of the features.
-    __host__ __device__ static constexpr int steps(int l) { return RECOMPUTE ? blocks(Spec::COUT[l]) : 1; }
-    __host__ __device__ static constexpr int lastStage()
+    __host__ __device__ static constexpr int preBefore(int l, int slots, int wg)   // registers of a thread before those of layer l
     {
-        int n = NL + 1;
-        for (int i = 0; i < NL - 1; ++i) n += steps(i);
-        return n;
+        int r = 0;
+        for (int i = 0; i < l; ++i)
+            if (preCol(i, slots) < 0) r += (Spec::COUT[i] / 8 + wg - 1) / wg * 4;
+        return r;
     }
-    __host__ __device__ static constexpr int stepLayer(int stage)   // layer whose delta stage `stage` computes (NL < stage < lastStage())
-    {
-        int s = NL + 1, l = NL - 2;
-        while (s + steps(l) <= stage) { s += steps(l); --l; }
-        return l;
-    }
-    __host__ __device__ static constexpr int stepIndex(int stage)
-    {
-        int s = NL + 1, l = NL - 2;
-        while (s + steps(l) <= stage) { s += steps(l); --l; }
-        return stage - s;
-    }
+    __host__ __device__ static constexpr int slotStride(int slots) { return slotCols() + spareCols(slots); }   // columns of a slot
+    // Slots and warpgroups per slot: as many slots as there is room for, the stages of a tile being latency (see above). 17 warps have 96
+    // registers a thread, 13 have 128.
+    __host__ __device__ static constexpr bool holds(int slots, int wg, int registers) { return fits(slots) && preBefore(NL - 1, slots, wg) <= registers; }
+    static constexpr int SLOTS = holds(4, 1, 40) ? 4 : holds(3, 1, 72) ? 3 : holds(2, 2, 48) ? 2 : 1;
+    static constexpr int WG = SLOTS >= 3 ? 1 : SLOTS == 2 ? 2 : 4;
+    static constexpr int WARPGROUPS = SLOTS * WG, THREADS = WARPGROUPS * 128 + 32;   // the last warp issues the weight gradients
+    __host__ __device__ static constexpr int preCol(int l) { return preCol(l, SLOTS); }
+    __host__ __device__ static constexpr int preBefore(int l) { return preBefore(l, SLOTS, WG); }
+    __host__ __device__ static constexpr int slotStride() { return slotStride(SLOTS); }
+    // Stages: 0 features, 1 .. NL - 1 activations, NL loss, then the deltas of the layers NL - 2 .. 0, then the adjoint of the features.
+    __host__ __device__ static constexpr int lastStage() { return 2 * NL; }
+    __host__ __device__ static constexpr int stepLayer(int stage) { return 2 * NL - 1 - stage; }   // layer whose delta stage `stage` computes (NL < stage < lastStage())
     // (TcLayout: the encode pass exists for the same networks)
-    __host__ __device__ static constexpr bool eligible() { return TL::eligible() && (fits(1, false) || fits(1, true)); }
+    __host__ __device__ static constexpr bool eligible() { return TL::eligible() && fits(1); }
 };
 
 // K-major tile or weight block read along its rows' channels (MN-major operand): 64-channel blocks `lbo` bytes apart,
@@ -160,6 +167,16 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8])
 #pragma unroll
     for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
 }
+// 4 packed words at consecutive columns
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4])
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_st4(uint32_t taddr, const uint32_t (&v)[4])
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // The whole issuing warp runs the issue code, so that descriptors and addresses live in uniform registers; only the
 // elected lane's instruction takes effect. (Behind a `lane == 0` branch every operand has to be moved to a uniform register
 // first: 16 MMAs with N = 64 take 773 instead of 596 clocks to issue.)
@@ -179,18 +196,6 @@ __device__ __forceinline__ void umma_commit_elected(uint32_t lead, uint32_t bar)
 {
     asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
                  "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar), "r"(lead) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-// without the suspension that a try_wait may take: for a warp that watches several barriers
-__device__ __forceinline__ bool mbar_poll(uint32_t bar, uint32_t parity)
-{
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
 }
 // Bounded wait. When one gives up it raises the CTA's abort flag; from then on nobody waits any more (`dead`), so that the
 // CTA runs through to its end.
@@ -299,55 +304,57 @@ __device__ __forceinline__ void store_piece(const LaunchArgs& p, long long point
 }
 
 // ---- MMAs (issued by one elected lane of a whole warp) --------------------------------------------------------------------------------------------
-template <class Spec, bool LOSS, int SLOTS>
+template <class Spec, bool LOSS>
 struct TrainIssue {
     using TL = TcLayout<Spec>;
     using TR = TrainLayout<Spec, LOSS>;
-    // outputs [FIRST, FIRST + N) of layer L = input * W^T, to column `dTmem`
-    template <int L, int FIRST, int N>
+    // outputs of layer L = input * W^T, to column `dTmem`
+    template <int L>
     static __device__ __forceinline__ void forward(uint32_t lead, uint32_t smem, uint32_t slotSmem, uint32_t dTmem)
     {
         constexpr int CIN = Spec::CIN[L], COUT = Spec::COUT[L];
-        const uint64_t a = umma_desc_sw128(slotSmem + TR::bufOffset(L)), b = umma_desc_sw128(smem + TL::wOffset(L) + FIRST * 128);
+        const uint64_t a = umma_desc_sw128(slotSmem + TR::bufOffset(L)), b = umma_desc_sw128(smem + TL::wOffset(L));
 #pragma unroll
         for (int k = 0; k < CIN / 16; ++k)
             umma_f16_elected(lead, dTmem, a + (((k >> 2) * TRAIN_BLOCK + (k & 3) * 32) >> 4), b + (((k >> 2) * (COUT * 128) + (k & 3) * 32) >> 4),
-                             umma_idesc_f16(TC_TILE, N), k > 0 ? 1u : 0u);
+                             umma_idesc_f16(TC_TILE, COUT), k > 0 ? 1u : 0u);
     }
-    // adjoint of inputs [FIRST, FIRST + N) of layer L = delta * W, to column `dTmem`
-    template <int L, int FIRST, int N>
+    // adjoint of the inputs of layer L = delta * W, to column `dTmem`
+    template <int L>
     static __device__ __forceinline__ void adjoint(uint32_t lead, uint32_t smem, uint32_t slotSmem, uint32_t dTmem)
     {
         constexpr int COUT = Spec::COUT[L];
-        const uint64_t a = umma_desc_sw128(slotSmem + TR::deltaOffset(L)), b = umma_desc_mn_sw128(smem + TL::wOffset(L) + FIRST / 64 * (COUT * 128), COUT * 128);
+        const uint64_t a = umma_desc_sw128(slotSmem + TR::deltaOffset(L)), b = umma_desc_mn_sw128(smem + TL::wOffset(L), COUT * 128);
 #pragma unroll
         for (int k = 0; k < COUT / 16; ++k)
-            umma_f16_elected(lead, dTmem, a + (((k >> 2) * TRAIN_BLOCK + (k & 3) * 32) >> 4), b + ((k * 2048) >> 4), umma_idesc_f16(TC_TILE, N) | UMMA_B_MN,
-                             k > 0 ? 1u : 0u);
+            umma_f16_elected(lead, dTmem, a + (((k >> 2) * TRAIN_BLOCK + (k & 3) * 32) >> 4), b + ((k * 2048) >> 4),
+                             umma_idesc_f16(TC_TILE, Spec::CIN[L]) | UMMA_B_MN, k > 0 ? 1u : 0u);
     }
     // weight (and bias) gradient of layer L
     template <int L>
     static __device__ __forceinline__ void gradient(uint32_t lead, uint32_t smem, uint32_t slotSmem, uint32_t wgTmem, uint32_t accumulate)
     {
         constexpr int CIN = Spec::CIN[L];
-        const uint32_t delta = slotSmem + TR::deltaOffset(L), input = slotSmem + TR::bufOffset(L), ones = smem + TR::onesStart(SLOTS);
-        // M is always 128: the block after a 64-channel operand is whatever lies there (inside the CTA's shared memory), its rows
-        // of the result are not read
+        const uint32_t delta = slotSmem + TR::deltaOffset(L), input = slotSmem + TR::bufOffset(L), ones = smem + TR::onesStart(TR::SLOTS);
+        // The 64 channels behind an operand of one block are the block of ones: the input's channel of ones where its own block is full,
+        // else rows of the result that are not read (M is always 128). It holds 16 points, which every MMA reads: its distance
+        // shrinks as the operand's address grows.
         constexpr bool OUT = TR::mIsOut(L);
-        const uint32_t inputLbo = CIN == 64 ? ones - input : TRAIN_BLOCK;
-        const uint64_t m = OUT ? umma_desc_mn_sw128(delta, TRAIN_BLOCK) : umma_desc_mn_sw128(input, inputLbo);
-        const uint64_t n = OUT ? umma_desc_mn_sw128(input, inputLbo) : umma_desc_mn_sw128(delta, TRAIN_BLOCK);
+        constexpr bool DELTA_WIDE = Spec::COUT[L] > 64, INPUT_WIDE = CIN > 64;
+        const uint64_t d = umma_desc_mn_sw128(delta, DELTA_WIDE ? TRAIN_BLOCK : ones - delta), i = umma_desc_mn_sw128(input, INPUT_WIDE ? TRAIN_BLOCK : ones - input);
+        constexpr uint64_t STEP = 2048 >> 4, WIDE_STEP = STEP, NARROW_STEP = STEP - (STEP << 16);
         constexpr int N = OUT ? CIN + (TR::bias(L) && CIN != 128 ? 16 : 0) : Spec::COUT[L];
 #pragma unroll
-        for (int k = 0; k < TC_TILE / 16; ++k)
-            umma_f16_elected(lead, wgTmem + TR::wgCol(L), m + ((k * 2048) >> 4), n + ((k * 2048) >> 4), umma_idesc_f16(TC_TILE, N) | UMMA_A_MN | UMMA_B_MN,
-                             k == 0 ? accumulate : 1u);
+        for (int k = 0; k < TC_TILE / 16; ++k) {
+            const uint64_t dk = d + k * (DELTA_WIDE ? WIDE_STEP : NARROW_STEP), ik = i + k * (INPUT_WIDE ? WIDE_STEP : NARROW_STEP);
+            umma_f16_elected(lead, wgTmem + TR::wgCol(L), OUT ? dk : ik, OUT ? ik : dk, umma_idesc_f16(TC_TILE, N) | UMMA_A_MN | UMMA_B_MN, k == 0 ? accumulate : 1u);
+        }
         if constexpr (TR::separateBias(L)) {
-            const uint64_t d = umma_desc_mn_sw128(delta, TRAIN_BLOCK), o = umma_desc_mn_sw128(ones, TRAIN_BLOCK);
+            const uint64_t o = umma_desc_mn_sw128(ones, TRAIN_BLOCK);   // (16 channels of it)
 #pragma unroll
             for (int k = 0; k < TC_TILE / 16; ++k)
-                umma_f16_elected(lead, wgTmem + TR::wgCol(L) + N, d + ((k * 2048) >> 4), o + ((k * 2048) >> 4),
-                                 umma_idesc_f16(TC_TILE, 16) | UMMA_A_MN | UMMA_B_MN, k == 0 ? accumulate : 1u);
+                umma_f16_elected(lead, wgTmem + TR::wgCol(L) + N, d + k * (DELTA_WIDE ? WIDE_STEP : NARROW_STEP), o, umma_idesc_f16(TC_TILE, 16) | UMMA_A_MN | UMMA_B_MN,
+                                 k == 0 ? accumulate : 1u);
         }
     }
     // what the next stage of the slot waits for after stage ST
@@ -356,16 +363,13 @@ struct TrainIssue {
     {
         constexpr int NL = Spec::NUM_LAYERS, NEXT = ST + 1;
         if constexpr (ST < NL) {
-            forward<ST, 0, Spec::COUT[ST]>(lead, smem, slotSmem, slotTmem + TR::dCol(ST));
+            forward<ST>(lead, smem, slotSmem, slotTmem);
             umma_commit_elected(lead, bars);
         } else if constexpr (NEXT < TR::lastStage()) {
-            constexpr int L = TR::stepLayer(NEXT), FIRST = 64 * TR::stepIndex(NEXT), LEFT = Spec::COUT[L] - FIRST;
-            constexpr int N = TR::RECOMPUTE && LEFT > 64 ? 64 : LEFT;
-            if constexpr (TR::RECOMPUTE) forward<L, FIRST, N>(lead, smem, slotSmem, slotTmem);
-            adjoint<L + 1, FIRST, N>(lead, smem, slotSmem, slotTmem + TR::adjCol());
+            adjoint<TR::stepLayer(NEXT) + 1>(lead, smem, slotSmem, slotTmem);
             umma_commit_elected(lead, bars);
         } else if constexpr (TR::FEATURE_ADJOINT) {
-            adjoint<0, 0, Spec::CIN[0]>(lead, smem, slotSmem, slotTmem + TR::featureAdjCol());
+            adjoint<0>(lead, smem, slotSmem, slotTmem);
             umma_commit_elected(lead, bars);
         }
     }
@@ -376,7 +380,7 @@ struct TrainIssue {
         constexpr int NL = Spec::NUM_LAYERS;
         if constexpr (ST < NL) return -1;
         else if constexpr (ST == NL) return NL - 1;
-        else return TR::stepIndex(ST) == TR::steps(TR::stepLayer(ST)) - 1 ? TR::stepLayer(ST) : -1;
+        else return ST < TR::lastStage() ? TR::stepLayer(ST) : -1;
     }
     // weight gradient of layer `layer`. `started`: layers whose accumulator holds sums already
     template <int L>
@@ -394,24 +398,58 @@ struct TrainIssue {
     }
 };
 
+// ---- requests for weight gradients: a ring of entries that the issuing warps of the slots fill and the weight-gradient warp empties ----
+// An entry carries its number, so that the reader of entry n knows it from the one before in its place. A slot asks for one layer at a
+// time, the next time only after the gradient before is done: the ring never overruns.
+constexpr int TRAIN_QUEUE = 16;
+__device__ __forceinline__ void train_request(uint32_t queue, int slot, int layer)
+{
+    uint32_t n;
+    asm volatile("atom.relaxed.cta.shared::cta.add.u32 %0, [%1], 1;" : "=r"(n) : "r"(queue) : "memory");
+    const uint32_t v = (n + 1) << 8 | static_cast<uint32_t>(slot) << 5 | static_cast<uint32_t>(layer);
+    asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(queue + 4 + (n % TRAIN_QUEUE) * 4), "r"(v) : "memory");
+}
+__device__ __forceinline__ uint32_t train_next_request(uint32_t queue, uint32_t n)
+{
+    uint32_t v;
+    asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(queue + 4 + (n % TRAIN_QUEUE) * 4) : "memory");
+    return v;
+}
+
 // ---- one tile slot, per thread --------------------------------------------------------------------------------------------
 template <class Spec, bool LOSS>
 struct TrainSlot {
-    static constexpr int WG = TRAIN_WARPGROUPS / TrainLayout<Spec, LOSS>::SLOTS;          // warpgroups of a slot
+    static constexpr int WG = TrainLayout<Spec, LOSS>::WG;                           // warpgroups of a slot
     static constexpr int PIECES = (Spec::CIN[0] / 8 + WG - 1) / WG;                 // 8-channel pieces of the input this thread writes
     static constexpr int TARGETS = Spec::NUM_OUTPUTS <= 4 ? Spec::NUM_OUTPUTS : 0;  // prefetched by the warpgroup that takes the loss
     uint32_t row;          // shared address of this thread's row in buffer 0
     uint32_t tmem;         // base column, lane field of this warp included
-    uint32_t bars;         // full: accumulator done; graded: weight gradient done; ready: a delta is complete
-    uint32_t counter;      // arrivals of the slot's warps
-    uint32_t smem, slotSmem, slotTmem, lead;   // what the MMAs of the slot are issued from
+    uint32_t bars;         // full: accumulator done; graded: weight gradient done
+    int slot;              // its warps meet on named barrier 2 + slot at the end of a stage
+    bool issuer;           // this warp issues the MMAs of the slot
+    uint32_t smem, lead;
     uint32_t full, graded; // parities
     long long point;
     bool valid;
     uint32_t features[PIECES][4];
     float target[TARGETS > 0 ? TARGETS : 1];
+    // pre-activations of this thread's channels, from a layer's forward to its backward stage (TrainLayout::preCol)
+    static constexpr int PRE = TrainLayout<Spec, LOSS>::preBefore(Spec::NUM_LAYERS - 1);
+    uint32_t pre[PRE > 0 ? PRE : 1];
 };
 
+// targets (or adjoints of the output) of a point, for the warpgroup that takes the loss
+template <class Spec, bool LOSS>
+__device__ __forceinline__ void train_fetch_target(const LaunchArgs& p, TrainSlot<Spec, LOSS>& sl, int wg, long long point)
+{
+    if constexpr (TrainSlot<Spec, LOSS>::TARGETS > 0) {
+        if (wg == 0 && point < p.numel) {
+#pragma unroll
+            for (int c = 0; c < Spec::NUM_OUTPUTS; ++c)
+                sl.target[c] = LOSS ? __ldg(p.target + point * p.tS0 + c * p.tS1) : __ldg(p.adjOutput + point * p.aoS0 + c * p.aoS1);
+        }
+    }
+}
 template <class Spec, bool LOSS, int K>
 __device__ __forceinline__ void train_fetch(const LaunchArgs& p, TrainSlot<Spec, LOSS>& sl, int wg, long long point)
 {
@@ -442,7 +480,7 @@ __device__ __forceinline__ void train_store_adjoint(const LaunchArgs& p, const T
     if constexpr (K * 8 < Spec::CIN[0]) {
         if (wg == K % TrainSlot<Spec, LOSS>::WG) {
             float x[8];
-            tmem_ld8(sl.tmem + TrainLayout<Spec, LOSS>::featureAdjCol() + K * 8, x);
+            tmem_ld8(sl.tmem + K * 8, x);
             tmem_wait_ld();
             uint32_t v[4];
 #pragma unroll
@@ -491,13 +529,6 @@ __device__ __forceinline__ void train_stage(const LaunchArgs& p, TrainSlot<Spec,
                 sts128(sl.row + sw128_row_offset(row, piece), v[0], v[1], v[2], v[3]);
             }
         }
-        if constexpr (TrainSlot<Spec, LOSS>::TARGETS > 0) {
-            if (wg == 0 && sl.valid) {
-#pragma unroll
-                for (int c = 0; c < Spec::NUM_OUTPUTS; ++c)
-                    sl.target[c] = LOSS ? __ldg(p.target + sl.point * p.tS0 + c * p.tS1) : __ldg(p.adjOutput + sl.point * p.aoS0 + c * p.aoS1);
-            }
-        }
     } else {
         if constexpr (ST < TR::lastStage() || TR::FEATURE_ADJOINT) {
             train_wait(sl.bars, sl.full, abortFlag, dead);
@@ -515,13 +546,22 @@ __device__ __forceinline__ void train_stage(const LaunchArgs& p, TrainSlot<Spec,
                 float v[8];
                 __half2 pre[4];
                 uint32_t w[4];
-                tmem_ld8(sl.tmem + TR::dCol(L) + col, v);
+                tmem_ld8(sl.tmem + col, v);
                 tmem_wait_ld();
                 train_pre<Spec, L>(v, bias, col, pre);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) w[i] = h2_as_u32(act_forward2<Act>(pre[i], col + 2 * i));
                 train_put(sl.row + TR::bufOffset(L + 1), row, col, w);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) w[i] = h2_as_u32(pre[i]);
+                if constexpr (TR::preCol(L) >= 0) {
+                    tmem_st4(sl.tmem + TR::slotCols() + TR::preCol(L) + col / 2, w);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) sl.pre[TR::preBefore(L) + k * 4 + i] = w[i];
+                }
             }
+            if constexpr (TR::preCol(L) >= 0) tmem_wait_st();
         } else if constexpr (ST == NL) {
             constexpr int L = NL - 1, COUT = Spec::COUT[L];
             using Act = typename Spec::template Act<L>;
@@ -532,7 +572,7 @@ __device__ __forceinline__ void train_stage(const LaunchArgs& p, TrainSlot<Spec,
                 float v[8];
                 __half2 pre[4];
                 uint32_t w[4];
-                tmem_ld8(sl.tmem + TR::dCol(L) + col, v);
+                tmem_ld8(sl.tmem + col, v);
                 tmem_wait_ld();
                 train_pre<Spec, L>(v, bias, col, pre);
 #pragma unroll
@@ -561,58 +601,64 @@ __device__ __forceinline__ void train_stage(const LaunchArgs& p, TrainSlot<Spec,
                     const __half2 d = act_adjoint2<Act>(pre[i], __floats2half2_rn(adj[0], adj[1]), col + 2 * i);
                     w[i] = sl.valid ? h2_as_u32(d) : 0u;
                 }
-                train_put<TR::SHARED_LAST ? 4 : 0>(sl.row + TR::bufOffset(TR::SHARED_LAST ? NL - 1 : NL), row, col, w);
+                train_put<TR::LAST_CHUNK>(sl.row + TR::bufOffset(TR::LAST_BUFFER), row, col, w);
             }
-            // the next tile of this slot: its features are fetched under the backward pass
-            train_fetch<Spec, LOSS, 0>(p, sl, wg, nextPoint);
         } else if constexpr (ST < TR::lastStage()) {
-            // outputs [FIRST, FIRST + N) of the delta of layer L from the adjoint of layer L + 1's input
-            constexpr int L = TR::stepLayer(ST), H = TR::stepIndex(ST), FIRST = 64 * H, LEFT = Spec::COUT[L] - FIRST,
-                          N = TR::RECOMPUTE && LEFT > 64 ? 64 : LEFT;
+            // delta of layer L from the adjoint of layer L + 1's input
+            constexpr int L = TR::stepLayer(ST), COUT = Spec::COUT[L];
             using Act = typename Spec::template Act<L>;
-            bool graded = H > 0;
+            // (all of them are computed under the gradient of layer L + 1, whose operand their buffer still is)
+            uint32_t d[(COUT / 8 + WG - 1) / WG][4];
 #pragma unroll
-            for (int k = 0; k < (N / 8 + WG - 1) / WG; ++k) {
+            for (int k = 0; k < (COUT / 8 + WG - 1) / WG; ++k) {
                 const int col = (wg + k * WG) * 8;
-                if (col >= N) continue;
-                float v[8], x[8];
-                __half2 pre[4];
-                uint32_t w[4];
-                tmem_ld8(sl.tmem + TR::dCol(L) + col, v);
-                tmem_ld8(sl.tmem + TR::adjCol() + col, x);
+                if (col >= COUT) continue;
+                float x[8];
+                tmem_ld8(sl.tmem + col, x);
+                if constexpr (TR::preCol(L) >= 0) {
+                    tmem_ld4(sl.tmem + TR::slotCols() + TR::preCol(L) + col / 2, d[k]);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) d[k][i] = sl.pre[TR::preBefore(L) + k * 4 + i];
+                }
                 tmem_wait_ld();
-                train_pre<Spec, L>(v, bias, FIRST + col, pre);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const __half2 d = act_adjoint2<Act>(pre[i], __floats2half2_rn(x[2 * i], x[2 * i + 1]), FIRST + col + 2 * i);
-                    w[i] = sl.valid ? h2_as_u32(d) : 0u;
+                    const __half2 y = act_adjoint2<Act>(u32_as_h2(d[k][i]), __floats2half2_rn(x[2 * i], x[2 * i + 1]), col + 2 * i);
+                    d[k][i] = sl.valid ? h2_as_u32(y) : 0u;
                 }
-                if (!graded) train_wait(sl.bars + 8, sl.graded, abortFlag, dead);   // the buffer still is an operand of layer L + 1's gradient
-                graded = true;
-                train_put(sl.row + TR::bufOffset(L + 1), row, FIRST + col, w);
             }
-            if (!graded) train_wait(sl.bars + 8, sl.graded, abortFlag, dead);       // (no columns here: stay in step with the barrier)
-            if constexpr (H == 0) sl.graded ^= 1u;
+            train_wait(sl.bars + 8, sl.graded, abortFlag, dead);
+#pragma unroll
+            for (int k = 0; k < (COUT / 8 + WG - 1) / WG; ++k) {
+                const int col = (wg + k * WG) * 8;
+                if (col < COUT) train_put(sl.row + TR::bufOffset(L + 1), row, col, d[k]);
+            }
+            sl.graded ^= 1u;
         } else {
             if constexpr (TR::FEATURE_ADJOINT) train_store_adjoint<Spec, LOSS, 0>(p, sl, wg);
             train_wait(sl.bars + 8, sl.graded, abortFlag, dead);   // buffer 0 is written next
             sl.graded ^= 1u;
         }
     }
+    // the next tile of this slot: its features are fetched under the last stage (earlier they would be spilled, and waited for to do so)
+    if constexpr (ST == TR::lastStage() - 1) {
+        train_fetch<Spec, LOSS, 0>(p, sl, wg, nextPoint);
+        train_fetch_target<Spec, LOSS>(p, sl, wg, nextPoint);
+    }
     if constexpr (ST < TR::lastStage()) {
-        using Issue = TrainIssue<Spec, LOSS, TR::SLOTS>;
+        using Issue = TrainIssue<Spec, LOSS>;
         tc_fence_before();
         fence_proxy_async();   // generic-proxy writes of the operands become visible to the tensor core
         __syncwarp();
-        uint32_t before = 0;
-        if ((threadIdx.x & 31) == 0)
-            asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;" : "=r"(before) : "r"(sl.counter) : "memory");
-        before = __shfl_sync(0xffffffffu, before, 0);
-        if ((before & (WG * 4 - 1)) == WG * 4 - 1) {
+        if (!sl.issuer) {
+            asm volatile("bar.arrive %0, %1;" ::"r"(2 + sl.slot), "n"(WG * 128) : "memory");
+        } else {
+            asm volatile("bar.sync %0, %1;" ::"r"(2 + sl.slot), "n"(WG * 128) : "memory");
             tc_fence_after();
-            if (!__any_sync(0xffffffffu, dead)) Issue::template critical<ST>(sl.lead, sl.smem, sl.slotSmem, sl.slotTmem, sl.bars);
+            if (!__any_sync(0xffffffffu, dead)) Issue::template critical<ST>(sl.lead, sl.smem, sl.smem + TR::slotStart() + sl.slot * TR::slotBytes(), sl.tmem & 0xffffu, sl.bars);
             if constexpr (Issue::template graded<ST>() >= 0)
-                if ((threadIdx.x & 31) == 0) mbar_arrive(sl.bars + 16);
+                if ((threadIdx.x & 31) == 0) train_request(sl.smem + TR::queueStart(), sl.slot, Issue::template graded<ST>());
         }
     }
 }
@@ -627,42 +673,34 @@ __device__ __forceinline__ void train_stages(const LaunchArgs& p, TrainSlot<Spec
     }
 }
 
-// The weight-gradient warp: whenever a slot's delta is complete, the MMAs of that layer's gradient. All slots add to the same
+// The weight-gradient warp: the MMAs of the layers' gradients in the order in which the deltas are completed. All slots add to the same
 // accumulators, so one thread issues them; nobody waits for them before the slot's next stage has computed its results.
-template <class Spec, bool LOSS, int SLOTS>
-__device__ __forceinline__ void train_gradients(uint32_t lead, uint32_t smem, uint32_t tmemBase, uint32_t bars, int myTiles, volatile int* abortFlag, bool& dead)
+template <class Spec, bool LOSS>
+__device__ __forceinline__ void train_gradients(uint32_t lead, uint32_t smem, uint32_t tmemBase, uint32_t bars, uint32_t queue, int myTiles, volatile int* abortFlag,
+                                                bool& dead)
 {
     using TR = TrainLayout<Spec, LOSS>;
-    constexpr int NL = Spec::NUM_LAYERS;
-    int layer[SLOTS], left[SLOTS], open = 0;
-    uint32_t parity = 0, started = 0, idle = 0;
-#pragma unroll
-    for (int j = 0; j < SLOTS; ++j) {
-        layer[j] = NL - 1;
-        left[j] = myTiles > j ? (myTiles - j + SLOTS - 1) / SLOTS * NL : 0;
-        open += left[j] > 0;
-    }
-    while (open > 0) {
-        ++idle;
-#pragma unroll
-        for (int j = 0; j < SLOTS; ++j) {
-            if (left[j] == 0 || !__all_sync(0xffffffffu, mbar_poll(bars + j * 24 + 16, (parity >> j) & 1u))) continue;
-            tc_fence_after();
-            // (opaque copies: the descriptors of all MMAs would be computed ahead of the loop and spilled)
-            uint32_t base = smem, tmem = tmemBase;
-            asm volatile("" : "+r"(base), "+r"(tmem));
-            TrainIssue<Spec, LOSS, SLOTS>::template weights<0>(lead, layer[j], base, base + TR::slotStart() + j * TR::slotBytes(), tmem + SLOTS * TR::slotCols(), started,
-                                                         bars + j * 24);
-            parity ^= 1u << j;
-            layer[j] = layer[j] == 0 ? NL - 1 : layer[j] - 1;
-            if (--left[j] == 0) --open;
-            idle = 0;
+    uint32_t started = 0;
+    const uint32_t requests = static_cast<uint32_t>(myTiles) * Spec::NUM_LAYERS;
+    for (uint32_t n = 0; n < requests; ++n) {
+        uint32_t v = 0, idle = 0;
+        while (true) {
+            v = __shfl_sync(0xffffffffu, train_next_request(queue, n), 0);
+            if ((v >> 8) == ((n + 1) & 0xffffffu)) break;
+            ++idle;
+            if (idle > 4 * TC_SPIN_LIMIT || ((idle & 1023u) == 1023u && __any_sync(0xffffffffu, *abortFlag != 0))) {
+                *abortFlag = 1;
+                dead = true;
+                return;
+            }
         }
-        if (idle > 4 * TC_SPIN_LIMIT || ((idle & 1023u) == 1023u && __any_sync(0xffffffffu, *abortFlag != 0))) {
-            *abortFlag = 1;
-            dead = true;
-            return;
-        }
+        tc_fence_after();
+        // (opaque copies: the descriptors of all MMAs would be computed ahead of the loop and spilled)
+        uint32_t base = smem, tmem = tmemBase;
+        asm volatile("" : "+r"(base), "+r"(tmem));
+        const int slot = static_cast<int>(v >> 5) & 7;
+        TrainIssue<Spec, LOSS>::template weights<0>(lead, static_cast<int>(v & 31u), base, base + TR::slotStart() + slot * TR::slotBytes(), tmem + TR::SLOTS * TR::slotStride(),
+                                                    started, bars + slot * 16);
     }
 }
 
@@ -678,7 +716,7 @@ __device__ __forceinline__ void train_flush(const LaunchArgs& p, uint32_t wgTmem
         float* gw = p.gradWeights + Spec::WOFF[L];
         float* gb = p.gradWeights + (BIAS ? Spec::BOFF[L] : 0);
         const bool vec = (reinterpret_cast<uintptr_t>(gw) & 15) == 0;   // (a caller's gradient vector may start anywhere)
-        for (int c = warpgroup; c < CHUNKS; c += TRAIN_WARPGROUPS) {
+        for (int c = warpgroup; c < CHUNKS; c += TR::WARPGROUPS) {
             const int col = c * 16;
             float v[16];
             tmem_ld16(wgTmem + TR::wgCol(L) + col, v);
@@ -726,7 +764,7 @@ __device__ __forceinline__ void train_init(const LaunchArgs& p, uint32_t smemBas
         constexpr int CIN = Spec::CIN[L], COUT = Spec::COUT[L];
         if constexpr (!ONES) {
             if constexpr (Spec::BOFF[L] >= 0)
-                for (int i = threadIdx.x; i < COUT; i += TRAIN_THREADS) sBias[TR::dBefore(L) + i] = p.weights[Spec::BOFF[L] + i];
+                for (int i = threadIdx.x; i < COUT; i += TR::THREADS) sBias[TR::dBefore(L) + i] = p.weights[Spec::BOFF[L] + i];
         } else if constexpr (CIN % 64 != 0) {
 #pragma unroll
             for (int s = 0; s < SLOTS; ++s)
@@ -737,7 +775,7 @@ __device__ __forceinline__ void train_init(const LaunchArgs& p, uint32_t smemBas
 }
 
 template <class Spec, bool LOSS, int SLOTS>
-__global__ void __launch_bounds__(TRAIN_THREADS, 1)
+__global__ void __launch_bounds__(TrainLayout<Spec, LOSS>::THREADS, 1)
 fused_train_tc_kernel(const __grid_constant__ LaunchArgs p, const __grid_constant__ TcWeightMaps<Spec> weightMaps)
 {
     using TL = TcLayout<Spec>;
@@ -745,26 +783,23 @@ fused_train_tc_kernel(const __grid_constant__ LaunchArgs p, const __grid_constan
     extern __shared__ unsigned char smemRaw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~static_cast<uintptr_t>(1023));
     __half* sBias = reinterpret_cast<__half*>(smem + TR::biasStart(SLOTS));
-    // full, graded and ready of every slot, the weight staging, the drain of every warp after a timeout; arrival counters
+    // full and graded of every slot, the weight staging, the drain of every warp after a timeout; requests for weight gradients
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + TR::barStart(SLOTS));
-    uint64_t* weightBar = bars + 3 * SLOTS;
+    uint64_t* weightBar = bars + 2 * SLOTS;
     uint64_t* drainBar = weightBar + 1;
-    uint32_t* counters = reinterpret_cast<uint32_t*>(drainBar + TRAIN_THREADS / 32);
-    uint32_t* tmemSlot = counters + SLOTS;
+    uint32_t* queue = reinterpret_cast<uint32_t*>(smem + TR::queueStart());   // number of requests so far, then the ring
+    uint32_t* tmemSlot = queue + 1 + TRAIN_QUEUE;
     volatile int* abortFlag = reinterpret_cast<int*>(tmemSlot + 1);
-    static_assert(8 * (3 * SLOTS + 1 + TRAIN_THREADS / 32) + 4 * (SLOTS + 2) <= 384, "barrier area");
+    static_assert(8 * (2 * SLOTS + 1 + TR::THREADS / 32) + 4 * (TRAIN_QUEUE + 3) <= 384, "barrier area");
+    static_assert(SLOTS <= 8 && Spec::NUM_LAYERS <= 32, "fields of a request");
     const uint32_t smemBase = smem_u32(smem);
     const int warp = threadIdx.x >> 5, warpgroup = warp >> 2, row = threadIdx.x & 127;
 
     if (threadIdx.x == 0) {
         mbar_init(smem_u32(weightBar), 1);
-        for (int w = 0; w < TRAIN_THREADS / 32; ++w) mbar_init(smem_u32(drainBar + w), 1);
-        for (int s = 0; s < SLOTS; ++s) {
-            mbar_init(smem_u32(bars + 3 * s), 1);                                // one tcgen05.commit per phase
-            mbar_init(smem_u32(bars + 3 * s + 1), 1);
-            mbar_init(smem_u32(bars + 3 * s + 2), 1);                            // the last warp of a stage that completes a delta
-            counters[s] = 0;
-        }
+        for (int w = 0; w < TR::THREADS / 32; ++w) mbar_init(smem_u32(drainBar + w), 1);
+        for (int s = 0; s < 2 * SLOTS; ++s) mbar_init(smem_u32(bars + s), 1);     // one tcgen05.commit per phase
+        for (int i = 0; i <= TRAIN_QUEUE; ++i) queue[i] = 0;
         *abortFlag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         mbar_expect_tx(smem_u32(weightBar), TL::weightCopyBytes());
@@ -772,12 +807,12 @@ fused_train_tc_kernel(const __grid_constant__ LaunchArgs p, const __grid_constan
     }
     // Operand buffers and the block behind them start as zeros with a channel of ones: in the buffers the first padding
     // channel of the input (stages write the channels before it only), in the last block channel 0.
-    for (int i = threadIdx.x; i < (TR::onesStart(SLOTS) + TRAIN_BLOCK - TR::slotStart()) / 16; i += TRAIN_THREADS)
+    for (int i = threadIdx.x; i < (TR::onesStart(SLOTS) + TRAIN_ONES - TR::slotStart()) / 16; i += TR::THREADS)
         reinterpret_cast<uint4*>(smem + TR::slotStart())[i] = make_uint4(0, 0, 0, 0);
     train_init<Spec, LOSS, 0, SLOTS, false>(p, smemBase, sBias, row);
     __syncthreads();
     if (warpgroup == 0) {
-        sts16(smemBase + TR::onesStart(SLOTS) + row * 128 + sw128_row_offset(row, 0), __ushort_as_half(0x3C00));
+        if (row < TRAIN_ONES / 128) sts16(smemBase + TR::onesStart(SLOTS) + row * 128 + sw128_row_offset(row, 0), __ushort_as_half(0x3C00));
         train_init<Spec, LOSS, 0, SLOTS, true>(p, smemBase, sBias, row);
     }
     if (warp == 0) {
@@ -790,7 +825,7 @@ fused_train_tc_kernel(const __grid_constant__ LaunchArgs p, const __grid_constan
     tc_fence_after();
     const uint32_t tmemBase = *tmemSlot;
     const uint32_t laneField = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    const uint32_t wgTmem = tmemBase + SLOTS * TR::slotCols();
+    const uint32_t wgTmem = tmemBase + SLOTS * TR::slotStride();
     const int numTiles = static_cast<int>((p.numel + TC_TILE - 1) / TC_TILE);
     const int stride = gridDim.x;
     const int myTiles = static_cast<int>(blockIdx.x) < numTiles ? (numTiles - static_cast<int>(blockIdx.x) + stride - 1) / stride : 0;
@@ -798,25 +833,25 @@ fused_train_tc_kernel(const __grid_constant__ LaunchArgs p, const __grid_constan
     const uint32_t lead = elect_one();
     train_wait(smem_u32(weightBar), 0, abortFlag, dead);
     __syncwarp();
-    if (warpgroup == TRAIN_WARPGROUPS) {
+    if (warpgroup == TR::WARPGROUPS) {
         const uint32_t smemU = __shfl_sync(0xffffffffu, smemBase, 0), tmemU = __shfl_sync(0xffffffffu, tmemBase, 0);
-        if (!__any_sync(0xffffffffu, dead)) train_gradients<Spec, LOSS, SLOTS>(lead, smemU, tmemU, smemU + TR::barStart(SLOTS), myTiles, abortFlag, dead);
+        if (!__any_sync(0xffffffffu, dead)) train_gradients<Spec, LOSS>(lead, smemU, tmemU, smemU + TR::barStart(SLOTS), smem_u32(queue), myTiles, abortFlag, dead);
     } else {
         // tile i of this CTA's sequence belongs to slot i % SLOTS
         const int slot = warpgroup / TrainSlot<Spec, LOSS>::WG, wg = warpgroup % TrainSlot<Spec, LOSS>::WG;
         auto pointOf = [&](int i) { return i < myTiles ? (blockIdx.x + static_cast<long long>(i) * stride) * TC_TILE + row : p.numel; };
         TrainSlot<Spec, LOSS> sl;
         sl.row = smemBase + TR::slotStart() + slot * TR::slotBytes() + row * 128;
-        sl.tmem = tmemBase + slot * TR::slotCols() + laneField;
-        sl.bars = smem_u32(bars + 3 * slot);
-        sl.counter = smem_u32(counters + slot);
+        sl.tmem = tmemBase + slot * TR::slotStride() + laneField;
+        sl.bars = smem_u32(bars + 2 * slot);
+        sl.slot = slot;
+        sl.issuer = wg == 0 && (warp & 3) == (slot & 3);   // (on different sub-partitions of the SM)
         sl.smem = smemBase;
-        sl.slotSmem = smemBase + TR::slotStart() + slot * TR::slotBytes();
-        sl.slotTmem = tmemBase + slot * TR::slotCols();
         sl.lead = lead;
         sl.full = sl.graded = 0;
         sl.point = pointOf(slot);
         train_fetch<Spec, LOSS, 0>(p, sl, wg, sl.point);
+        train_fetch_target<Spec, LOSS>(p, sl, wg, sl.point);
         float lossAcc = 0.f;
         for (int i = slot; i < myTiles; i += SLOTS) {
             sl.valid = sl.point < p.numel;
@@ -825,7 +860,7 @@ fused_train_tc_kernel(const __grid_constant__ LaunchArgs p, const __grid_constan
             sl.point = next;
         }
         tc_fence_before();
-        asm volatile("bar.sync 1, %0;" ::"n"(TRAIN_WARPGROUPS * 128) : "memory");   // every slot's weight gradients are in
+        asm volatile("bar.sync 1, %0;" ::"n"(TR::WARPGROUPS * 128) : "memory");   // every slot's weight gradients are in
         if (myTiles > 0 && !__any_sync(0xffffffffu, *abortFlag != 0)) {
             tc_fence_after();
             train_flush<Spec, LOSS, 0>(p, wgTmem + laneField, warpgroup, row);
@@ -869,7 +904,7 @@ struct TrainLaunchers {
         if (m != cudaSuccess) return m;
         const long long tiles = (a.numel + TC_TILE - 1) / TC_TILE;
         const long long blocks = tiles < a.numSMs ? tiles : a.numSMs;
-        k<<<static_cast<unsigned>(blocks), TRAIN_THREADS, smem, s>>>(a, *maps);
+        k<<<static_cast<unsigned>(blocks), TR::THREADS, smem, s>>>(a, *maps);
         return cudaGetLastError();
     }
 };

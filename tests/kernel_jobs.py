@@ -28,6 +28,8 @@ def jobs():
         out.append(("net", json.dumps(cfg), 0))
         out.append(("net", json.dumps(cfg), 1))
     out.append(("net", json.dumps(tt.two_grid_config()), 3))
+    for cfg in tt.slot_configs().values():
+        out.append(("net", json.dumps(cfg), 0))
     for d in (2, 4):
         out.append(("net", json.dumps(tt.dims_config(d)), 0))
     import test_gpu_full_size as tf

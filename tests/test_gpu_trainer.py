@@ -289,6 +289,57 @@ def test_train_kernel_matches_separate_kernels(name, n):
         assert norm > 0 and float((ga - gb).norm()) <= 1e-2 * norm, f"{name} n={n} segment {i}: {float((ga - gb).norm()) / norm}"
 
 
+def slot_configs():
+    """name -> network by the tile slots of its training kernel: four (of one warpgroup; last delta in the first input's block), three, two
+    (of two warpgroups) and one (of four); pre-activations in tensor memory, in registers, and both."""
+    return {
+        "four": specs.config3(log2_hashmap_size=12),
+        "three": specs.identity_net(40, [64, 64, 3], ["celu", "sine", "identity"], bias=[True, False, True]),
+        "two": specs.config4(log2_hashmap_size=10, dense_resolution=16),
+        "one": specs.identity_net(9, [128, 112, 5], ["relu", "celu", "identity"]),
+    }
+
+
+@pytest.mark.parametrize("n", [129, 9 * 148 * 128 + 77])
+@pytest.mark.parametrize("name", list(slot_configs().keys()))
+def test_train_kernel_tile_slots(name, n):
+    """Tiles that follow each other in the slots of a CTA (nine or ten tiles per CTA) and the adjoint of the inputs, against the separate
+    kernels; tolerance as above. The autograd pass takes the other instantiation of the same kernel."""
+    import torch
+    from qmlp import bindings
+    from qmlp.trainer import FusedTrainer
+    import qmlp
+    cfg = slot_configs()[name]
+    spec = oracle.parse_spec(cfg)
+    x = torch.from_numpy(helpers.uniform(33, 1, (n, spec.num_inputs), 0.0, 1.0)).cuda()
+    t = torch.from_numpy(helpers.uniform(33, 2, (n, spec.num_outputs), -1.0, 1.0)).cuda()
+    params = torch.from_numpy(helpers.xavier_parameters(spec, cfg, bias_scale=0.1).astype(np.float32)).cuda()
+    tables = [torch.from_numpy(tb).cuda() if tb is not None else None for tb in helpers.grid_tables(spec, scale=0.5)]
+    results = []
+    try:
+        for path in (0, 1):
+            bindings.QuickMLP.set_kernel_path(path)
+            tr = FusedTrainer(bindings.Network(json.dumps(cfg)), grid_half_copy=False)
+            tr.set_parameters(params, tables)
+            tr.backend.gradients(x, t, n, tr.loss_sum)
+            module = qmlp.FusedNetwork(json.dumps(cfg), weight_dtype=torch.float32)
+            with torch.no_grad():
+                module.weights.copy_(params)
+                for p, tb in zip(module.encoding_parameters, [tb for tb in tables]):
+                    if tb is not None:
+                        p.copy_(tb)
+            xg = x.clone().requires_grad_(not any(tb is not None for tb in tables))
+            torch.nn.functional.mse_loss(module(xg), t).backward()
+            torch.cuda.synchronize()
+            results.append([tr.loss_sum.clone(), tr.gradient.clone(), module.weights.grad] + ([xg.grad] if xg.requires_grad else []))
+    finally:
+        bindings.QuickMLP.set_kernel_path(0)
+    for i, (a, b) in enumerate(zip(*results)):
+        norm = float(b.norm())
+        assert norm > 0 and float((a - b).norm()) <= 1e-2 * norm, f"{name} n={n} result {i}: {float((a - b).norm()) / norm}"
+    assert bindings.QuickMLP.device_status() == 0
+
+
 def test_scatter_with_copies_of_hot_levels():
     """A batch that hits the lines of the coarse levels often enough for copies of their gradients: one launch over all levels,
     and launches over ranges of levels that begin before, inside and behind the levels with copies, against the scatter
