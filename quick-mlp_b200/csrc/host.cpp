@@ -320,7 +320,40 @@ void EncodingHashGrid::planReplicas(int64_t points, int group, kernel::GradRepli
     // under one set of tuning switches serves a call under another.
     if (isLine()) return;
     const double reductions = static_cast<double>(points) * (1 << (dim_ - 1));
+    // By cell (kernel::GridCellUnits) while the records of a level take up to 16 bytes per point and those of all levels, which a scatter
+    // works on at the same time, stay in L2 beside the gradients of the others (80 MB). A point and level save about 11 ps, a byte of records
+    // costs 0.4 ps to clear and to add up, and the launch that adds up costs as much as half a million points save: 3-D grid of 16^3 to
+    // 7006^3 vertices, four levels by cell, step of 2^20 points 821 -> 786 us; three levels, autograd call of 2^18 points 309 -> 292; two
+    // levels, step of 2^17 points 204 -> 209; two levels of 64^3 with four features (16 bytes per point), step of 2^21 points 1500 -> 1487; 16
+    // levels of 54^3 (160 MB), 2^20 points 382 -> 630. Dense levels only: rows of a small hashed level that many vertices share would be added up
+    // one vertex after the other (10^6 points, 1024 rows, terms of one sign: error against 64 bits 1.4e-7 -> 2.2e-7).
+    const int64_t record = static_cast<int64_t>(features_) << dim_;   // elements of a cell
+    const bool records = dim_ >= 2 && dim_ <= 4 && (features_ == 2 || features_ == 4 || features_ == 8) && record <= 64;
+    auto cellsOf = [&](int l) {
+        double n = 1;
+        for (int k = 0; k < dim_; ++k) n *= table_[l].resolution;
+        return n;
+    };
+    auto fewCells = [&](int l) { return records && !table_[l].hashed && cellsOf(l) * static_cast<double>(record) * 4 <= 16.0 * static_cast<double>(points); };
+    int few = 0;
+    for (int l = 0; l < levels_ && group + l < kernel::MAX_GRID_LEVELS; ++l) few += fewCells(l) ? 1 : 0;
+    const bool byCell = static_cast<double>(points) * few >= static_cast<double>(1 << 19);
+    int64_t recordElements = 0;
+    for (int g = 0; g < group; ++g) recordElements = r.byCell[g] ? r.total : recordElements;   // (an upper bound: of the grids before)
     for (int l = 0; l < levels_ && group + l < kernel::MAX_GRID_LEVELS; ++l) {
+        if (byCell && fewCells(l)) {
+            // as many copies as leave a record 256 points (10^6 points on 256 cells of 64 bytes: 40 us, 4096 cells 17, 16384 cells 15)
+            int lg = 0;
+            for (double hits = static_cast<double>(points) / cellsOf(l); hits > 256 && lg < 6; hits /= 2) ++lg;
+            const int64_t n = static_cast<int64_t>(cellsOf(l)) * record << lg, at = (r.total + 3) / 4 * 4;   // (written 16 bytes at a time)
+            if (recordElements + n <= (20ll << 20) && at + n <= (1ll << 28)) {
+                r.byCell[group + l] = static_cast<unsigned char>(1 + lg);
+                r.offset[group + l] = static_cast<unsigned int>(at);
+                r.total = at + n;
+                recordElements += n;
+                continue;
+            }
+        }
         const int64_t elements = (l + 1 < levels_ ? table_[l + 1].memoryOffset : numParameters_) - table_[l].memoryOffset;
         double perLine = reductions / std::max<double>(1.0, static_cast<double>(elements) / 32);
         int lg = 0;

@@ -574,6 +574,141 @@ __device__ __forceinline__ void grid_half_scatter(const GridP& g, float* grad, c
     grid_half_adjoint<D, F, false, true, false, PD>(g, grad, lv, pos, side, adjF, none);
 }
 
+// ---- gradients by cell (GradReplicas::byCell) -----------------------------------------------------------------------
+// A level with few cells, compared with the points of a batch, adds its gradient up by cell first: a record of the 2^D corners' rows
+// per cell, so that a point's contributions are one contiguous piece of memory which several lanes send in one request. The records are then
+// added up at the vertices. 2^20 random points, two features, 3-D: 64 bytes by four lanes 12 us, the four pairs of rows of the
+// table 25 us (a level of 16^3 to 121^3 vertices; launches not counted).
+template <int D, int F>
+struct GridCellUnits {
+    static constexpr int ROWS = 1 << D, ELEMENTS = ROWS * F;
+    static constexpr bool USED = D >= 2 && D <= 4 && (F == 2 || F == 4 || F == 8) && ELEMENTS <= 64;
+    static constexpr int UNITS = ELEMENTS / 4;                  // of 16 bytes
+    static constexpr int LANES = UNITS < 8 ? UNITS : 8;         // that share a point
+};
+// The lanes of a group take the group's points in turn. `pos`: this lane's own point; adjoint(r, a): the adjoint of the features of the
+// group's r-th point (all lanes of the warp take part). False if this lane's point lies in no cell that has a record.
+template <int D, int F, class Adjoint>
+__device__ __forceinline__ bool grid_cells_scatter(float* records, const GridLevelP& lv, const float (&pos)[D], bool valid, const Adjoint& adjoint)
+{
+    using C = GridCellUnits<D, F>;
+    GridCell<D> c;
+    grid_cell<D>(pos, lv.resolution, c);
+    bool regular = true;   // high corner = low corner + 1, or the border: not so for a point below the box
+    unsigned int own = c.lo[0];
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+        regular = regular && c.hi[k] == min(c.lo[k] + 1u, static_cast<unsigned int>(lv.resolution - 1));
+        if (k > 0) own = c.lo[k] + own * static_cast<unsigned int>(lv.resolution);
+    }
+    if (!valid || !regular) own = 0xffffffffu;
+    const int lane = threadIdx.x % C::LANES;
+#pragma unroll
+    for (int r = 0; r < C::LANES; ++r) {
+        const unsigned int cell = __shfl_sync(0xffffffffu, own, r, C::LANES);
+        float f[D], a[F];
+#pragma unroll
+        for (int k = 0; k < D; ++k) f[k] = __shfl_sync(0xffffffffu, c.f[k], r, C::LANES);
+        adjoint(r, a);
+        if (cell == 0xffffffffu) continue;
+        float* at = records + static_cast<size_t>(cell) * C::ELEMENTS + lane * 4;
+#pragma unroll
+        for (int u = 0; u < C::UNITS; u += C::LANES) {
+            const int unit = u + lane;
+            if constexpr (F == 2) {   // two rows, neighbours in dimension 0 (weights: the product of grid_corner_weight)
+                float w = 1.f;
+#pragma unroll
+                for (int k = D - 1; k >= 1; --k) w *= ((unit >> (k - 1)) & 1) ? f[k] : (1.f - f[k]);
+                const float w0 = w * (1.f - f[0]), w1 = w * f[0];
+                red_add_v4_f32(at + u * 4, w0 * a[0], w0 * a[1], w1 * a[0], w1 * a[1]);
+            } else {
+                const int corner = unit / (F / 4);
+                float w = 1.f;
+#pragma unroll
+                for (int k = D - 1; k >= 0; --k) w *= ((corner >> k) & 1) ? f[k] : (1.f - f[k]);
+                if constexpr (F == 4) {
+                    red_add_v4_f32(at + u * 4, w * a[0], w * a[1], w * a[2], w * a[3]);
+                } else {
+                    const bool upper = (unit & 1) != 0;
+                    red_add_v4_f32(at + u * 4, w * (upper ? a[4] : a[0]), w * (upper ? a[5] : a[1]), w * (upper ? a[6] : a[2]), w * (upper ? a[7] : a[3]));
+                }
+            }
+        }
+    }
+    return own != 0xffffffffu || !valid;
+}
+template <int D>
+__host__ __device__ inline unsigned int grid_cell_count(int resolution)
+{
+    unsigned int n = 1;
+    for (int k = 0; k < D; ++k) n *= static_cast<unsigned int>(resolution);
+    return n;
+}
+// records of a level -> its gradient: the cells around a vertex (grid-stride over blockIdx.x, 256 threads)
+template <int D, int F>
+__device__ __forceinline__ void grid_sum_cells(const GridP& g, const GradReplicas& r, int group, int l)
+{
+    using C = GridCellUnits<D, F>;
+    const GridLevelP& lv = g.levels[l];
+    const unsigned int n = grid_cell_count<D>(lv.resolution), res = static_cast<unsigned int>(lv.resolution);
+    const int copies = 1 << (r.byCell[group] - 1);
+    const float* base = r.base + r.offset[group];
+    for (unsigned int i = blockIdx.x * 256u + threadIdx.x; i < n; i += gridDim.x * 256u) {
+        unsigned int v[D], rest = i;
+#pragma unroll
+        for (int k = D - 1; k >= 0; --k) {
+            const unsigned int q = rest / res;
+            v[k] = rest - q * res;
+            rest = q;
+        }
+        double sum[F];   // (up to 512 terms of like size: added in fp32 they would cost more than the reductions did)
+#pragma unroll
+        for (int e = 0; e < F; ++e) sum[e] = 0.0;
+        // In every dimension the vertex is the low corner of its own cell, the high corner of the one before, and at the border
+        // also the high corner of its own.
+        bool border = false;
+#pragma unroll
+        for (int k = 0; k < D; ++k) border = border || v[k] == res - 1;
+        int combinations = 1;
+        for (int k = 0; k < D; ++k) combinations *= border ? 3 : 2;
+        for (int t = 0; t < combinations; ++t) {
+            unsigned int cell = 0, corner = 0;
+            bool there = true;
+            int digits = t;
+#pragma unroll
+            for (int k = 0; k < D; ++k) {
+                const int what = border ? digits % 3 : digits & 1;
+                digits = border ? digits / 3 : digits >> 1;
+                there = there && !(what == 1 && v[k] == 0) && !(what == 2 && v[k] != res - 1);
+                cell = (v[k] - (what == 1 ? 1u : 0u)) + cell * res;
+                corner |= (what != 0 ? 1u : 0u) << k;
+            }
+            if (!there) continue;
+            const float* at = base + (static_cast<size_t>(cell) * C::ROWS + corner) * F;
+            for (int c = 0; c < copies; ++c, at += static_cast<size_t>(n) * C::ELEMENTS) {
+                if constexpr (F == 2) {
+                    const float2 x = *reinterpret_cast<const float2*>(at);
+                    sum[0] += x.x; sum[1] += x.y;
+                } else {
+#pragma unroll
+                    for (int e = 0; e < F; e += 4) {
+                        const float4 x = *reinterpret_cast<const float4*>(at + e);
+                        sum[e] += x.x; sum[e + 1] += x.y; sum[e + 2] += x.z; sum[e + 3] += x.w;
+                    }
+                }
+            }
+        }
+        bool any = false;
+        float total[F];
+#pragma unroll
+        for (int e = 0; e < F; ++e) {
+            total[e] = static_cast<float>(sum[e]);
+            any = any || total[e] != 0.f;   // (also true of NaN)
+        }
+        if (any) grid_scatter_row<F>(g.grad, grid_checked_index<D, F>(g, lv, grid_vertex_index<D, F>(v, lv)), g.vecOk != 0, 1.f, total);
+    }
+}
+
 // elements of level l of a table of `levels` levels (levels with copies are small: 32 bits hold every index into them)
 __device__ __forceinline__ int grid_level_elements(const GridP& g, int l, int levels)
 {
@@ -588,10 +723,37 @@ __device__ __forceinline__ float* grid_grad_of_cta(const GridP& g, const GradRep
     if (BOUNDS_CHECK && n <= 0) return g.grad;   // (a table declared shorter than it is)
     return r.base + r.offset[group] + (blockIdx.x & ((1u << r.log2Copies[group]) - 1u)) * n - g.levels[l].offset;
 }
+// where this CTA adds up level `group` by cell, null: it does not
+template <int D, int F>
+__device__ __forceinline__ float* grid_records_of_cta(const GridP& g, const GradReplicas& r, int group, int l)
+{
+    if constexpr (GridCellUnits<D, F>::USED) {
+        if (group < MAX_GRID_LEVELS && r.byCell[group] != 0)
+            return r.base + r.offset[group] +
+                   static_cast<size_t>(blockIdx.x & ((1u << (r.byCell[group] - 1)) - 1u)) * grid_cell_count<D>(g.levels[l].resolution) * GridCellUnits<D, F>::ELEMENTS;
+    }
+    return nullptr;
+}
+// blocks of 256 threads for grid_sum_copies
+template <int D, int F>
+inline unsigned int grid_sum_blocks(const GridP& g, const GradReplicas& r, int group, int l)
+{
+    if (group >= MAX_GRID_LEVELS || !GridCellUnits<D, F>::USED || r.byCell[group] == 0) return 32;
+    const unsigned int n = (grid_cell_count<D>(g.levels[l].resolution) + 255) / 256;
+    return n < 32 ? 32 : (n > 1024 ? 1024 : n);
+}
 // sum of the copies of a level -> its gradient (grid-stride over blockIdx.x, 256 threads)
+template <int D, int F>
 __device__ __forceinline__ void grid_sum_copies(const GridP& g, const GradReplicas& r, int group, int l, int levels)
 {
-    if (group >= MAX_GRID_LEVELS || r.log2Copies[group] == 0 || g.grad == nullptr) return;
+    if (group >= MAX_GRID_LEVELS || g.grad == nullptr) return;
+    if constexpr (GridCellUnits<D, F>::USED) {
+        if (r.byCell[group] != 0) {
+            grid_sum_cells<D, F>(g, r, group, l);
+            return;
+        }
+    }
+    if (r.log2Copies[group] == 0) return;
     const int copies = 1 << r.log2Copies[group], n = grid_level_elements(g, l, levels);
     const float* src = r.base + r.offset[group];
     for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {

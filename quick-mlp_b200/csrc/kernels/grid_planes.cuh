@@ -203,6 +203,32 @@ __device__ __forceinline__ void scatter_group(const LaunchArgs& p, int g, const 
                 }
             }
             const GridLevelP& lv = grid.levels[l];
+            if (float* records = grid_records_of_cta<D, F>(grid, p.replicas, g, l)) {
+                if constexpr (GridCellUnits<D, F>::USED) {
+                    float pos[D];
+                    grid_position<D, Enc::START>(grid, side ? in1 : in0, pos);
+                    const auto unpack = [&](const uint32_t (&w)[(F + 1) / 2], float (&a)[F]) {
+#pragma unroll
+                        for (int i = 0; i < F / 2; ++i) {
+                            const float2 x = __half22float2(u32_as_h2(w[i]));
+                            a[2 * i] = x.x;
+                            a[2 * i + 1] = x.y;
+                        }
+                    };
+                    const bool done = grid_cells_scatter<D, F>(records, lv, pos, valid, [&](int r, float (&a)[F]) {
+                        uint32_t w[(F + 1) / 2];
+#pragma unroll
+                        for (int i = 0; i < (F + 1) / 2; ++i) w[i] = __shfl_sync(0xffffffffu, own[i], r, GridCellUnits<D, F>::LANES);
+                        unpack(w, a);
+                    });
+                    if (!done) {
+                        float a[F], none[D];
+                        unpack(own, a);
+                        grid_level_adjoint<D, F, false, true, false>(grid, lv, pos, a, none);
+                    }
+                }
+                return;
+            }
             float* grad = grid_grad_of_cta(grid, p.replicas, g, l, Enc::L);
 #pragma unroll
             for (int s = 0; s < 2; ++s) {
@@ -261,9 +287,20 @@ __device__ __forceinline__ void sum_group(const LaunchArgs& p, int g)
         if (g >= SG::before() + SG::own()) {
             sum_group<Spec, E + 1>(p, g);
         } else if constexpr (Enc::IS_GRID) {
-            grid_sum_copies(p.grids[Enc::SLOT], p.replicas, g, g - SG::before(), Enc::L);
+            grid_sum_copies<Enc::D, Enc::F>(p.grids[Enc::SLOT], p.replicas, g, g - SG::before(), Enc::L);
         }
     }
+}
+template <class Spec, int E>
+inline unsigned int sum_blocks(const LaunchArgs& a, int g)
+{
+    if constexpr (E < Spec::NUM_ENCODINGS) {
+        using Enc = typename Spec::template Enc<E>;
+        using SG = ScatterGroups<Spec, E>;
+        if (g >= SG::before() + SG::own()) return sum_blocks<Spec, E + 1>(a, g);
+        if constexpr (Enc::IS_GRID) return grid_sum_blocks<Enc::D, Enc::F>(a.grids[Enc::SLOT], a.replicas, g, g - SG::before());
+    }
+    return 0;
 }
 template <class Spec>
 __global__ void __launch_bounds__(256) sum_copies_kernel(const __grid_constant__ LaunchArgs p)
@@ -291,7 +328,7 @@ struct PlaneLaunchers {
             int sums = 0;   // the levels up to the last one that has copies
             long long from = a.replicas.total, to = a.replicas.total;
             for (int g = 0; g < groups && g < MAX_GRID_LEVELS; ++g) {
-                if (a.replicas.log2Copies[g] == 0) continue;
+                if (a.replicas.log2Copies[g] == 0 && a.replicas.byCell[g] == 0) continue;
                 if (g >= begin && g < end) {
                     if (sums == 0) from = a.replicas.offset[g];
                     sums = g - begin + 1;
@@ -306,7 +343,12 @@ struct PlaneLaunchers {
             }
             scatter_planes_kernel<Spec><<<static_cast<unsigned>(bx), SCATTER_THREADS, 0, s>>>(a);
             if (sums > 0) {
-                sum_copies_kernel<Spec><<<dim3(32, sums), 256, 0, s>>>(a);
+                unsigned int blocks = 32;
+                for (int g = begin; g < begin + sums; ++g) {
+                    const unsigned int n = sum_blocks<Spec, 0>(a, g);
+                    blocks = n > blocks ? n : blocks;
+                }
+                sum_copies_kernel<Spec><<<dim3(blocks, sums), 256, 0, s>>>(a);
                 if (launches) *launches = 2;
             }
             return cudaGetLastError();

@@ -73,6 +73,7 @@ struct GradReplicas {
     long long total;                        // elements
     unsigned int offset[MAX_GRID_LEVELS];        // first element of a level's copies; levels counted over all grids of the network
     unsigned char log2Copies[MAX_GRID_LEVELS];   // 0: the level has no copies
+    unsigned char byCell[MAX_GRID_LEVELS];       // 1 + log2 of the copies of a level whose gradient is added up by cell first (GridCellUnits); else 0
 };
 
 struct LaunchArgs {

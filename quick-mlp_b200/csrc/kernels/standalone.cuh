@@ -180,12 +180,40 @@ __global__ void __launch_bounds__(EncodingTile<Enc>::WARPS * 32) grid_encoding_a
         for (int l = 0; l < Enc::L; ++l) {
             const GridLevelP& lv = g.levels[l];
             float* grad = g.grad;
-            if constexpr (PARAM_GRAD) grad = grid_grad_of_cta(g, p.replicas, l, l, Enc::L);
+            float* records = nullptr;
+            if constexpr (PARAM_GRAD) {
+                grad = grid_grad_of_cta(g, p.replicas, l, l, Enc::L);
+                records = grid_records_of_cta<D, F>(g, p.replicas, l, l);
+            }
+            if constexpr (PARAM_GRAD && GridCellUnits<D, F>::USED) {
+                if (records != nullptr) {
+                    constexpr int C = Enc::CONCAT ? F : 0;
+                    float own[D];
+#pragma unroll
+                    for (int k = 0; k < D; ++k) own[k] = side ? pos[1][k] : pos[0][k];
+                    const bool done = grid_cells_scatter<D, F>(records, lv, own, row0 + lane <= last, [&](int r, float (&a)[F]) {
+                        T::get(tile + (lane / GridCellUnits<D, F>::LANES * GridCellUnits<D, F>::LANES + r) * T::STRIDE, l * C, a);
+                    });
+                    if (!done) {
+                        float a[F], none[D];
+                        T::get(tile + lane * T::STRIDE, l * C, a);
+                        grid_level_adjoint<D, F, Enc::HALF_TABLE, true, false>(g, lv, own, a, none);
+                    }
+                    if constexpr (!INPUT_GRAD) continue;
+                }
+            }
 #pragma unroll
             for (int s = 0; s < 2; ++s) {
                 if (i0 + s > last) continue;
                 float adjF[F];
                 T::get(tile + ((lane & ~1) + s) * T::STRIDE, Enc::CONCAT ? l * F : 0, adjF);
+                if constexpr (PARAM_GRAD && INPUT_GRAD && GridCellUnits<D, F>::USED) {
+                    if (records != nullptr) {   // (the table's gradient is done)
+                        if (lv.hashed) grid_half_adjoint<D, F, Enc::HALF_TABLE, false, true, 0>(g, grad, lv, pos[s], side, adjF, adjPos[s]);
+                        else grid_half_adjoint<D, F, Enc::HALF_TABLE, false, true, D - 1>(g, grad, lv, pos[s], side, adjF, adjPos[s]);
+                        continue;
+                    }
+                }
                 if (lv.hashed) grid_half_adjoint<D, F, Enc::HALF_TABLE, PARAM_GRAD, INPUT_GRAD, 0>(g, grad, lv, pos[s], side, adjF, adjPos[s]);
                 else grid_half_adjoint<D, F, Enc::HALF_TABLE, PARAM_GRAD, INPUT_GRAD, D - 1>(g, grad, lv, pos[s], side, adjF, adjPos[s]);
             }
@@ -207,7 +235,7 @@ __global__ void __launch_bounds__(EncodingTile<Enc>::WARPS * 32) grid_encoding_a
 template <class Enc>
 __global__ void __launch_bounds__(256) sum_replicas_kernel(const __grid_constant__ LaunchArgs p)
 {
-    grid_sum_copies(p.grids[0], p.replicas, blockIdx.y, blockIdx.y, Enc::L);
+    grid_sum_copies<Enc::D, Enc::F>(p.grids[0], p.replicas, blockIdx.y, blockIdx.y, Enc::L);
 }
 
 template <class EncSpec>
@@ -245,7 +273,14 @@ struct EncodingLaunchers {
                     if (e != cudaSuccess) return e;
                 }
                 grid_encoding_adjoint_kernel<Enc, INPUT_GRAD, PARAM_GRAD><<<blocksFor(a, threads), threads, 0, s>>>(a);
-                if (copies) sum_replicas_kernel<Enc><<<dim3(32, Enc::L), 256, 0, s>>>(a);
+                if (copies) {
+                    unsigned int blocks = 32;
+                    for (int l = 0; l < Enc::L; ++l) {
+                        const unsigned int n = grid_sum_blocks<Enc::D, Enc::F>(a.grids[0], a.replicas, l, l);
+                        blocks = n > blocks ? n : blocks;
+                    }
+                    sum_replicas_kernel<Enc><<<dim3(blocks, Enc::L), 256, 0, s>>>(a);
+                }
                 count = copies ? 2 : 1;
                 return cudaGetLastError();
             }

@@ -216,3 +216,34 @@ def test_adjoint_with_gradient_copies(name, n):
     (gx0, gt0), (gx1, gt1) = results
     assert torch.equal(gx0, gx1)
     helpers.assert_close(gt1.cpu().numpy(), gt0.cpu().numpy(), f"{name} n={n}", rtol=2.0 ** -9, atol=1e-5 * float(gt0.abs().max()))
+
+
+@pytest.mark.parametrize("name,n", [("dense2d_multires", 131073), ("hash3d_f2", 262147), ("hash4d_f4", 265001), ("hash2d_f8", 530001)])
+def test_adjoint_added_up_by_cell(name, n):
+    """Batches that are large enough for the gradient of the small levels to be added up by cell first, against the same call without
+    scratch: points below the box (other corners than a cell's), above it and on its borders. Tolerance as above; no row
+    gets more than 2^18 terms of a few times the largest adjoint, most of them of one sign."""
+    import ctypes as C
+    import torch
+    from qmlp._capi import check, lib, wrap
+    cfg, e, oe = _enc(name)
+    x = helpers.uniform(10, 1, (n, oe.n_in), -0.02, 1.02)
+    x[::97] = np.round(x[::97])
+    x = torch.from_numpy(x).cuda()
+    adj = torch.from_numpy(helpers.uniform(10, 2, (n, oe.num_outputs), 0.0, 1.0)).cuda()
+    table = torch.from_numpy(helpers.uniform(10, 3, (oe.num_parameters,), -1.0, 1.0)).cuda()
+    for mode in (2, 3):
+        need = C.c_size_t()
+        check(lib().qmlp_encoding_adjoint_memory(e._h, n, mode, C.byref(need)))
+        assert need.value > 0
+        results = []
+        for tmp in (None, torch.full((need.value,), 0x7e, dtype=torch.uint8, device="cuda")):
+            gx, gt = torch.zeros_like(x), torch.zeros_like(table)
+            p, g, ai = wrap(table), wrap(gt), wrap(gx)
+            check(lib().qmlp_encoding_adjoint_with_memory(e._h, wrap(x), wrap(adj), ai, None, C.byref(p), C.byref(g), mode,
+                                                          tmp.data_ptr() if tmp is not None else None, need.value if tmp is not None else 0))
+            torch.cuda.synchronize()
+            results.append((gx, gt))
+        (gx0, gt0), (gx1, gt1) = results
+        assert torch.equal(gx0, gx1)
+        helpers.assert_close(gt1.cpu().numpy(), gt0.cpu().numpy(), f"{name} n={n}", rtol=2.0 ** -9, atol=1e-5 * float(gt0.abs().max()))
