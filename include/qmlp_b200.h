@@ -234,6 +234,11 @@ QMLP_API int qmlp_encoding_zero_gradients(qmlp_encoding_t* enc, qmlp_stream_t st
  * `parameters` may be NULL (use the bound parameter). */
 QMLP_API int qmlp_encoding_forward(qmlp_encoding_t* enc, const qmlp_tensor_t* input, qmlp_tensor_t* output,
                                    qmlp_stream_t stream, const qmlp_tensor_t* parameters);
+/* The same with optional scratch memory (qmlp_encoding_forward_memory() bytes for these parameters, 256-byte aligned, contents
+ * irrelevant): large batches on small grid levels then read copies of the levels in which the rows of a cell lie side by side. */
+QMLP_API int qmlp_encoding_forward_memory(qmlp_encoding_t* enc, int64_t num_elements, const qmlp_tensor_t* parameters, size_t* bytes);
+QMLP_API int qmlp_encoding_forward_with_memory(qmlp_encoding_t* enc, const qmlp_tensor_t* input, qmlp_tensor_t* output,
+                                               qmlp_stream_t stream, const qmlp_tensor_t* parameters, void* tmp_memory, size_t tmp_bytes);
 /* IEncoding::adjoint, src_cpp/src/iencoding.cpp:97-196 */
 QMLP_API int qmlp_encoding_adjoint(qmlp_encoding_t* enc, const qmlp_tensor_t* input, const qmlp_tensor_t* adj_output,
                                    qmlp_tensor_t* adj_input, qmlp_stream_t stream, const qmlp_tensor_t* parameters,

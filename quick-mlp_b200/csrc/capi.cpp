@@ -226,8 +226,8 @@ size_t replicaBytes(const Network& n, int64_t points)
 size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 void bindReplicas(const Network& n, kernel::LaunchArgs& a, void* memory)
 {
-    n.planReplicas(a.numel, a.replicas);
-    if (a.replicas.total > 0) a.replicas.base = static_cast<float*>(memory);
+    n.planReplicas(a.numel, a.level->replicas);
+    if (a.level->replicas.total > 0) a.level->replicas.base = static_cast<float*>(memory);
 }
 
 } // namespace
@@ -484,11 +484,17 @@ static void inferenceLocked(Network& n, const qmlp_tensor_t* input, qmlp_tensor_
     a.output = static_cast<float*>(output->data);
     a.outS0 = output->strides[0];
     a.outS1 = output->strides[1];
+    const int64_t rowBytes = static_cast<int64_t>(n.encodedChannels()) * 2;
     int64_t need = a.numGrids > 0 ? planeChunk(n, a.numel) : 0;
     if (need > 0) {
-        const int64_t rowBytes = static_cast<int64_t>(n.encodedChannels()) * 2;
-        __half* planes = static_cast<__half*>(memory);
-        if (memory == nullptr || memoryBytes < static_cast<size_t>(need * rowBytes)) {
+        // copies of small levels by cell only in the caller's memory, behind the planes
+        const size_t planeBytes = align256(static_cast<size_t>(need * rowBytes));
+        __half* planes = memory != nullptr && memoryBytes >= planeBytes ? static_cast<__half*>(memory) : nullptr;
+        if (planes != nullptr) {
+            const size_t cellBytes = n.planCells(a.numel, a.level->cells);
+            if (cellBytes > 0 && memoryBytes >= planeBytes + cellBytes) a.level->cells.base = static_cast<unsigned char*>(memory) + planeBytes;
+        }
+        if (planes == nullptr) {
             n.claimDevice();
             if (n.planeCapacity < need) {
                 if (n.planes) {
@@ -514,7 +520,7 @@ static void inferenceLocked(Network& n, const qmlp_tensor_t* input, qmlp_tensor_
             a.output = out0 + c0 * a.outS0;
             a.planes = planes;
             a.planeStride = need;
-            a.flags = kernel::FLAG_HALF_SUMS;
+            a.flags = kernel::FLAG_HALF_SUMS | (c0 == 0 ? kernel::FLAG_FILL_CELLS : 0);
             int launches = 0;
             int e;
             {
@@ -546,7 +552,9 @@ int qmlp_network_inference_memory(qmlp_network_t* net, int64_t num_elements, siz
     if (!bytes) throw std::runtime_error("null argument");
     Network& n = *net->impl;
     std::lock_guard<std::mutex> lock(n.mutex);
-    *bytes = static_cast<size_t>(planeChunk(n, num_elements)) * n.encodedChannels() * 2;
+    const int64_t chunk = planeChunk(n, num_elements);
+    kernel::CellTables cells;
+    *bytes = chunk > 0 ? align256(static_cast<size_t>(chunk) * n.encodedChannels() * 2) + n.planCells(num_elements, cells) : 0;
     QMLP_CATCH
 }
 
@@ -950,8 +958,27 @@ static void encodingArgs(Encoding& e, kernel::LaunchArgs& a, const qmlp_tensor_t
     }
 }
 
+int qmlp_encoding_forward_memory(qmlp_encoding_t* enc, int64_t num_elements, const qmlp_tensor_t* parameters, size_t* bytes)
+{
+    QMLP_TRY
+    if (!bytes) throw std::runtime_error("null argument");
+    *bytes = 0;
+    if (auto* g = dynamic_cast<EncodingHashGrid*>(enc->impl.get())) {
+        const bool given = parameters != nullptr && parameters->ndim > 0;
+        kernel::CellTables c{};
+        *bytes = g->planCells(num_elements, 0, (given ? parameters->precision : g->paramInference.precision) == QMLP_HALF, c, 0);
+    }
+    QMLP_CATCH
+}
+
 int qmlp_encoding_forward(qmlp_encoding_t* enc, const qmlp_tensor_t* input, qmlp_tensor_t* output, qmlp_stream_t stream,
                           const qmlp_tensor_t* parameters)
+{
+    return qmlp_encoding_forward_with_memory(enc, input, output, stream, parameters, nullptr, 0);
+}
+
+int qmlp_encoding_forward_with_memory(qmlp_encoding_t* enc, const qmlp_tensor_t* input, qmlp_tensor_t* output, qmlp_stream_t stream,
+                                      const qmlp_tensor_t* parameters, void* tmp_memory, size_t tmp_bytes)
 {
     QMLP_TRY
     Encoding& e = *enc->impl;
@@ -973,6 +1000,14 @@ int qmlp_encoding_forward(qmlp_encoding_t* enc, const qmlp_tensor_t* input, qmlp
         a.output = static_cast<float*>(output->data);
         a.outS0 = output->strides[0];
         a.outS1 = output->strides[1];
+        if (auto* g = dynamic_cast<EncodingHashGrid*>(&e); g && tmp_memory) {
+            if ((reinterpret_cast<uintptr_t>(tmp_memory) & 255) != 0) throw std::runtime_error("scratch memory must be 256-byte aligned");
+            const size_t need = g->planCells(a.numel, 0, e.paramInference.precision == QMLP_HALF, a.level->cells, 0);
+            if (need > 0 && need <= tmp_bytes) {
+                a.level->cells.base = static_cast<unsigned char*>(tmp_memory);
+                a.flags = kernel::FLAG_FILL_CELLS;
+            }
+        }
         if (a.numel > 0) {
             auto m = e.standaloneModule(e.paramInference.precision == QMLP_HALF && e.isGrid());
             checkLaunch(m->launch(kernel::KERNEL_ENCODING_FORWARD, &a, static_cast<cudaStream_t>(stream), nullptr), "kernel launch failed");
@@ -1048,9 +1083,9 @@ int qmlp_encoding_adjoint_with_memory(qmlp_encoding_t* enc, const qmlp_tensor_t*
         a.flags = (gIn ? 1 : 0) | (gP ? 2 : 0);
         if (auto* g = dynamic_cast<EncodingHashGrid*>(&e); g && gP && tmp_memory) {
             if ((reinterpret_cast<uintptr_t>(tmp_memory) & 15) != 0) throw std::runtime_error("scratch memory must be 16-byte aligned");
-            g->planReplicas(a.numel, 0, a.replicas);
-            if (a.replicas.total > 0 && static_cast<size_t>(a.replicas.total) * sizeof(float) <= tmp_bytes) a.replicas.base = static_cast<float*>(tmp_memory);
-            else std::memset(&a.replicas, 0, sizeof a.replicas);
+            g->planReplicas(a.numel, 0, a.level->replicas);
+            if (a.level->replicas.total > 0 && static_cast<size_t>(a.level->replicas.total) * sizeof(float) <= tmp_bytes) a.level->replicas.base = static_cast<float*>(tmp_memory);
+            else std::memset(&a.level->replicas, 0, sizeof a.level->replicas);
         }
         if (a.numel > 0 && a.flags != 0) {
             auto m = e.standaloneModule(e.paramInference.precision == QMLP_HALF && e.isGrid());
@@ -1152,7 +1187,7 @@ int qmlp_convert_half(const float* src, uint16_t* dst, int64_t count, qmlp_strea
 // of a split step; the copies of points and targets in bin order and the bin tables of the
 // spatially binned step (only for networks with a grid encoding).
 struct TrainerLayout {
-    size_t adjOut = 0, planes = 0, replicas = 0, weightSums = 0, sortedInput = 0, sortedTarget = 0, bins = 0, total = 0;
+    size_t adjOut = 0, planes = 0, replicas = 0, cells = 0, weightSums = 0, sortedInput = 0, sortedTarget = 0, bins = 0, total = 0;
     int binCount = 0;
 };
 static TrainerLayout trainerLayout(const Network& n, int64_t points)
@@ -1167,6 +1202,9 @@ static TrainerLayout trainerLayout(const Network& n, int64_t points)
     b = align(b + adjointPlaneBytes(n, n32, QMLP_GRADIENTS_NETWORK_WEIGHTS | QMLP_GRADIENTS_INPUT_ENCODINGS));
     l.replicas = b;
     b = align(b + replicaBytes(n, points));
+    l.cells = b;
+    kernel::CellTables cells;
+    b = align(b + n.planCells(points, cells, /*widest=*/true));   // (the size does not depend on what is bound)
     l.weightSums = b;
     b = align(b + static_cast<size_t>(n.parameterCount()) * sizeof(float));
     const int dims = n.sortDimensions();
@@ -1322,6 +1360,7 @@ int qmlp_trainer_gradients_part(qmlp_trainer_t* tr, const qmlp_tensor_t* input, 
     for (int i = 0; i < n.numEncodings(); ++i) anyGrid = anyGrid || n.encoding(i)->hasParameters();
     __half* planes = anyGrid ? reinterpret_cast<__half*>(ws + lay.planes) : nullptr;
     bindReplicas(n, a, ws + lay.replicas);
+    if (n.planCells(numel, a.level->cells) > 0) a.level->cells.base = ws + lay.cells;
     // Gather-dominated batches (same rule as inference): the encodings are computed one grid level at a time into
     // the plane region of the workspace, which is free until the backward kernel writes the adjoint planes there,
     // and the forward kernel reads its layer-0 operand from the planes.
@@ -1405,7 +1444,11 @@ int qmlp_trainer_gradients_part(qmlp_trainer_t* tr, const qmlp_tensor_t* input, 
                 tr->weightsWait = true;
             }
             if (what & 5) {
-                if (anyGrid) launchModule(n, *m, kernel::KERNEL_ENCODE_PLANES, a, stream);
+                if (anyGrid) {
+                    kernel::LaunchArgs e = a;
+                    e.flags |= kernel::FLAG_FILL_CELLS;
+                    launchModule(n, *m, kernel::KERNEL_ENCODE_PLANES, e, stream);
+                }
                 launchModule(n, *m, kernel::KERNEL_TRAIN, a, stream);
             }
             if (what == 8) {
@@ -1422,6 +1465,7 @@ int qmlp_trainer_gradients_part(qmlp_trainer_t* tr, const qmlp_tensor_t* input, 
         if (wantPlanes) {
             a.planes = planes;
             a.planeStride = n32;
+            a.flags = kernel::FLAG_FILL_CELLS;
             auto m = n.module(n.currentHalfMask());
             int launches = 0;
             int e;

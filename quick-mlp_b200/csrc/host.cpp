@@ -1,12 +1,14 @@
 // Activations, encodings, network spec, parameter layout and source generation for the per-spec instantiation.
 #include "host.hpp"
 
+#include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstring>
 #include <fstream>
 #include <random>
 #include <cctype>
+#include <cstdlib>
 #include <set>
 #include <sstream>
 #include <sys/stat.h>
@@ -365,6 +367,24 @@ void EncodingHashGrid::planReplicas(int64_t points, int group, kernel::GradRepli
     }
 }
 
+size_t EncodingHashGrid::planCells(int64_t points, int group, bool halfTable, kernel::CellTables& c, size_t bytes) const
+{
+    // Rows of four and more features in levels with at most a quarter as many cells as the batch has points, copies of up to 128 MB (they are
+    // read at random: from L2), from 3/4 million points on: 4-D grid of fp16 rows, 2^24 points 10120 -> 9520 us; 2-D pyramid of fp32 rows,
+    // 10^6 points 155 -> 143, 2^18 points 71 -> 76 (the host's launch); mixed network, step of 2^21 points 1487 -> 1474, 2^19 points 448 -> 453.
+    // Rows of two features gain nothing: 3-D grid, step of 2^20 points 786 -> 797 (fp16 rows), 823 -> 825 (fp32).
+    const int64_t cellBytes = (static_cast<int64_t>(features_) << dim_) * (halfTable ? 2 : 4);   // (kernel::GridCellRows)
+    if (isLine() || dim_ < 2 || (features_ != 4 && features_ != 8) || cellBytes < 64 || cellBytes > 256 || points < (3 << 18)) return bytes;
+    for (int l = 0; l < levels_ && group + l < kernel::MAX_GRID_LEVELS; ++l) {
+        double cells = 1;
+        for (int k = 0; k < dim_; ++k) cells *= table_[l].resolution;
+        if (cells * 4 > static_cast<double>(points) || cells * static_cast<double>(cellBytes) > static_cast<double>(128 << 20)) continue;
+        c.offset[group + l] = static_cast<unsigned int>(bytes / 256 + 1);
+        bytes += (static_cast<size_t>(cells) * cellBytes + 255) / 256 * 256;
+    }
+    return bytes;
+}
+
 void EncodingHashGrid::setParameter(const qmlp_tensor_t* t, int usage)
 {
     BoundTensor b;
@@ -670,6 +690,21 @@ void Network::planReplicas(int64_t points, kernel::GradReplicas& r) const
             h->planReplicas(points, group, r);
             group += static_cast<int>(h->levelTable().size());
         }
+}
+
+size_t Network::planCells(int64_t points, kernel::CellTables& c, bool widest) const
+{
+    std::memset(&c, 0, sizeof c);
+    size_t bytes = 0;
+    int group = 0;
+    for (const auto& e : encodings_)
+        if (auto* h = dynamic_cast<const EncodingHashGrid*>(e.get())) {
+            if (h->isLine()) continue;
+            if (widest) bytes = std::max(h->planCells(points, group, false, c, bytes), h->planCells(points, group, true, c, bytes));
+            else bytes = h->planCells(points, group, h->paramInference.precision == QMLP_HALF, c, bytes);
+            group += static_cast<int>(h->levelTable().size());
+        }
+    return bytes;
 }
 
 int Network::gridLevels() const

@@ -171,6 +171,9 @@ public:
     // copies of the gradients of small levels for a batch of `points` (kernel::GradReplicas; base is left as it is),
     // appended to `r` from level `group` (counted over all grids of a network) on
     void planReplicas(int64_t points, int group, kernel::GradReplicas& r) const;
+    // copies of small levels by cell for a batch of `points` (kernel::CellTables; base is left as it is), appended to `c` from
+    // level `group` on behind the first `bytes` bytes; returns the bytes then used
+    size_t planCells(int64_t points, int group, bool halfTable, kernel::CellTables& c, size_t bytes) const;
     int features() const { return features_; }
     int dimension() const { return dim_; }
     Json gridJson() const;   // the hash grid's own configuration (id "HashGrid")
@@ -258,6 +261,9 @@ public:
     int64_t gridTableBytes() const;   // bytes of all bound grid tables (what the gather walks through)
     int gathersPerPoint() const;      // table rows fetched per point by all plain grid encodings: sum of levels * 2^D
     void planReplicas(int64_t points, kernel::GradReplicas& r) const;   // of all grid encodings; zeroes `r` first
+    // copies by cell of all grid encodings for tables of the type that is bound; zeroes `c` first, returns the bytes. `widest`: the
+    // bytes that are enough whatever is bound
+    size_t planCells(int64_t points, kernel::CellTables& c, bool widest = false) const;
     int gridLevels() const;           // levels of all grid encodings
     int sortDimensions() const;       // dimension of the grid whose bounding box bins the points of a training step (0: none)
     // level-major encoding pass (inference of networks with tables larger than L2): chunk buffer, allocated at the

@@ -601,8 +601,10 @@ struct TcLaunchers {
     static cudaError_t inference(const LaunchArgs& a, cudaStream_t s) { return run<false>(a, s); }
     static cudaError_t inferencePlanes(const LaunchArgs& a, cudaStream_t s) { return run<true>(a, s); }
     // level-major encoding pass: blockIdx.y = level (slow), blockIdx.x strides over the points of the chunk
-    static cudaError_t encodePlanes(const LaunchArgs& a, cudaStream_t s)
+    static cudaError_t encodePlanes(const LaunchArgs& a, cudaStream_t s, int* launches)
     {
+        const cudaError_t filled = fill_cells<Spec>(a, s, launches);
+        if (filled != cudaSuccess) return filled;
         constexpr int groups = plane_group_count<Spec>();
         long long bx = (a.numel + 255) / 256;
         const long long cap = static_cast<long long>(a.numSMs) * 8;

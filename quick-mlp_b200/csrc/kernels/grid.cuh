@@ -333,6 +333,11 @@ struct GridHalfCell {
     __device__ __forceinline__ GridHalfCell(const float (&pos)[D], int resolution, int side)
     {
         grid_cell<D>(pos, resolution, c);
+        take(side);
+    }
+    __device__ __forceinline__ GridHalfCell(const GridCell<D>& cell, int side) : c(cell) { take(side); }
+    __device__ __forceinline__ void take(int side)
+    {
         vp = side ? c.hi[PD] : c.lo[PD];
         wp = side ? c.f[PD] : 1.f - c.f[PD];
     }
@@ -504,6 +509,178 @@ __device__ __forceinline__ void grid_pair_sums(const GridP& g, const GridLevelP&
     for (int i = 0; i < F; ++i) feat[i] = (side ? f1[i] : f0[i]) + __shfl_xor_sync(0xffffffffu, side ? f0[i] : f1[i], 1);
 }
 
+// ---- copies by cell (CellTables) ------------------------------------------------------------------------------------
+// A level with few cells, compared with the points of a batch, is copied so that the 2^D rows of a cell lie side by side: the lanes
+// of a pair then read one contiguous piece of memory, one request, where the rows of the table take 2^(D-1) (the request
+// rate bounds the gathers, see above). The rows of a cell stand as the lanes of a pair fetch them, in accesses of up to
+// 32 bytes: low side of the pairing dimension, high side, low side, ...; within a side by the bits of the other dimensions. The
+// terms and their order are those of the table's rows.
+template <int D, int F, bool HALF>
+struct GridCellRows {
+    static constexpr int H = 1 << (D - 1), ROW = F * (HALF ? 2 : 4), WORDS = ROW / 4;   // rows per side; bytes and words of a row
+    static constexpr int BYTES = 2 * H * ROW;
+    static constexpr bool USED = D >= 2 && (F == 4 || F == 8) && BYTES >= 64 && BYTES <= 256;   // (the host's rule: EncodingHashGrid::planCells)
+    static constexpr int ACCESS = H * ROW < 32 ? H * ROW : 32, PER_ACCESS = ACCESS / ROW, ACCESSES = H / PER_ACCESS;
+};
+
+// Cells are numbered by their low corner, neighbours along the dimension whose vertices are neighbouring rows first (the copy is
+// filled with coalesced reads).
+template <int D>
+__device__ __forceinline__ unsigned int grid_cell_number(const GridCell<D>& c, const GridLevelP& lv)
+{
+    unsigned int n;
+    if (lv.hashed) {
+        n = c.lo[D - 1];
+#pragma unroll
+        for (int k = D - 2; k >= 0; --k) n = c.lo[k] + n * static_cast<unsigned int>(lv.resolution);
+    } else {
+        n = c.lo[0];
+#pragma unroll
+        for (int k = 1; k < D; ++k) n = c.lo[k] + n * static_cast<unsigned int>(lv.resolution);
+    }
+    return n;
+}
+// The copy holds the cells of points inside the box: high corner = low corner + 1, or the border. A point below the box has
+// other corners.
+template <int D>
+__device__ __forceinline__ bool grid_cell_regular(const GridCell<D>& c, const GridLevelP& lv)
+{
+    bool ok = true;
+#pragma unroll
+    for (int k = 0; k < D; ++k) ok = ok && c.hi[k] == min(c.lo[k] + 1u, static_cast<unsigned int>(lv.resolution - 1));
+    return ok;
+}
+
+// this lane's rows (one side of the pairing dimension) of a cell
+template <int D, int F, bool HALF>
+__device__ __forceinline__ void grid_cell_load(const unsigned char* cells, unsigned int cell, int side,
+                                               uint32_t (&raw)[1 << (D - 1)][GridCellRows<D, F, HALF>::WORDS])
+{
+    using C = GridCellRows<D, F, HALF>;
+    const unsigned char* at = cells + static_cast<size_t>(cell) * C::BYTES + side * C::ACCESS;
+#pragma unroll
+    for (int u = 0; u < C::ACCESSES; ++u) {
+        uint32_t v[8];
+        static_assert(C::ACCESS == 32);
+        ldg_nc_u256(at + u * 2 * C::ACCESS, v);
+#pragma unroll
+        for (int r = 0; r < C::PER_ACCESS; ++r)
+#pragma unroll
+            for (int i = 0; i < C::WORDS; ++i) raw[u * C::PER_ACCESS + r][i] = v[r * C::WORDS + i];
+    }
+}
+
+// feat += w * row
+template <int F, bool HALF>
+__device__ __forceinline__ void grid_add_row(float w, const uint32_t (&r)[F * (HALF ? 2 : 4) / 4], float (&feat)[F])
+{
+    if constexpr (HALF) {
+#pragma unroll
+        for (int i = 0; i < F / 2; ++i) {
+            const float2 x = __half22float2(u32_as_h2(r[i]));
+            feat[2 * i] += w * x.x;
+            feat[2 * i + 1] += w * x.y;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < F; ++i) feat[i] += w * __uint_as_float(r[i]);
+    }
+}
+
+// grid_pair_forward from the copy. False, for the whole warp, if one of its points has other corners than the copy holds.
+template <int D, int F, bool HALF, bool EXCHANGE, int PD>
+__device__ __forceinline__ bool grid_pair_from_cells(const unsigned char* cells, const GridLevelP& lv, const float (&pos0)[D], const float (&pos1)[D], int side,
+                                                     float (&feat)[F])
+{
+    using C = GridCellRows<D, F, HALF>;
+    GridCell<D> c0, c1;
+    grid_cell<D>(pos0, lv.resolution, c0);
+    grid_cell<D>(pos1, lv.resolution, c1);
+#pragma unroll
+    for (int k = 0; k < D; ++k) asm volatile("" : "+f"(c0.f[k]), "+f"(c1.f[k]));   // (computed here, beside the product they come from, as in the other path)
+    if (!__all_sync(0xffffffffu, grid_cell_regular<D>(c0, lv) && grid_cell_regular<D>(c1, lv))) return false;
+    uint32_t raw0[C::H][C::WORDS], raw1[C::H][C::WORDS];
+    grid_cell_load<D, F, HALF>(cells, grid_cell_number<D>(c0, lv), side, raw0);
+    grid_cell_load<D, F, HALF>(cells, grid_cell_number<D>(c1, lv), side, raw1);
+    if constexpr (EXCHANGE) {
+        GridCell<D> own;
+#pragma unroll
+        for (int i = 0; i < D; ++i) own.f[i] = side ? c1.f[i] : c0.f[i];
+#pragma unroll
+        for (int i = 0; i < F; ++i) feat[i] = 0.f;
+        grid_pair_blend<D, F, PD, C::WORDS>(own, side, raw0, raw1, feat,
+                                           [](float w, const uint32_t (&r)[C::WORDS], float (&f)[F]) { grid_add_row<F, HALF>(w, r, f); });
+    } else {
+        const GridHalfCell<D, PD> h0(c0, side), h1(c1, side);
+        float f0[F], f1[F];
+#pragma unroll
+        for (int i = 0; i < F; ++i) f0[i] = f1[i] = 0.f;
+#pragma unroll
+        for (int h = 0; h < C::H; ++h) {
+            grid_add_row<F, HALF>(h0.weight(h), raw0[h], f0);
+            grid_add_row<F, HALF>(h1.weight(h), raw1[h], f1);
+        }
+#pragma unroll
+        for (int i = 0; i < F; ++i) feat[i] = (side ? f1[i] : f0[i]) + __shfl_xor_sync(0xffffffffu, side ? f0[i] : f1[i], 1);
+    }
+    return true;
+}
+
+// copy of level `group` (counted over all grids), null: none
+__device__ __forceinline__ const unsigned char* grid_cells(const CellTables& t, int group)
+{
+    if (t.base == nullptr || group >= MAX_GRID_LEVELS || t.offset[group] == 0) return nullptr;
+    return t.base + static_cast<size_t>(t.offset[group] - 1) * 256;
+}
+
+constexpr int FILL_THREADS = 256;
+// blocks that fill the copy of a level: a thread writes one access
+template <int D, int F, bool HALF>
+__host__ __device__ inline unsigned int grid_fill_blocks(int resolution)
+{
+    unsigned int n = 1;
+    for (int k = 0; k < D; ++k) n *= static_cast<unsigned int>(resolution);
+    return (n * (2 * GridCellRows<D, F, HALF>::ACCESSES) + FILL_THREADS - 1) / FILL_THREADS;
+}
+template <int D, int F, bool HALF>
+__device__ __forceinline__ void grid_fill_cells(const GridP& g, const GridLevelP& lv, unsigned char* cells, unsigned int block)
+{
+    using C = GridCellRows<D, F, HALF>;
+    const unsigned int t = block * FILL_THREADS + threadIdx.x, side = t & 1u, u = (t >> 1) % C::ACCESSES, res = static_cast<unsigned int>(lv.resolution);
+    unsigned int n = (t >> 1) / C::ACCESSES, lo[D];
+    // (the dimension that varies first: grid_cell_number)
+#pragma unroll
+    for (int j = 0; j < D; ++j) {
+        const unsigned int q = n / res, r = n - q * res;
+        if (lv.hashed) lo[j] = r;
+        else lo[D - 1 - j] = r;
+        n = q;
+    }
+    if (n != 0) return;   // past the last cell
+    GridCell<D> c;
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+        c.lo[k] = lo[k];
+        c.hi[k] = min(lo[k] + 1u, res - 1u);
+    }
+    uint32_t v[8];
+#pragma unroll
+    for (int r = 0; r < C::PER_ACCESS; ++r) {
+        const unsigned int h = u * C::PER_ACCESS + r;
+        const int b = static_cast<int>(lv.hashed ? (h << 1 | side) : (h | side << (D - 1)));
+        const unsigned int e = grid_corner_index<D, F>(g, c, lv, b);
+        float row[F];
+        grid_load_row<F, HALF>(g.table, e, g.vecOk != 0, row);
+#pragma unroll
+        for (int i = 0; i < C::WORDS; ++i) {
+            if constexpr (HALF) v[r * C::WORDS + i] = h2_as_u32(__floats2half2_rn(row[2 * i], row[2 * i + 1]));
+            else v[r * C::WORDS + i] = __float_as_uint(row[i]);
+        }
+    }
+    unsigned char* at = cells + static_cast<size_t>(t) * C::ACCESS;   // (accesses in the order of the threads)
+    stg_u256(at, v);
+}
+
 // Features of one level for this lane's own point; all lanes of the warp take part. The lanes exchange rows or, unless EXACT,
 // half sums. With half sums a feature next to the middle of two fp16 numbers can be rounded to the other one, which moves a
 // ReLU input across zero now and then and with it the gradients behind it (3-D grid of 16 levels, 25 843 points: one
@@ -512,10 +689,16 @@ __device__ __forceinline__ void grid_pair_sums(const GridP& g, const GridLevelP&
 // 280 us in all), above that the half sums (two fp32 features, 100 000 points: 41.0 against 42.8 us; 4-D grid of four fp16
 // features, 2^24 points: 10.5 against 11.7 ms).
 template <int D, int F, bool HALF, bool EXACT>
-__device__ __forceinline__ void grid_pair_forward(const GridP& g, const GridLevelP& lv, const float (&pos0)[D], const float (&pos1)[D], int side,
-                                                  float (&feat)[F])
+__device__ __forceinline__ void grid_pair_forward(const GridP& g, const GridLevelP& lv, const unsigned char* cells, const float (&pos0)[D], const float (&pos1)[D],
+                                                  int side, float (&feat)[F])
 {
     constexpr int WORDS = (1 << (D - 1)) * ((HALF && F % 2 == 0) ? F / 2 : F);
+    if constexpr (GridCellRows<D, F, HALF>::USED) {
+        if (cells != nullptr) {
+            if (lv.hashed ? grid_pair_from_cells<D, F, HALF, EXACT || WORDS <= 4, 0>(cells, lv, pos0, pos1, side, feat)
+                          : grid_pair_from_cells<D, F, HALF, EXACT || WORDS <= 4, D - 1>(cells, lv, pos0, pos1, side, feat)) return;
+        }
+    }
     if constexpr (EXACT || WORDS <= 4) {
         if (lv.hashed) grid_pair_exchange<D, F, HALF, 0>(g, lv, pos0, pos1, side, feat);
         else grid_pair_exchange<D, F, HALF, D - 1>(g, lv, pos0, pos1, side, feat);

@@ -38,6 +38,27 @@ __host__ __device__ constexpr int plane_group_count()
     return PlaneGroups<Spec, Spec::NUM_ENCODINGS - 1>::before() + PlaneGroups<Spec, Spec::NUM_ENCODINGS - 1>::own();
 }
 
+// levels of the plain grids, counted over all encodings
+template <class Spec, int E>
+struct ScatterGroups {
+    using Enc = typename Spec::template Enc<E>;
+    __host__ __device__ static constexpr int own()
+    {
+        if constexpr (Enc::IS_GRID) return Enc::L;
+        else return 0;
+    }
+    __host__ __device__ static constexpr int before()
+    {
+        if constexpr (E == 0) return 0;
+        else return ScatterGroups<Spec, E - 1>::before() + ScatterGroups<Spec, E - 1>::own();
+    }
+};
+template <class Spec>
+__host__ __device__ constexpr int scatter_group_count()
+{
+    return ScatterGroups<Spec, Spec::NUM_ENCODINGS - 1>::before() + ScatterGroups<Spec, Spec::NUM_ENCODINGS - 1>::own();
+}
+
 template <int W>
 __device__ __forceinline__ void store_halfs(const LaunchArgs& p, __half* dst, const float (&v)[W])
 {
@@ -95,7 +116,7 @@ __device__ __forceinline__ void encode_group(const LaunchArgs& p, int g, const R
             for (int l = first; l < end; ++l) {
                 const GridLevelP& lv = grid.levels[l];
                 float f[F];
-                grid_pair_forward<D, F, Enc::HALF_TABLE, EXACT>(grid, lv, pos0, pos1, side, f);
+                grid_pair_forward<D, F, Enc::HALF_TABLE, EXACT>(grid, lv, grid_cells(p.level->cells, ScatterGroups<Spec, E>::before() + l), pos0, pos1, side, f);
 #pragma unroll
                 for (int i = 0; i < F; ++i) feat[i] += f[i];
             }
@@ -143,31 +164,58 @@ __global__ void __launch_bounds__(256, plane_min_blocks<Spec>()) encode_planes_k
     }
 }
 
+// ---- copies by cell (CellTables) --------------------------------------------------------------------------------------
+// visit(encoding index constant, level of the grid, level over all grids) for every level that has a copy
+template <class Spec, int E = 0, class Visit>
+__host__ __device__ __forceinline__ void each_cell_level(const LaunchArgs& p, const Visit& visit)
+{
+    if constexpr (E < Spec::NUM_ENCODINGS) {
+        using Enc = typename Spec::template Enc<E>;
+        if constexpr (Enc::IS_GRID) {
+            if constexpr (GridCellRows<Enc::D, Enc::F, Enc::HALF_TABLE>::USED) {
+                for (int l = 0; l < Enc::L; ++l) {
+                    const int group = ScatterGroups<Spec, E>::before() + l;
+                    if (group < MAX_GRID_LEVELS && p.level->cells.offset[group] != 0) visit(Enc{}, l, group);
+                }
+            }
+        }
+        each_cell_level<Spec, E + 1>(p, visit);
+    }
+}
+// one block after the other for every level that has a copy
+template <class Spec>
+__global__ void __launch_bounds__(FILL_THREADS) fill_cells_kernel(const __grid_constant__ LaunchArgs p)
+{
+    unsigned int block = blockIdx.x;
+    each_cell_level<Spec>(p, [&](auto enc, int l, int group) {
+        using Enc = decltype(enc);
+        const GridP& grid = p.grids[Enc::SLOT];
+        const unsigned int n = grid_fill_blocks<Enc::D, Enc::F, Enc::HALF_TABLE>(grid.levels[l].resolution);
+        if (block < n)
+            grid_fill_cells<Enc::D, Enc::F, Enc::HALF_TABLE>(grid, grid.levels[l], p.level->cells.base + static_cast<size_t>(p.level->cells.offset[group] - 1) * 256, block);
+        block -= n;   // (wraps: the levels after this block's own are past its number)
+    });
+}
+template <class Spec>
+inline cudaError_t fill_cells(const LaunchArgs& a, cudaStream_t s, int* launches)
+{
+    if (a.level->cells.base == nullptr || !(a.flags & FLAG_FILL_CELLS)) return cudaSuccess;
+    unsigned int blocks = 0;
+    each_cell_level<Spec>(a, [&](auto enc, int l, int) {
+        using Enc = decltype(enc);
+        blocks += grid_fill_blocks<Enc::D, Enc::F, Enc::HALF_TABLE>(a.grids[Enc::SLOT].levels[l].resolution);
+    });
+    if (blocks == 0) return cudaSuccess;
+    fill_cells_kernel<Spec><<<blocks, FILL_THREADS, 0, s>>>(a);
+    if (launches) ++*launches;
+    return cudaGetLastError();
+}
+
 // ---- level-major scatter of the table gradients --------------------------------------------------------------------
 // Counterpart of the encoding pass for the backward direction: the backward kernel leaves the adjoint of every grid
 // feature in the planes (write_adjoint_planes), and this kernel turns them into table gradients: light threads, many
 // CTAs per SM, nothing but coalesced plane reads and reductions (the backward kernel itself runs 16 warps per SM at 128
 // registers and alternates between MMA and scatter phases). A "group" is one level of one grid.
-template <class Spec, int E>
-struct ScatterGroups {
-    using Enc = typename Spec::template Enc<E>;
-    __host__ __device__ static constexpr int own()
-    {
-        if constexpr (Enc::IS_GRID) return Enc::L;
-        else return 0;
-    }
-    __host__ __device__ static constexpr int before()
-    {
-        if constexpr (E == 0) return 0;
-        else return ScatterGroups<Spec, E - 1>::before() + ScatterGroups<Spec, E - 1>::own();
-    }
-};
-template <class Spec>
-__host__ __device__ constexpr int scatter_group_count()
-{
-    return ScatterGroups<Spec, Spec::NUM_ENCODINGS - 1>::before() + ScatterGroups<Spec, Spec::NUM_ENCODINGS - 1>::own();
-}
-
 // lanes in pairs: both lanes of a pair scatter half of the corners of the even lane's point, then of the odd lane's
 template <class Spec, int E>
 __device__ __forceinline__ void scatter_group(const LaunchArgs& p, int g, const RowReader& in0, const RowReader& in1, long long point, bool valid)
@@ -203,7 +251,7 @@ __device__ __forceinline__ void scatter_group(const LaunchArgs& p, int g, const 
                 }
             }
             const GridLevelP& lv = grid.levels[l];
-            if (float* records = grid_records_of_cta<D, F>(grid, p.replicas, g, l)) {
+            if (float* records = grid_records_of_cta<D, F>(grid, p.level->replicas, g, l)) {
                 if constexpr (GridCellUnits<D, F>::USED) {
                     float pos[D];
                     grid_position<D, Enc::START>(grid, side ? in1 : in0, pos);
@@ -229,7 +277,7 @@ __device__ __forceinline__ void scatter_group(const LaunchArgs& p, int g, const 
                 }
                 return;
             }
-            float* grad = grid_grad_of_cta(grid, p.replicas, g, l, Enc::L);
+            float* grad = grid_grad_of_cta(grid, p.level->replicas, g, l, Enc::L);
 #pragma unroll
             for (int s = 0; s < 2; ++s) {
                 float pos[D], adjF[F];
@@ -287,7 +335,7 @@ __device__ __forceinline__ void sum_group(const LaunchArgs& p, int g)
         if (g >= SG::before() + SG::own()) {
             sum_group<Spec, E + 1>(p, g);
         } else if constexpr (Enc::IS_GRID) {
-            grid_sum_copies<Enc::D, Enc::F>(p.grids[Enc::SLOT], p.replicas, g, g - SG::before(), Enc::L);
+            grid_sum_copies<Enc::D, Enc::F>(p.grids[Enc::SLOT], p.level->replicas, g, g - SG::before(), Enc::L);
         }
     }
 }
@@ -298,7 +346,7 @@ inline unsigned int sum_blocks(const LaunchArgs& a, int g)
         using Enc = typename Spec::template Enc<E>;
         using SG = ScatterGroups<Spec, E>;
         if (g >= SG::before() + SG::own()) return sum_blocks<Spec, E + 1>(a, g);
-        if constexpr (Enc::IS_GRID) return grid_sum_blocks<Enc::D, Enc::F>(a.grids[Enc::SLOT], a.replicas, g, g - SG::before());
+        if constexpr (Enc::IS_GRID) return grid_sum_blocks<Enc::D, Enc::F>(a.grids[Enc::SLOT], a.level->replicas, g, g - SG::before());
     }
     return 0;
 }
@@ -326,19 +374,19 @@ struct PlaneLaunchers {
             // launches of other ranges may run at the same time.
             const int begin = a.scatterLevelEnd > 0 ? a.scatterLevelBegin : 0, end = a.scatterLevelEnd > 0 ? a.scatterLevelEnd : groups;
             int sums = 0;   // the levels up to the last one that has copies
-            long long from = a.replicas.total, to = a.replicas.total;
+            long long from = a.level->replicas.total, to = a.level->replicas.total;
             for (int g = 0; g < groups && g < MAX_GRID_LEVELS; ++g) {
-                if (a.replicas.log2Copies[g] == 0 && a.replicas.byCell[g] == 0) continue;
+                if (a.level->replicas.log2Copies[g] == 0 && a.level->replicas.byCell[g] == 0) continue;
                 if (g >= begin && g < end) {
-                    if (sums == 0) from = a.replicas.offset[g];
+                    if (sums == 0) from = a.level->replicas.offset[g];
                     sums = g - begin + 1;
                 } else if (g >= end) {
-                    to = a.replicas.offset[g];
+                    to = a.level->replicas.offset[g];
                     break;
                 }
             }
             if (sums > 0) {
-                const cudaError_t e = cudaMemsetAsync(a.replicas.base + from, 0, (to - from) * sizeof(float), s);
+                const cudaError_t e = cudaMemsetAsync(a.level->replicas.base + from, 0, (to - from) * sizeof(float), s);
                 if (e != cudaSuccess) return e;
             }
             scatter_planes_kernel<Spec><<<static_cast<unsigned>(bx), SCATTER_THREADS, 0, s>>>(a);

@@ -13,7 +13,7 @@ namespace kernel {
 constexpr int MAX_GRID_LEVELS = 32;
 constexpr int MAX_GRIDS = 4;
 // Grid slots of the launch arguments as this translation unit sees them. The generated source of a network defines how many
-// it uses, so that a launch copies no more: the slots are the last member, and an instantiation reads a prefix of what the
+// it uses, so that a launch copies no more: the slots (and what goes with levels) are the last members, and an instantiation reads a prefix of what the
 // library passes.
 #ifdef QMLP_GRIDS
 constexpr int GRID_SLOTS = QMLP_GRIDS;
@@ -64,6 +64,16 @@ constexpr int FLAG_GRAD_ENCODINGS = 4;
 constexpr int FLAG_SPLIT_SCATTER = 8;
 // KERNEL_ENCODE_PLANES for a pass without gradients: see grid_pair_forward
 constexpr int FLAG_HALF_SUMS = 16;
+// KERNEL_ENCODE_PLANES, KERNEL_ENCODING_FORWARD: fill the copies by cell (CellTables) first
+constexpr int FLAG_FILL_CELLS = 32;
+
+// Copies of small grid levels by cell: the rows of a cell's 2^D corners side by side, so that a point fetches one piece of memory
+// per level instead of 2^(D-1) pairs of rows (kernels/grid.cuh, GridCellRows). Filled from the tables by every call that
+// uses them.
+struct CellTables {
+    unsigned char* base;                    // 256-byte aligned (null: none)
+    unsigned int offset[MAX_GRID_LEVELS];   // first byte of a level's cells / 256, + 1; levels counted over all grids of the network; 0: no copy
+};
 
 // Copies of the gradients of small grid levels. Reductions to one 128-byte line execute one after the other in its L2 slice
 // (about nine clocks each): a level of a few lines that a large batch keeps hitting holds the whole kernel up. Such
@@ -74,6 +84,11 @@ struct GradReplicas {
     unsigned int offset[MAX_GRID_LEVELS];        // first element of a level's copies; levels counted over all grids of the network
     unsigned char log2Copies[MAX_GRID_LEVELS];   // 0: the level has no copies
     unsigned char byCell[MAX_GRID_LEVELS];       // 1 + log2 of the copies of a level whose gradient is added up by cell first (GridCellUnits); else 0
+};
+
+struct LevelArgs {
+    GradReplicas replicas;   // KERNEL_ENCODING_ADJOINT, KERNEL_SCATTER_PLANES
+    CellTables cells;        // KERNEL_ENCODE_PLANES, KERNEL_ENCODING_FORWARD
 };
 
 struct LaunchArgs {
@@ -106,7 +121,7 @@ struct LaunchArgs {
     float* sortedTarget;                           // (numel, NUM_OUTPUTS) row-major, may be null
     int scatterLevelBegin, scatterLevelEnd;        // KERNEL_SCATTER_PLANES: grid levels (counted over all grids) to scatter; 0, 0 = all
     int runAggregation;                            // 0: every point of every level scatters straight to the gradient table
-    GradReplicas replicas;                         // KERNEL_ENCODING_ADJOINT, KERNEL_SCATTER_PLANES
+    LevelArgs level[GRID_SLOTS > 0 ? 1 : 0];       // (a network without grids carries none)
     GridP grids[GRID_SLOTS];                       // the last member (GRID_SLOTS)
 };
 
@@ -156,4 +171,4 @@ extern "C" {
 typedef int (*qmlp_spec_launch_fn)(int kernel, const void* args, cudaStream_t stream, int* launches);
 typedef int (*qmlp_spec_abi_fn)(void);
 }
-#define QMLP_SPEC_ABI_VERSION 12
+#define QMLP_SPEC_ABI_VERSION 13

@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(EncodingTile<Enc>::WARPS * 32) grid_encoding_f
         for (int l = 0; l < Enc::L; ++l) {
             const GridLevelP& lv = g.levels[l];
             float feat[F];
-            grid_pair_forward<D, F, Enc::HALF_TABLE, false>(g, lv, pos0, pos1, side, feat);
+            grid_pair_forward<D, F, Enc::HALF_TABLE, false>(g, lv, grid_cells(p.level->cells, l), pos0, pos1, side, feat);
 #pragma unroll
             for (int i = 0; i < F; ++i) sum[i] = Enc::CONCAT ? feat[i] : sum[i] + feat[i];
             if constexpr (Enc::CONCAT) T::put(tile + lane * T::STRIDE, l * F, sum);
@@ -182,8 +182,8 @@ __global__ void __launch_bounds__(EncodingTile<Enc>::WARPS * 32) grid_encoding_a
             float* grad = g.grad;
             float* records = nullptr;
             if constexpr (PARAM_GRAD) {
-                grad = grid_grad_of_cta(g, p.replicas, l, l, Enc::L);
-                records = grid_records_of_cta<D, F>(g, p.replicas, l, l);
+                grad = grid_grad_of_cta(g, p.level->replicas, l, l, Enc::L);
+                records = grid_records_of_cta<D, F>(g, p.level->replicas, l, l);
             }
             if constexpr (PARAM_GRAD && GridCellUnits<D, F>::USED) {
                 if (records != nullptr) {
@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(EncodingTile<Enc>::WARPS * 32) grid_encoding_a
 template <class Enc>
 __global__ void __launch_bounds__(256) sum_replicas_kernel(const __grid_constant__ LaunchArgs p)
 {
-    grid_sum_copies<Enc::D, Enc::F>(p.grids[0], p.replicas, blockIdx.y, blockIdx.y, Enc::L);
+    grid_sum_copies<Enc::D, Enc::F>(p.grids[0], p.level->replicas, blockIdx.y, blockIdx.y, Enc::L);
 }
 
 template <class EncSpec>
@@ -249,10 +249,12 @@ struct EncodingLaunchers {
         if (blocks > cap) blocks = cap;
         return static_cast<unsigned>(blocks < 1 ? 1 : blocks);
     }
-    static cudaError_t forward(const LaunchArgs& a, cudaStream_t s)
+    static cudaError_t forward(const LaunchArgs& a, cudaStream_t s, int& count)
     {
         if constexpr (Enc::IS_GRID) {
             if constexpr (EncodingTile<Enc>::USED) {
+                const cudaError_t e = fill_cells<EncSpec>(a, s, &count);
+                if (e != cudaSuccess) return e;
                 constexpr int threads = EncodingTile<Enc>::WARPS * 32;
                 grid_encoding_forward_kernel<Enc><<<blocksFor(a, threads), threads, 0, s>>>(a);
                 return cudaGetLastError();
@@ -267,16 +269,16 @@ struct EncodingLaunchers {
         if constexpr (Enc::IS_GRID) {
             if constexpr (EncodingTile<Enc>::USED) {
                 constexpr int threads = EncodingTile<Enc>::WARPS * 32;
-                const bool copies = PARAM_GRAD && a.replicas.total > 0;
+                const bool copies = PARAM_GRAD && a.level->replicas.total > 0;
                 if (copies) {
-                    const cudaError_t e = cudaMemsetAsync(a.replicas.base, 0, a.replicas.total * sizeof(float), s);
+                    const cudaError_t e = cudaMemsetAsync(a.level->replicas.base, 0, a.level->replicas.total * sizeof(float), s);
                     if (e != cudaSuccess) return e;
                 }
                 grid_encoding_adjoint_kernel<Enc, INPUT_GRAD, PARAM_GRAD><<<blocksFor(a, threads), threads, 0, s>>>(a);
                 if (copies) {
                     unsigned int blocks = 32;
                     for (int l = 0; l < Enc::L; ++l) {
-                        const unsigned int n = grid_sum_blocks<Enc::D, Enc::F>(a.grids[0], a.replicas, l, l);
+                        const unsigned int n = grid_sum_blocks<Enc::D, Enc::F>(a.grids[0], a.level->replicas, l, l);
                         blocks = n > blocks ? n : blocks;
                     }
                     sum_replicas_kernel<Enc><<<dim3(blocks, Enc::L), 256, 0, s>>>(a);
@@ -294,7 +296,7 @@ struct EncodingLaunchers {
         cudaError_t e = cudaErrorInvalidValue;
         int count = 1;
         if (kernel == KERNEL_ENCODING_FORWARD) {
-            e = forward(a, s);
+            e = forward(a, s, count);
         } else if (kernel == KERNEL_ENCODING_ADJOINT) {
             const bool ig = (a.flags & 1) != 0, pg = (a.flags & 2) != 0;
             if (ig && pg) e = adjoint<true, true>(a, s, count);

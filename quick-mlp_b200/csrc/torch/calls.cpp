@@ -33,7 +33,7 @@ using OptTensor = std::optional<Tensor>;
     X(last_error) X(network_num_encodings) X(network_channels_in) X(network_channels_out) X(network_encoding)             \
     X(network_destroy) X(network_set_parameter) X(network_inference_memory) X(network_inference_with_memory) X(network_inference_host) X(network_forward_memory)  \
     X(network_forward) X(network_adjoint_memory) X(network_adjoint) X(network_recompute_memory) X(network_forward_recompute) X(network_adjoint_recompute) X(network_parameter_count) X(encoding_create)         \
-    X(encoding_num_output_channels) X(encoding_has_parameters) X(encoding_set_parameter) X(encoding_forward)              \
+    X(encoding_num_output_channels) X(encoding_has_parameters) X(encoding_set_parameter) X(encoding_forward_memory) X(encoding_forward_with_memory)              \
     X(encoding_adjoint_memory) X(encoding_adjoint_with_memory) X(activation_create) X(activation_forward) X(activation_adjoint) X(trainer_workspace_bytes)       \
     X(trainer_gradients_part) X(trainer_update) X(convert_half)
 
@@ -323,8 +323,12 @@ Tensor encodingForward(const Tensor& input, const OptTensor& parameters, std::st
     const qmlp_tensor_t in = wrap(input), p = parameters.has_value() ? wrap(*parameters) : qmlp_tensor_t{};
     Tensor output = at::empty({input.size(0), e.channels}, floatLike(input));
     qmlp_tensor_t out = wrap(output);
+    const qmlp_tensor_t* bound = parameters.has_value() ? &p : nullptr;
+    size_t bytes = 0;   // copies of small levels by cell
+    check(api.encoding_forward_memory(e.handle, input.size(0), bound, &bytes));
+    const Tensor tmp = bytes > 0 ? at::empty({static_cast<int64_t>(bytes)}, floatLike(input).dtype(torch::kUInt8)) : Tensor();
     std::lock_guard<std::mutex> lock(e.mutex);
-    check(api.encoding_forward(e.handle, &in, &out, currentStream(), parameters.has_value() ? &p : nullptr));
+    check(api.encoding_forward_with_memory(e.handle, &in, &out, currentStream(), bound, bytes > 0 ? tmp.data_ptr() : nullptr, bytes));
     return output;
 }
 // what is not asked for is returned as an empty tensor

@@ -105,6 +105,8 @@ SIGNATURES = {
     "qmlp_encoding_zero_gradients": (C.c_int, [_P, _P]),
     "qmlp_encoding_forward": (C.c_int, [_P, _TP, _TP, _P, _TP]),
     "qmlp_encoding_adjoint": (C.c_int, [_P, _TP, _TP, _TP, _P, _TP, _TP, C.c_int]),
+    "qmlp_encoding_forward_memory": (C.c_int, [_P, C.c_int64, _TP, C.POINTER(C.c_size_t)]),
+    "qmlp_encoding_forward_with_memory": (C.c_int, [_P, _TP, _TP, _P, _TP, _P, C.c_size_t]),
     "qmlp_encoding_adjoint_memory": (C.c_int, [_P, C.c_int64, C.c_int, C.POINTER(C.c_size_t)]),
     "qmlp_encoding_adjoint_with_memory": (C.c_int, [_P, _TP, _TP, _TP, _P, _TP, _TP, C.c_int, _P, C.c_size_t]),
     "qmlp_encoding_compile": (C.c_int, [_P, C.c_int]),

@@ -39,6 +39,8 @@ def jobs():
         out.append(("enc", json.dumps(cfg), 0))
     for name, cfg in te.encoding_cases().items():
         out.append(("enc", json.dumps(cfg), 0))
+    for name in ("hash4d_f4", "hash2d_f8"):
+        out.append(("enc", json.dumps(te.encoding_cases()[name]), 1))   # fp16 tables
     for cfg in (specs.hashgrid(3, 6, 1, 14, 8, 300), specs.hashgrid(4, 4, 1, 16, 8, 64), specs.hashgrid(2, 5, 1, -1, 4, 64)):
         out.append(("enc", json.dumps(cfg), 0))
     for a in ("relu", "celu", "sine", "identity", json.dumps(tn.LEAKY)):

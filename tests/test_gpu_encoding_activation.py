@@ -247,3 +247,76 @@ def test_adjoint_added_up_by_cell(name, n):
         (gx0, gt0), (gx1, gt1) = results
         assert torch.equal(gx0, gx1)
         helpers.assert_close(gt1.cpu().numpy(), gt0.cpu().numpy(), f"{name} n={n}", rtol=2.0 ** -9, atol=1e-5 * float(gt0.abs().max()))
+
+
+@pytest.mark.parametrize("name,half", [("dense2d_multires", False), ("hash4d_f4", True), ("hash4d_f4", False), ("hash2d_f8", False), ("hash2d_f8", True)])
+def test_forward_from_copies_by_cell(name, half):
+    """Batches that are large enough for copies of the small levels by cell against the same call without scratch: points below the box (a warp
+    that holds one reads the table), above it and on its borders; a table at an odd offset. The terms are the same; a compiler that
+    forms the cell fraction with one rounding in one place and two in another moves it by R * 2^-24, R up to 256 here, and with it a feature
+    by that times the largest slope of a cell, 2, in each dimension; points outside extrapolate, and so does the rounding."""
+    import ctypes as C
+    import torch
+    from qmlp._capi import check, lib, wrap
+    cfg, e, oe = _enc(name)
+    n = (3 << 18) + 77
+    x = helpers.uniform(11, 1, (n, oe.n_in), 0.0, 1.0)
+    x[::1013] -= 0.5
+    x[::1009] += 0.5
+    x[::97] = np.round(x[::97])
+    x = torch.from_numpy(x).cuda()
+    for shift in (0, 1):
+        data = torch.from_numpy(helpers.uniform(11, 3, (oe.num_parameters + 1,), -1.0, 1.0)).cuda()
+        table = (data.half() if half else data)[shift:shift + oe.num_parameters]
+        need = C.c_size_t()
+        p = wrap(table)
+        check(lib().qmlp_encoding_forward_memory(e._h, n, C.byref(p), C.byref(need)))
+        assert need.value > 0
+        check(lib().qmlp_encoding_forward_memory(e._h, 1000, C.byref(p), C.byref(C.c_size_t())))
+        results = []
+        for tmp in (None, torch.full((need.value,), 0x7e, dtype=torch.uint8, device="cuda")):
+            out = torch.zeros((n, oe.num_outputs), device="cuda")
+            check(lib().qmlp_encoding_forward_with_memory(e._h, wrap(x), wrap(out), None, C.byref(p), tmp.data_ptr() if tmp is not None else None,
+                                                          need.value if tmp is not None else 0))
+            torch.cuda.synchronize()
+            results.append(out)
+        inside = ((x >= 0) & (x <= 1)).all(dim=1)
+        a, b = results[0][inside], results[1][inside]
+        assert float((a - b).abs().max()) <= 256 * 2.0 ** -24 * 2 * oe.n_in
+        a, b = results[0][~inside].double(), results[1][~inside].double()
+        assert float((a - b).abs().max()) <= 1e-4 * float(a.abs().max())
+
+
+def test_network_inference_from_copies_by_cell():
+    """The level-major pass with and without copies by cell (memory for the planes alone): the same features up to the rounding of a cell
+    fraction (above), which an fp16 rounding of a feature shows as 2^-11 now and then, and four layers pass on."""
+    import ctypes as C
+    import torch
+    from qmlp import bindings
+    from qmlp._capi import check, lib, wrap
+    from test_gpu_network import network_cases
+    cfg, rng, _ = network_cases()["config5_small"]
+    spec = oracle.parse_spec(cfg)
+    net = bindings.Network(json.dumps(cfg))
+    n = (3 << 18) + 5
+    x = torch.from_numpy(helpers.uniform(12, 1, (n, spec.num_inputs), -0.001, 1.0)).cuda()
+    w = torch.from_numpy(helpers.xavier_parameters(spec, cfg, bias_scale=0.1)).cuda().half()
+    t = torch.from_numpy(helpers.grid_tables(spec, scale=1.0)[0]).cuda().half()
+    net.inference(x[:64], w, [t])   # binds the parameters
+    try:
+        bindings.QuickMLP.set_kernel_path(2)
+        need = C.c_size_t()
+        check(lib().qmlp_network_inference_memory(net._h, n, C.byref(need)))
+        planes = (n + 65535) // 65536 * 65536 * sum(net.encoding(i).num_output_channels() for i in range(net.num_encodings())) * 2
+        assert need.value > planes
+        results = []
+        for size in (planes, need.value):
+            tmp = torch.full((size,), 0x7e, dtype=torch.uint8, device="cuda")
+            out = torch.zeros((n, spec.num_outputs), device="cuda")
+            o = wrap(out)
+            check(lib().qmlp_network_inference_with_memory(net._h, wrap(x), C.byref(o), None, tmp.data_ptr(), size))
+            torch.cuda.synchronize()
+            results.append(out)
+        assert float((results[0] - results[1]).norm()) <= 1e-4 * float(results[0].norm()) > 0
+    finally:
+        bindings.QuickMLP.set_kernel_path(0)
