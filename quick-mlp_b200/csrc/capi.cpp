@@ -154,8 +154,13 @@ void launchModule(Network& n, KernelModule& m, int kernelId, const kernel::Launc
 {
     TimedLaunch timed(kernelId, static_cast<cudaStream_t>(stream));
     int launches = 0;
-    const kernel::LaunchArgs b = withScratchSizes(n, kernelId, a);
-    checkLaunch(m.launch(kernelId, &b, static_cast<cudaStream_t>(stream), &launches), "kernel launch failed");
+    // (only bounds-checking instantiations read the sizes; the copy is 3 KB of a small call)
+    if (Library::instance().boundsCheck) {
+        const kernel::LaunchArgs b = withScratchSizes(n, kernelId, a);
+        checkLaunch(m.launch(kernelId, &b, static_cast<cudaStream_t>(stream), &launches), "kernel launch failed");
+    } else {
+        checkLaunch(m.launch(kernelId, &a, static_cast<cudaStream_t>(stream), &launches), "kernel launch failed");
+    }
     n.launchCount += launches;
 }
 
