@@ -104,8 +104,9 @@ QMLP_API int qmlp_device_status(int* status);
  * offset and plane offset against the declared sizes, skip what lies outside and set a bit of the status word
  * (qmlp_device_status) instead of faulting - the role of the reference's debug asserts in WrappedArray
  * (src_cpp/include/qmlp/kernels/common.cuh:174-218); "bounds_shrink": n declares every size n elements smaller than it
- * is (test hook: the check fires while every access still lands in real memory). Stand in for the reference's tuning options
- * (src_cpp/src/fused_network.cpp:45-69). */
+ * is (test hook: the check fires while every access still lands in real memory); "spin_limit": the layer kernel of a training
+ * step gives up an on-chip wait after n polls (test hook of the same instantiations, which then report bit 0; -1: as without
+ * it). Stand in for the reference's tuning options (src_cpp/src/fused_network.cpp:45-69). */
 QMLP_API int qmlp_set_tuning(const char* key, int value);
 /* Per-kernel device timing: while enabled, every kernel the library launches is bracketed by a CUDA event pair on its
  * stream; qmlp_read_kernel_timing waits for the recorded launches, sums them per kernel (ids: the library's kernel

@@ -146,6 +146,7 @@ kernel::LaunchArgs withScratchSizes(const Network& n, int kernelId, const kernel
     const long long shrink = Library::instance().boundsShrink;
     b.fwdTmpHalfs = a.fwdTmp ? std::max<long long>(1, n32 * stashHalfs - shrink) : 0;
     b.adjTmpHalfs = a.adjTmp ? std::max<long long>(1, n32 * n.deltaHalfsPerPoint() - shrink) : 0;
+    b.spinLimit = Library::instance().spinLimit < 0 ? 1u << 24 : static_cast<unsigned int>(Library::instance().spinLimit);
     b.planeHalfs = a.planes ? std::max<long long>(1, a.planeStride * n.encodedChannels() - shrink) : 0;
     return b;
 }
@@ -312,7 +313,8 @@ int qmlp_set_tuning(const char* key, int value)
     else if (k == "scatter_runs") lib.runAggregation = value;
     else if (k == "bounds_check") lib.boundsCheck = value > 0;
     else if (k == "bounds_shrink") lib.boundsShrink = value > 0 ? value : 0;
-    else throw std::runtime_error("unknown tuning key '" + k + "' (sort_points, split_scatter, scatter_runs, bounds_check, bounds_shrink)");
+    else if (k == "spin_limit") lib.spinLimit = std::min(value, 1 << 24);
+    else throw std::runtime_error("unknown tuning key '" + k + "' (sort_points, split_scatter, scatter_runs, bounds_check, bounds_shrink, spin_limit)");
     QMLP_CATCH
 }
 

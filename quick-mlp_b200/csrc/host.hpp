@@ -52,6 +52,7 @@ struct Library {
     // size the host declares; an access outside is skipped and reported through the status word
     bool boundsCheck = false;
     int64_t boundsShrink = 0; // test hook: declare tables and scratch buffers this many elements smaller than they are
+    int spinLimit = -1;       // test hook: polls after which a wait of the training kernel's bounds-checking instantiations gives up (-1: as ever)
     int* statusWord();     // device word of the current device that kernels set when a bounded wait gives up
 };
 

@@ -197,12 +197,19 @@ __device__ __forceinline__ void umma_commit_elected(uint32_t lead, uint32_t bar)
     asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
                  "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar), "r"(lead) : "memory");
 }
+// polls of a wait before it gives up (bounds-checking instantiations: the host's, a test hook)
+__device__ __forceinline__ uint32_t train_spin_limit(const LaunchArgs& p)
+{
+    if constexpr (BOUNDS_CHECK) return p.spinLimit;
+    (void)p;
+    return TC_SPIN_LIMIT;
+}
 // Bounded wait. When one gives up it raises the CTA's abort flag; from then on nobody waits any more (`dead`), so that the
 // CTA runs through to its end.
-__device__ __forceinline__ void train_wait(uint32_t bar, uint32_t parity, volatile int* abortFlag, bool& dead)
+__device__ __forceinline__ void train_wait(uint32_t bar, uint32_t parity, volatile int* abortFlag, bool& dead, uint32_t limit = TC_SPIN_LIMIT)
 {
     if (dead) return;
-    for (uint32_t i = 0; i < TC_SPIN_LIMIT; ++i) {
+    for (uint32_t i = 0; i < limit; ++i) {
         if (mbar_test(bar, parity)) return;
         if ((i & 1023u) == 1023u && *abortFlag != 0) break;
     }
@@ -512,7 +519,7 @@ __device__ __forceinline__ void train_put(uint32_t rowAddr, int row, int col, co
 }
 
 // One stage of a slot's tile (TrainLayout::lastStage). Every stage but the last is followed by the MMAs of the next one: the
-// warps count their arrivals, and the last one issues.
+// slot's warps meet, and one of them (the same one for all stages) issues.
 template <class Spec, bool LOSS, int ST>
 __device__ __forceinline__ void train_stage(const LaunchArgs& p, TrainSlot<Spec, LOSS>& sl, const __half* bias, int wg, int row, long long nextPoint,
                                             float& lossAcc, volatile int* abortFlag, bool& dead)
@@ -531,7 +538,7 @@ __device__ __forceinline__ void train_stage(const LaunchArgs& p, TrainSlot<Spec,
         }
     } else {
         if constexpr (ST < TR::lastStage() || TR::FEATURE_ADJOINT) {
-            train_wait(sl.bars, sl.full, abortFlag, dead);
+            train_wait(sl.bars, sl.full, abortFlag, dead, train_spin_limit(p));
             sl.full ^= 1u;
         }
         __syncwarp();   // tcgen05.ld is warp-collective
@@ -628,7 +635,7 @@ __device__ __forceinline__ void train_stage(const LaunchArgs& p, TrainSlot<Spec,
                     d[k][i] = sl.valid ? h2_as_u32(y) : 0u;
                 }
             }
-            train_wait(sl.bars + 8, sl.graded, abortFlag, dead);
+            train_wait(sl.bars + 8, sl.graded, abortFlag, dead, train_spin_limit(p));
 #pragma unroll
             for (int k = 0; k < (COUT / 8 + WG - 1) / WG; ++k) {
                 const int col = (wg + k * WG) * 8;
@@ -637,7 +644,7 @@ __device__ __forceinline__ void train_stage(const LaunchArgs& p, TrainSlot<Spec,
             sl.graded ^= 1u;
         } else {
             if constexpr (TR::FEATURE_ADJOINT) train_store_adjoint<Spec, LOSS, 0>(p, sl, wg);
-            train_wait(sl.bars + 8, sl.graded, abortFlag, dead);   // buffer 0 is written next
+            train_wait(sl.bars + 8, sl.graded, abortFlag, dead, train_spin_limit(p));   // buffer 0 is written next
             sl.graded ^= 1u;
         }
     }
@@ -651,10 +658,13 @@ __device__ __forceinline__ void train_stage(const LaunchArgs& p, TrainSlot<Spec,
         tc_fence_before();
         fence_proxy_async();   // generic-proxy writes of the operands become visible to the tensor core
         __syncwarp();
-        if (!sl.issuer) {
-            asm volatile("bar.arrive %0, %1;" ::"r"(2 + sl.slot), "n"(WG * 128) : "memory");
-        } else {
-            asm volatile("bar.sync %0, %1;" ::"r"(2 + sl.slot), "n"(WG * 128) : "memory");
+        // All warps of the slot wait here, the others for an accumulator that is not computed before anyway. After a wait that gave up this
+        // keeps them in step: no warp leaves a tile early, so each takes part in every meeting once. (If they only arrived, a warp that
+        // waits for nothing any more would arrive for later stages too and leave the issuing warp alone in one of them for good. Layers
+        // of 32 -> 64 -> 64 -> 1, 2^20 points / 48 -> 128 -> 64 -> 16 -> 4, 2^21 points: arriving only 94.7 / 564 us, meeting 94.7 / 576,
+        // an arrival counter whose last warp issues 98.8 / 586.)
+        asm volatile("bar.sync %0, %1;" ::"r"(2 + sl.slot), "n"(WG * 128) : "memory");
+        if (sl.issuer) {
             tc_fence_after();
             if (!__any_sync(0xffffffffu, dead)) Issue::template critical<ST>(sl.lead, sl.smem, sl.smem + TR::slotStart() + sl.slot * TR::slotBytes(), sl.tmem & 0xffffu, sl.bars);
             if constexpr (Issue::template graded<ST>() >= 0)
@@ -676,8 +686,8 @@ __device__ __forceinline__ void train_stages(const LaunchArgs& p, TrainSlot<Spec
 // The weight-gradient warp: the MMAs of the layers' gradients in the order in which the deltas are completed. All slots add to the same
 // accumulators, so one thread issues them; nobody waits for them before the slot's next stage has computed its results.
 template <class Spec, bool LOSS>
-__device__ __forceinline__ void train_gradients(uint32_t lead, uint32_t smem, uint32_t tmemBase, uint32_t bars, uint32_t queue, int myTiles, volatile int* abortFlag,
-                                                bool& dead)
+__device__ __forceinline__ void train_gradients(const LaunchArgs& p, uint32_t lead, uint32_t smem, uint32_t tmemBase, uint32_t bars, uint32_t queue, int myTiles,
+                                                volatile int* abortFlag, bool& dead)
 {
     using TR = TrainLayout<Spec, LOSS>;
     uint32_t started = 0;
@@ -688,12 +698,13 @@ __device__ __forceinline__ void train_gradients(uint32_t lead, uint32_t smem, ui
             v = __shfl_sync(0xffffffffu, train_next_request(queue, n), 0);
             if ((v >> 8) == ((n + 1) & 0xffffffu)) break;
             ++idle;
-            if (idle > 4 * TC_SPIN_LIMIT || ((idle & 1023u) == 1023u && __any_sync(0xffffffffu, *abortFlag != 0))) {
+            if (idle > 4 * train_spin_limit(p) || ((idle & 1023u) == 1023u && __any_sync(0xffffffffu, *abortFlag != 0))) {
                 *abortFlag = 1;
                 dead = true;
                 return;
             }
         }
+        __syncwarp();   // (orders the elected lane's MMAs behind lane 0's acquire)
         tc_fence_after();
         // (opaque copies: the descriptors of all MMAs would be computed ahead of the loop and spilled)
         uint32_t base = smem, tmem = tmemBase;
@@ -831,11 +842,11 @@ fused_train_tc_kernel(const __grid_constant__ LaunchArgs p, const __grid_constan
     const int myTiles = static_cast<int>(blockIdx.x) < numTiles ? (numTiles - static_cast<int>(blockIdx.x) + stride - 1) / stride : 0;
     bool dead = false;
     const uint32_t lead = elect_one();
-    train_wait(smem_u32(weightBar), 0, abortFlag, dead);
+    train_wait(smem_u32(weightBar), 0, abortFlag, dead, train_spin_limit(p));
     __syncwarp();
     if (warpgroup == TR::WARPGROUPS) {
         const uint32_t smemU = __shfl_sync(0xffffffffu, smemBase, 0), tmemU = __shfl_sync(0xffffffffu, tmemBase, 0);
-        if (!__any_sync(0xffffffffu, dead)) train_gradients<Spec, LOSS>(lead, smemU, tmemU, smemU + TR::barStart(SLOTS), smem_u32(queue), myTiles, abortFlag, dead);
+        if (!__any_sync(0xffffffffu, dead)) train_gradients<Spec, LOSS>(p, lead, smemU, tmemU, smemU + TR::barStart(SLOTS), smem_u32(queue), myTiles, abortFlag, dead);
     } else {
         // tile i of this CTA's sequence belongs to slot i % SLOTS
         const int slot = warpgroup / TrainSlot<Spec, LOSS>::WG, wg = warpgroup % TrainSlot<Spec, LOSS>::WG;
@@ -872,7 +883,8 @@ fused_train_tc_kernel(const __grid_constant__ LaunchArgs p, const __grid_constan
         }
     }
     __syncthreads();         // (nobody raises the flag any more)
-    if (*abortFlag != 0) {   // gave up: let this warp's MMAs in flight finish
+    if (*abortFlag != 0) {   // gave up: let the copies of the weights and this warp's MMAs in flight finish
+        mbar_wait(smem_u32(weightBar), 0);
         umma_commit_elected(lead, smem_u32(drainBar + warp));
         mbar_wait(smem_u32(drainBar + warp), 0);
         __syncwarp();

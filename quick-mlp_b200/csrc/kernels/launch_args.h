@@ -112,6 +112,7 @@ struct LaunchArgs {
     __half* planes;                                // encoded features (or their adjoints) of a chunk of points, one plane per grid level
     long long planeStride;                         // points per plane (capacity of the chunk buffer)
     long long fwdTmpHalfs, adjTmpHalfs, planeHalfs; // sizes of the three scratch buffers in halfs (QMLP_BOUNDS_CHECK builds; 0: unknown)
+    unsigned int spinLimit;                        // polls before a wait of the training kernel gives up (QMLP_BOUNDS_CHECK builds)
     // spatially binned training step (kernels/sorted_scatter.cuh): KERNEL_SORT_POINTS copies the points (and targets)
     // into Morton-bin order; the kernels after it read the sorted copies through `input` / `target`
     unsigned int* binCounts;                       // points per bin (sort_bin_count() entries), zeroed by the launcher
@@ -171,4 +172,4 @@ extern "C" {
 typedef int (*qmlp_spec_launch_fn)(int kernel, const void* args, cudaStream_t stream, int* launches);
 typedef int (*qmlp_spec_abi_fn)(void);
 }
-#define QMLP_SPEC_ABI_VERSION 13
+#define QMLP_SPEC_ABI_VERSION 14

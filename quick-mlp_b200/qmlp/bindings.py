@@ -50,7 +50,7 @@ class QuickMLP:
         """Tuning switches of the fused training step ("sort_points", "split_scatter", "scatter_runs"; -1 = automatic) and
         of the kernel instantiation ("bounds_check": 1 = kernels that test every table row, stash and plane offset and
         report through device_status() instead of faulting; "bounds_shrink": test hook, declares all sizes that many
-        elements smaller)."""
+        elements smaller; "spin_limit": test hook, polls before a wait of the training kernel gives up)."""
         check(lib().qmlp_set_tuning(key.encode(), int(value)))
 
     @staticmethod

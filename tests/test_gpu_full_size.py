@@ -386,6 +386,44 @@ def test_bounds_check_reaches_the_step_and_the_recomputing_pair(bounds_check):
         assert all(bool(torch.isfinite(r).all()) for r in result)
 
 
+@pytest.mark.parametrize("name", ["config3", "config4"])
+def test_training_kernel_ends_when_a_wait_gives_up(bounds_check, name):
+    """Waits of the layer kernel that run out after 0, 1 or 16 polls (test hook), with one and with two warpgroups to a tile and
+    six tiles per CTA: the kernel ends and reports it, also where some of a slot's warps have given up and others have not. Afterwards the
+    same call is right again."""
+    import torch
+    from qmlp import bindings
+    from qmlp.trainer import FusedTrainer
+    cfg = specs.config3(log2_hashmap_size=12) if name == "config3" else specs.config4()
+    spec = oracle.parse_spec(cfg)
+    n = 6 * 148 * 128 + 77
+    x = torch.from_numpy(helpers.uniform(86, 1, (n, 3))).cuda()
+    t = torch.from_numpy(helpers.uniform(86, 2, (n, spec.num_outputs), -1.0, 1.0)).cuda()
+    params = torch.from_numpy(helpers.xavier_parameters(spec, cfg, bias_scale=0.05)).cuda()
+    tables = [torch.from_numpy(tb).cuda() if tb is not None else None for tb in helpers.grid_tables(spec, scale=0.5)]
+    tr = FusedTrainer(bindings.Network(json.dumps(cfg)), grid_half_copy=name == "config3")
+    tr.set_parameters(params, tables)
+
+    def gradients():
+        tr.gradient.zero_()
+        tr.backend.gradients(x, t, n, tr.loss_sum)
+        return tr.gradient.clone()
+    before = gradients()
+    assert bindings.QuickMLP.device_status() == 0
+    try:
+        for limit in (0, 1, 16):
+            bindings.QuickMLP.set_tuning("spin_limit", limit)
+            for _ in range(3):
+                gradients()
+            status = bindings.QuickMLP.device_status()
+            assert status & ~1 == 0 and (status == 1 or limit > 0), f"limit {limit}: {status}"
+    finally:
+        bindings.QuickMLP.set_tuning("spin_limit", -1)
+    after = gradients()
+    assert bindings.QuickMLP.device_status() == 0
+    assert float((after - before).norm()) <= 1e-5 * float(before.norm())   # (the order of fp32 sums)
+
+
 def test_scratch_memory_does_not_depend_on_the_switches():
     """Scratch sized with bounds_check on serves a call with it off: the workspace a trainer keeps for a number of points, and
     the adjoint scratch an autograd node asked for in its forward call. 2^18 points: the coarse levels have copies."""
