@@ -183,7 +183,7 @@ QMLP_API int qmlp_network_forward_static_scratch(qmlp_network_t* net, const qmlp
 QMLP_API int qmlp_static_scratch(void** device_address, size_t* bytes);
 /* FusedNetwork::zeroGradients, src_cpp/src/fused_network.cpp:738-744 (asynchronous on `stream` here). */
 QMLP_API int qmlp_network_zero_gradients(qmlp_network_t* net, qmlp_stream_t stream);
-/* FusedNetwork::adjointMemory, src_cpp/src/fused_network.cpp:997-1010 */
+/* FusedNetwork::adjointMemory, src_cpp/src/fused_network.cpp:997-1010. Memory for a number of points serves every smaller batch. */
 QMLP_API int qmlp_network_adjoint_memory(qmlp_network_t* net, int64_t num_elements, int adjoint_flags, size_t* bytes);
 /* FusedNetwork::adjoint, src_cpp/src/fused_network.cpp:1012-1145. Gradients are accumulated (+=). */
 QMLP_API int qmlp_network_adjoint(qmlp_network_t* net, const qmlp_tensor_t* input, const qmlp_tensor_t* adj_output,
@@ -292,7 +292,8 @@ QMLP_API void qmlp_trainer_destroy(qmlp_trainer_t* tr);
  * (segment 0 = network, 1 + i = encoding i; -1 when the encoding has no parameters). */
 QMLP_API int64_t qmlp_trainer_fused_count(const qmlp_trainer_t* tr);
 QMLP_API int64_t qmlp_trainer_segment_start(const qmlp_trainer_t* tr, int segment);
-/* Scratch bytes a step over `num_elements` points needs (stash + adjoint stash + output + output gradient). */
+/* Scratch bytes a step over `num_elements` points needs (stash + adjoint stash + output + output gradient); they serve every smaller
+ * batch. */
 QMLP_API int qmlp_trainer_workspace_bytes(qmlp_trainer_t* tr, int64_t num_elements, size_t* bytes);
 /* Bind the fused buffers: fp32 master parameters, fp32 gradient, Adam first/second moments (all fused_count floats)
  * and the half working copy (fused_count halfs: fp16 network weights, and fp16 grid tables when grid_half_copy). */

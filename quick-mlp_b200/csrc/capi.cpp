@@ -222,13 +222,9 @@ size_t adjointPlaneBytes(const Network& n, int64_t n32, int flags)
     const bool wanted = anyGrid && (flags & QMLP_GRADIENTS_INPUT_ENCODINGS) != 0;
     return wanted ? static_cast<size_t>(n32) * n.encodedChannels() * 2 : 0;
 }
-// behind the planes, 256-byte aligned: copies of the gradients of hot levels (kernel::GradReplicas)
-size_t replicaBytes(const Network& n, int64_t points)
-{
-    kernel::GradReplicas r;
-    n.planReplicas(points, r);
-    return static_cast<size_t>(r.total) * sizeof(float);
-}
+// behind the planes, 256-byte aligned: copies of the gradients of hot levels (kernel::GradReplicas). Memory for a number of points
+// serves every smaller batch: the calls that use it are not told its size.
+size_t replicaBytes(const Network& n, int64_t points) { return static_cast<size_t>(n.replicaElements(points)) * sizeof(float); }
 size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 void bindReplicas(const Network& n, kernel::LaunchArgs& a, void* memory)
 {
@@ -1034,9 +1030,9 @@ int qmlp_encoding_adjoint_memory(qmlp_encoding_t* enc, int64_t num_elements, int
     *bytes = 0;
     auto* g = dynamic_cast<EncodingHashGrid*>(enc->impl.get());
     if (g && (adjoint_mode & QMLP_ENCODING_PARAM_GRADIENTS)) {
-        kernel::GradReplicas r{};
-        g->planReplicas(num_elements, 0, r);
-        *bytes = static_cast<size_t>(r.total) * sizeof(float);
+        int64_t records = 0, copies = 0;
+        g->boundReplicas(num_elements, 0, records, copies);
+        *bytes = static_cast<size_t>(replicaElements(records, copies)) * sizeof(float);
     }
     QMLP_CATCH
 }

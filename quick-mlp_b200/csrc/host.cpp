@@ -313,42 +313,65 @@ std::string EncodingHashGrid::deviceType(int outOffset, int slot, bool halfTable
                   outOffset, slot, halfTable ? "true" : "false");
 }
 
+// Elements of the records of all levels: what a scatter works on at the same time stays in L2 beside the gradients of the other levels (80 MB).
+constexpr int64_t RECORD_BUDGET = 20ll << 20;
+// elements of all copies together (32-bit offsets)
+constexpr int64_t REPLICA_LIMIT = 1ll << 28;
+
+// log2 of the copies of the records by cell of a level (kernel::GridCellUnits): as many as leave a record 256 points (10^6 points on 256
+// cells of 64 bytes: 40 us, 4096 cells 17, 16384 cells 15). -1: the level has too many cells for the batch.
+// By cell while the records of a level take up to 16 bytes per point. A point and level save about 11 ps, a byte of records
+// costs 0.4 ps to clear and to add up, and the launch that adds up costs as much as half a million points save: 3-D grid of 16^3 to
+// 7006^3 vertices, four levels by cell, step of 2^20 points 821 -> 786 us; three levels, autograd call of 2^18 points 309 -> 292; two
+// levels, step of 2^17 points 204 -> 209; two levels of 64^3 with four features (16 bytes per point), step of 2^21 points 1500 -> 1487; 16
+// levels of 54^3 (160 MB), 2^20 points 382 -> 630. Dense levels only: rows of a small hashed level that many vertices share would be added up
+// one vertex after the other (10^6 points, 1024 rows, terms of one sign: error against 64 bits 1.4e-7 -> 2.2e-7).
+int EncodingHashGrid::recordCopies(int64_t points, int level, int64_t& elements) const
+{
+    const int64_t record = static_cast<int64_t>(features_) << dim_;   // elements of a cell
+    if (dim_ < 2 || dim_ > 4 || (features_ != 2 && features_ != 4 && features_ != 8) || record > 64 || table_[level].hashed) return -1;
+    double cells = 1;
+    for (int k = 0; k < dim_; ++k) cells *= table_[level].resolution;
+    if (cells * static_cast<double>(record) * 4 > 16.0 * static_cast<double>(points)) return -1;
+    int lg = 0;
+    for (double hits = static_cast<double>(points) / cells; hits > 256 && lg < 6; hits /= 2) ++lg;
+    elements = static_cast<int64_t>(cells) * record << lg;
+    return lg;
+}
+bool EncodingHashGrid::recordsWorthwhile(int64_t points, int group) const
+{
+    int few = 0;
+    int64_t elements;
+    for (int l = 0; l < levels_ && group + l < kernel::MAX_GRID_LEVELS; ++l) few += recordCopies(points, l, elements) >= 0 ? 1 : 0;
+    return static_cast<double>(points) * few >= static_cast<double>(1 << 19);
+}
+// log2 of the copies of a level's gradient. A point sends 2^(D-1) reductions per level (neighbouring corners leave as one) to the lines of
+// the level. Up to 2048 per line they hide behind the rest of the kernel (a line takes about nine clocks each); above that, as many
+// copies as bring a line back to that number, 64 at most.
+int EncodingHashGrid::gradientCopies(int64_t points, int level, int64_t& elements) const
+{
+    elements = (level + 1 < levels_ ? table_[level + 1].memoryOffset : numParameters_) - table_[level].memoryOffset;
+    double perLine = static_cast<double>(points) * (1 << (dim_ - 1)) / std::max<double>(1.0, static_cast<double>(elements) / 32);
+    int lg = 0;
+    for (; perLine > 2048 && lg < 6; perLine /= 2) ++lg;
+    elements <<= lg;
+    return lg;
+}
+
 void EncodingHashGrid::planReplicas(int64_t points, int group, kernel::GradReplicas& r) const
 {
-    // A point sends 2^(D-1) reductions per level (neighbouring corners leave as one) to the lines of the level. Up to
-    // 2048 per line they hide behind the rest of the kernel (a line takes about nine clocks each); above that, as many
-    // copies as bring a line back to that number, 64 at most.
     // The plan, and with it the size of the scratch memory, depends on the grid and the number of points alone: memory sized
     // under one set of tuning switches serves a call under another.
     if (isLine()) return;
-    const double reductions = static_cast<double>(points) * (1 << (dim_ - 1));
-    // By cell (kernel::GridCellUnits) while the records of a level take up to 16 bytes per point and those of all levels, which a scatter
-    // works on at the same time, stay in L2 beside the gradients of the others (80 MB). A point and level save about 11 ps, a byte of records
-    // costs 0.4 ps to clear and to add up, and the launch that adds up costs as much as half a million points save: 3-D grid of 16^3 to
-    // 7006^3 vertices, four levels by cell, step of 2^20 points 821 -> 786 us; three levels, autograd call of 2^18 points 309 -> 292; two
-    // levels, step of 2^17 points 204 -> 209; two levels of 64^3 with four features (16 bytes per point), step of 2^21 points 1500 -> 1487; 16
-    // levels of 54^3 (160 MB), 2^20 points 382 -> 630. Dense levels only: rows of a small hashed level that many vertices share would be added up
-    // one vertex after the other (10^6 points, 1024 rows, terms of one sign: error against 64 bits 1.4e-7 -> 2.2e-7).
-    const int64_t record = static_cast<int64_t>(features_) << dim_;   // elements of a cell
-    const bool records = dim_ >= 2 && dim_ <= 4 && (features_ == 2 || features_ == 4 || features_ == 8) && record <= 64;
-    auto cellsOf = [&](int l) {
-        double n = 1;
-        for (int k = 0; k < dim_; ++k) n *= table_[l].resolution;
-        return n;
-    };
-    auto fewCells = [&](int l) { return records && !table_[l].hashed && cellsOf(l) * static_cast<double>(record) * 4 <= 16.0 * static_cast<double>(points); };
-    int few = 0;
-    for (int l = 0; l < levels_ && group + l < kernel::MAX_GRID_LEVELS; ++l) few += fewCells(l) ? 1 : 0;
-    const bool byCell = static_cast<double>(points) * few >= static_cast<double>(1 << 19);
+    const bool byCell = recordsWorthwhile(points, group);
     int64_t recordElements = 0;
     for (int g = 0; g < group; ++g) recordElements = r.byCell[g] ? r.total : recordElements;   // (an upper bound: of the grids before)
     for (int l = 0; l < levels_ && group + l < kernel::MAX_GRID_LEVELS; ++l) {
-        if (byCell && fewCells(l)) {
-            // as many copies as leave a record 256 points (10^6 points on 256 cells of 64 bytes: 40 us, 4096 cells 17, 16384 cells 15)
-            int lg = 0;
-            for (double hits = static_cast<double>(points) / cellsOf(l); hits > 256 && lg < 6; hits /= 2) ++lg;
-            const int64_t n = static_cast<int64_t>(cellsOf(l)) * record << lg, at = (r.total + 3) / 4 * 4;   // (written 16 bytes at a time)
-            if (recordElements + n <= (20ll << 20) && at + n <= (1ll << 28)) {
+        int64_t n = 0;
+        int lg = byCell ? recordCopies(points, l, n) : -1;
+        if (lg >= 0) {
+            const int64_t at = (r.total + 3) / 4 * 4;   // (written 16 bytes at a time)
+            if (recordElements + n <= RECORD_BUDGET && at + n <= REPLICA_LIMIT) {
                 r.byCell[group + l] = static_cast<unsigned char>(1 + lg);
                 r.offset[group + l] = static_cast<unsigned int>(at);
                 r.total = at + n;
@@ -356,14 +379,23 @@ void EncodingHashGrid::planReplicas(int64_t points, int group, kernel::GradRepli
                 continue;
             }
         }
-        const int64_t elements = (l + 1 < levels_ ? table_[l + 1].memoryOffset : numParameters_) - table_[l].memoryOffset;
-        double perLine = reductions / std::max<double>(1.0, static_cast<double>(elements) / 32);
-        int lg = 0;
-        for (; perLine > 2048 && lg < 6; perLine /= 2) ++lg;
-        if (lg == 0 || r.total + (elements << lg) > (1ll << 28)) continue;   // (32-bit offsets)
+        lg = gradientCopies(points, l, n);
+        if (lg == 0 || r.total + n > REPLICA_LIMIT) continue;
         r.log2Copies[group + l] = static_cast<unsigned char>(lg);
         r.offset[group + l] = static_cast<unsigned int>(r.total);
-        r.total += elements << lg;
+        r.total += n;
+    }
+}
+
+void EncodingHashGrid::boundReplicas(int64_t points, int group, int64_t& records, int64_t& copies) const
+{
+    // Level by level what either kind may take, each of which grows with the points; which levels the budget leaves out does not.
+    if (isLine()) return;
+    const bool byCell = recordsWorthwhile(points, group);
+    for (int l = 0; l < levels_ && group + l < kernel::MAX_GRID_LEVELS; ++l) {
+        int64_t n = 0;
+        if (byCell && recordCopies(points, l, n) >= 0) records += n;
+        if (gradientCopies(points, l, n) > 0) copies += n;
     }
 }
 
@@ -690,6 +722,25 @@ void Network::planReplicas(int64_t points, kernel::GradReplicas& r) const
             h->planReplicas(points, group, r);
             group += static_cast<int>(h->levelTable().size());
         }
+}
+
+int64_t replicaElements(int64_t records, int64_t copies)
+{
+    const int64_t n = std::min(records, RECORD_BUDGET) + copies;
+    return n > 0 ? std::min(n + 4 * kernel::MAX_GRID_LEVELS, REPLICA_LIMIT) : 0;   // (every level starts on a multiple of 4)
+}
+
+int64_t Network::replicaElements(int64_t points) const
+{
+    int64_t records = 0, copies = 0;
+    int group = 0;
+    for (const auto& e : encodings_)
+        if (auto* h = dynamic_cast<const EncodingHashGrid*>(e.get())) {
+            if (h->isLine()) continue;
+            h->boundReplicas(points, group, records, copies);
+            group += static_cast<int>(h->levelTable().size());
+        }
+    return qmlp::replicaElements(records, copies);
 }
 
 size_t Network::planCells(int64_t points, kernel::CellTables& c, bool widest) const

@@ -172,6 +172,8 @@ public:
     // copies of the gradients of small levels for a batch of `points` (kernel::GradReplicas; base is left as it is),
     // appended to `r` from level `group` (counted over all grids of a network) on
     void planReplicas(int64_t points, int group, kernel::GradReplicas& r) const;
+    // adds what the plans of all batches of up to `points` need at most: elements of records by cell and of copies (replicaElements)
+    void boundReplicas(int64_t points, int group, int64_t& records, int64_t& copies) const;
     // copies of small levels by cell for a batch of `points` (kernel::CellTables; base is left as it is), appended to `c` from
     // level `group` on behind the first `bytes` bytes; returns the bytes then used
     size_t planCells(int64_t points, int group, bool halfTable, kernel::CellTables& c, size_t bytes) const;
@@ -187,7 +189,14 @@ protected:
     std::vector<float> boxMin_, boxSize_, boxInvSize_;
     std::vector<GridLevel> table_;
     int64_t numParameters_ = 0;
+
+private:
+    int recordCopies(int64_t points, int level, int64_t& elements) const;
+    bool recordsWorthwhile(int64_t points, int group) const;
+    int gradientCopies(int64_t points, int level, int64_t& elements) const;
 };
+// elements of scratch for the sums that EncodingHashGrid::boundReplicas leaves behind
+int64_t replicaElements(int64_t records, int64_t copies);
 
 // EncodingLineIntegration, src_cpp/include/qmlp/encoding_line_integration.h / src_cpp/src/encoding_line_integration.cpp:
 // ray start + direction in, the child volume (a hash grid on the sample position) integrated along the ray out.
@@ -262,6 +271,7 @@ public:
     int64_t gridTableBytes() const;   // bytes of all bound grid tables (what the gather walks through)
     int gathersPerPoint() const;      // table rows fetched per point by all plain grid encodings: sum of levels * 2^D
     void planReplicas(int64_t points, kernel::GradReplicas& r) const;   // of all grid encodings; zeroes `r` first
+    int64_t replicaElements(int64_t points) const;                      // elements that serve the plan of every batch of up to `points`
     // copies by cell of all grid encodings for tables of the type that is bound; zeroes `c` first, returns the bytes. `widest`: the
     // bytes that are enough whatever is bound
     size_t planCells(int64_t points, kernel::CellTables& c, bool widest = false) const;

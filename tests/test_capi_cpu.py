@@ -194,3 +194,50 @@ def test_stash_block_layout_helper():
     assert np.array_equal(rows, want.astype(np.float32))
     both = helpers.stash_rows_all(np.concatenate([flat, flat]), n32, [c, c])
     assert np.array_equal(both.reshape(2, n32, c)[1], want.astype(np.float32))
+
+
+def scratch_networks():
+    """name -> network whose levels have records by cell, copies of the gradient and copies by cell in different mixtures"""
+    def net(num_inputs, *encodings):
+        return specs.grid_net(num_inputs, list(encodings), [64, 1], ["relu", "identity"])
+    return {
+        "pyramid": net(2, specs.hashgrid(2, 12, 4, -1, 16, 2048)),
+        "grid4d": specs.config5(),
+        "mixed": specs.config4(),
+        "rows_of_one_and_four": net(3, specs.hashgrid(2, 6, 1, -1, 5, 300), specs.hashgrid(3, 8, 4, 14, 8, 200)),
+        "wide_rows": net(3, specs.hashgrid(2, 4, 8, -1, 100, 1000), specs.hashgrid(3, 4, 8, 10, 20, 100)),
+    }
+
+
+@pytest.mark.parametrize("name", list(scratch_networks()))
+def test_scratch_for_a_larger_batch_serves_a_smaller_one(name):
+    """A program sizes its scratch memory once, for its largest batch (the calls that use it are not told its size)."""
+    from qmlp import bindings
+    from qmlp._capi import TrainerConfig
+    lib = _lib()
+    net = bindings.Network(json.dumps(scratch_networks()[name]))
+    config = TrainerConfig(1e-2, 0.9, 0.999, 1e-8, 0, 0)
+    handle = C.c_void_p()
+    assert lib.qmlp_trainer_create(net._h, C.byref(config), C.byref(handle)) == 0
+    size = C.c_size_t()
+
+    def workspace(n):
+        assert lib.qmlp_trainer_workspace_bytes(handle, n, C.byref(size)) == 0
+        return size.value
+
+    def encoding(n, call, *args):
+        total = []
+        for i in range(net.num_encodings()):
+            assert call(net.encoding(i)._h, n, *args, C.byref(size)) == 0
+            total.append(size.value)
+        return total
+    points = sorted({int(64 * 1.07 ** i) for i in range(190)} | {3686400, 3686464, 16769600, 16777984} | {(1 << k) + d for k in range(6, 25) for d in (-1, 0, 1)})
+    try:
+        last = None
+        for n in points:
+            now = [net.adjoint_memory(n, 7), net.adjoint_memory(n, 6), workspace(n)]
+            now += encoding(n, lib.qmlp_encoding_adjoint_memory, 2) + encoding(n, lib.qmlp_encoding_forward_memory, None)
+            assert last is None or all(a >= b for a, b in zip(now, last)), f"{n} points: {now}, fewer: {last}"
+            last = now
+    finally:
+        lib.qmlp_trainer_destroy(handle)
