@@ -368,22 +368,20 @@ void EncodingHashGrid::planReplicas(int64_t points, int group, kernel::GradRepli
     for (int g = 0; g < group; ++g) recordElements = r.byCell[g] ? r.total : recordElements;   // (an upper bound: of the grids before)
     for (int l = 0; l < levels_ && group + l < kernel::MAX_GRID_LEVELS; ++l) {
         int64_t n = 0;
+        // (Rows of four features and the records are written 16 bytes at a time, and the levels before may have an odd number of
+        // elements: rows of one feature of another grid.)
+        const int64_t at = (r.total + 3) / 4 * 4;
         int lg = byCell ? recordCopies(points, l, n) : -1;
-        if (lg >= 0) {
-            const int64_t at = (r.total + 3) / 4 * 4;   // (written 16 bytes at a time)
-            if (recordElements + n <= RECORD_BUDGET && at + n <= REPLICA_LIMIT) {
-                r.byCell[group + l] = static_cast<unsigned char>(1 + lg);
-                r.offset[group + l] = static_cast<unsigned int>(at);
-                r.total = at + n;
-                recordElements += n;
-                continue;
-            }
+        if (lg >= 0 && recordElements + n <= RECORD_BUDGET && at + n <= REPLICA_LIMIT) {
+            r.byCell[group + l] = static_cast<unsigned char>(1 + lg);
+            recordElements += n;
+        } else {
+            lg = gradientCopies(points, l, n);
+            if (lg == 0 || at + n > REPLICA_LIMIT) continue;
+            r.log2Copies[group + l] = static_cast<unsigned char>(lg);
         }
-        lg = gradientCopies(points, l, n);
-        if (lg == 0 || r.total + n > REPLICA_LIMIT) continue;
-        r.log2Copies[group + l] = static_cast<unsigned char>(lg);
-        r.offset[group + l] = static_cast<unsigned int>(r.total);
-        r.total += n;
+        r.offset[group + l] = static_cast<unsigned int>(at);
+        r.total = at + n;
     }
 }
 

@@ -289,6 +289,40 @@ def test_train_kernel_matches_separate_kernels(name, n):
         assert norm > 0 and float((ga - gb).norm()) <= 1e-2 * norm, f"{name} n={n} segment {i}: {float((ga - gb).norm()) / norm}"
 
 
+def odd_rows_config():
+    """A grid of one feature per row, whose first level has an odd number of rows, in front of one of four features."""
+    return specs.grid_net(3, [specs.hashgrid(2, 3, 1, -1, 5, 21), specs.hashgrid(3, 2, 4, -1, 4, 12)], [64, 2], ["relu", "identity"])
+
+
+@pytest.mark.parametrize("n", [16384, 20001])
+def test_copies_of_gradients_behind_odd_levels(n):
+    """Copies of hot levels' gradients that follow copies with an odd number of elements: rows of four features are written 16
+    bytes at a time. Against the kernels without copies; tolerance as above."""
+    import torch
+    from qmlp import bindings
+    from qmlp.trainer import FusedTrainer
+    cfg = odd_rows_config()
+    spec = oracle.parse_spec(cfg)
+    x = torch.from_numpy(helpers.uniform(34, 1, (n, 3), 0.0, 1.0)).cuda()
+    t = torch.from_numpy(helpers.uniform(34, 2, (n, 2), -1.0, 1.0)).cuda()
+    params = torch.from_numpy(helpers.xavier_parameters(spec, cfg, bias_scale=0.1).astype(np.float32)).cuda()
+    tables = [torch.from_numpy(tb).cuda() for tb in helpers.grid_tables(spec, scale=0.5)]
+    results = []
+    try:
+        for path in (0, 1):
+            bindings.QuickMLP.set_kernel_path(path)
+            tr = FusedTrainer(bindings.Network(json.dumps(cfg)), grid_half_copy=False)
+            tr.set_parameters(params, tables)
+            tr.backend.gradients(x, t, n, tr.loss_sum)
+            torch.cuda.synchronize()
+            results.append([tr.segment(tr.gradient, i).clone() for i in range(3)])
+    finally:
+        bindings.QuickMLP.set_kernel_path(0)
+    for i, (a, b) in enumerate(zip(*results)):
+        norm = float(b.norm())
+        assert norm > 0 and float((a - b).norm()) <= 1e-2 * norm, f"segment {i}: {float((a - b).norm()) / norm}"
+
+
 def slot_configs():
     """name -> network by the tile slots of its training kernel: four (of one warpgroup; last delta in the first input's block), three, two
     (of two warpgroups) and one (of four); pre-activations in tensor memory, in registers, and both."""
