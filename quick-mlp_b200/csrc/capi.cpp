@@ -969,7 +969,7 @@ int qmlp_encoding_forward_memory(qmlp_encoding_t* enc, int64_t num_elements, con
     if (auto* g = dynamic_cast<EncodingHashGrid*>(enc->impl.get())) {
         const bool given = parameters != nullptr && parameters->ndim > 0;
         kernel::CellTables c{};
-        *bytes = g->planCells(num_elements, 0, (given ? parameters->precision : g->paramInference.precision) == QMLP_HALF, c, 0);
+        *bytes = g->planCells(num_elements, 0, (given ? parameters->precision : g->paramInference.precision) == QMLP_HALF, true, c, 0);
     }
     QMLP_CATCH
 }
@@ -1005,7 +1005,7 @@ int qmlp_encoding_forward_with_memory(qmlp_encoding_t* enc, const qmlp_tensor_t*
         a.outS1 = output->strides[1];
         if (auto* g = dynamic_cast<EncodingHashGrid*>(&e); g && tmp_memory) {
             if ((reinterpret_cast<uintptr_t>(tmp_memory) & 255) != 0) throw std::runtime_error("scratch memory must be 256-byte aligned");
-            const size_t need = g->planCells(a.numel, 0, e.paramInference.precision == QMLP_HALF, a.level->cells, 0);
+            const size_t need = g->planCells(a.numel, 0, e.paramInference.precision == QMLP_HALF, true, a.level->cells, 0);
             if (need > 0 && need <= tmp_bytes) {
                 a.level->cells.base = static_cast<unsigned char*>(tmp_memory);
                 a.flags = kernel::FLAG_FILL_CELLS;

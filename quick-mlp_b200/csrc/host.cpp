@@ -397,18 +397,38 @@ void EncodingHashGrid::boundReplicas(int64_t points, int group, int64_t& records
     }
 }
 
-size_t EncodingHashGrid::planCells(int64_t points, int group, bool halfTable, kernel::CellTables& c, size_t bytes) const
+size_t EncodingHashGrid::planCells(int64_t points, int group, bool halfTable, bool alone, kernel::CellTables& c, size_t bytes) const
 {
-    // Rows of four and more features in levels with at most a quarter as many cells as the batch has points, copies of up to 128 MB (they are
-    // read at random: from L2), from 3/4 million points on: 4-D grid of fp16 rows, 2^24 points 10120 -> 9520 us; 2-D pyramid of fp32 rows,
-    // 10^6 points 155 -> 143, 2^18 points 71 -> 76 (the host's launch); mixed network, step of 2^21 points 1487 -> 1474, 2^19 points 448 -> 453.
-    // Rows of two features gain nothing: 3-D grid, step of 2^20 points 786 -> 797 (fp16 rows), 823 -> 825 (fp32).
+    // Rows of four and more features, from 3/4 million points on, in levels with at most a twelfth as many cells as the batch has points, or copies
+    // of up to 8 bytes per point: every call writes them first. Uniform points / 128 samples along rays, time without over time with
+    // copies: two levels of 2^20 points, 3-D fp32 rows of 40^3 1.26 / 1.05, 50^3 1.12 / 0.88, 57^3 1.01 / 0.87; 2-D of 256^2 1.10 / 1.02, 360^2
+    // 1.08 / 1.05, 510^2 0.98 / 0.91; 2^22 points, 4-D fp16 rows, level by level: 16^4 1.52 / 1.00, 22^4 1.52 / 0.87, 31^4 1.01 / 0.64; mixed
+    // network, 2^20 points, fp16 50^3 1.10 / 0.86, fp32 50^3 1.00 / 0.84. Rows of two features gain nothing: 3-D grid, step of 2^20 points
+    // 786 -> 797 (fp16 rows), 823 -> 825 (fp32).
+    // All copies of a grid together: a pass that goes level by level reads one at a time (512 MB, the size of its planes). A stand-alone
+    // encoding reads all levels at once, and they have to stay in L2 beside its table: 2-D of 360^2, four levels (33 MB) 1.12, six of eight (50 MB)
+    // 0.77; of 256^2, eight levels (34 MB) 1.21, twelve of 16 (50 MB) 0.76; 16 levels of 57^3 (379 MB) 0.85. Unless the table itself does not: then one
+    // piece per point instead of 2^(D-1) pairs comes from DRAM, which is worth four points per cell: nine of 16 levels of 95^3, 2^22 points, 8021 -> 4829 us
+    // (rays 2728 -> 2241); 2-D, eight features, 16 levels of 512^2 to 1000^2 5120 -> 2812 (4151 -> 2704). No more memory than the
+    // features take there.
     const int64_t cellBytes = (static_cast<int64_t>(features_) << dim_) * (halfTable ? 2 : 4);   // (kernel::GridCellRows)
     if (isLine() || dim_ < 2 || (features_ != 4 && features_ != 8) || cellBytes < 64 || cellBytes > 256 || points < (3 << 18)) return bytes;
-    for (int l = 0; l < levels_ && group + l < kernel::MAX_GRID_LEVELS; ++l) {
+    const bool beyondL2 = alone && numParameters_ * (halfTable ? 2 : 4) > (96ll << 20);
+    const double limit = !alone ? 512.0 * (1 << 20) : beyondL2 ? 4.0 * numOutputChannels() * static_cast<double>(points) : 36.0 * (1 << 20);
+    auto cellsOf = [&](int l) {
         double cells = 1;
         for (int k = 0; k < dim_; ++k) cells *= table_[l].resolution;
-        if (cells * 4 > static_cast<double>(points) || cells * static_cast<double>(cellBytes) > static_cast<double>(128 << 20)) continue;
+        return cells;
+    };
+    // coarsest levels first: more points only ever add a level, and memory for a batch serves every smaller one
+    std::vector<int> order;
+    for (int l = 0; l < levels_ && group + l < kernel::MAX_GRID_LEVELS; ++l) order.push_back(l);
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return table_[a].resolution < table_[b].resolution; });
+    const size_t begin = bytes;
+    for (int l : order) {
+        const double cells = cellsOf(l), size = cells * static_cast<double>(cellBytes), n = static_cast<double>(points);
+        if (!(beyondL2 ? cells * 4 <= n : cells * 12 <= n || size <= 8 * n) || size > static_cast<double>(128 << 20)) break;
+        if (static_cast<double>(bytes - begin) + size > limit) break;
         c.offset[group + l] = static_cast<unsigned int>(bytes / 256 + 1);
         bytes += (static_cast<size_t>(cells) * cellBytes + 255) / 256 * 256;
     }
@@ -749,8 +769,8 @@ size_t Network::planCells(int64_t points, kernel::CellTables& c, bool widest) co
     for (const auto& e : encodings_)
         if (auto* h = dynamic_cast<const EncodingHashGrid*>(e.get())) {
             if (h->isLine()) continue;
-            if (widest) bytes = std::max(h->planCells(points, group, false, c, bytes), h->planCells(points, group, true, c, bytes));
-            else bytes = h->planCells(points, group, h->paramInference.precision == QMLP_HALF, c, bytes);
+            if (widest) bytes = std::max(h->planCells(points, group, false, false, c, bytes), h->planCells(points, group, true, false, c, bytes));
+            else bytes = h->planCells(points, group, h->paramInference.precision == QMLP_HALF, false, c, bytes);
             group += static_cast<int>(h->levelTable().size());
         }
     return bytes;

@@ -175,8 +175,9 @@ public:
     // adds what the plans of all batches of up to `points` need at most: elements of records by cell and of copies (replicaElements)
     void boundReplicas(int64_t points, int group, int64_t& records, int64_t& copies) const;
     // copies of small levels by cell for a batch of `points` (kernel::CellTables; base is left as it is), appended to `c` from
-    // level `group` on behind the first `bytes` bytes; returns the bytes then used
-    size_t planCells(int64_t points, int group, bool halfTable, kernel::CellTables& c, size_t bytes) const;
+    // level `group` on behind the first `bytes` bytes; returns the bytes then used. `alone`: for the stand-alone encoding, which reads
+    // all levels of a point in turn, not level by level
+    size_t planCells(int64_t points, int group, bool halfTable, bool alone, kernel::CellTables& c, size_t bytes) const;
     int features() const { return features_; }
     int dimension() const { return dim_; }
     Json gridJson() const;   // the hash grid's own configuration (id "HashGrid")

@@ -241,3 +241,34 @@ def test_scratch_for_a_larger_batch_serves_a_smaller_one(name):
             last = now
     finally:
         lib.qmlp_trainer_destroy(handle)
+
+
+def test_copies_by_cell_have_a_limit():
+    """Copies of small levels by cell that a stand-alone encoding asks for: what stays in the L2 beside a table that does, no level whose copy
+    costs more than it saves, and no more than the features themselves for a table that does not stay there; networks, which go
+    level by level: 512 MB a grid."""
+    from qmlp import bindings
+    from qmlp._capi import TrainerConfig
+    lib = _lib()
+    size = C.c_size_t()
+
+    def forward(cfg, n):
+        e = bindings.Encoding(json.dumps(cfg))
+        assert lib.qmlp_encoding_forward_memory(e._h, n, None, C.byref(size)) == 0
+        return size.value
+    assert 0 < forward(specs.hashgrid(3, 16, 4, -1, 32, 40), 1 << 20) <= 36 << 20
+    assert forward(specs.hashgrid(3, 16, 4, -1, 54, 60), 1 << 20) == 0
+    assert forward(specs.hashgrid(2, 8, 4, -1, 490, 500), 1 << 20) == 0
+    assert 0 < forward(specs.hashgrid(3, 16, 4, -1, 90, 100), 1 << 22) <= (1 << 22) * 64 * 4
+    assert forward(specs.hashgrid(2, 5, 4, -1, 16, 256), 1000003) > 65536 * 64
+    cfg = specs.config5()
+    cfg["encodings"] = [specs.hashgrid(4, 16, 4, 22, 31, 31, per_level_scale=1.0)]
+
+    def workspace(cfg, n):
+        net, handle, config = bindings.Network(json.dumps(cfg)), C.c_void_p(), TrainerConfig(1e-2, 0.9, 0.999, 1e-8, 1, 0)
+        assert lib.qmlp_trainer_create(net._h, C.byref(config), C.byref(handle)) == 0
+        assert lib.qmlp_trainer_workspace_bytes(handle, n, C.byref(size)) == 0
+        lib.qmlp_trainer_destroy(handle)
+        return size.value
+    few, many = workspace(specs.config5(), 1 << 24), workspace(cfg, 1 << 24)   # (the other parts differ by records and copies of gradients)
+    assert many - few <= (512 << 20) + (4 << 20) * 20
