@@ -151,18 +151,23 @@ kernel::LaunchArgs withScratchSizes(const Network& n, int kernelId, const kernel
     return b;
 }
 
-void launchModule(Network& n, KernelModule& m, int kernelId, const kernel::LaunchArgs& a, qmlp_stream_t stream)
+// The runtime's status; counts the launches. (Only bounds-checking instantiations read the sizes: the copy is 3 KB of a small call.)
+int tryLaunch(Network& n, KernelModule& m, int kernelId, const kernel::LaunchArgs& a, qmlp_stream_t stream)
 {
     TimedLaunch timed(kernelId, static_cast<cudaStream_t>(stream));
-    int launches = 0;
-    // (only bounds-checking instantiations read the sizes; the copy is 3 KB of a small call)
+    int launches = 0, e;
     if (Library::instance().boundsCheck) {
         const kernel::LaunchArgs b = withScratchSizes(n, kernelId, a);
-        checkLaunch(m.launch(kernelId, &b, static_cast<cudaStream_t>(stream), &launches), "kernel launch failed");
+        e = m.launch(kernelId, &b, static_cast<cudaStream_t>(stream), &launches);
     } else {
-        checkLaunch(m.launch(kernelId, &a, static_cast<cudaStream_t>(stream), &launches), "kernel launch failed");
+        e = m.launch(kernelId, &a, static_cast<cudaStream_t>(stream), &launches);
     }
-    n.launchCount += launches;
+    if (e == 0) n.launchCount += launches;
+    return e;
+}
+void launchModule(Network& n, KernelModule& m, int kernelId, const kernel::LaunchArgs& a, qmlp_stream_t stream)
+{
+    checkLaunch(tryLaunch(n, m, kernelId, a, stream), "kernel launch failed");
 }
 
 void launchNet(Network& n, int kernelId, const kernel::LaunchArgs& a, qmlp_stream_t stream)
@@ -524,16 +529,9 @@ static void inferenceLocked(Network& n, const qmlp_tensor_t* input, qmlp_tensor_
             a.planes = planes;
             a.planeStride = need;
             a.flags = kernel::FLAG_HALF_SUMS | (c0 == 0 ? kernel::FLAG_FILL_CELLS : 0);
-            int launches = 0;
-            int e;
-            {
-                TimedLaunch timed(kernel::KERNEL_ENCODE_PLANES, static_cast<cudaStream_t>(stream));
-                const kernel::LaunchArgs sized = withScratchSizes(n, kernel::KERNEL_ENCODE_PLANES, a);
-                e = m->launch(kernel::KERNEL_ENCODE_PLANES, &sized, static_cast<cudaStream_t>(stream), &launches);
-            }
+            const int e = tryLaunch(n, *m, kernel::KERNEL_ENCODE_PLANES, a, stream);
             if (e == static_cast<int>(cudaErrorNotSupported) && c0 == 0) { n.planesUnsupported = true; ok = false; break; }
             checkLaunch(e, "kernel launch failed");
-            n.launchCount += launches;
             launchModule(n, *m, kernel::KERNEL_INFERENCE_PLANES, a, stream);
         }
         if (ok) return;
@@ -1447,11 +1445,8 @@ int qmlp_trainer_gradients_part(qmlp_trainer_t* tr, const qmlp_tensor_t* input, 
                 tr->weightsWait = true;
             }
             if (what & 5) {
-                if (anyGrid) {
-                    kernel::LaunchArgs e = a;
-                    e.flags |= kernel::FLAG_FILL_CELLS;
-                    launchModule(n, *m, kernel::KERNEL_ENCODE_PLANES, e, stream);
-                }
+                a.flags |= kernel::FLAG_FILL_CELLS;   // (the encode pass alone reads it)
+                if (anyGrid) launchModule(n, *m, kernel::KERNEL_ENCODE_PLANES, a, stream);
                 launchModule(n, *m, kernel::KERNEL_TRAIN, a, stream);
             }
             if (what == 8) {
@@ -1470,18 +1465,11 @@ int qmlp_trainer_gradients_part(qmlp_trainer_t* tr, const qmlp_tensor_t* input, 
             a.planeStride = n32;
             a.flags = kernel::FLAG_FILL_CELLS;
             auto m = n.module(n.currentHalfMask());
-            int launches = 0;
-            int e;
-            {
-                TimedLaunch timed(kernel::KERNEL_ENCODE_PLANES, static_cast<cudaStream_t>(stream));
-                const kernel::LaunchArgs sized = withScratchSizes(n, kernel::KERNEL_ENCODE_PLANES, a);
-                e = m->launch(kernel::KERNEL_ENCODE_PLANES, &sized, static_cast<cudaStream_t>(stream), &launches);
-            }
+            const int e = tryLaunch(n, *m, kernel::KERNEL_ENCODE_PLANES, a, stream);
             if (e == static_cast<int>(cudaErrorNotSupported)) {
                 n.planesUnsupported = true;
             } else {
                 checkLaunch(e, "kernel launch failed");
-                n.launchCount += launches;
                 launchNet(n, kernel::KERNEL_FORWARD_LOSS_PLANES, a, stream);
                 done = true;
             }
