@@ -91,9 +91,9 @@ QMLP_API int qmlp_set_kernel_include_dir(const char* dir);
  * src_cpp/src/fused_network.cpp:45-69). */
 QMLP_API int qmlp_set_kernel_path(int path);
 /* Synchronises the current device and returns (then clears) its kernel status word: 0 = every kernel ran to completion;
- * bit 0 (1) = a kernel gave up on a bounded on-chip wait and its results are invalid; bits 1, 2, 3 (2, 4, 8) = a kernel
- * instantiated with bounds checks (qmlp_set_tuning("bounds_check", 1)) met a table row, a stash offset or a plane offset
- * outside the size the host declared and skipped that access. The reference has no counterpart (its
+ * bit 0 (1) = a kernel gave up on a bounded on-chip wait and its results are invalid; bits 1, 2, 3, 4 (2, 4, 8, 16) = a
+ * kernel instantiated with bounds checks (qmlp_set_tuning("bounds_check", 1)) met a table row, a stash offset, a plane offset or a
+ * record or copy of a grid cell outside the size the host declared and skipped that access. The reference has no counterpart (its
  * kernels contain no waits); debugging aids there are printf paths (src_cpp/include/qmlp/kernels/layer.cuh:28-41). */
 QMLP_API int qmlp_device_status(int* status);
 /* Tuning switches of the fused training step, for measurements; -1 restores the library's own choice.
@@ -101,7 +101,7 @@ QMLP_API int qmlp_device_status(int* status);
  * its own kernel (1) or inside the backward kernel (0); "scatter_runs": 0 sends every table-gradient contribution of
  * the sorted scatter straight to the table instead of summing runs of points that share a cell first. "bounds_check": 1
  * makes networks and encodings use (and build, on first use) instantiations whose kernels test every table row, stash
- * offset and plane offset against the declared sizes, skip what lies outside and set a bit of the status word
+ * offset, plane offset and record or copy of a grid cell against the declared sizes, skip what lies outside and set a bit of the status word
  * (qmlp_device_status) instead of faulting - the role of the reference's debug asserts in WrappedArray
  * (src_cpp/include/qmlp/kernels/common.cuh:174-218); "bounds_shrink": n declares every size n elements smaller than it
  * is (test hook: the check fires while every access still lands in real memory); "spin_limit": the layer kernel of a training

@@ -147,6 +147,8 @@ kernel::LaunchArgs withScratchSizes(const Network& n, int kernelId, const kernel
     b.fwdTmpHalfs = a.fwdTmp ? std::max<long long>(1, n32 * stashHalfs - shrink) : 0;
     b.adjTmpHalfs = a.adjTmp ? std::max<long long>(1, n32 * n.deltaHalfsPerPoint() - shrink) : 0;
     b.spinLimit = Library::instance().spinLimit < 0 ? 1u << 24 : static_cast<unsigned int>(Library::instance().spinLimit);
+    b.level->replicas.capacity = std::max<long long>(0, a.level->replicas.total - shrink);
+    b.level->cells.bytes = std::max<long long>(0, a.level->cells.bytes - shrink);
     b.planeHalfs = a.planes ? std::max<long long>(1, a.planeStride * n.encodedChannels() - shrink) : 0;
     return b;
 }
@@ -500,6 +502,7 @@ static void inferenceLocked(Network& n, const qmlp_tensor_t* input, qmlp_tensor_
         __half* planes = memory != nullptr && memoryBytes >= planeBytes ? static_cast<__half*>(memory) : nullptr;
         if (planes != nullptr) {
             const size_t cellBytes = n.planCells(a.numel, a.level->cells);
+            a.level->cells.bytes = static_cast<long long>(cellBytes);
             if (cellBytes > 0 && memoryBytes >= planeBytes + cellBytes) a.level->cells.base = static_cast<unsigned char*>(memory) + planeBytes;
         }
         if (planes == nullptr) {
@@ -1006,6 +1009,7 @@ int qmlp_encoding_forward_with_memory(qmlp_encoding_t* enc, const qmlp_tensor_t*
             const size_t need = g->planCells(a.numel, 0, e.paramInference.precision == QMLP_HALF, true, a.level->cells, 0);
             if (need > 0 && need <= tmp_bytes) {
                 a.level->cells.base = static_cast<unsigned char*>(tmp_memory);
+                a.level->cells.bytes = std::max<long long>(0, static_cast<long long>(need) - Library::instance().boundsShrink);
                 a.flags = kernel::FLAG_FILL_CELLS;
             }
         }
@@ -1087,6 +1091,7 @@ int qmlp_encoding_adjoint_with_memory(qmlp_encoding_t* enc, const qmlp_tensor_t*
             g->planReplicas(a.numel, 0, a.level->replicas);
             if (a.level->replicas.total > 0 && static_cast<size_t>(a.level->replicas.total) * sizeof(float) <= tmp_bytes) a.level->replicas.base = static_cast<float*>(tmp_memory);
             else std::memset(&a.level->replicas, 0, sizeof a.level->replicas);
+            a.level->replicas.capacity = std::max<long long>(0, a.level->replicas.total - Library::instance().boundsShrink);
         }
         if (a.numel > 0 && a.flags != 0) {
             auto m = e.standaloneModule(e.paramInference.precision == QMLP_HALF && e.isGrid());
@@ -1361,7 +1366,8 @@ int qmlp_trainer_gradients_part(qmlp_trainer_t* tr, const qmlp_tensor_t* input, 
     for (int i = 0; i < n.numEncodings(); ++i) anyGrid = anyGrid || n.encoding(i)->hasParameters();
     __half* planes = anyGrid ? reinterpret_cast<__half*>(ws + lay.planes) : nullptr;
     bindReplicas(n, a, ws + lay.replicas);
-    if (n.planCells(numel, a.level->cells) > 0) a.level->cells.base = ws + lay.cells;
+    a.level->cells.bytes = static_cast<long long>(n.planCells(numel, a.level->cells));
+    if (a.level->cells.bytes > 0) a.level->cells.base = ws + lay.cells;
     // Gather-dominated batches (same rule as inference): the encodings are computed one grid level at a time into
     // the plane region of the workspace, which is free until the backward kernel writes the adjoint planes there,
     // and the forward kernel reads its layer-0 operand from the planes.

@@ -345,7 +345,7 @@ __device__ __forceinline__ void encode_pair(const LaunchArgs& p, const RowReader
             for (int l = 0; l < Enc::L; ++l) {
                 const GridLevelP& lv = g.levels[l];
                 float feat[F];
-                grid_pair_forward<D, F, Enc::HALF_TABLE, EXACT>(g, lv, nullptr, pos0, pos1, side, feat);
+                grid_pair_forward<D, F, Enc::HALF_TABLE, EXACT>(g, lv, CellCopy{nullptr, nullptr}, pos0, pos1, side, feat);
 #pragma unroll
                 for (int i = 0; i < F; ++i) {
                     if constexpr (Enc::CONCAT) out(Enc::OUT_OFF + l * F + i, feat[i]);

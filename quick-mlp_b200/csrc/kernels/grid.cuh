@@ -58,8 +58,8 @@ __device__ __forceinline__ unsigned int grid_vertex_index(const unsigned int (&v
     return idx * F + lv.offset;
 }
 
-// Every table access of every kernel passes its element index through here, so this is where a QMLP_BOUNDS_CHECK build tests
-// it: a row that does not lie inside its level is reported through the status word and replaced by the level's first row
+// Every table access of every kernel passes its element index through here (records and copies by cell: grid_cell_inside), so this is
+// where a QMLP_BOUNDS_CHECK build tests it: a row that does not lie inside its level is reported through the status word and replaced by the level's first row
 // (which the copies of a level's gradient hold too), and the kernel carries on.
 template <int D, int F>
 __device__ __forceinline__ unsigned int grid_checked_index(const GridP& g, const GridLevelP& lv, unsigned int e)
@@ -79,6 +79,24 @@ __device__ __forceinline__ unsigned int grid_checked_index(const GridP& g, const
     }
     (void)g; (void)lv;
     return e;
+}
+
+// QMLP_BOUNDS_CHECK builds: is `cell` a cell of the level, and does what is read or written for it end where the scratch memory does? If
+// not, the status word says so and the caller does without. Compiles to `true` in regular builds.
+template <int D>
+__device__ __forceinline__ bool grid_cell_inside(const GridLevelP& lv, unsigned int cell, const void* upTo, const void* end, int* status)
+{
+    if constexpr (BOUNDS_CHECK) {
+        unsigned long long cells = 1;
+#pragma unroll
+        for (int k = 0; k < D; ++k) cells *= static_cast<unsigned long long>(lv.resolution);
+        if (cell >= cells || static_cast<const char*>(upTo) > static_cast<const char*>(end)) {
+            if (status != nullptr) atomicOr(status, STATUS_CELL);
+            return false;
+        }
+    }
+    (void)lv; (void)cell; (void)upTo; (void)end; (void)status;
+    return true;
 }
 
 // element index of corner `bits` of a cell (bit k set -> high corner in dimension k)
@@ -551,6 +569,12 @@ __device__ __forceinline__ bool grid_cell_regular(const GridCell<D>& c, const Gr
     return ok;
 }
 
+// a level's copy (at null: none) and the end of the memory that holds it
+struct CellCopy {
+    const unsigned char* at;
+    const unsigned char* end;
+};
+
 // this lane's rows (one side of the pairing dimension) of a cell
 template <int D, int F, bool HALF>
 __device__ __forceinline__ void grid_cell_load(const unsigned char* cells, unsigned int cell, int side,
@@ -589,8 +613,8 @@ __device__ __forceinline__ void grid_add_row(float w, const uint32_t (&r)[F * (H
 
 // grid_pair_forward from the copy. False, for the whole warp, if one of its points has other corners than the copy holds.
 template <int D, int F, bool HALF, bool EXCHANGE, int PD>
-__device__ __forceinline__ bool grid_pair_from_cells(const unsigned char* cells, const GridLevelP& lv, const float (&pos0)[D], const float (&pos1)[D], int side,
-                                                     float (&feat)[F])
+__device__ __forceinline__ bool grid_pair_from_cells(const CellCopy& copy, const GridLevelP& lv, int* status, const float (&pos0)[D], const float (&pos1)[D],
+                                                     int side, float (&feat)[F])
 {
     using C = GridCellRows<D, F, HALF>;
     GridCell<D> c0, c1;
@@ -599,9 +623,15 @@ __device__ __forceinline__ bool grid_pair_from_cells(const unsigned char* cells,
 #pragma unroll
     for (int k = 0; k < D; ++k) asm volatile("" : "+f"(c0.f[k]), "+f"(c1.f[k]));   // (computed here, beside the product they come from, as in the other path)
     if (!__all_sync(0xffffffffu, grid_cell_regular<D>(c0, lv) && grid_cell_regular<D>(c1, lv))) return false;
+    const unsigned int n0 = grid_cell_number<D>(c0, lv), n1 = grid_cell_number<D>(c1, lv);
+    if constexpr (BOUNDS_CHECK) {
+        const unsigned char *up0 = copy.at + (static_cast<size_t>(n0) + 1) * C::BYTES, *up1 = copy.at + (static_cast<size_t>(n1) + 1) * C::BYTES;
+        const bool inside = grid_cell_inside<D>(lv, n0, up0, copy.end, status) && grid_cell_inside<D>(lv, n1, up1, copy.end, status);
+        if (!__all_sync(0xffffffffu, inside)) return false;
+    }
     uint32_t raw0[C::H][C::WORDS], raw1[C::H][C::WORDS];
-    grid_cell_load<D, F, HALF>(cells, grid_cell_number<D>(c0, lv), side, raw0);
-    grid_cell_load<D, F, HALF>(cells, grid_cell_number<D>(c1, lv), side, raw1);
+    grid_cell_load<D, F, HALF>(copy.at, n0, side, raw0);
+    grid_cell_load<D, F, HALF>(copy.at, n1, side, raw1);
     if constexpr (EXCHANGE) {
         GridCell<D> own;
 #pragma unroll
@@ -626,11 +656,11 @@ __device__ __forceinline__ bool grid_pair_from_cells(const unsigned char* cells,
     return true;
 }
 
-// copy of level `group` (counted over all grids), null: none
-__device__ __forceinline__ const unsigned char* grid_cells(const CellTables& t, int group)
+// copy of level `group` (counted over all grids)
+__device__ __forceinline__ CellCopy grid_cells(const CellTables& t, int group)
 {
-    if (t.base == nullptr || group >= MAX_GRID_LEVELS || t.offset[group] == 0) return nullptr;
-    return t.base + static_cast<size_t>(t.offset[group] - 1) * 256;
+    if (t.base == nullptr || group >= MAX_GRID_LEVELS || t.offset[group] == 0) return {nullptr, nullptr};
+    return {t.base + static_cast<size_t>(t.offset[group] - 1) * 256, t.base + t.bytes};
 }
 
 constexpr int FILL_THREADS = 256;
@@ -643,7 +673,7 @@ __host__ __device__ inline unsigned int grid_fill_blocks(int resolution)
     return (n * (2 * GridCellRows<D, F, HALF>::ACCESSES) + FILL_THREADS - 1) / FILL_THREADS;
 }
 template <int D, int F, bool HALF>
-__device__ __forceinline__ void grid_fill_cells(const GridP& g, const GridLevelP& lv, unsigned char* cells, unsigned int block)
+__device__ __forceinline__ void grid_fill_cells(const GridP& g, const GridLevelP& lv, unsigned char* cells, const unsigned char* end, unsigned int block)
 {
     using C = GridCellRows<D, F, HALF>;
     const unsigned int t = block * FILL_THREADS + threadIdx.x, side = t & 1u, u = (t >> 1) % C::ACCESSES, res = static_cast<unsigned int>(lv.resolution);
@@ -678,6 +708,7 @@ __device__ __forceinline__ void grid_fill_cells(const GridP& g, const GridLevelP
         }
     }
     unsigned char* at = cells + static_cast<size_t>(t) * C::ACCESS;   // (accesses in the order of the threads)
+    if (!grid_cell_inside<D>(lv, 0, at + C::ACCESS, end, g.status)) return;
     stg_u256(at, v);
 }
 
@@ -689,14 +720,14 @@ __device__ __forceinline__ void grid_fill_cells(const GridP& g, const GridLevelP
 // 280 us in all), above that the half sums (two fp32 features, 100 000 points: 41.0 against 42.8 us; 4-D grid of four fp16
 // features, 2^24 points: 10.5 against 11.7 ms).
 template <int D, int F, bool HALF, bool EXACT>
-__device__ __forceinline__ void grid_pair_forward(const GridP& g, const GridLevelP& lv, const unsigned char* cells, const float (&pos0)[D], const float (&pos1)[D],
+__device__ __forceinline__ void grid_pair_forward(const GridP& g, const GridLevelP& lv, const CellCopy& copy, const float (&pos0)[D], const float (&pos1)[D],
                                                   int side, float (&feat)[F])
 {
     constexpr int WORDS = (1 << (D - 1)) * ((HALF && F % 2 == 0) ? F / 2 : F);
     if constexpr (GridCellRows<D, F, HALF>::USED) {
-        if (cells != nullptr) {
-            if (lv.hashed ? grid_pair_from_cells<D, F, HALF, EXACT || WORDS <= 4, 0>(cells, lv, pos0, pos1, side, feat)
-                          : grid_pair_from_cells<D, F, HALF, EXACT || WORDS <= 4, D - 1>(cells, lv, pos0, pos1, side, feat)) return;
+        if (copy.at != nullptr) {
+            if (lv.hashed ? grid_pair_from_cells<D, F, HALF, EXACT || WORDS <= 4, 0>(copy, lv, g.status, pos0, pos1, side, feat)
+                          : grid_pair_from_cells<D, F, HALF, EXACT || WORDS <= 4, D - 1>(copy, lv, g.status, pos0, pos1, side, feat)) return;
         }
     }
     if constexpr (EXACT || WORDS <= 4) {
@@ -772,19 +803,16 @@ struct GridCellUnits {
 // The lanes of a group take the group's points in turn. `pos`: this lane's own point; adjoint(r, a): the adjoint of the features of the
 // group's r-th point (all lanes of the warp take part). False if this lane's point lies in no cell that has a record.
 template <int D, int F, class Adjoint>
-__device__ __forceinline__ bool grid_cells_scatter(float* records, const GridLevelP& lv, const float (&pos)[D], bool valid, const Adjoint& adjoint)
+__device__ __forceinline__ bool grid_cells_scatter(float* records, const float* end, int* status, const GridLevelP& lv, const float (&pos)[D], bool valid,
+                                                   const Adjoint& adjoint)
 {
     using C = GridCellUnits<D, F>;
     GridCell<D> c;
     grid_cell<D>(pos, lv.resolution, c);
-    bool regular = true;   // high corner = low corner + 1, or the border: not so for a point below the box
     unsigned int own = c.lo[0];
 #pragma unroll
-    for (int k = 0; k < D; ++k) {
-        regular = regular && c.hi[k] == min(c.lo[k] + 1u, static_cast<unsigned int>(lv.resolution - 1));
-        if (k > 0) own = c.lo[k] + own * static_cast<unsigned int>(lv.resolution);
-    }
-    if (!valid || !regular) own = 0xffffffffu;
+    for (int k = 1; k < D; ++k) own = c.lo[k] + own * static_cast<unsigned int>(lv.resolution);
+    if (!valid || !grid_cell_regular<D>(c, lv)) own = 0xffffffffu;
     const int lane = threadIdx.x % C::LANES;
 #pragma unroll
     for (int r = 0; r < C::LANES; ++r) {
@@ -794,6 +822,7 @@ __device__ __forceinline__ bool grid_cells_scatter(float* records, const GridLev
         for (int k = 0; k < D; ++k) f[k] = __shfl_sync(0xffffffffu, c.f[k], r, C::LANES);
         adjoint(r, a);
         if (cell == 0xffffffffu) continue;
+        if (!grid_cell_inside<D>(lv, cell, records + (static_cast<size_t>(cell) + 1) * C::ELEMENTS, end, status)) continue;
         float* at = records + static_cast<size_t>(cell) * C::ELEMENTS + lane * 4;
 #pragma unroll
         for (int u = 0; u < C::UNITS; u += C::LANES) {
@@ -836,6 +865,7 @@ __device__ __forceinline__ void grid_sum_cells(const GridP& g, const GradReplica
     const unsigned int n = grid_cell_count<D>(lv.resolution), res = static_cast<unsigned int>(lv.resolution);
     const int copies = 1 << (r.byCell[group] - 1);
     const float* base = r.base + r.offset[group];
+    if (!grid_cell_inside<D>(lv, 0, base + static_cast<size_t>(copies) * n * C::ELEMENTS, r.base + r.capacity, g.status)) return;
     for (unsigned int i = blockIdx.x * 256u + threadIdx.x; i < n; i += gridDim.x * 256u) {
         unsigned int v[D], rest = i;
 #pragma unroll
@@ -844,7 +874,7 @@ __device__ __forceinline__ void grid_sum_cells(const GridP& g, const GradReplica
             v[k] = rest - q * res;
             rest = q;
         }
-        double sum[F];   // (up to 512 terms of like size: added in fp32 they would cost more than the reductions did)
+        double sum[F];   // (2^D cells, 3^D at the upper border, of up to 64 copies each: added in fp32 the terms would cost more than the reductions did)
 #pragma unroll
         for (int e = 0; e < F; ++e) sum[e] = 0.0;
         // In every dimension the vertex is the low corner of its own cell, the high corner of the one before, and at the border

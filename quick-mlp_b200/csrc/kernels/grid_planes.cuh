@@ -192,7 +192,8 @@ __global__ void __launch_bounds__(FILL_THREADS) fill_cells_kernel(const __grid_c
         const GridP& grid = p.grids[Enc::SLOT];
         const unsigned int n = grid_fill_blocks<Enc::D, Enc::F, Enc::HALF_TABLE>(grid.levels[l].resolution);
         if (block < n)
-            grid_fill_cells<Enc::D, Enc::F, Enc::HALF_TABLE>(grid, grid.levels[l], p.level->cells.base + static_cast<size_t>(p.level->cells.offset[group] - 1) * 256, block);
+            grid_fill_cells<Enc::D, Enc::F, Enc::HALF_TABLE>(grid, grid.levels[l], p.level->cells.base + static_cast<size_t>(p.level->cells.offset[group] - 1) * 256,
+                                                                   p.level->cells.base + p.level->cells.bytes, block);
         block -= n;   // (wraps: the levels after this block's own are past its number)
     });
 }
@@ -263,7 +264,7 @@ __device__ __forceinline__ void scatter_group(const LaunchArgs& p, int g, const 
                             a[2 * i + 1] = x.y;
                         }
                     };
-                    const bool done = grid_cells_scatter<D, F>(records, lv, pos, valid, [&](int r, float (&a)[F]) {
+                    const bool done = grid_cells_scatter<D, F>(records, p.level->replicas.base + p.level->replicas.capacity, grid.status, lv, pos, valid, [&](int r, float (&a)[F]) {
                         uint32_t w[(F + 1) / 2];
 #pragma unroll
                         for (int i = 0; i < (F + 1) / 2; ++i) w[i] = __shfl_sync(0xffffffffu, own[i], r, GridCellUnits<D, F>::LANES);

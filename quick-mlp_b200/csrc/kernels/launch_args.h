@@ -44,9 +44,9 @@ struct GridP {
 };
 
 // Bits of the library's device status word (qmlp_device_status). Bit 0 is set by a kernel that gave up on a bounded wait;
-// the others only by instantiations compiled with QMLP_BOUNDS_CHECK, which test every table row, stash offset and plane
-// offset against the size the host declared, skip an access that would leave it and report here instead of faulting.
-constexpr int STATUS_WAIT_TIMEOUT = 1, STATUS_TABLE_ROW = 2, STATUS_STASH = 4, STATUS_PLANES = 8;
+// the others only by instantiations compiled with QMLP_BOUNDS_CHECK, which test every table row, stash offset, plane
+// offset and record or copy of a grid cell against the size the host declared, skip an access that would leave it and report here instead of faulting.
+constexpr int STATUS_WAIT_TIMEOUT = 1, STATUS_TABLE_ROW = 2, STATUS_STASH = 4, STATUS_PLANES = 8, STATUS_CELL = 16;
 #ifdef QMLP_BOUNDS_CHECK
 constexpr bool BOUNDS_CHECK = true;
 #else
@@ -72,6 +72,7 @@ constexpr int FLAG_FILL_CELLS = 32;
 // uses them.
 struct CellTables {
     unsigned char* base;                    // 256-byte aligned (null: none)
+    long long bytes;                        // of all copies (QMLP_BOUNDS_CHECK builds)
     unsigned int offset[MAX_GRID_LEVELS];   // first byte of a level's cells / 256, + 1; levels counted over all grids of the network; 0: no copy
 };
 
@@ -81,6 +82,7 @@ struct CellTables {
 struct GradReplicas {
     float* base;                            // copies of all such levels, level by level (null: none)
     long long total;                        // elements
+    long long capacity;                     // the same, for QMLP_BOUNDS_CHECK builds (the size the host declares)
     unsigned int offset[MAX_GRID_LEVELS];        // first element of a level's copies; levels counted over all grids of the network
     unsigned char log2Copies[MAX_GRID_LEVELS];   // 0: the level has no copies
     unsigned char byCell[MAX_GRID_LEVELS];       // 1 + log2 of the copies of a level whose gradient is added up by cell first (GridCellUnits); else 0
@@ -172,4 +174,4 @@ extern "C" {
 typedef int (*qmlp_spec_launch_fn)(int kernel, const void* args, cudaStream_t stream, int* launches);
 typedef int (*qmlp_spec_abi_fn)(void);
 }
-#define QMLP_SPEC_ABI_VERSION 14
+#define QMLP_SPEC_ABI_VERSION 15

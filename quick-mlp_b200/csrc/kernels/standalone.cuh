@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(EncodingTile<Enc>::WARPS * 32) grid_encoding_a
                     float own[D];
 #pragma unroll
                     for (int k = 0; k < D; ++k) own[k] = side ? pos[1][k] : pos[0][k];
-                    const bool done = grid_cells_scatter<D, F>(records, lv, own, row0 + lane <= last, [&](int r, float (&a)[F]) {
+                    const bool done = grid_cells_scatter<D, F>(records, p.level->replicas.base + p.level->replicas.capacity, g.status, lv, own, row0 + lane <= last, [&](int r, float (&a)[F]) {
                         T::get(tile + (lane / GridCellUnits<D, F>::LANES * GridCellUnits<D, F>::LANES + r) * T::STRIDE, l * C, a);
                     });
                     if (!done) {

@@ -424,6 +424,37 @@ def test_training_kernel_ends_when_a_wait_gives_up(bounds_check, name):
     assert float((after - before).norm()) <= 1e-5 * float(before.norm())   # (the order of fp32 sums)
 
 
+@pytest.mark.parametrize("name,n", [("config3", (1 << 19) + 77), ("config4", (3 << 18) + 77)])
+def test_bounds_check_reaches_records_and_copies_by_cell(bounds_check, name, n):
+    """A step that adds up gradients by cell (both networks) and reads levels from copies by cell (rows of four features): silent with honest
+    sizes, with sizes declared 3000 smaller reported by a bit of its own, and skipped. Tolerance against the instantiation without
+    checks, which may round a cell fraction otherwise, as for the kernels of the step: a relu input next to zero."""
+    import torch
+    from qmlp import bindings
+    from qmlp.trainer import FusedTrainer
+    cfg = FULL[name]()
+    spec = oracle.parse_spec(cfg)
+    x = torch.from_numpy(helpers.uniform(87, 1, (n, 3), -0.001, 1.001)).cuda()
+    t = torch.from_numpy(helpers.uniform(87, 2, (n, spec.num_outputs), -1.0, 1.0)).cuda()
+    params = torch.from_numpy(helpers.xavier_parameters(spec, cfg, bias_scale=0.05)).cuda()
+    tables = [torch.from_numpy(tb).cuda() if tb is not None else None for tb in helpers.grid_tables(spec, scale=0.5)]
+    tr = FusedTrainer(bindings.Network(json.dumps(cfg)), grid_half_copy=name == "config3")
+    tr.set_parameters(params, tables)
+    tr.backend.gradients(x, t, n, tr.loss_sum)
+    assert bindings.QuickMLP.device_status() == 0
+    gradient = tr.gradient.clone()
+    bindings.QuickMLP.set_tuning("bounds_shrink", 3000)
+    tr.gradient.zero_()
+    tr.backend.gradients(x, t, n, tr.loss_sum)
+    assert bindings.QuickMLP.device_status() & 17 == 16
+    assert bool(torch.isfinite(tr.gradient).all())
+    bindings.QuickMLP.set_tuning("bounds_shrink", 0)
+    bindings.QuickMLP.set_tuning("bounds_check", 0)
+    tr.gradient.zero_()
+    tr.backend.gradients(x, t, n, tr.loss_sum)
+    assert float((tr.gradient - gradient).norm()) <= 1e-2 * float(gradient.norm())
+
+
 def test_scratch_memory_does_not_depend_on_the_switches():
     """Scratch sized with bounds_check on serves a call with it off: the workspace a trainer keeps for a number of points, and
     the adjoint scratch an autograd node asked for in its forward call. 2^18 points: the coarse levels have copies."""
