@@ -28,6 +28,7 @@ def jobs():
         out.append(("net", json.dumps(cfg), 0))
         out.append(("net", json.dumps(cfg), 1))
     out.append(("net", json.dumps(tt.two_grid_config()), 3))
+    out.append(("net", json.dumps(tt.two_grid_config()), 0))
     out.append(("net", json.dumps(tt.odd_rows_config()), 0))
     for cfg in tt.slot_configs().values():
         out.append(("net", json.dumps(cfg), 0))

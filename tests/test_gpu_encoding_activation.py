@@ -320,3 +320,77 @@ def test_network_inference_from_copies_by_cell():
         assert float((results[0] - results[1]).norm()) <= 1e-4 * float(results[0].norm()) > 0
     finally:
         bindings.QuickMLP.set_kernel_path(0)
+
+
+def test_two_chunks_of_an_inference_from_copies_by_cell():
+    """Copies that the first chunk of an inference fills serve the second. Tolerance as above."""
+    import ctypes as C
+    import torch
+    from qmlp import bindings
+    from qmlp._capi import check, lib, wrap
+    from test_gpu_network import network_cases
+    cfg, rng, _ = network_cases()["config5_small"]
+    spec = oracle.parse_spec(cfg)
+    net = bindings.Network(json.dumps(cfg))
+    n, chunk = (1 << 22) + 4099, 1 << 22
+    x = torch.rand((n, spec.num_inputs), device="cuda", generator=torch.Generator(device="cuda").manual_seed(13))
+    w = torch.from_numpy(helpers.xavier_parameters(spec, cfg, bias_scale=0.1)).cuda().half()
+    t = torch.from_numpy(helpers.grid_tables(spec, scale=1.0)[0]).cuda().half()
+    net.inference(x[:64], w, [t])   # binds the parameters
+    try:
+        bindings.QuickMLP.set_kernel_path(2)
+        need = C.c_size_t()
+        check(lib().qmlp_network_inference_memory(net._h, n, C.byref(need)))
+        planes = chunk * sum(net.encoding(i).num_output_channels() for i in range(net.num_encodings())) * 2
+        assert need.value > planes
+        results = []
+        for size in (planes, need.value):
+            tmp = torch.full((size,), 0x7e, dtype=torch.uint8, device="cuda")
+            out = torch.zeros((n, spec.num_outputs), device="cuda")
+            o = wrap(out)
+            check(lib().qmlp_network_inference_with_memory(net._h, wrap(x), C.byref(o), None, tmp.data_ptr(), size))
+            torch.cuda.synchronize()
+            results.append(out)
+        for part in (slice(0, chunk), slice(chunk, n)):
+            assert float((results[0][part] - results[1][part]).norm()) <= 1e-4 * float(results[0][part].norm()) > 0
+    finally:
+        bindings.QuickMLP.set_kernel_path(0)
+
+
+@pytest.mark.parametrize("name", ["dense2d_multires", "hash2d_f8"])
+def test_points_and_adjoints_that_are_not_finite(name):
+    """NaN and infinite coordinates and adjoints with copies and records by cell: the same entries as without scratch are not finite, the others
+    agree (tolerances as above)."""
+    import ctypes as C
+    import torch
+    from qmlp._capi import check, lib, wrap
+    cfg, e, oe = _enc(name)
+    n = (3 << 18) + 77
+    x = helpers.uniform(14, 1, (n, oe.n_in), 0.0, 1.0)
+    adj = helpers.uniform(14, 2, (n, oe.num_outputs), 0.1, 1.0)
+    for k, v in enumerate((np.nan, np.inf, -np.inf)):
+        x[1000 + k, 0] = v
+        x[2000 + k, -1] = v
+        adj[200001 + 31 * k, k] = v
+    x, adj = torch.from_numpy(x).cuda(), torch.from_numpy(adj).cuda()
+    table = torch.from_numpy(helpers.uniform(14, 3, (oe.num_parameters,), -1.0, 1.0)).cuda()
+    p, forward, adjoint = wrap(table), C.c_size_t(), C.c_size_t()
+    check(lib().qmlp_encoding_forward_memory(e._h, n, C.byref(p), C.byref(forward)))
+    check(lib().qmlp_encoding_adjoint_memory(e._h, n, 2, C.byref(adjoint)))
+    assert forward.value > 0 and adjoint.value > 0
+    results = []
+    for scratch in (False, True):
+        out, gt = torch.zeros((n, oe.num_outputs), device="cuda"), torch.zeros_like(table)
+        g = wrap(gt)
+        tmp = torch.full((max(forward.value, adjoint.value),), 0x7e, dtype=torch.uint8, device="cuda")
+        at = tmp.data_ptr() if scratch else None
+        check(lib().qmlp_encoding_forward_with_memory(e._h, wrap(x), wrap(out), None, C.byref(p), at, forward.value if scratch else 0))
+        check(lib().qmlp_encoding_adjoint_with_memory(e._h, wrap(x), wrap(adj), None, None, C.byref(p), C.byref(g), 2, at, adjoint.value if scratch else 0))
+        torch.cuda.synchronize()
+        results.append((out, gt))
+    for (a, b), rtol in zip(zip(*results), (0.0, 2.0 ** -9)):
+        finite = torch.isfinite(a)
+        assert torch.equal(finite, torch.isfinite(b)) and 0 < int((~finite).sum()) < a.numel() // 2
+        a, b = a[finite], b[finite]
+        atol = 256 * 2.0 ** -24 * 2 * oe.n_in if rtol == 0 else 1e-5 * float(a.abs().max())
+        assert bool(((a - b).abs() <= rtol * a.abs() + atol).all())

@@ -374,6 +374,50 @@ def test_train_kernel_tile_slots(name, n):
     assert bindings.QuickMLP.device_status() == 0
 
 
+@pytest.mark.parametrize("half", [False, True])
+def test_step_with_records_and_copies_by_cell(half):
+    """A batch that is large enough for levels of both grids to be read from copies by cell and for the dense level's gradient to be added up by
+    cell, with points below and above the box, against the separate kernels; tolerance as above. Then a smaller batch in the same
+    workspace against a trainer that has seen no other."""
+    import torch
+    from qmlp import bindings
+    from qmlp.trainer import FusedTrainer
+    cfg = two_grid_config()
+    spec = oracle.parse_spec(cfg)
+    n, small = (3 << 18) + 77, 300001
+    x = torch.from_numpy(helpers.uniform(35, 1, (n, 3), -0.002, 1.002)).cuda()
+    t = torch.from_numpy(helpers.uniform(35, 2, (n, spec.num_outputs), -1.0, 1.0)).cuda()
+    params = torch.from_numpy(helpers.xavier_parameters(spec, cfg, bias_scale=0.1).astype(np.float32)).cuda()
+    tables = [torch.from_numpy(tb).cuda() for tb in helpers.grid_tables(spec, scale=0.5)]
+
+    def trainer():
+        tr = FusedTrainer(bindings.Network(json.dumps(cfg)), grid_half_copy=half)
+        tr.set_parameters(params, tables)
+        return tr
+
+    def gradients(tr, count):
+        tr.gradient.zero_()
+        tr.loss_sum.zero_()
+        before = tr.network.launch_count()
+        tr.backend.gradients(x[:count], t[:count], count, tr.loss_sum)
+        torch.cuda.synchronize()
+        return tr.network.launch_count() - before, [tr.loss_sum.clone()] + [tr.segment(tr.gradient, i).clone() for i in range(3)]
+    tr = trainer()
+    launches, fused = gradients(tr, n)
+    assert launches == 5      # copies by cell, encode, layers, scatter, sum of the records
+    again = gradients(tr, small)[1]
+    alone = gradients(trainer(), small)[1]
+    try:
+        bindings.QuickMLP.set_kernel_path(1)
+        separate = gradients(trainer(), n)[1]
+    finally:
+        bindings.QuickMLP.set_kernel_path(0)
+    for what, results, tolerance in (("separate kernels", (fused, separate), 1e-2), ("fresh workspace", (again, alone), 1e-5)):   # (1e-5: order of fp32 sums)
+        for i, (a, b) in enumerate(zip(*results)):
+            norm = float(b.norm())
+            assert norm > 0 and float((a - b).norm()) <= tolerance * norm, f"{what} result {i}: {float((a - b).norm()) / norm}"
+
+
 def test_scatter_with_copies_of_hot_levels():
     """A batch that hits the lines of the coarse levels often enough for copies of their gradients: one launch over all levels,
     and launches over ranges of levels that begin before, inside and behind the levels with copies, against the scatter
