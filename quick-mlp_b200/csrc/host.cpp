@@ -8,7 +8,6 @@
 #include <fstream>
 #include <random>
 #include <cctype>
-#include <cstdlib>
 #include <set>
 #include <sstream>
 #include <sys/stat.h>

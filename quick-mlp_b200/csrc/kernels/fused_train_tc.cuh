@@ -28,13 +28,13 @@
 //     the slot overwrites their operands, and that stage computes all its deltas before it waits.
 // Measured, step of 32 -> 64 -> 64 -> 1 on 2^20 points: 94 (forward) + 123 (backward) + 127 us (weight gradients) -> 137 us with two slots
 // of two warpgroups -> 111 us with four of one; 48 -> 128 -> 64 -> 16 -> 4 on 2^21 points: 709 (with the gather) + 1022 (with the scatter)
-// + 473 -> 577 us with accumulators computed a second time -> 563 us. What it spends (clocks of the first example, measured in the kernel):
+// + 473 -> 577 us with accumulators computed a second time -> 576 us (111 and 564 while a slot's warps did not wait for each other at the
+// end of a stage). What it spends (clocks of the first example, measured in the kernel):
 // a tile's MMAs 1970, 54 % of the time per tile (K = 16 takes 40 to 49 clocks from shared memory however few columns, 33 from tensor
 // memory, for which there are no columns left); a slot's stage 2000: 450 waiting for the accumulator behind other slots' MMAs, 1000
 // of epilogue, 130 fences, 300 to issue. Features fetched before the last stage are spilled, and a spill waits for the load (1500 clocks).
-// Weight gradients issued by the slots' own warps under a lock instead of by a warp of their own (128 instead of 96 registers): waits that ran
-// out and sums that were lost; not to be tried again.
-// Every wait is bounded; on a timeout the CTA runs through without waiting and the status word is set.
+// Every wait on the tensor core or a copy is bounded. After one that gave up the CTA runs through without them and sets the status word; what its
+// warps still wait for then is each other, at barriers that each of them reaches.
 //
 // The second instantiation (LOSS false) is the backward pass of a forward call that stashed the encoded features only: the layers
 // are computed a second time on the tensor core instead of being written by the forward kernel and read twice. 32 -> 64 -> 64 -> 1
@@ -134,7 +134,9 @@ struct TrainLayout {
     }
     __host__ __device__ static constexpr int slotStride(int slots) { return slotCols() + spareCols(slots); }   // columns of a slot
     // Slots and warpgroups per slot: as many slots as there is room for, the stages of a tile being latency (see above). 17 warps have 96
-    // registers a thread, 13 have 128.
+    // registers a thread, 13 have 128. Also at few tiles per CTA, where half the threads work on each: 32 -> 64 -> 64 -> 1, 0.4 / 1 / 2 / 4 / 8 / 16
+    // tiles per CTA, two slots of two warpgroups 14.8 / 18.9 / 22.9 / 27.0 / 33.2 / 51.3 us, four of one 14.8 / 19.0 / 22.9 / 25.0 / 29.2 / 43.4;
+    // 3 -> 64 x 4 -> 1 22.3 / 27.1 / 34.7 / 49.3 / 78.2 / 135 and 22.2 / 27.0 / 29.1 / 38.6 / 57.2 / 92.1.
     __host__ __device__ static constexpr bool holds(int slots, int wg, int registers) { return fits(slots) && preBefore(NL - 1, slots, wg) <= registers; }
     static constexpr int SLOTS = holds(4, 1, 40) ? 4 : holds(3, 1, 72) ? 3 : holds(2, 2, 48) ? 2 : 1;
     static constexpr int WG = SLOTS >= 3 ? 1 : SLOTS == 2 ? 2 : 4;
